@@ -1,17 +1,20 @@
-"""Builds libcutile_b200.so for sm_100a with nvcc (cross-compiles without a GPU).
+"""Builds libcutile_b200.so for sm_100a with nvcc (cross-compiles without a GPU) and the host extension _host.so.
 
 Usage: python build.py [--force] [--verbose]
 The library is written next to the Python mirror (../cutile_b200/) so that an
 in-tree checkout is self-contained.
 """
+import importlib.util
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 OUT_DIR = os.path.join(os.path.dirname(HERE), "cutile_b200")
 LIB = os.path.join(OUT_DIR, "libcutile_b200.so")
+HOST = os.path.join(OUT_DIR, "_host.so")  # native call path of the Python package (host.cpp)
 OBJ_DIR = os.path.join(HERE, "build")
 INCLUDE = os.path.join(os.path.dirname(os.path.dirname(HERE)), "include")
 
@@ -59,7 +62,28 @@ def build(force=False, verbose=False):
         if r.returncode:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link failed")
+    build_host(force, verbose)
     return LIB
+
+
+def build_host(force=False, verbose=False):
+    """The CPython extension: compiled against the headers of the torch that imports it, linked to LIB next to it."""
+    src = os.path.join(HERE, "host.cpp")
+    if not (force or _stale(HOST, [src, os.path.join(INCLUDE, "cutile_b200.h")])):
+        return
+    spec = importlib.util.find_spec("torch")  # its folder, without importing it
+    torch_dir = os.path.dirname(spec.origin)
+    cuda = os.path.dirname(os.path.dirname(NVCC))
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-D_GLIBCXX_USE_CXX11_ABI=1",
+           "-I", sysconfig.get_paths()["include"], "-I", os.path.join(torch_dir, "include"),
+           "-I", os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"), "-I", os.path.join(cuda, "include"),
+           src, "-o", HOST, "-L", OUT_DIR, "-l:libcutile_b200.so", "-L", os.path.join(torch_dir, "lib"),
+           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if verbose or r.returncode:
+        sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
+    if r.returncode:
+        raise RuntimeError("the host extension failed to build")
 
 
 if __name__ == "__main__":

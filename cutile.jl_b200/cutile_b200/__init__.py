@@ -6,6 +6,8 @@ argument order; tensors are torch CUDA tensors laid out like the Julia arrays
 (so torch shapes are the Julia shapes reversed).  All arithmetic happens in the
 CUDA library; nothing here computes on the host.
 """
+import torch  # noqa: F401  (its libraries are loaded before the extension that is linked against them)
+
 from . import _lib  # noqa: F401  (fails loudly when the shared library is missing)
 from ._lib import CtbError, version_info, check_device_status  # noqa: F401
 from . import softmax, layernorm, matmul, batchmatmul, fmha, moe, multi, vadd, transpose, fft, tiled  # noqa: F401

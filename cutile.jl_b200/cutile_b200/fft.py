@@ -9,7 +9,7 @@ import math
 import numpy as np
 import torch
 
-from . import _lib
+from . import _host, _lib
 from ._util import handles, ptr
 
 
@@ -64,6 +64,11 @@ class FftPlan:
 
     def __call__(self, input, out=None, **hints):
         """FFT along the last torch dimension (the first Julia dimension) of a complex64 [batch, N] tensor."""
+        if not hints:
+            F0, F1, F2 = self.factors
+            r = _host.fft(input, out, self.tables, self.N, F0, F1, F2, self.D)
+            if r is not None:
+                return r
         if input.dtype != torch.complex64 or input.dim() != 2 or input.shape[1] != self.N or not input.is_contiguous():
             raise _lib.CtbError(_lib.BAD_ARG, "FftPlan: input must be a contiguous complex64 [batch, %d] tensor" % self.N)
         if out is None:

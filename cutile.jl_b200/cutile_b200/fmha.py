@@ -8,7 +8,7 @@ import math
 
 import torch
 
-from . import _lib
+from . import _host, _lib
 from ._util import handles, ptr, dtype_code
 
 
@@ -35,6 +35,10 @@ def cutile_fmha(Q, K, V, *, qk_scale=None, input_pos=0, tile_m=128, tile_n=128, 
                 **hints):
     """cutile_fmha(Q, K, V; qk_scale, input_pos, tile_m, tile_n, query_group_size, causal),
     examples/fmha.jl:146-168: allocates and returns Out."""
+    if not hints:
+        r = _host.fmha(Q, K, V, None, qk_scale, input_pos, tile_m, tile_n, query_group_size, causal)
+        if r is not None:
+            return r
     B, H, Sq, D = Q.shape
     Dv, Skv = V.shape[3], V.shape[2]
     if qk_scale is None:

@@ -4,12 +4,14 @@ Memory order of the Julia arrays: X, Y, DX, DY (N, M) are torch [M, N];
 W, B, FINAL_DW, FINAL_DB are [N]; Mean, Rstd are [M]; the partial buffers
 DW, DB (N, GROUP_SIZE_M) are torch [GROUP_SIZE_M, N].
 """
-from . import _lib
+from . import _host, _lib
 from ._util import handles, ptr, rows
 
 
 def layer_norm_fwd(X, W, B, Y, Mean, Rstd, eps, TILE_N, **hints):
     """layer_norm_fwd(X, W, B, Y, Mean, Rstd, eps, TILE_N), examples/layernorm.jl:27-68."""
+    if not hints and _host.layernorm_fwd(X, W, B, Y, Mean, Rstd, eps, TILE_N):
+        return
     ctx, stream = handles(X, hints)
     ldx, M, N = rows(X, "X")
     ldy, My, Ny = rows(Y, "Y")
@@ -23,6 +25,8 @@ def layer_norm_bwd_dx_partial_dwdb(DX, DY, DW, DB, X, W, Mean, Rstd, Locks, GROU
     """layer_norm_bwd_dx_partial_dwdb(...), examples/layernorm.jl:118-171.
     `Locks` is accepted for signature compatibility and never touched; DW/DB
     need no zero-fill."""
+    if not hints and _host.layernorm_bwd(DX, DY, DW, DB, X, W, Mean, Rstd, GROUP_SIZE_M, TILE_N):
+        return
     ctx, stream = handles(X, hints)
     ldx, M, N = rows(X, "X")
     lddy, _, _ = rows(DY, "DY")
@@ -38,6 +42,8 @@ def layer_norm_bwd_dx_partial_dwdb(DX, DY, DW, DB, X, W, Mean, Rstd, Locks, GROU
 
 def layer_norm_bwd_dwdb(DW, DB, FINAL_DW, FINAL_DB, TILE_M, TILE_N, **hints):
     """layer_norm_bwd_dwdb(DW, DB, FINAL_DW, FINAL_DB, TILE_M, TILE_N), examples/layernorm.jl:186-205."""
+    if not hints and _host.layernorm_dwdb(DW, DB, FINAL_DW, FINAL_DB, TILE_M, TILE_N):
+        return
     ctx, stream = handles(DW, hints)
     G, N = DW.shape
     _lib.check(_lib.lib.ctb_layernorm_bwd_dwdb(ctx, stream, ptr(DW), ptr(DB), ptr(FINAL_DW), ptr(FINAL_DB), N, G,

@@ -3,12 +3,14 @@
 Memory order of the Julia arrays: A(M, K) is torch [K, M]; B(K, N) is torch
 [N, K]; C(M, N) is torch [N, M].
 """
-from . import _lib
+from . import _host, _lib
 from ._util import handles, ptr, rows, dtype_code
 
 
 def matmul_kernel(A, B, C, tm, tn, tk, **hints):
     """matmul_kernel(A, B, C, tm, tn, tk), examples/matmul.jl:28-60."""
+    if not hints and _host.matmul(A, B, C, tm, tn, tk):
+        return C
     ctx, stream = handles(A, hints)
     lda, K, M = rows(A, "A")
     ldb, N, Kb = rows(B, "B")

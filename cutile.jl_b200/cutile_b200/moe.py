@@ -9,7 +9,7 @@ import ctypes as C
 
 import torch
 
-from . import _lib
+from . import _host, _lib
 from ._util import handles, ptr
 
 
@@ -23,6 +23,10 @@ def _ids_bits(t):
 
 def moe_router(hidden_states, W_r, topk, return_logits=False):
     """Router of the benchmark configuration: returns (topk_weights [topk, T] f16, topk_ids [topk, T] int32)."""
+    if not return_logits:
+        r = _host.moe_router(hidden_states, W_r, topk)
+        if r is not None:
+            return r
     ctx, stream = handles(hidden_states)
     T, H = hidden_states.shape
     E = W_r.shape[0]
@@ -93,6 +97,9 @@ def silu_and_mul_kernel(A, B, C, TILE_N, **hints):
 def cutile_moe(hidden_states, w1, w2, topk_weights, topk_ids, tile_m, tile_n, tile_k):
     """cutile_moe(hidden_states, w1, w2, topk_weights, topk_ids, tile_m, tile_n, tile_k),
     examples/moe.jl:218-257: returns the (H, T) result as torch [T, H] f16."""
+    r = _host.moe_ffn(hidden_states, w1, w2, topk_weights, topk_ids, tile_m, tile_n, tile_k)
+    if r is not None:
+        return r
     ctx, stream = handles(hidden_states)
     T, H = hidden_states.shape
     E, H2, I = w2.shape

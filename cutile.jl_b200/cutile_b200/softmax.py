@@ -3,11 +3,13 @@
 Tensors are in the memory order of the Julia arrays: Julia `input(N, M)` is a
 torch tensor of shape [M, N] (each row is one softmax problem of N elements).
 """
-from . import _lib
+from . import _host, _lib
 from ._util import handles, ptr, rows, dtype_code, next_power_of_2  # noqa: F401
 
 
 def _run(output, input, variant, tile_size, hints):
+    if not hints and _host.softmax(output, input, variant, tile_size):
+        return output
     ctx, stream = handles(input, hints)
     ldi, M, N = rows(input, "input")
     ldo, Mo, No = rows(output, "output")

@@ -7,10 +7,11 @@ whole expression as ONE kernel; ``materialize(expr)`` is the allocating form (``
 and the reduced dimensions kept with extent 1.
 """
 import ctypes as C
+import functools
 
 import torch
 
-from . import _lib
+from . import _host, _lib
 from ._util import handles, ptr, dtype_code
 
 _OPS = {"input": 0, "const": 1, "identity": 16, "neg": 17, "abs": 18, "sqrt": 19, "exp": 20, "exp2": 21, "log": 22,
@@ -19,61 +20,29 @@ _OPS = {"input": 0, "const": 1, "identity": 16, "neg": 17, "abs": 18, "sqrt": 19
 MAX_DIMS = 3
 
 
-class Expr:
-    """A node of a broadcast expression: ("leaf", tensor) | ("const", value) | (unary name, Expr) | (binary name, Expr, Expr)."""
 
-    def __init__(self, *node):
-        self.node = node
-
-    @staticmethod
-    def wrap(x):
-        if isinstance(x, Expr):
-            return x
-        if isinstance(x, torch.Tensor):
-            return Tiled(x)
-        if isinstance(x, (int, float)):
-            return Expr("const", float(x))
-        raise TypeError(f"a Tiled broadcast takes Tiled arrays and numbers, not {type(x).__name__}")  # no device storage
-
-    def _bin(self, name, other, swap=False):
-        o = Expr.wrap(other)
-        return Expr(name, o, self) if swap else Expr(name, self, o)
-
-    __add__ = lambda self, o: self._bin("add", o)
-    __radd__ = lambda self, o: self._bin("add", o, True)
-    __sub__ = lambda self, o: self._bin("sub", o)
-    __rsub__ = lambda self, o: self._bin("sub", o, True)
-    __mul__ = lambda self, o: self._bin("mul", o)
-    __rmul__ = lambda self, o: self._bin("mul", o, True)
-    __truediv__ = lambda self, o: self._bin("div", o)
-    __rtruediv__ = lambda self, o: self._bin("div", o, True)
-    __pow__ = lambda self, o: self._bin("pow", o)
-    __neg__ = lambda self: Expr("neg", self)
-    __abs__ = lambda self: Expr("abs", self)
+def _leaf_error(tensor):
+    """Raises what makes `tensor` no array leaf (called by the native Tiled type when it refuses one)."""
+    if not isinstance(tensor, torch.Tensor) or not tensor.is_cuda:
+        raise ValueError("Tiled: the array must live in device memory")  # the reference's ArgumentError for host leaves
+    if tensor.dim() > MAX_DIMS:
+        raise _lib.CtbError(_lib.UNSUPPORTED, "Tiled: at most three dimensions")
+    if not tensor.is_contiguous():
+        raise _lib.CtbError(_lib.BAD_ARG, "Tiled: the array must be dense")
 
 
-class Tiled(Expr):
-    """``ct.Tiled(A)``: an array leaf."""
-
-    def __init__(self, tensor):
-        if not isinstance(tensor, torch.Tensor) or not tensor.is_cuda:
-            raise ValueError("Tiled: the array must live in device memory")  # the reference's ArgumentError for host leaves
-        if tensor.dim() > MAX_DIMS:
-            raise _lib.CtbError(_lib.UNSUPPORTED, "Tiled: at most three dimensions")
-        if not tensor.is_contiguous():
-            raise _lib.CtbError(_lib.BAD_ARG, "Tiled: the array must be dense")
-        Expr.__init__(self, "leaf", tensor)
-        self.tensor = tensor
+_host.setup(_lib.context, _lib.check, _leaf_error)
+Expr, Tiled = _host.Expr, _host.Tiled  # expression nodes (csrc/host.cpp)
 
 
 def _unary(name):
-    return lambda x: Expr(name, Expr.wrap(x))
+    return functools.partial(_host.unary, name)
 
 
 sin, cos, exp, exp2, log, log2, sqrt, tanh, inv, abs2 = (_unary(n) for n in
                                                          ("sin", "cos", "exp", "exp2", "log", "log2", "sqrt", "tanh", "inv", "abs2"))
-tmax = lambda a, b: Expr.wrap(a)._bin("max", b)
-tmin = lambda a, b: Expr.wrap(a)._bin("min", b)
+tmax = functools.partial(_host.binary, "max")
+tmin = functools.partial(_host.binary, "min")
 
 
 def _jshape(t):
@@ -131,6 +100,8 @@ def _compile(expr):
 
 def assign(dest, expr, **hints):
     """``ct.Tiled(dest) .= expr``: evaluates the whole expression in one kernel; returns dest."""
+    if not hints and _host.assign(dest, expr):
+        return dest
     expr = Expr.wrap(expr)
     if not isinstance(dest, torch.Tensor) or not dest.is_cuda:
         raise ValueError("Tiled: the destination must live in device memory")
@@ -180,6 +151,10 @@ def tmapreduce(f, op, a, dims=None, out=None, **hints):
     """``mapreduce(f, op, ct.Tiled(A); dims)``: f a unary function name ("identity", "abs", "abs2", ...), op one of
     "add", "mul", "max", "min"; dims Julia's 1-based dimensions (an int or a tuple; None = all).  Returns a tensor with
     extent 1 along the reduced dimensions (a 0-dimensional tensor for dims=None, like Julia's scalar)."""
+    if out is None and not hints:
+        r = _host.mapreduce(f, op, a, dims)
+        if r is not None:
+            return r
     t = a.tensor if isinstance(a, Tiled) else Tiled(a).tensor
     if dims is None:
         jd = tuple(range(1, t.dim() + 1))

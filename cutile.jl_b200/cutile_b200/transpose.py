@@ -2,12 +2,14 @@
 
 Memory order of the Julia arrays: x(M, N) is torch [N, M]; y(N, M) is torch [M, N].
 """
-from . import _lib
+from . import _host, _lib
 from ._util import handles, ptr, rows, dtype_code
 
 
 def transpose_kernel(x, y, tm, tn, **hints):
     """transpose_kernel(x, y, tm, tn), examples/transpose.jl:11-19: y = transpose(x)."""
+    if not hints and _host.transpose(x, y, tm, tn):
+        return y
     ctx, stream = handles(x, hints)
     ldx, N, M = rows(x, "x")
     ldy, My, Ny = rows(y, "y")

@@ -1,0 +1,57 @@
+"""The native call path of the package (csrc/host.cpp): expression nodes without a GPU, and on a GPU that calls it takes
+itself and calls it leaves to the Python checks give the same results."""
+import numpy as np
+import pytest
+
+
+def test_expression_nodes():
+    import torch
+    from cutile_b200 import tiled as T
+    e = T.Expr.wrap(2) + 3
+    assert e.node[0] == "add" and e.node[1].node == ("const", 2.0) and isinstance(e, T.Expr)
+    assert (2.0 * e).node[0] == "mul" and (2.0 * e).node[2] is e
+    assert [(-e).node[0], abs(e).node[0], (e ** 2).node[0], T.tanh(e).node[0], T.tmax(e, 1).node[0]] == \
+        ["neg", "abs", "pow", "tanh", "max"]
+    with pytest.raises(TypeError):
+        2 ** e
+    with pytest.raises(TypeError):
+        e + range(3)
+    with pytest.raises(ValueError, match="device memory"):
+        T.Tiled(torch.ones(3))
+    for _ in range(20000):  # a tree this deep is released without recursion
+        e = e + 1.0
+    del e
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n", [(1, 4), (64, 1000), (33, 4096)])
+def test_native_and_checked_calls_agree(cuda, m, n):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x = torch.randn(m, n, device="cuda", generator=g)
+    outs = []
+    for hints in ({}, {"occupancy": 2}):  # launch keywords take the Python path
+        o = torch.full_like(x, float("nan"))
+        assert cuda.softmax.softmax_chunked_kernel(o, x, n, 1024, **hints) is o
+        a = torch.full_like(x, float("nan"))
+        cuda.tiled.assign(a, cuda.tiled.Tiled(x) * 2.0 + cuda.tiled.tanh(cuda.tiled.Tiled(x[:1].contiguous())), **hints)
+        s = cuda.tiled.tsum(cuda.tiled.Tiled(x), dims=1, **hints)
+        v = cuda.vadd.vec_add_kernel_2d(x, o, torch.empty_like(x), 32, 32, **hints)
+        outs.append([t.cpu().numpy() for t in (o, a, s, v)])
+    for p, q in zip(*outs):
+        assert p.shape == q.shape and np.array_equal(p, q)
+
+
+@pytest.mark.gpu
+def test_native_path_follows_the_current_stream(cuda):
+    import torch
+    x = torch.randn(4096, 4096, device="cuda")
+    want = torch.softmax(x, 1)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        y = x * 1.0
+        o = torch.empty_like(y)
+        cuda.softmax.softmax_tma_kernel(o, y, 4096)
+    side.synchronize()
+    assert (o - want).abs().max().item() < 1e-6
