@@ -5,6 +5,7 @@
 #include <cuda_fp16.h>
 
 #include "ctx.h"
+#include "ptx.cuh"
 
 using namespace ctb_internal;
 
@@ -42,6 +43,7 @@ struct Vec16<__half> {
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256) vadd_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ c,
                                                    long long n, long long rows, long long lda, long long ldb, long long ldc) {
+  ctb::grid_dependency_sync();
   constexpr int V = Vec16<T>::N;
   const long long per_row = VEC ? n / V : n;  // work units per row
   const long long total = per_row * rows;
@@ -65,6 +67,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) transpose_kernel(const T* __restrict__ x, T* __restrict__ y, int m, int n, long long ldx,
                                                         long long ldy, int tiles_m, long long tiles) {
   __shared__ T tile[kTT][kTT + 16 / sizeof(T) + 1];
+  ctb::grid_dependency_sync();
   constexpr int V = 16 / sizeof(T);
   const bool vec_in = (ldx % V == 0) && ((uintptr_t)x % 16 == 0), vec_out = (ldy % V == 0) && ((uintptr_t)y % 16 == 0);
   for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {
@@ -132,7 +135,7 @@ int ctb_vadd(ctb_ctx* ctx, void* stream, const void* a, const void* b, void* c, 
   const long long units = (vec ? n / V : n) * rows;
   const int grid = (int)std::max<long long>(1, std::min<long long>((units + 255) / 256, (long long)ctx->sm_count * 16));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-#define CTB_VADD(T, VECV) vadd_kernel<T, VECV><<<grid, 256, 0, st>>>((const T*)a, (const T*)b, (T*)c, n, rows, lda, ldb, ldc)
+#define CTB_VADD(T, VECV) launch_kernel(vadd_kernel<T, VECV>, grid, 256, 0, st, 0, (const T*)a, (const T*)b, (T*)c, n, rows, lda, ldb, ldc)
   if (dtype == CTB_F32) { if (vec) CTB_VADD(float, true); else CTB_VADD(float, false); }
   else { if (vec) CTB_VADD(__half, true); else CTB_VADD(__half, false); }
 #undef CTB_VADD
@@ -154,9 +157,9 @@ int ctb_transpose(ctb_ctx* ctx, void* stream, const void* x, void* y, int64_t m,
   const int grid = (int)std::max<long long>(1, std::min<long long>(tiles, (long long)ctx->sm_count * 8));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (dtype == CTB_F32)
-    transpose_kernel<float><<<grid, 256, 0, st>>>((const float*)x, (float*)y, (int)m, (int)n, ldx, ldy, tiles_m, tiles);
+    launch_kernel(transpose_kernel<float>, grid, 256, 0, st, 0, (const float*)x, (float*)y, (int)m, (int)n, ldx, ldy, tiles_m, tiles);
   else
-    transpose_kernel<__half><<<grid, 256, 0, st>>>((const __half*)x, (__half*)y, (int)m, (int)n, ldx, ldy, tiles_m, tiles);
+    launch_kernel(transpose_kernel<__half>, grid, 256, 0, st, 0, (const __half*)x, (__half*)y, (int)m, (int)n, ldx, ldy, tiles_m, tiles);
   CTB_CHECK_LAUNCH("ctb_transpose launch");
   return CTB_OK;
 }

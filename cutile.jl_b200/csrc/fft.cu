@@ -16,6 +16,7 @@
 #include <type_traits>
 
 #include "ctx.h"
+#include "ptx.cuh"
 
 using namespace ctb_internal;
 
@@ -146,6 +147,7 @@ fft_kernel(const float2* __restrict__ x, float2* __restrict__ y, const float2* _
   float* Ws0 = reinterpret_cast<float*>(B + padded);  // 16-byte aligned planes (read with 16-byte loads)
   float* Ws1 = Ws0 + ((2 * F0 * F0 + 3) & ~3);
   float* Ws2 = Ws1 + ((2 * F1 * F1 + 3) & ~3);
+  ctb::grid_dependency_sync();
   load_dft(Ws0, W0, F0);
   load_dft(Ws1, W1, F1);
   load_dft(Ws2, W2, F2);
@@ -215,7 +217,7 @@ extern "C" int ctb_fft(ctb_ctx* ctx, void* stream, const void* x, void* y, const
   }
   const int lines = (int)(N / std::min(F0, std::min(F1, F2)));
   const int threads = std::min(256, std::max(32, (lines + 31) / 32 * 32));
-  fft_kernel<<<(unsigned)batch, threads, smem, static_cast<cudaStream_t>(stream)>>>(
+  launch_kernel(fft_kernel, (unsigned)batch, threads, smem, static_cast<cudaStream_t>(stream), 0,
       (const float2*)x, (float2*)y, (const float2*)W0, (const float2*)W1, (const float2*)W2, (const float2*)T0, (const float2*)T1,
       F0, F1, F2);
   CTB_CHECK_LAUNCH("ctb_fft launch");

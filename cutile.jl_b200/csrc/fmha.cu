@@ -202,6 +202,7 @@ __global__ void __launch_bounds__(kThreadsD, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  grid_dependency_sync();
   const uint32_t tmem = tmem_base_s;
   volatile int* abort = &abort_s;
 
@@ -606,7 +607,7 @@ extern "C" int ctb_fmha_fwd(ctb_ctx* ctx, void* stream, const void* Q, const voi
   auto kern = dtype == CTB_BF16 ? fmha_kernel<true> : fmha_kernel<false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return cuda_fail(e, "ctb_fmha_fwd: shared memory opt-in");
-  kern<<<grid, kThreadsD, smem, static_cast<cudaStream_t>(stream)>>>(tq, tk, tv, to, p, ctx->dev_status);
+  launch_kernel(kern, grid, kThreadsD, smem, static_cast<cudaStream_t>(stream), 0, tq, tk, tv, to, p, ctx->dev_status);
   CTB_CHECK_LAUNCH("ctb_fmha_fwd launch");
   return CTB_OK;
 }

@@ -127,6 +127,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  grid_dependency_sync();
   const uint32_t tmem_base = tmem_base_s;
   volatile int* abort = &abort_s;
   const int nk = (p.K + G::BK - 1) / G::BK;
@@ -256,6 +257,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 template <typename T>
 __global__ void __launch_bounds__(256)
     gemm_splitk_reduce_kernel(const float* __restrict__ partial, T* __restrict__ C, const Params p) {
+  grid_dependency_sync();
   constexpr int kTileElems = kTileM * kTileN;
   const long long total = (long long)p.num_tiles * (kTileElems / 4);
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -349,6 +351,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   cluster_arrive();  // the peer's barriers exist before anything is signalled on them
   cluster_wait();
   tc_fence_after();
+  grid_dependency_sync();
   const uint32_t tmem_base = tmem_base_s;
   volatile int* abort = &abort_s;
   const int nk = (p.K + G::BK - 1) / G::BK;
@@ -503,6 +506,7 @@ int pair_clusters(ctb_ctx* ctx, size_t smem) {
 __global__ void __launch_bounds__(256) tf32_round_kernel(const uint4* __restrict__ in, uint4* __restrict__ out, long long n4,
                                                          const uint32_t* __restrict__ in_tail, uint32_t* __restrict__ out_tail,
                                                          int tail) {
+  grid_dependency_sync();
   auto rne = [](uint32_t u) {
     const bool nan = ((u >> 23) & 0xFFu) == 0xFFu && (u & 0x7FFFFFu) != 0;
     const uint32_t r = (u + 0xFFFu + ((u >> 13) & 1u)) & 0xFFFFE000u;
@@ -539,10 +543,10 @@ int launch(ctb_ctx* ctx, cudaStream_t st, const T* A, const T* B, T* C, int M, i
     float* A2 = reinterpret_cast<float*>(static_cast<unsigned char*>(ws) + oa);
     float* B2 = reinterpret_cast<float*>(static_cast<unsigned char*>(ws) + ob);
     const int rgrid = ctx->sm_count * 8;
-    tf32_round_kernel<<<rgrid, 256, 0, st>>>(reinterpret_cast<const uint4*>(A), reinterpret_cast<uint4*>(A2), ea / 4,
+    launch_kernel(tf32_round_kernel, rgrid, 256, 0, st, 0, reinterpret_cast<const uint4*>(A), reinterpret_cast<uint4*>(A2), ea / 4,
                                             reinterpret_cast<const uint32_t*>(A) + (ea & ~3ll),
                                             reinterpret_cast<uint32_t*>(A2) + (ea & ~3ll), (int)(ea & 3));
-    tf32_round_kernel<<<rgrid, 256, 0, st>>>(reinterpret_cast<const uint4*>(B), reinterpret_cast<uint4*>(B2), eb / 4,
+    launch_kernel(tf32_round_kernel, rgrid, 256, 0, st, 0, reinterpret_cast<const uint4*>(B), reinterpret_cast<uint4*>(B2), eb / 4,
                                             reinterpret_cast<const uint32_t*>(B) + (eb & ~3ll),
                                             reinterpret_cast<uint32_t*>(B2) + (eb & ~3ll), (int)(eb & 3));
     CTB_CHECK_LAUNCH("ctb_gemm operand rounding launch");
@@ -593,7 +597,7 @@ int launch(ctb_ctx* ctx, cudaStream_t st, const T* A, const T* B, T* C, int M, i
       const int clusters = pair_clusters<T>(ctx, smem);
       if (clusters > 0) {
         const int grid = 2 * (int)std::min<long long>(pairs, clusters);
-        k<<<grid, kThreads, smem, st>>>(ta, tb2, C, p, ctx->dev_status);
+        launch_kernel(k, grid, kThreads, smem, st, 0, ta, tb2, C, p, ctx->dev_status);
         CTB_CHECK_LAUNCH("ctb_gemm launch");
         return CTB_OK;
       }
@@ -620,12 +624,12 @@ int launch(ctb_ctx* ctx, cudaStream_t st, const T* A, const T* B, T* C, int M, i
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return cuda_fail(e, "ctb_gemm: shared memory opt-in");
   const int grid = (int)std::min<long long>(nt * p.splits, ctx->sm_count);
-  k<<<grid, kThreads, smem, st>>>(ta, tb, C, p, ctx->dev_status);
+  launch_kernel(k, grid, kThreads, smem, st, 0, ta, tb, C, p, ctx->dev_status);
   CTB_CHECK_LAUNCH("ctb_gemm launch");
   if (p.splits > 1) {
     const long long work = nt * kTileM * kTileN / 4;
     const int rgrid = (int)std::min<long long>((work + 255) / 256, (long long)ctx->sm_count * 8);
-    gemm_splitk_reduce_kernel<T><<<rgrid, 256, 0, st>>>(p.partial, C, p);
+    launch_kernel(gemm_splitk_reduce_kernel<T>, rgrid, 256, 0, st, 0, p.partial, C, p);
     CTB_CHECK_LAUNCH("ctb_gemm split-K reduction launch");
   }
   return CTB_OK;

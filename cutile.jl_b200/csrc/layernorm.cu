@@ -68,6 +68,7 @@ __global__ void __launch_bounds__(kFwdThreads)
     fence_mbar_init();
   }
   __syncthreads();
+  grid_dependency_sync();
   const int first = blockIdx.x, step = gridDim.x;
   const int nrows = first < M ? (M - first + step - 1) / step : 0;
   if (tid == 0) {
@@ -157,6 +158,7 @@ __global__ void __launch_bounds__(kFwdThreads) ln_fwd_generic_kernel(const float
                                                                      int N, int M, long long ldx, long long ldy,
                                                                      float eps) {
   __shared__ float red[kFwdThreads / 32];
+  grid_dependency_sync();
   const int tid = threadIdx.x;
   const float fn = (float)N;
   for (int row = blockIdx.x; row < M; row += gridDim.x) {
@@ -212,6 +214,7 @@ __global__ void __launch_bounds__(kBwdThreads)
     fence_mbar_init();
   }
   __syncthreads();
+  grid_dependency_sync();
 
   const int first = g + G * rank, step = G * C;
   const int nrows = first < M ? (M - first + step - 1) / step : 0;
@@ -356,6 +359,7 @@ __global__ void __launch_bounds__(kBwdThreads)
                           const float* __restrict__ Mean, const float* __restrict__ Rstd, int N, int M, long long ldx,
                           long long lddy, long long lddx, int G) {
   __shared__ float red[2][kBwdWarps];
+  grid_dependency_sync();
   const int tid = threadIdx.x, g = blockIdx.x;
   const float inv_n = 1.0f / (float)N;
   float dw[kGenCols], db[kGenCols];
@@ -419,6 +423,7 @@ constexpr int kRedCols = 32, kRedSlices = 8;
 __global__ void __launch_bounds__(kRedCols * kRedSlices)
     ln_bwd_reduce_kernel(const float* __restrict__ DW, const float* __restrict__ DB, float* __restrict__ FDW,
                          float* __restrict__ FDB, int N, int G) {
+  grid_dependency_sync();
   __shared__ float sw[kRedSlices][kRedCols], sb[kRedSlices][kRedCols];
   const int cx = threadIdx.x & (kRedCols - 1), sl = threadIdx.x / kRedCols;
   const int c = blockIdx.x * kRedCols + cx;
@@ -464,20 +469,8 @@ int launch_bwd(ctb_ctx* ctx, cudaStream_t st, float* DX, const float* DY, float*
   if (per_sm > 2048 / kBwdThreads) per_sm = 2048 / kBwdThreads;
   int C = 8;
   while (C > 1 && ((long long)G * C > (long long)ctx->sm_count * per_sm || (long long)G * C * 2 > M)) C >>= 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(G * C);
-  cfg.blockDim = dim3(kBwdThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = C;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  e = cudaLaunchKernelEx(&cfg, k, DX, DY, DW, DB, X, W, Mean, Rstd, N, M, ldx, lddy, lddx, G, row_stride,
-                         ctx->dev_status);
+  e = launch_kernel(k, G * C, kBwdThreads, smem, st, C, DX, DY, DW, DB, X, W, Mean, Rstd, N, M, ldx, lddy, lddx, G, row_stride,
+                    ctx->dev_status);
   if (e != cudaSuccess) return cuda_fail(e, "ctb_layernorm_bwd_dx_partial_dwdb launch");
   return CTB_OK;
 }
@@ -515,7 +508,7 @@ int ctb_layernorm_fwd(ctb_ctx* ctx, void* stream, const float* X, const float* W
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kFwdThreads, smem);                                \
     if (per_sm < 1) per_sm = 1;                                                                                  \
     const int grid = (int)std::min<int64_t>(M, (int64_t)ctx->sm_count * per_sm);                                 \
-    k<<<grid, kFwdThreads, smem, st>>>(X, W, B, Y, Mean, Rstd, n, m, ldx, ldy, eps, stage_bytes, ctx->dev_status); \
+    launch_kernel(k, grid, kFwdThreads, smem, st, 0, X, W, B, Y, Mean, Rstd, n, m, ldx, ldy, eps, stage_bytes, ctx->dev_status); \
   }
     if (nv <= 1) CTB_LN_FWD(1)
     else if (nv <= 2) CTB_LN_FWD(2)
@@ -524,7 +517,7 @@ int ctb_layernorm_fwd(ctb_ctx* ctx, void* stream, const float* X, const float* W
 #undef CTB_LN_FWD
   } else {
     const int grid = (int)std::min<int64_t>(M, (int64_t)ctx->sm_count * 8);
-    ln_fwd_generic_kernel<<<grid, kFwdThreads, 0, st>>>(X, W, B, Y, Mean, Rstd, n, m, ldx, ldy, eps);
+    launch_kernel(ln_fwd_generic_kernel, grid, kFwdThreads, 0, st, 0, X, W, B, Y, Mean, Rstd, n, m, ldx, ldy, eps);
   }
   CTB_CHECK_LAUNCH("ctb_layernorm_fwd launch");
   return CTB_OK;
@@ -560,7 +553,7 @@ int ctb_layernorm_bwd_dx_partial_dwdb(ctb_ctx* ctx, void* stream, float* DX, con
   if (N > kBwdThreads * kGenCols)
     return fail(CTB_UNSUPPORTED, "ctb_layernorm_bwd_dx_partial_dwdb: N=%lld exceeds %d", (long long)N,
                 kBwdThreads * kGenCols);
-  ln_bwd_generic_kernel<<<G, kBwdThreads, 0, st>>>(DX, DY, DW, DB, X, W, Mean, Rstd, n, m, ldx, lddy, lddx, G);
+  launch_kernel(ln_bwd_generic_kernel, G, kBwdThreads, 0, st, 0, DX, DY, DW, DB, X, W, Mean, Rstd, n, m, ldx, lddy, lddx, G);
   CTB_CHECK_LAUNCH("ctb_layernorm_bwd_dx_partial_dwdb launch");
   return CTB_OK;
 }
@@ -573,8 +566,7 @@ int ctb_layernorm_bwd_dwdb(ctb_ctx* ctx, void* stream, const float* DW, const fl
   if (!is_pow2(tile_m) || !is_pow2(tile_n))
     return fail(CTB_UNSUPPORTED_TILE, "ctb_layernorm_bwd_dwdb: TILE_M/TILE_N must be powers of two");
   CTB_CHECK_DEV(DW); CTB_CHECK_DEV(DB); CTB_CHECK_DEV(FINAL_DW); CTB_CHECK_DEV(FINAL_DB);
-  ln_bwd_reduce_kernel<<<(int)((N + kRedCols - 1) / kRedCols), kRedCols * kRedSlices, 0,
-                         static_cast<cudaStream_t>(stream)>>>(DW, DB, FINAL_DW, FINAL_DB, (int)N, group_size_m);
+  launch_kernel(ln_bwd_reduce_kernel, (int)((N + kRedCols - 1) / kRedCols), kRedCols * kRedSlices, 0, static_cast<cudaStream_t>(stream), 0, DW, DB, FINAL_DW, FINAL_DB, (int)N, group_size_m);
   CTB_CHECK_LAUNCH("ctb_layernorm_bwd_dwdb launch");
   return CTB_OK;
 }
@@ -647,19 +639,8 @@ int launch_bwd_static(const StaticDev& d, cudaStream_t st, float* DX, const floa
   per_sm = std::max(1, std::min(per_sm, 2048 / kBwdThreads));
   int C = 8;
   while (C > 1 && ((long long)G * C > (long long)d.sm_count * per_sm || (long long)G * C * 2 > M)) C >>= 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(G * C);
-  cfg.blockDim = dim3(kBwdThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = C;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  e = cudaLaunchKernelEx(&cfg, k, DX, DY, DW, DB, X, W, Mean, Rstd, N, M, ldx, lddy, lddx, G, row_stride, d.status);
+  e = launch_kernel(k, G * C, kBwdThreads, smem, st, C, DX, DY, DW, DB, X, W, Mean, Rstd, N, M, ldx, lddy, lddx, G, row_stride,
+                    d.status);
   if (e != cudaSuccess) return cuda_fail(e, "ctb_layernorm_bwd_static launch");
   return CTB_OK;
 }
@@ -695,7 +676,7 @@ extern "C" int ctb_layernorm_bwd_static(void* stream, float* DX, const float* DY
   else if (nv <= 2) r = launch_bwd_static<2>(*d, st, DX, DY, DW, DB, X, W, Mean, Rstd, n, m, ldx, lddy, lddx);
   else r = launch_bwd_static<4>(*d, st, DX, DY, DW, DB, X, W, Mean, Rstd, n, m, ldx, lddy, lddx);
   if (r) return r;
-  ln_bwd_reduce_kernel<<<(n + kRedCols - 1) / kRedCols, kRedCols * kRedSlices, 0, st>>>(DW, DB, FINAL_DW, FINAL_DB, n,
+  launch_kernel(ln_bwd_reduce_kernel, (n + kRedCols - 1) / kRedCols, kRedCols * kRedSlices, 0, st, 0, DW, DB, FINAL_DW, FINAL_DB, n,
                                                                                       kStaticGroups);
   CTB_CHECK_LAUNCH("ctb_layernorm_bwd_static reduce launch");
   return CTB_OK;

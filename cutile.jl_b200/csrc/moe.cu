@@ -123,6 +123,7 @@ __global__ void __launch_bounds__(kRouterThreads)
                       __half* __restrict__ gates, float* __restrict__ logits_out, int T, int H, int E, int topk,
                       int eg, int tw) {
   extern __shared__ __align__(16) unsigned char rsm_raw[];
+  grid_dependency_sync();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nchunk = (H + 255) / 256, Hp = nchunk * 256;
   const int ew = kRouterWarps / tw, G = TT * tw;
@@ -276,6 +277,7 @@ __global__ void __launch_bounds__(kAlignThreads)
                      int* __restrict__ sorted_token_ids, int* __restrict__ sorted_expert_ids,
                      int* __restrict__ num_blocks, int capacity_blocks, int skip_empty, int* status,
                      const unsigned char* __restrict__ warm, long long warm_bytes) {
+  grid_dependency_sync();
   cg::cluster_group cluster = cg::this_cluster();
   const int C = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
   if ((int)blockIdx.x >= C) {
@@ -536,6 +538,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  grid_dependency_sync();
   const uint32_t tmem = tmem_base_s;
   volatile int* abort = &abort_s;
   const int nblocks = p.num_blocks_host >= 0 ? p.num_blocks_host : *p.num_blocks_dev;
@@ -862,6 +865,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 // out(:, t) = sum over the top-k slot outputs of token t.  The slot outputs are f16 like the reference's cache3
 // (examples/moe.jl:230,256); they are added in f32 in ascending slot order and rounded once.
 __global__ void moe_combine_kernel(const __half* __restrict__ slots, __half* __restrict__ out, int T, int H, int topk) {
+  grid_dependency_sync();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;  // over T*H/8
   const int h8 = H / 8;
   if (i >= (long long)T * h8) return;
@@ -889,6 +893,7 @@ __global__ void moe_combine_kernel(const __half* __restrict__ slots, __half* __r
 __global__ void moe_gather_rows_kernel(uint4* __restrict__ dst, const uint4* __restrict__ src,
                                        const int* __restrict__ ids, long long n, int vecs, int replicas,
                                        long long src_rows) {
+  grid_dependency_sync();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n * vecs) return;
   const long long r = i / vecs;
@@ -900,6 +905,7 @@ __global__ void moe_gather_rows_kernel(uint4* __restrict__ dst, const uint4* __r
 // dst row ids[i]-1 = src row i (ids out of range are skipped)
 __global__ void moe_scatter_rows_kernel(uint4* __restrict__ dst, const uint4* __restrict__ src,
                                         const int* __restrict__ ids, long long n, int vecs, long long dst_rows) {
+  grid_dependency_sync();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n * vecs) return;
   const long long r = i / vecs;
@@ -911,6 +917,7 @@ __global__ void moe_scatter_rows_kernel(uint4* __restrict__ dst, const uint4* __
 __global__ void moe_silu_and_mul_kernel(const __half* __restrict__ A, const __half* __restrict__ B,
                                         __half* __restrict__ C, int n, long long cols, long long lda, long long ldb,
                                         long long ldc) {
+  grid_dependency_sync();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= cols * n) return;
   const long long col = i / n;
@@ -1032,7 +1039,7 @@ int launch_gemm(ctb_ctx* ctx, cudaStream_t st, int epi, const __half* A, long lo
 #define CTB_LAUNCH_MOE(EPI, NWV)                                                                              \
   e = cudaFuncSetAttribute(moe_gemm_kernel<EPI, NWV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
   if (e != cudaSuccess) return cuda_fail(e, "moe gemm: shared memory opt-in");                                \
-  moe_gemm_kernel<EPI, NWV><<<grid, kGemmThreads, smem, st>>>(tw, p, ctx->dev_status);
+  launch_kernel(moe_gemm_kernel<EPI, NWV>, grid, kGemmThreads, smem, st, 0, tw, p, ctx->dev_status);
   if (epi == EPI_SWIGLU) { CTB_LAUNCH_MOE(EPI_SWIGLU, 2) }
   else if (nw == 2) { CTB_LAUNCH_MOE(EPI_F16, 2) }
   else { CTB_LAUNCH_MOE(EPI_F16, 1) }
@@ -1063,27 +1070,15 @@ int launch_align(ctb_ctx* ctx, cudaStream_t st, const void* topk_ids, int ids_bi
   }
   const int extra = warm ? std::max(1, (ctx->sm_count - C) / C) : 0;  // whole clusters that only warm the L2
   const unsigned char* warm_p = static_cast<const unsigned char*>(warm);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(C * (1 + extra));
-  cfg.blockDim = dim3(kAlignThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = C;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cfg.numAttrs = C > 1 ? 1 : 0;  // a single CTA is launched as an ordinary grid (a cluster of one by default)
+  const int grid = C * (1 + extra);
   cudaError_t e;
   if (ids_bits == 32)
-    e = cudaLaunchKernelEx(&cfg, moe_align_kernel<int>, (const int*)topk_ids, T, topk, E, tile_m, sorted_token_ids,
-                           sorted_expert_ids, num_blocks, capacity, skip_empty, ctx->dev_status, warm_p, warm_bytes);
+    e = launch_kernel(moe_align_kernel<int>, grid, kAlignThreads, smem, st, C, (const int*)topk_ids, T, topk, E, tile_m,
+                      sorted_token_ids, sorted_expert_ids, num_blocks, capacity, skip_empty, ctx->dev_status, warm_p, warm_bytes);
   else
-    e = cudaLaunchKernelEx(&cfg, moe_align_kernel<long long>, (const long long*)topk_ids, T, topk, E, tile_m,
-                           sorted_token_ids, sorted_expert_ids, num_blocks, capacity, skip_empty, ctx->dev_status, warm_p,
-                           warm_bytes);
+    e = launch_kernel(moe_align_kernel<long long>, grid, kAlignThreads, smem, st, C, (const long long*)topk_ids, T, topk, E,
+                      tile_m, sorted_token_ids, sorted_expert_ids, num_blocks, capacity, skip_empty, ctx->dev_status, warm_p,
+                      warm_bytes);
   if (e != cudaSuccess) return cuda_fail(e, "moe align launch");
   return CTB_OK;
 }
@@ -1189,7 +1184,7 @@ int ctb_moe_router(ctb_ctx* ctx, void* stream, const void* hidden, const void* W
 #define CTB_LAUNCH_ROUTER(TTV)                                                                                  \
   ce = cudaFuncSetAttribute(moe_router_kernel<TTV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);    \
   if (ce != cudaSuccess) return cuda_fail(ce, "ctb_moe_router: shared memory opt-in");                          \
-  moe_router_kernel<TTV><<<grid, kRouterThreads, smem, static_cast<cudaStream_t>(stream)>>>(                    \
+  launch_kernel(moe_router_kernel<TTV>, grid, kRouterThreads, smem, static_cast<cudaStream_t>(stream), 0,                     \
       (const __half*)hidden, (const __half*)W_r, topk_ids, (__half*)topk_weights, logits, (int)T, (int)H, (int)E, \
       topk, eg, tw);
   if (TT == 4) { CTB_LAUNCH_ROUTER(4) } else { CTB_LAUNCH_ROUTER(2) }
@@ -1245,7 +1240,7 @@ int ctb_moe_silu_and_mul(ctb_ctx* ctx, void* stream, const void* A, const void* 
   if (cols == 0) return CTB_OK;
   CTB_CHECK_DEV(A); CTB_CHECK_DEV(B); CTB_CHECK_DEV(C);
   const long long tot = n * cols;
-  moe_silu_and_mul_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_kernel(moe_silu_and_mul_kernel, (unsigned)((tot + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream), 0,
       (const __half*)A, (const __half*)B, (__half*)C, (int)n, cols, lda, ldb, ldc);
   CTB_CHECK_LAUNCH("ctb_moe_silu_and_mul launch");
   return CTB_OK;
@@ -1295,7 +1290,7 @@ int ctb_moe_ffn(ctb_ctx* ctx, void* stream, const void* hidden, const void* w1, 
                   (int)topk);
   if (r) return r;
   const long long n8 = T * (H / 8);
-  moe_combine_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, st>>>(slots, (__half*)out, (int)T, (int)H, (int)topk);
+  launch_kernel(moe_combine_kernel, (unsigned)((n8 + 255) / 256), 256, 0, st, 0, slots, (__half*)out, (int)T, (int)H, (int)topk);
   CTB_CHECK_LAUNCH("ctb_moe_ffn combine launch");
   return CTB_OK;
 }
@@ -1386,7 +1381,7 @@ int ctb_moe_gather_rows(ctb_ctx* ctx, void* stream, void* dst, const void* src, 
   if ((uintptr_t)dst % 16 || (uintptr_t)src % 16) return fail(CTB_BAD_ALIGN, "ctb_moe_gather_rows: 16-byte alignment");
   const int vecs = (int)(row_elems / 8);
   const long long tot = n_ids * vecs;
-  moe_gather_rows_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_kernel(moe_gather_rows_kernel, (unsigned)((tot + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream), 0,
       (uint4*)dst, (const uint4*)src, ids, n_ids, vecs, num_token_replicas, src_rows);
   CTB_CHECK_LAUNCH("ctb_moe_gather_rows launch");
   return CTB_OK;
@@ -1402,7 +1397,7 @@ int ctb_moe_scatter_rows(ctb_ctx* ctx, void* stream, void* dst, const void* src,
   if ((uintptr_t)dst % 16 || (uintptr_t)src % 16) return fail(CTB_BAD_ALIGN, "ctb_moe_scatter_rows: 16-byte alignment");
   const int vecs = (int)(row_elems / 8);
   const long long tot = n_ids * vecs;
-  moe_scatter_rows_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_kernel(moe_scatter_rows_kernel, (unsigned)((tot + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream), 0,
       (uint4*)dst, (const uint4*)src, ids, n_ids, vecs, dst_rows);
   CTB_CHECK_LAUNCH("ctb_moe_scatter_rows launch");
   return CTB_OK;
@@ -1416,7 +1411,7 @@ int ctb_moe_combine(ctb_ctx* ctx, void* stream, const void* slots, void* out, in
   CTB_CHECK_DEV(slots); CTB_CHECK_DEV(out);
   if ((uintptr_t)slots % 16 || (uintptr_t)out % 16) return fail(CTB_BAD_ALIGN, "ctb_moe_combine: 16-byte alignment");
   const long long n8 = T * (H / 8);
-  moe_combine_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_kernel(moe_combine_kernel, (unsigned)((n8 + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream), 0,
       (const __half*)slots, (__half*)out, (int)T, (int)H, (int)topk);
   CTB_CHECK_LAUNCH("ctb_moe_combine launch");
   return CTB_OK;

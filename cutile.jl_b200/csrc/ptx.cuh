@@ -41,6 +41,16 @@ __device__ __forceinline__ bool elect_one() {
 #define CTB_WARP_WAIT(...) (__all_sync(0xffffffffu, mbar_wait(__VA_ARGS__)))
 #define CTB_WARP_WAIT1(...) (__shfl_sync(0xffffffffu, (threadIdx.x & 31) == 0 ? (int)mbar_wait(__VA_ARGS__) : 1, 0) != 0)
 
+// Start of a kernel's work on global memory.  Kernels launched through launch_kernel (ctx.h) carry programmatic stream
+// serialization: its CTAs may become resident while the kernel before it on the stream still runs,
+// and this wait ends when that kernel has completed and its stores are visible.  The trigger before it lets the next
+// kernel's CTAs do the same.  Barrier set-up, TMEM allocation and descriptor prefetch stand before the call and so run
+// under the tail of the previous kernel.
+__device__ __forceinline__ void grid_dependency_sync() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");

@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(kThreads) softmax_staged_kernel(T* __restrict_
     fence_mbar_init();
   }
   __syncthreads();
+  grid_dependency_sync();
 
   const int first = blockIdx.x, step = gridDim.x;
   const int nrows = first < M ? (M - first + step - 1) / step : 0;
@@ -208,6 +209,7 @@ __global__ void __launch_bounds__(kRowThreads) softmax_row_smem_kernel(T* __rest
     fence_mbar_init();
   }
   __syncthreads();
+  grid_dependency_sync();
   P* buf = reinterpret_cast<P*>(smem);
   auto block_reduce = [&](float v, bool is_max) {
     v = is_max ? warp_max(v) : warp_sum(v);
@@ -284,6 +286,7 @@ template <typename T, int VEC, int CACHE>
 __global__ void __launch_bounds__(kThreads) softmax_online_kernel(T* __restrict__ out, const T* __restrict__ in,
                                                                   int N, int M, long long ld_out, long long ld_in) {
   __shared__ float red[kWarps];
+  grid_dependency_sync();
   const int tid = threadIdx.x;
   const int nvec = (N + VEC - 1) / VEC;  // VEC==4 only when N % 4 == 0
   const int nstep = (nvec + kThreads - 1) / kThreads;
@@ -374,7 +377,7 @@ int launch(ctb_ctx* ctx, cudaStream_t st, T* out, const T* in, int N, int M, lon
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads, smem);
     if (per_sm < 1) per_sm = 1;
     const int grid = min(M, ctx->sm_count * per_sm);
-    k<<<grid, kThreads, smem, st>>>(out, in, N, M, ldo, ldi, stage_bytes, ctx->dev_status);
+    launch_kernel(k, grid, kThreads, smem, st, 0, out, in, N, M, ldo, ldi, stage_bytes, ctx->dev_status);
   } else if (bulk_ok && row_bytes <= 200 * 1024) {
     const size_t smem = (row_bytes + 127) & ~size_t(127);
     auto k = softmax_row_smem_kernel<T>;
@@ -382,14 +385,14 @@ int launch(ctb_ctx* ctx, cudaStream_t st, T* out, const T* in, int N, int M, lon
     if (e != cudaSuccess) return cuda_fail(e, "ctb_softmax: shared memory opt-in");
     const int per_sm = std::max(1, (int)((size_t)220 * 1024 / (smem + 2048)));
     const int grid = min(M, ctx->sm_count * std::min(per_sm, 4));
-    k<<<grid, kRowThreads, smem, st>>>(out, in, N, M, ldo, ldi, ctx->dev_status);
+    launch_kernel(k, grid, kRowThreads, smem, st, 0, out, in, N, M, ldo, ldi, ctx->dev_status);
   } else {
     int per_sm = 8;
     const int grid = min(M, ctx->sm_count * per_sm);
     if (vec_ok)
-      softmax_online_kernel<T, 4, 8><<<grid, kThreads, 0, st>>>(out, in, N, M, ldo, ldi);
+      launch_kernel(softmax_online_kernel<T, 4, 8>, grid, kThreads, 0, st, 0, out, in, N, M, ldo, ldi);
     else
-      softmax_online_kernel<T, 1, 8><<<grid, kThreads, 0, st>>>(out, in, N, M, ldo, ldi);
+      launch_kernel(softmax_online_kernel<T, 1, 8>, grid, kThreads, 0, st, 0, out, in, N, M, ldo, ldi);
   }
   CTB_CHECK_LAUNCH("ctb_softmax launch");
   return CTB_OK;
