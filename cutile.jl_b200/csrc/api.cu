@@ -63,6 +63,11 @@ int* sched_slot(ctb_ctx* ctx) {
   return ctx->sched_pool + 2 * (n % kSchedSlots);
 }
 
+int* ticket_slots(ctb_ctx* ctx) {
+  const unsigned n = __atomic_fetch_add(&ctx->tickets_next, 1u, __ATOMIC_RELAXED);
+  return ctx->tickets + (size_t)kTickets * (n % kTicketSlots);
+}
+
 EncodeTiledFn encode_tiled() {
   static EncodeTiledFn fn = nullptr;
   static std::once_flag once;
@@ -134,6 +139,8 @@ int ctb_create(ctb_ctx** out, int device) {
   c->workspace_bytes = 0;
   c->sched_pool = nullptr;
   c->sched_next = 0;
+  c->tickets = nullptr;
+  c->tickets_next = 0;
   c->flag_wait_ns = 2000000000ull;
   c->tf32_rne = 0;
   c->comm = nullptr;
@@ -141,6 +148,8 @@ int ctb_create(ctb_ctx** out, int device) {
   if (e == cudaSuccess) e = cudaMemset(c->dev_status, 0, sizeof(int));
   if (e == cudaSuccess) e = cudaMalloc(&c->sched_pool, 2 * kSchedSlots * sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(c->sched_pool, 0, 2 * kSchedSlots * sizeof(int));
+  if (e == cudaSuccess) e = cudaMalloc(&c->tickets, kTicketSlots * kTickets * sizeof(int));
+  if (e == cudaSuccess) e = cudaMemset(c->tickets, 0, kTicketSlots * kTickets * sizeof(int));
   if (e != cudaSuccess) {
     delete c;
     return cuda_fail(e, "ctb_create: status word");
@@ -156,6 +165,7 @@ void ctb_destroy(ctb_ctx* ctx) {
   if (ctx->workspace) cudaFree(ctx->workspace);
   if (ctx->dev_status) cudaFree(ctx->dev_status);
   if (ctx->sched_pool) cudaFree(ctx->sched_pool);
+  if (ctx->tickets) cudaFree(ctx->tickets);
   delete ctx;
 }
 

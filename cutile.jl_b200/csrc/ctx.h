@@ -23,6 +23,10 @@ struct ctb_ctx {
   // that overlap on the device (different streams) do not share one.
   int* sched_pool;
   unsigned sched_next;
+  // Arrival counters of reductions whose last CTA finishes the job: kTicketSlots sets of kTickets ints, zero between
+  // launches (the last CTA returns its counter to zero).  Launches take the sets in turn.
+  int* tickets;
+  unsigned tickets_next;
   void* comm;             // ctb_internal::Comm* once an NCCL communicator is attached (multi.cu)
   unsigned long long flag_wait_ns;  // how long a kernel waits for another rank's flag before it gives up
   int tf32_rne;           // 1: f32 GEMM operands are rounded to TF32 (nearest even) by a pass of their own first
@@ -46,8 +50,11 @@ int moe_experts_rows(ctb_ctx* ctx, cudaStream_t st, const void* rows, int64_t ld
                      const void* gates, int64_t R, int64_t H, int64_t I, int64_t E_local, const void* w1_local,
                      const void* w2_local, int tile_m, void* C, int64_t ldc, void* const* c_peer, int64_t c_split);
 constexpr int kSchedSlots = 256;
+constexpr int kTickets = 4096, kTicketSlots = 16;
 // The next pair of work counters of the context (see ctb_ctx::sched_pool).
 int* sched_slot(ctb_ctx* ctx);
+// The next set of kTickets arrival counters of the context (see ctb_ctx::tickets).
+int* ticket_slots(ctb_ctx* ctx);
 
 // cuTensorMapEncodeTiled, resolved through the runtime so that the library has
 // no link-time dependency on libcuda and loads on machines without a driver.
