@@ -12,6 +12,7 @@
 #include <math.h>
 
 #include <algorithm>
+#include <cmath>
 #include <type_traits>
 
 #include "ctx.h"
@@ -26,122 +27,357 @@ constexpr int kMaxInputs = CTB_TILED_MAX_INPUTS;
 constexpr int kMaxConsts = CTB_TILED_MAX_CONSTS;
 constexpr int kStack = 4;
 
-// One instruction word of the accumulator machine.  The accumulator A is the top of a four-entry register stack.
+// One instruction word of the accumulator machine.  The accumulator A is the top of a four-entry stack.
 //   kind LOAD : push; A = operand
 //   kind UNARY: A = code(A)
 //   kind BIN  : A = A code operand, or operand code A when the REV bit is set; an operand from the stack is popped
 // operand source: the stack entry below A (BIN only), inputs[arg] or constants[arg].
-enum : unsigned { K_LOAD = 0, K_UNARY = 1, K_BIN = 2 };
-enum : unsigned { SRC_STACK = 0, SRC_INPUT = 1, SRC_CONST = 2 };
+// Bits 24..31 of a word repeat kind, source, reversed and code as one dense index.
+enum : unsigned { K_LOAD = 0, K_UNARY = 1, K_BIN = 2, K_STORE = 3 };
+enum : unsigned { SRC_STACK = 0, SRC_INPUT = 1, SRC_CONST = 2, SRC_TEMP = 3 };  // STORE, TEMP: shared subexpressions only
 constexpr unsigned kRevBit = 1u << 4;
-// Bits 24..31: the index the vector kernel switches on, dense so that the switch is one jump through a table:
-// 0, 1 = push an input / a constant; 2..13 = the unary codes NEG..ABS2; then the seven binary codes for each of the six
-// (operand source, reversed) pairs.
-constexpr unsigned kDispatchUnary = 2, kDispatchBinary = 14;
-__host__ __device__ constexpr unsigned bin_variant(unsigned src, bool rev) {
-  return (src == SRC_INPUT ? 0u : src == SRC_CONST ? 1u : 2u) * 2u + (rev ? 1u : 0u);
+constexpr unsigned dispatch_index(unsigned kind, unsigned src, bool rev, unsigned code) {
+  return kind == K_LOAD    ? (src == SRC_INPUT ? 0u : 1u)
+         : kind == K_UNARY ? 2u + (code - CTB_TILED_NEG)
+                           : 14u + 7u * ((src == SRC_INPUT ? 0u : src == SRC_CONST ? 1u : 2u) * 2u + (rev ? 1u : 0u)) +
+                                 (code - CTB_TILED_ADD);
 }
-__host__ __device__ constexpr unsigned dispatch_index(unsigned kind, unsigned src, bool rev, unsigned code) {
-  return kind == K_LOAD ? (src == SRC_INPUT ? 0u : 1u)
-         : kind == K_UNARY ? kDispatchUnary + (code - CTB_TILED_NEG)
-                           : kDispatchBinary + 7u * bin_variant(src, rev) + (code - CTB_TILED_ADD);
-}
-__host__ __device__ constexpr unsigned make_ins(unsigned kind, unsigned src, bool rev, unsigned code, unsigned arg) {
+constexpr unsigned make_ins(unsigned kind, unsigned src, bool rev, unsigned code, unsigned arg) {
   return kind | (src << 2) | (rev ? kRevBit : 0u) | (code << 8) | (arg << 16) | (dispatch_index(kind, src, rev, code) << 24);
 }
 
+// The kernel runs a lowered form without a stack: a value that waits (a stack entry, or a subexpression that occurs more
+// than once) sits in one of up to kTemps temporaries.  A lowered word is operation | argument << 8 | tail bits: the result
+// may still pass through A = p A + q (kTailFma) and be stored to temporary (word >> kTailStore) - 1 before the next word.
+// What bounds long programs is the dispatch (about 24 issue slots and 200-400 clocks of latency per word and thread; the
+// elements in flight are limited by registers), so words do much: adding, subtracting, multiplying by a constant and
+// negation are one fused multiply-add with (p, q) chosen so that the result is the operator's own (A + c = 1 A + c,
+// c - A = -1 A + c, A c = c A - 0, each rounded once) and ride on the word before them, subtracting an array is adding -1
+// times it, and the eight operations that most expressions consist of are three compares deep behind one.
+constexpr unsigned kSubtract = 1u << 10;    // L_ADD_*: A - operand
+constexpr unsigned kOperandFma = 1u << 11;  // L_MUL_*, L_ADD_*: the operand enters as p operand + q
+constexpr unsigned kTailFma = 1u << 12;
+constexpr int kTailStore = 13;
+enum : unsigned {
+  L_FMA = 0,                                       // A = p A + q
+  L_LOAD_INPUT, L_LOAD_TEMP,                       // A = operand
+  L_MUL_INPUT, L_MUL_TEMP, L_ADD_INPUT, L_ADD_TEMP,  // A = A * operand, A +- operand
+  L_LOAD_CONST,                                    // A = q
+  L_HOT,                                           // number of the operations above
+  L_UNARY = L_HOT,                                 // + code - NEG
+  L_BINARY = L_UNARY + (CTB_TILED_ABS2 - CTB_TILED_NEG + 1),  // + 10 * source + 2 * (SUB, DIV, MAX, MIN, POW) + reversed
+  L_COUNT = L_BINARY + 30
+};
+constexpr int kColdCodes[5] = {CTB_TILED_SUB, CTB_TILED_DIV, CTB_TILED_MAX, CTB_TILED_MIN, CTB_TILED_POW};
+constexpr int kTemps = 4;
+constexpr int kMaxIns = kMaxOps + kMaxOps / 2;
+
 struct Program {
   int n_ins;
-  unsigned ins[kMaxOps];
-  float consts[kMaxConsts];
+  int n_temps;
+  unsigned ins[kMaxIns + 1];  // one word of padding: the kernel fetches a word ahead
+  float2 pq[kMaxIns];
 };
 
+// How an operand is read (chosen on the host).
+enum : int {
+  OP_LINEAR = 0,  // laid out like the destination, aligned: a vector of four elements per group
+  OP_SCALAR = 1,  // a single element
+  OP_ROW = 2,     // expanded, first extent a multiple of four: one aligned vector, or one element, per group
+  OP_SHIFTED = 3, // laid out like the destination, not aligned: element by element
+  OP_ELEM = 4,    // anything else: element by element, each with its own coordinates
+  OP_VECTOR = 5,  // OP_ROW that varies along the first dimension only (a bias): one aligned vector per group
+  OP_FIXED = 6    // varies along the first dimension only, and the grid is such that every group of a thread lies at the
+                  // same place of it: four elements per thread, read once
+};
 struct Operands {
   const void* ptr[kMaxInputs];
   long long stride[kMaxInputs][3];
+  int mode[kMaxInputs];
+  unsigned slot[kMaxInputs];  // offset in shared memory
 };
 
 // ---- postfix program -> accumulator-machine instructions (host) ---------------------------------------------------
 struct Node {
   int op, arg, left, right;  // left/right: node indices, -1 for none
   int need;                  // stack entries the subtree needs when it is evaluated into A
+  int uses, temp;            // times it is an operand; temporary that holds it once evaluated, -1 for none
 };
-inline bool is_leaf(const Node& n) { return n.op == CTB_TILED_INPUT || n.op == CTB_TILED_CONST; }
-inline unsigned leaf_src(const Node& n) { return n.op == CTB_TILED_INPUT ? SRC_INPUT : SRC_CONST; }
+inline bool is_input(const Node& n) { return n.op == CTB_TILED_INPUT; }
 
 struct Compiler {
   Node nodes[kMaxOps];
-  int n_nodes = 0;
-  Program* out = nullptr;
-  void put(unsigned w) { out->ins[out->n_ins++] = w; }
-  void emit(int i) {
+  int n_nodes = 0, n_words = 0;
+  bool lowering = false;
+  const float* constants = nullptr;  // lowering only
+  unsigned words[kMaxIns];           // with a stack; kind STORE only for shared subexpressions
+  float2 affine[kMaxIns];            // of words with an operand p leaf + q, else (0, 0)
+  void put(unsigned w) {
+    affine[n_words] = make_float2(0.f, 0.f);
+    words[n_words++] = w;
+  }
+  bool plain(int i) const { return nodes[i].op == CTB_TILED_INPUT || nodes[i].op == CTB_TILED_CONST || nodes[i].temp >= 0; }
+  bool leaf(int i) const { return plain(i); }
+  // Is node i = p leaf + q with one rounding, the leaf an input or a temporary?  Such an operand of + - * needs no
+  // evaluation of its own when lowered.
+  bool affine_leaf(int i, int* of, float* p, float* q) const {
+    if (!lowering || plain(i)) return false;
     const Node& n = nodes[i];
-    if (is_leaf(n)) {
-      put(make_ins(K_LOAD, leaf_src(n), false, 0, (unsigned)n.arg));
-    } else if (n.right < 0) {
+    auto array = [&](int k) { return plain(k) && (nodes[k].temp >= 0 || nodes[k].op == CTB_TILED_INPUT); };
+    if (n.op == CTB_TILED_NEG && array(n.left)) {
+      *of = n.left; *p = -1.f; *q = -0.f;
+      return true;
+    }
+    if (n.op < CTB_TILED_ADD || n.op > CTB_TILED_MUL) return false;
+    const bool left = array(n.left);
+    const int a = left ? n.left : n.right, k = left ? n.right : n.left;
+    if (!array(a) || nodes[k].op != CTB_TILED_CONST) return false;
+    const float v = constants[nodes[k].arg];
+    *of = a;
+    if (n.op == CTB_TILED_MUL) { *p = v; *q = -0.f; }
+    else if (n.op == CTB_TILED_ADD) { *p = 1.f; *q = v; }
+    else { *p = left ? 1.f : -1.f; *q = left ? -v : v; }
+    return true;
+  }
+  unsigned leaf_src(int i) const { return nodes[i].temp >= 0 ? SRC_TEMP : is_input(nodes[i]) ? SRC_INPUT : SRC_CONST; }
+  unsigned leaf_arg(int i) const { return (unsigned)(nodes[i].temp >= 0 ? nodes[i].temp : nodes[i].arg); }
+  // stack entries of every node from those of its operands (operands come before their operators)
+  void set_needs() {
+    for (int i = 0; i < n_nodes; ++i) {
+      Node& n = nodes[i];
+      n.need = 1;
+      if (n.left < 0) continue;
+      const int l = leaf(n.left) ? 1 : nodes[n.left].need;
+      if (n.right < 0) { n.need = l; continue; }
+      const int r = leaf(n.right) ? 1 : nodes[n.right].need;
+      int of;
+      float p, q;
+      const bool in_place = n.op <= CTB_TILED_MUL && !leaf(n.left) && !leaf(n.right);
+      if (in_place && affine_leaf(n.right, &of, &p, &q)) { n.need = l; continue; }
+      if (in_place && n.op != CTB_TILED_SUB && affine_leaf(n.left, &of, &p, &q)) { n.need = r; continue; }
+      n.need = leaf(n.right) ? l : leaf(n.left) ? r : std::max(std::max(l, r), std::min(l, r) + 1);
+    }
+  }
+  void emit(int i) {  // the value of a node (a leaf only when it is the whole expression) into A
+    const Node& n = nodes[i];
+    if (leaf(i)) {
+      put(make_ins(K_LOAD, leaf_src(i), false, 0, leaf_arg(i)));
+    } else {
+      emit_op(i);
+    }
+  }
+  void emit_op(int i) {
+    const Node& n = nodes[i];
+    if (n.right < 0) {
       emit(n.left);
       if (n.op != CTB_TILED_IDENTITY) put(make_ins(K_UNARY, 0, false, (unsigned)n.op, 0));
-    } else {
-      const Node &l = nodes[n.left], &r = nodes[n.right];
-      const bool commutes = n.op == CTB_TILED_ADD || n.op == CTB_TILED_MUL;  // a op b == b op a bit for bit
-      if (is_leaf(r)) {         // A = left; A = A op leaf
-        emit(n.left);
-        put(make_ins(K_BIN, leaf_src(r), false, (unsigned)n.op, (unsigned)r.arg));
-      } else if (is_leaf(l)) {  // A = right; A = leaf op A
-        emit(n.right);
-        put(make_ins(K_BIN, leaf_src(l), !commutes, (unsigned)n.op, (unsigned)l.arg));
-      } else if (l.need > r.need) {  // the deeper side first: A = right, below it left; A = below op A
-        emit(n.left);
-        emit(n.right);
-        put(make_ins(K_BIN, SRC_STACK, !commutes, (unsigned)n.op, 0));
-      } else {                  // A = left, below it right; A = A op below
-        emit(n.right);
-        emit(n.left);
-        put(make_ins(K_BIN, SRC_STACK, false, (unsigned)n.op, 0));
+      return;
+    }
+    const bool commutes = n.op == CTB_TILED_ADD || n.op == CTB_TILED_MUL;  // a op b == b op a bit for bit
+    int of;
+    float p, q;
+    if (n.op <= CTB_TILED_MUL && !leaf(n.left) && !leaf(n.right)) {
+      const bool right = affine_leaf(n.right, &of, &p, &q);
+      if (right || (commutes && affine_leaf(n.left, &of, &p, &q))) {  // A = one side; A = A op (p leaf + q)
+        emit(right ? n.left : n.right);
+        put(make_ins(K_BIN, leaf_src(of), false, (unsigned)n.op, leaf_arg(of)));
+        affine[n_words - 1] = make_float2(p, q);
+        return;
       }
+    }
+    if (leaf(n.right)) {        // A = left; A = A op leaf
+      emit(n.left);
+      put(make_ins(K_BIN, leaf_src(n.right), false, (unsigned)n.op, leaf_arg(n.right)));
+    } else if (leaf(n.left)) {  // A = right; A = leaf op A
+      emit(n.right);
+      put(make_ins(K_BIN, leaf_src(n.left), !commutes, (unsigned)n.op, leaf_arg(n.left)));
+    } else if (nodes[n.left].need > nodes[n.right].need) {  // the deeper side first: A = right, below it left; A = below op A
+      emit(n.left);
+      emit(n.right);
+      put(make_ins(K_BIN, SRC_STACK, !commutes, (unsigned)n.op, 0));
+    } else {                    // A = left, below it right; A = A op below
+      emit(n.right);
+      emit(n.left);
+      put(make_ins(K_BIN, SRC_STACK, false, (unsigned)n.op, 0));
     }
   }
 };
 
-// Returns 0, or a negative number -(k+1) naming the offending postfix operation k with *why set; -1000 when the
-// expression needs more than kStack live values.  *need: the stack entries the instructions use (1 = the accumulator
-// alone).
-int compile_program(const int32_t* program, int n_ops, int n_inputs, int n_constants, Program* out, const char** why,
-                    int* need = nullptr) {
-  Compiler c;
-  c.out = out;
-  out->n_ins = 0;
+// Parses the postfix program into c (the root is the last node).  Returns 0, or a negative number -(k+1) naming the
+// offending operation k with *why set.  share: equal subexpressions become one node (value numbering).
+int parse_program(const int32_t* program, int n_ops, int n_inputs, int n_constants, bool share, Compiler* c, int* root,
+                  const char** why) {
   int stack[kMaxOps], depth = 0;
   for (int k = 0; k < n_ops; ++k) {
     const int op = program[2 * k], arg = program[2 * k + 1];
-    Node n = {op, arg, -1, -1, 1};
+    Node n = {op, 0, -1, -1, 1, 0, -1};
     if (op == CTB_TILED_INPUT) {
       if (arg < 0 || arg >= n_inputs) { *why = "names an input that was not given"; return -(k + 1); }
+      n.arg = arg;
     } else if (op == CTB_TILED_CONST) {
       if (arg < 0 || arg >= n_constants) { *why = "names a constant that was not given"; return -(k + 1); }
+      n.arg = arg;
     } else if (op >= CTB_TILED_IDENTITY && op <= CTB_TILED_ABS2) {
       if (depth < 1) { *why = "finds an empty stack"; return -(k + 1); }
       n.left = stack[--depth];
-      n.need = c.nodes[n.left].need;
     } else if (op >= CTB_TILED_ADD && op <= CTB_TILED_POW) {
       if (depth < 2) { *why = "needs two values on the stack"; return -(k + 1); }
       n.right = stack[--depth];
       n.left = stack[--depth];
-      const Node &l = c.nodes[n.left], &r = c.nodes[n.right];
-      if (is_leaf(r)) n.need = l.need;
-      else if (is_leaf(l)) n.need = r.need;
-      else n.need = std::max(std::max(l.need, r.need), std::min(l.need, r.need) + 1);
     } else {
       *why = "is not an operation code";
       return -(k + 1);
     }
-    c.nodes[c.n_nodes] = n;
-    stack[depth++] = c.n_nodes++;
+    int at = c->n_nodes;
+    if (share) {
+      at = 0;
+      auto same = [&](const Node& m) { return m.op == n.op && m.arg == n.arg && m.left == n.left && m.right == n.right; };
+      while (at < c->n_nodes && !same(c->nodes[at])) ++at;
+    }
+    if (at == c->n_nodes) {
+      if (n.left >= 0) ++c->nodes[n.left].uses;
+      if (n.right >= 0) ++c->nodes[n.right].uses;
+      c->nodes[c->n_nodes++] = n;
+    }
+    stack[depth++] = at;
   }
   if (depth != 1) { *why = "the program must leave exactly one value"; return -(n_ops + 1); }
-  if (c.nodes[stack[0]].need > kStack) return -1000;
-  if (need) *need = c.nodes[stack[0]].need;
-  c.emit(stack[0]);
+  *root = stack[0];
+  return 0;
+}
+
+// The instructions with a stack, without sharing (what ctb_tiled_compile reports); -1000 when the expression needs more
+// than kStack live values.
+int compile_program(const int32_t* program, int n_ops, int n_inputs, int n_constants, Compiler* c, const char** why) {
+  int root;
+  const int bad = parse_program(program, n_ops, n_inputs, n_constants, false, c, &root, why);
+  if (bad) return bad;
+  c->set_needs();
+  if (c->nodes[root].need > kStack) return -1000;
+  c->emit(root);
+  return 0;
+}
+
+// The lowered program of the kernel.  Subexpressions that occur more than once are evaluated first, each into a temporary
+// of its own (v = x + b is computed once in 0.5 v (1 + tanh(c (v + k v v v))): 11 instructions instead of 22), those that
+// save most first, as far as the temporaries reach; the rest is evaluated where it occurs.
+int lower_program(const int32_t* program, int n_ops, int n_inputs, const float* constants, int n_constants, Program* out,
+                  const char** why) {
+  Compiler c;
+  c.lowering = true;
+  c.constants = constants;
+  int root;
+  const int bad = parse_program(program, n_ops, n_inputs, n_constants, true, &c, &root, why);
+  if (bad) return bad;
+  int cost[kMaxOps];  // operators in the tree below a node
+  for (int i = 0; i < c.n_nodes; ++i) {
+    const Node& n = c.nodes[i];
+    cost[i] = n.left < 0 ? 0 : 1 + cost[n.left] + (n.right < 0 ? 0 : cost[n.right]);
+  }
+  auto stack_need = [&]() {  // over the root and every shared subexpression
+    c.set_needs();
+    int need = c.nodes[root].need;
+    for (int i = 0; i < c.n_nodes; ++i)
+      if (c.nodes[i].temp >= 0) need = std::max(need, c.nodes[i].need);
+    return need;
+  };
+  if (stack_need() > kStack) return -1000;
+  int shared = 0;
+  bool tried[kMaxOps] = {};
+  for (;;) {
+    int best = -1;
+    for (int i = 0; i < c.n_nodes; ++i)
+      if (!tried[i] && i != root && c.nodes[i].uses > 1 && cost[i] > 0 &&
+          (best < 0 || cost[i] * (c.nodes[i].uses - 1) > cost[best] * (c.nodes[best].uses - 1)))
+        best = i;
+    if (best < 0) break;
+    tried[best] = true;
+    c.nodes[best].temp = 0;  // any value: the leaf test
+    if (stack_need() - 1 + shared + 1 > kTemps) c.nodes[best].temp = -1;
+    else ++shared;
+  }
+  int next = stack_need() - 1;  // stack entries take the first temporaries
+  out->n_temps = next + shared;
+  for (int i = 0; i < c.n_nodes; ++i)
+    if (c.nodes[i].temp >= 0) c.nodes[i].temp = next++;
+  for (int i = 0; i < c.n_nodes; ++i)
+    if (c.nodes[i].temp >= 0) {
+      c.emit_op(i);
+      c.put(make_ins(K_STORE, 0, false, 0, (unsigned)c.nodes[i].temp));
+    }
+  c.emit(root);
+  // stack -> temporaries: the value at depth d of the stack (0 = bottom) waits in temporary d
+  out->n_ins = 0;
+  int depth = 0, held = -1;  // held: the temporary whose value A holds as well, -1 for none
+  bool tail_free = false;  // the last word can still take a multiply-add
+  auto put = [&](unsigned op, unsigned arg, float q, bool uses_q) {
+    out->pq[out->n_ins].x = 0.f;
+    out->pq[out->n_ins].y = q;
+    out->ins[out->n_ins++] = op | (arg << 8);
+    held = -1;
+    tail_free = !uses_q;
+  };
+  auto fma = [&](float p, float q) {  // A = p A + q
+    if (!tail_free) put(L_FMA, 0, 0.f, true);
+    else out->ins[out->n_ins - 1] |= kTailFma;
+    out->pq[out->n_ins - 1].x = p;
+    out->pq[out->n_ins - 1].y = q;
+    tail_free = false;
+    held = -1;
+  };
+  auto store = [&](int t) {  // with the word that computed the value
+    if (out->ins[out->n_ins - 1] >> kTailStore) fma(1.f, -0.f);  // that one stores already: A = A
+    out->ins[out->n_ins - 1] |= (unsigned)(t + 1) << kTailStore;
+    tail_free = false;
+    held = t;
+  };
+  for (int k = 0; k < c.n_words; ++k) {
+    const unsigned w = c.words[k], kind = w & 3u, src = (w >> 2) & 3u, code = (w >> 8) & 0xffu, arg = (w >> 16) & 0xffu;
+    const bool rev = (w & kRevBit) != 0;
+    if (kind == K_LOAD) {
+      if (depth > 0) store(depth - 1);
+      ++depth;
+      if (src == SRC_INPUT) put(L_LOAD_INPUT, arg, 0.f, false);
+      else if (src == SRC_CONST) put(L_LOAD_CONST, 0, constants[arg], true);
+      else if ((int)arg != held) put(L_LOAD_TEMP, arg, 0.f, false);
+    } else if (kind == K_UNARY) {
+      if (code == CTB_TILED_NEG) fma(-1.f, -0.f);
+      else put(L_UNARY + code - CTB_TILED_NEG, 0, 0.f, false);
+    } else if (kind == K_STORE) {
+      store((int)arg);
+      depth = 0;
+    } else {
+      unsigned from = src, index = arg;
+      if (src == SRC_STACK) {
+        --depth;
+        from = SRC_TEMP;
+        index = (unsigned)(depth - 1);
+      }
+      const bool in = from == SRC_INPUT;
+      const float2 aff = c.affine[k];
+      if (aff.x != 0.f || aff.y != 0.f || std::signbit(aff.y)) {
+        put(code == CTB_TILED_MUL ? (in ? L_MUL_INPUT : L_MUL_TEMP) : (in ? L_ADD_INPUT : L_ADD_TEMP),
+            index | (code == CTB_TILED_SUB ? kSubtract >> 8 : 0u) | kOperandFma >> 8, aff.y, true);
+        out->pq[out->n_ins - 1].x = aff.x;
+        out->n_temps = std::max(out->n_temps, 1);  // the kernel without temporaries does not look for it
+      } else if (from == SRC_CONST && code <= CTB_TILED_MUL) {
+        const float v = constants[index];
+        if (code == CTB_TILED_ADD) fma(1.f, v);
+        else if (code == CTB_TILED_MUL) fma(v, -0.f);
+        else if (rev) fma(-1.f, v);
+        else fma(1.f, -v);
+      } else if (code == CTB_TILED_MUL) {
+        put(in ? L_MUL_INPUT : L_MUL_TEMP, index, 0.f, false);
+      } else if (code == CTB_TILED_ADD || (code == CTB_TILED_SUB && !rev)) {
+        put(in ? L_ADD_INPUT : L_ADD_TEMP, index | (code == CTB_TILED_ADD ? 0u : kSubtract >> 8), 0.f, false);
+      } else {
+        unsigned pos = 0;
+        while (kColdCodes[pos] != (int)code) ++pos;
+        put(L_BINARY + 10u * (in ? 0u : from == SRC_CONST ? 1u : 2u) + 2u * pos + (rev ? 1u : 0u), index,
+            from == SRC_CONST ? constants[index] : 0.f, from == SRC_CONST);
+      }
+    }
+  }
   return 0;
 }
 
@@ -183,178 +419,6 @@ template <typename T>
 __device__ __forceinline__ void store1(void* p, long long i, float v) {
   if constexpr (sizeof(T) == 4) static_cast<float*>(p)[i] = v;
   else static_cast<__half*>(p)[i] = __float2half_rn(v);
-}
-
-// The general path, for arrays the vector path below cannot take (a first extent that is not a multiple of four, rows
-// that do not start on 16-byte boundaries): instantiated with V = 1, G = 1, NIN = 4, DEEP = true, one element per
-// thread and trip, operands and stack in registers.  (V = 4 groups of four neighbouring elements, G groups per thread
-// and NIN operands held are the knobs of the register-only vector kernel this one was before the operands moved to
-// shared memory; they still compile.)
-// DENSE: every operand either has the destination's shape (dense) or is a single element: one linear index, no
-// division.  Otherwise the group index is split into its three coordinates (32-bit arithmetic; the host checks
-// that the element count fits).  The operands are read once per element into registers.
-template <typename T, int V, int G, bool DENSE, int NIN, bool DEEP>
-__global__ void __launch_bounds__(256)
-    tiled_broadcast_kernel(void* __restrict__ dest, const Operands in, const Program prog, int n_inputs, long long d0,
-                           long long d1, long long d2) {
-  constexpr int E = V * G;
-  constexpr int ES = DEEP ? E : 1;  // extent of the stack entries below the accumulator
-  const long long n0 = d0 / V, total = n0 * d1 * d2;
-  const long long grid_stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += grid_stride * G) {
-    long long o[G];  // element offset of each group in the destination
-    bool live[G];
-    float x[NIN][E];
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-      const long long ig = i + g * grid_stride;
-      live[g] = ig < total;
-      long long off[NIN];
-      long long st0[NIN];
-      if (DENSE) {
-        o[g] = ig * V;
-#pragma unroll
-        for (int a = 0; a < NIN; ++a) {
-          st0[a] = in.stride[a][0];
-          off[a] = st0[a] ? o[g] : 0;
-        }
-      } else {
-        const unsigned u = (unsigned)ig, un0 = (unsigned)n0, ud1 = (unsigned)d1;
-        const unsigned r = u / un0, i0 = (u - r * un0) * V, i2 = r / ud1, i1 = r - i2 * ud1;
-        o[g] = i0 + d0 * (i1 + d1 * (long long)i2);
-#pragma unroll
-        for (int a = 0; a < NIN; ++a) {
-          st0[a] = in.stride[a][0];
-          off[a] = i0 * st0[a] + i1 * in.stride[a][1] + i2 * in.stride[a][2];
-        }
-      }
-#pragma unroll
-      for (int a = 0; a < NIN; ++a) {
-        float* xa = &x[a][g * V];
-        if (a < n_inputs && live[g]) {
-          if (V == 4 && st0[a] == 1) {
-            if constexpr (sizeof(T) == 4) {
-              const float4 q = __ldcs(reinterpret_cast<const float4*>(static_cast<const float*>(in.ptr[a]) + off[a]));
-              xa[0] = q.x; xa[1 % V] = q.y; xa[2 % V] = q.z; xa[3 % V] = q.w;
-            } else {
-              const uint2 q = __ldcs(reinterpret_cast<const uint2*>(static_cast<const __half*>(in.ptr[a]) + off[a]));
-              const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&q.x));
-              const float2 hi = __half22float2(*reinterpret_cast<const __half2*>(&q.y));
-              xa[0] = lo.x; xa[1 % V] = lo.y; xa[2 % V] = hi.x; xa[3 % V] = hi.y;
-            }
-          } else {
-#pragma unroll
-            for (int v = 0; v < V; ++v) xa[v] = load1<T>(in.ptr[a], off[a] + v * st0[a]);
-          }
-        } else {
-#pragma unroll
-          for (int v = 0; v < V; ++v) xa[v] = 0.f;
-        }
-      }
-    }
-    float s0[E], s1[ES], s2[ES], s3[ES];  // the stack, top (the accumulator) first
-#pragma unroll
-    for (int v = 0; v < E; ++v) s0[v] = 0.f;
-#pragma unroll
-    for (int v = 0; v < ES; ++v) s1[v] = s2[v] = s3[v] = 0.f;
-    for (int k = 0; k < prog.n_ins; ++k) {
-      const unsigned w = prog.ins[k];
-      const unsigned kind = w & 3u, src = (w >> 2) & 3u, code = (w >> 8) & 0xffu, arg = (w >> 16) & 0xffu;
-      if (kind == K_UNARY) {
-        // one dispatch per instruction and thread, not per element
-#define CTB_U(CODE, EXPR)               \
-  case CODE:                            \
-    _Pragma("unroll") for (int v = 0; v < E; ++v) { const float t = s0[v]; s0[v] = (EXPR); } \
-    break;
-        switch (code) {
-          CTB_U(CTB_TILED_NEG, -t)
-          CTB_U(CTB_TILED_ABS, fabsf(t))
-          CTB_U(CTB_TILED_SQRT, sqrtf(t))
-          CTB_U(CTB_TILED_EXP, expf(t))
-          CTB_U(CTB_TILED_EXP2, exp2f(t))
-          CTB_U(CTB_TILED_LOG, logf(t))
-          CTB_U(CTB_TILED_LOG2, log2f(t))
-          CTB_U(CTB_TILED_SIN, sinf(t))
-          CTB_U(CTB_TILED_COS, cosf(t))
-          CTB_U(CTB_TILED_TANH, tanhf(t))
-          CTB_U(CTB_TILED_INV, 1.0f / t)
-          CTB_U(CTB_TILED_ABS2, t * t)
-          default: break;
-        }
-#undef CTB_U
-        continue;
-      }
-      float t[E];  // the operand
-      if (src == SRC_INPUT) {
-        const unsigned which = NIN == 1 ? 0u : NIN == 2 ? (arg & 1u) : (arg & 3u);
-#pragma unroll
-        for (int a = 0; a < NIN; ++a) {
-          if (which == (unsigned)a) {
-#pragma unroll
-            for (int v = 0; v < E; ++v) t[v] = x[a][v];
-          }
-        }
-      } else if (src == SRC_CONST) {
-        const float c = prog.consts[arg & (kMaxConsts - 1)];
-#pragma unroll
-        for (int v = 0; v < E; ++v) t[v] = c;
-      } else {  // the entry below the accumulator, popped (DEEP programs only)
-#pragma unroll
-        for (int v = 0; v < E; ++v) {
-          t[v] = s1[v % ES];
-          if (DEEP) { s1[v % ES] = s2[v % ES]; s2[v % ES] = s3[v % ES]; }
-        }
-      }
-      if (kind == K_LOAD) {
-#pragma unroll
-        for (int v = 0; v < E; ++v) {
-          if (DEEP) { s3[v % ES] = s2[v % ES]; s2[v % ES] = s1[v % ES]; s1[v % ES] = s0[v]; }
-          s0[v] = t[v];
-        }
-        continue;
-      }
-      if (w & kRevBit) {
-#pragma unroll
-        for (int v = 0; v < E; ++v) {
-          const float q = s0[v]; s0[v] = t[v]; t[v] = q;
-        }
-      }
-#define CTB_B(CODE, EXPR)               \
-  case CODE:                            \
-    _Pragma("unroll") for (int v = 0; v < E; ++v) { const float a = s0[v], b = t[v]; s0[v] = (EXPR); } \
-    break;
-      switch (code) {
-        CTB_B(CTB_TILED_ADD, a + b)
-        CTB_B(CTB_TILED_SUB, a - b)
-        CTB_B(CTB_TILED_MUL, a * b)
-        CTB_B(CTB_TILED_DIV, a / b)
-        CTB_B(CTB_TILED_MAX, fmaxf(a, b))
-        CTB_B(CTB_TILED_MIN, fminf(a, b))
-        default:
-#pragma unroll
-          for (int v = 0; v < E; ++v) s0[v] = powf(s0[v], t[v]);
-          break;
-      }
-#undef CTB_B
-    }
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-      if (!live[g]) continue;
-      const float* r = &s0[g * V];
-      if (V == 4) {
-        if constexpr (sizeof(T) == 4) {
-          __stcs(reinterpret_cast<float4*>(static_cast<float*>(dest) + o[g]), make_float4(r[0], r[1 % V], r[2 % V], r[3 % V]));
-        } else {
-          uint2 q;
-          *reinterpret_cast<__half2*>(&q.x) = __floats2half2_rn(r[0], r[1 % V]);
-          *reinterpret_cast<__half2*>(&q.y) = __floats2half2_rn(r[2 % V], r[3 % V]);
-          __stcs(reinterpret_cast<uint2*>(static_cast<__half*>(dest) + o[g]), q);
-        }
-      } else {
-        store1<T>(dest, o[g], r[0]);
-      }
-    }
-  }
 }
 
 // ---- sine and cosine for the vector path ---------------------------------------------------------------------------
@@ -410,9 +474,9 @@ __device__ __forceinline__ void sincos_all(float (&a)[E]) {
   }
 }
 
-// ---- the vector path: operands staged in shared memory by cp.async, two trips deep ----------------------------------
+// ---- the kernel: operands staged in shared memory by cp.async, two trips deep ---------------------------------------
 __device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-// 16 or 8 bytes global -> shared, asynchronous; src_bytes = 0 writes zeros and reads nothing
+// 16 or 8 bytes global -> shared, asynchronous; the bytes beyond src_bytes become zeros and are not read
 template <int BYTES>
 __device__ __forceinline__ void cp_async_group(unsigned dst, const void* src, unsigned src_bytes) {
   if constexpr (BYTES == 16)
@@ -423,46 +487,111 @@ __device__ __forceinline__ void cp_async_group(unsigned dst, const void* src, un
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+// one element global -> shared (asynchronous for 4-byte elements); zero when !live
+template <typename T>
+__device__ __forceinline__ void copy_element(unsigned dst, const T* src, bool live) {
+  if constexpr (sizeof(T) == 4) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(live ? 4u : 0u) : "memory");
+  } else {
+    const unsigned short v = live ? *reinterpret_cast<const unsigned short*>(src) : (unsigned short)0;
+    asm volatile("st.shared.u16 [%0], %1;" ::"r"(dst), "h"(v) : "memory");
+  }
+}
 
-// The element-wise part of one instruction, for all of a thread's elements.  The operation, its direction and the
+// A thread's values live in 64-bit registers of two neighbouring elements each: + and * then take half an instruction per
+// element (with single floats in between, the moves into aligned register pairs and back cost more than the arithmetic).
+using Pair = unsigned long long;
+__device__ __forceinline__ Pair pair(float lo, float hi) {
+  Pair r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpair(Pair p) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(p));
+  return r;
+}
+__device__ __forceinline__ Pair fma_pair(Pair a, Pair b, Pair c) {
+  Pair d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ Pair mul_pair(Pair a, Pair b) {
+  Pair d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
+// The element-wise part of an instruction that is neither + nor *.  The operation, its direction and the
 // kind of operand are template parameters and every instruction has its own straight-line code under the kernel's
-// dispatch: with run-time tests on them around the element loops a multiplication by a constant executed 8.2
-// instructions per element (counted with ncu by differencing programs), with straight-line code 4.5.
+// dispatch.
 template <int CODE, bool REV>
 __device__ __forceinline__ float binary_op(float p, float q) {
   const float a = REV ? q : p, b = REV ? p : q;
-  if constexpr (CODE == CTB_TILED_ADD) return a + b;
-  else if constexpr (CODE == CTB_TILED_SUB) return a - b;
-  else if constexpr (CODE == CTB_TILED_MUL) return a * b;
+  if constexpr (CODE == CTB_TILED_SUB) return a - b;
   else if constexpr (CODE == CTB_TILED_DIV) return a / b;
   else if constexpr (CODE == CTB_TILED_MAX) return fmaxf(a, b);
   else if constexpr (CODE == CTB_TILED_MIN) return fminf(a, b);
   else return powf(a, b);
 }
-template <int CODE, bool REV, int E>
-__device__ __forceinline__ void apply_binary(float (&s0)[E], const float (&t)[E]) {
+template <int CODE, bool REV, int H, typename Get>
+__device__ __forceinline__ void apply_binary(Pair (&s0)[H], Get t) {  // t(h): the operand of pair h
 #pragma unroll
-  for (int v = 0; v < E; ++v) s0[v] = binary_op<CODE, REV>(s0[v], t[v]);
-}
-template <int CODE, bool REV, int E>
-__device__ __forceinline__ void apply_binary(float (&s0)[E], float c) {
-#pragma unroll
-  for (int v = 0; v < E; ++v) s0[v] = binary_op<CODE, REV>(s0[v], c);
-}
-template <int CODE, int E>
-__device__ __forceinline__ void apply_unary(float (&s0)[E]) {
-  if constexpr (CODE == CTB_TILED_SIN) {
-    sincos_all<false>(s0);
-  } else if constexpr (CODE == CTB_TILED_COS) {
-    sincos_all<true>(s0);
-  } else {
-#pragma unroll
-    for (int v = 0; v < E; ++v) s0[v] = unary(CODE, s0[v]);  // CODE is a constant: the switch inside folds
+  for (int h = 0; h < H; ++h) {
+    const float2 a = unpair(s0[h]), b = unpair(t(h));
+    s0[h] = pair(binary_op<CODE, REV>(a.x, b.x), binary_op<CODE, REV>(a.y, b.y));
   }
 }
+// tanh of two elements.  The library's tanhf branches per element (20 instructions measured); here both forms are
+// evaluated, the polynomials two elements at a time (12.5): |x| <= 1.25: x + x s P(s) with s = x^2 and P a weighted
+// minimax fit of degree 7 (fit error 1.0e-8 relative), above: 1 - 2 / (e^(2|x|) + 1).  Evaluated in C with the errors
+// that the exp2 and reciprocal units may add, the result is within 1.6 ulp everywhere.
+__device__ __forceinline__ Pair tanh_pair(Pair x) {
+  constexpr float kP[8] = {-0x1.555528p-2f, 0x1.110984p-3f, -0x1.b93bb2p-5f, 0x1.5fe566p-6f,
+                           -0x1.077b52p-7f, 0x1.4a90acp-9f, -0x1.1f4f08p-11f, 0x1.e7bc34p-15f};
+  constexpr float kTwoLog2e = 2.885390081777927f, kSwitch = 1.25f;
+  const float2 xs = unpair(x);
+  const float2 af = make_float2(fabsf(xs.x), fabsf(xs.y));
+  const Pair a = pair(af.x, af.y), s = mul_pair(a, a);
+  Pair poly = pair(kP[7], kP[7]);
+#pragma unroll
+  for (int k = 6; k >= 0; --k) poly = fma_pair(s, poly, pair(kP[k], kP[k]));
+  poly = fma_pair(mul_pair(a, s), poly, a);
+  const float2 t = unpair(mul_pair(a, pair(kTwoLog2e, kTwoLog2e)));
+  const float2 e1 = make_float2(ctb::ex2_approx_ftz(t.x) + 1.f, ctb::ex2_approx_ftz(t.y) + 1.f);
+  const Pair big = fma_pair(pair(ctb::rcp_approx_ftz(e1.x), ctb::rcp_approx_ftz(e1.y)), pair(-2.f, -2.f), pair(1.f, 1.f));
+  const float2 ps = unpair(poly), bs = unpair(big);
+  return pair(copysignf(af.x > kSwitch ? bs.x : ps.x, xs.x), copysignf(af.y > kSwitch ? bs.y : ps.y, xs.y));
+}
 
-// Calls f(integral_constant<IDX>) for the run-time idx in [LO, HI) through a balanced tree of compares: six uniform
-// branches for the 56 instructions (measured 4 % faster on a four-instruction program than a switch over the same cases).
+template <int CODE, int H>
+__device__ __forceinline__ void apply_unary(Pair (&s0)[H]) {
+  if constexpr (CODE == CTB_TILED_TANH) {
+#pragma unroll
+    for (int h = 0; h < H; ++h) s0[h] = tanh_pair(s0[h]);
+    return;
+  }
+  float f[2 * H];
+#pragma unroll
+  for (int h = 0; h < H; ++h) {
+    const float2 a = unpair(s0[h]);
+    f[2 * h] = a.x;
+    f[2 * h + 1] = a.y;
+  }
+  if constexpr (CODE == CTB_TILED_SIN) {
+    sincos_all<false>(f);
+  } else if constexpr (CODE == CTB_TILED_COS) {
+    sincos_all<true>(f);
+  } else {
+#pragma unroll
+    for (int v = 0; v < 2 * H; ++v) f[v] = unary(CODE, f[v]);  // CODE is a constant: the switch inside folds
+  }
+#pragma unroll
+  for (int h = 0; h < H; ++h) s0[h] = pair(f[2 * h], f[2 * h + 1]);
+}
+
+// Calls f(integral_constant<IDX>) for the run-time idx in [LO, HI) through a balanced tree of compares (measured 4 %
+// faster on a four-instruction program than a switch over the same cases).
 template <unsigned LO, unsigned HI, typename F>
 __device__ __forceinline__ void tree_dispatch(unsigned idx, F&& f) {
   if constexpr (HI - LO == 1) {
@@ -473,196 +602,374 @@ __device__ __forceinline__ void tree_dispatch(unsigned idx, F&& f) {
     else tree_dispatch<MID, HI>(idx, f);
   }
 }
-constexpr unsigned kDispatchCount = kDispatchBinary + 7 * 6;
 
-// Every operand is contiguous along the first dimension with 16-byte aligned rows, or expanded along it (the host
-// checks).  A group is four neighbouring elements; a thread owns G groups per trip, a whole grid apart.  The
-// operands of the NEXT trip are copied global -> shared by cp.async (no registers, nothing waits on them) while the
-// instructions run on the current trip's copies, so the latency of HBM is off the critical path whatever the
-// occupancy; registers hold only the accumulator, the current operand and, for DEEP programs, the three stack
-// entries.  A thread reads only the shared memory it filled itself: no CTA barrier anywhere.
-// Shared memory: [2 buffers][n_inputs][G][256 threads] groups of 4 * sizeof(T) bytes.
-// Addresses: with DENSE operands a thread keeps one running pointer per array and adds a trip's bytes to it; a trip
-// whose G groups all exist (all but a thread's last) runs without a bounds test.
-template <typename T, int G, bool DENSE, bool DEEP>
-__global__ void __launch_bounds__(256)
-    tiled_broadcast_pipe_kernel(void* __restrict__ dest, const Operands in, const Program prog, int n_inputs, long long d0,
-                                long long d1, long long d2) {
-  constexpr int V = 4, E = V * G, VB = V * (int)sizeof(T);
-  constexpr int ES = DEEP ? E : 1;
+// f(temporary k) for the run-time index k < NT
+template <int NT, int Q = 0, int N, int H, typename F>
+__device__ __forceinline__ void with_temp(Pair (&tmp)[N][H], unsigned k, F f) {
+  if constexpr (Q + 1 < NT) {
+    if (k == (unsigned)Q) f(tmp[Q]);
+    else with_temp<NT, Q + 1>(tmp, k, f);
+  } else if constexpr (NT > 0) {
+    f(tmp[NT - 1]);
+  }
+}
+
+// Division of an index below 2^31 by a fixed extent: q = u * mul >> shift (mul = floor(2^shift / d) + 1, exact there).
+struct FastDiv {
+  unsigned d, mul;
+  int shift;
+  __device__ __forceinline__ unsigned div(unsigned u) const { return (unsigned)(((unsigned long long)u * mul) >> shift); }
+};
+inline FastDiv fast_div(unsigned d) {
+  int l = 0;
+  while ((1ull << l) < d) ++l;
+  return {d, (unsigned)((1ull << (31 + l)) / d + 1), 31 + l};
+}
+struct Extents {
+  long long n;          // elements of the destination
+  long long full_below; // a trip that starts at a group below this has all its groups
+  FastDiv row, col;     // row: groups (OP_ROW, OP_VECTOR) or elements (OP_ELEM) of the first dimension; col: the second extent
+  unsigned d0;          // OP_FIXED: the first extent
+  int fixed_vec;        // OP_FIXED: the four elements are one aligned vector
+  int dest_vec;         // the destination is aligned for vector stores
+};
+
+// A group is four neighbouring elements of the destination, whatever the extents are (the last one may be partial); a
+// thread owns G groups per trip, a whole grid apart.  The operands of the NEXT trip are copied global -> shared by
+// cp.async (no registers, nothing waits on them) while the instructions run on the current trip's copies, so the latency
+// of HBM is off the critical path whatever the occupancy; registers hold the accumulator, the current operand and NT
+// temporaries.  A thread reads only the shared memory it filled itself: no CTA barrier anywhere.
+// Shared memory: per operand [2 buffers][G][256 threads] groups of 4 * sizeof(T) bytes, OP_FIXED [256 threads].
+// A trip whose G groups all exist (all but a thread's last) runs without a bounds test.  LINEAR: every operand is laid out
+// like the destination, single or fixed (OP_LINEAR, OP_SCALAR, OP_SHIFTED, OP_FIXED), no coordinates are computed.
+// What bounds it: HBM for short expressions (A .+ b 6200 GB/s on 8192 x 4096 f32), instruction issue and dispatch latency
+// for long ones: a word costs about 24 issue slots of dispatch per thread (16 elements) and half a slot per element for +
+// and *.  0.5 v (1 + tanh(c (v + k v^3))), v = A .+ b, on 8192 x 4096 f32: 254 us with a stack of registers, one
+// instruction per operator and v evaluated five times; 183 with v in a temporary; 109 with pairs in 64-bit registers
+// (107 -> 69 instructions per element); 82 with the words below (7 words, one temporary, b read once); 68.5 with equal
+// trips.
+template <typename T, int G, int NT, bool LINEAR>
+__global__ void __launch_bounds__(256, NT == 0 || NT == 2 ? 4 : 3)
+    tiled_broadcast_kernel(void* __restrict__ dest, const Operands in, const Program prog, int n_inputs, const Extents x) {
+  ctb::grid_dependency_sync();
+  constexpr int V = 4, H = V * G / 2, ES = (int)sizeof(T), VB = V * ES;
+  constexpr int NTR = NT > 0 ? NT : 1;
   extern __shared__ __align__(16) unsigned char tiled_smem[];
-  const long long n0 = d0 / V, total = n0 * d1 * d2;
+  const long long total = (x.n + V - 1) / V;  // groups
   const long long grid_stride = (long long)gridDim.x * blockDim.x;
-  const long long group_bytes = grid_stride * VB;  // from one of a thread's groups to the next, in a dense array
   const unsigned tid = threadIdx.x;
-  const unsigned buf_bytes = (unsigned)n_inputs * G * 256 * VB;
   const unsigned smem0 = smem_addr(tiled_smem) + tid * VB;
-  auto slot = [&](unsigned buf, unsigned a, unsigned g) { return smem0 + buf * buf_bytes + (a * G + g) * (256 * VB); };
+  auto slot = [&](unsigned buf, unsigned a) { return smem0 + in.slot[a] + buf * (G * 256 * VB); };
 
   long long i = (long long)blockIdx.x * blockDim.x + tid;
-  // running pointers (DENSE): this thread's first group of the trip to copy next / to store next
-  const char* src_p[kMaxInputs];
-#pragma unroll
-  for (int a = 0; a < kMaxInputs; ++a) src_p[a] = static_cast<const char*>(in.ptr[a]) + i * VB;
-  char* dst_p = static_cast<char*>(dest) + i * VB;
 
-  // element offset of group ig in the destination (the general case)
-  auto dest_offset = [&](long long ig) -> long long {
-    const unsigned u = (unsigned)ig, un0 = (unsigned)n0, ud1 = (unsigned)d1;
-    const unsigned r = u / un0, i0 = (u - r * un0) * V, i2 = r / ud1, i1 = r - i2 * ud1;
-    return i0 + d0 * (i1 + d1 * (long long)i2);
-  };
   auto issue = [&](long long at, unsigned buf, auto full_tag) {
     constexpr bool FULL = decltype(full_tag)::value;
+    auto live_of = [&](int g) -> int {  // elements of the trip's group g that exist
+      return FULL ? V : (int)max(0ll, min((long long)V, x.n - (at + g * grid_stride) * V));
+    };
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-      const long long ig = at + g * grid_stride;
-      const bool live = FULL || ig < total;
-      unsigned i0 = 0, i1 = 0, i2 = 0;
-      if (!DENSE) {
-        const unsigned u = live ? (unsigned)ig : 0u, un0 = (unsigned)n0, ud1 = (unsigned)d1;
-        const unsigned r = u / un0;
-        i0 = (u - r * un0) * V, i2 = r / ud1, i1 = r - i2 * ud1;
-      }
+    for (int a = 0; a < kMaxInputs; ++a) {
+      if (a >= n_inputs) break;  // uniform, and so are the modes
+      const int mode = in.mode[a];
+      const T* base = static_cast<const T*>(in.ptr[a]);
+      const unsigned to = slot(buf, a);
+      if (mode == OP_LINEAR) {
+        const char* src = reinterpret_cast<const char*>(base) + at * VB;
 #pragma unroll
-      for (int a = 0; a < kMaxInputs; ++a) {
-        if (a < n_inputs) {  // uniform
-          const bool contiguous = in.stride[a][0] == 1;
-          const char* src;
-          if (DENSE) {
-            src = contiguous ? src_p[a] + g * group_bytes : static_cast<const char*>(in.ptr[a]);
+        for (int g = 0; g < G; ++g) {
+          const int live = live_of(g);
+          cp_async_group<VB>(to + g * (256 * VB), live ? src + g * (grid_stride * VB) : reinterpret_cast<const char*>(base), live * ES);
+        }
+      } else if (!LINEAR && mode == OP_VECTOR) {
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+          const int live = live_of(g);
+          const unsigned u = live ? (unsigned)at + g * (unsigned)grid_stride : 0u;
+          const unsigned i0 = u - x.row.div(u) * x.row.d;
+          cp_async_group<VB>(to + g * (256 * VB), base + (unsigned long long)i0 * V, live * ES);
+        }
+      } else if (mode == OP_SHIFTED) {
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+          const int live = live_of(g);
+          const T* src = base + (at + g * grid_stride) * V;
+#pragma unroll
+          for (int e = 0; e < V; ++e) copy_element<T>(to + g * (256 * VB) + e * ES, e < live ? src + e : base, e < live);
+        }
+      } else if (!LINEAR && mode == OP_ROW) {  // the extent is a multiple of four: a group exists as a whole or not at all
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+          const int live = live_of(g);
+          const unsigned u = live ? (unsigned)at + g * (unsigned)grid_stride : 0u;
+          const unsigned r = x.row.div(u), i0 = (u - r * x.row.d) * V, i2 = x.col.div(r), i1 = r - i2 * x.col.d;
+          const T* src = base + (i0 * in.stride[a][0] + i1 * in.stride[a][1] + i2 * in.stride[a][2]);
+          if (in.stride[a][0]) {
+            cp_async_group<VB>(to + g * (256 * VB), src, live * ES);
           } else {
-            src = static_cast<const char*>(in.ptr[a]) +
-                  (i0 * in.stride[a][0] + i1 * in.stride[a][1] + i2 * in.stride[a][2]) * (long long)sizeof(T);
+#pragma unroll
+            for (int e = 0; e < V; ++e) copy_element<T>(to + g * (256 * VB) + e * ES, src, live != 0);
           }
-          if (contiguous) {
-            if (FULL) cp_async_group<VB>(slot(buf, a, g), src, VB);
-            else cp_async_group<VB>(slot(buf, a, g), live ? src : static_cast<const char*>(in.ptr[a]), live ? VB : 0);
-          } else if (live) {  // expanded along the first dimension: one element, four copies
-            const T v = *reinterpret_cast<const T*>(src);
-            T* dst = reinterpret_cast<T*>(tiled_smem + (slot(buf, a, g) - smem_addr(tiled_smem)));
-            dst[0] = v; dst[1] = v; dst[2] = v; dst[3] = v;
+        }
+      } else if (!LINEAR && mode == OP_ELEM) {
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+          const int live = live_of(g);
+          const unsigned u = live ? ((unsigned)at + g * (unsigned)grid_stride) * V : 0u;
+          const unsigned r = x.row.div(u);
+          unsigned i0 = u - r * x.row.d, i2 = x.col.div(r), i1 = r - i2 * x.col.d;
+#pragma unroll
+          for (int e = 0; e < V; ++e) {
+            const T* src = base + (i0 * in.stride[a][0] + i1 * in.stride[a][1] + i2 * in.stride[a][2]);
+            copy_element<T>(to + g * (256 * VB) + e * ES, e < live ? src : base, e < live);
+            if (++i0 == x.row.d) {
+              i0 = 0;
+              if (++i1 == x.col.d) { i1 = 0; ++i2; }
+            }
           }
         }
       }
     }
-    if (DENSE) {
-#pragma unroll
-      for (int a = 0; a < kMaxInputs; ++a) src_p[a] += group_bytes * G;
-    }
     cp_async_commit();
   };
-  // the four elements of every group of operand `a`, from shared memory
-  auto fetch = [&](unsigned buf, unsigned a, float (&t)[E]) {
-    const unsigned base = slot(buf, a & (kMaxInputs - 1), 0);
+  // the elements of every group of operand `a`
+  auto fetch = [&](unsigned buf, unsigned arg, Pair (&t)[H]) {
+    const unsigned a = arg & (kMaxInputs - 1);
+    if (in.mode[a] == OP_SCALAR) {
+      const float c = load1<T>(in.ptr[a], 0);
+#pragma unroll
+      for (int h = 0; h < H; ++h) t[h] = pair(c, c);
+      return;
+    }
+    if (in.mode[a] == OP_FIXED) {
+      Pair lo, hi;
+      if constexpr (sizeof(T) == 4) {
+        asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(lo), "=l"(hi) : "r"(smem0 + in.slot[a]));
+      } else {
+        uint2 q;
+        asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(q.x), "=r"(q.y) : "r"(smem0 + in.slot[a]));
+        const float2 l = __half22float2(*reinterpret_cast<const __half2*>(&q.x));
+        const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&q.y));
+        lo = pair(l.x, l.y);
+        hi = pair(h.x, h.y);
+      }
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        t[2 * g] = lo;
+        t[2 * g + 1] = hi;
+      }
+      return;
+    }
+    const unsigned base = slot(buf, a);
 #pragma unroll
     for (int g = 0; g < G; ++g) {
       if constexpr (sizeof(T) == 4) {
-        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                     : "=f"(t[4 * g]), "=f"(t[4 * g + 1]), "=f"(t[4 * g + 2]), "=f"(t[4 * g + 3])
-                     : "r"(base + g * (256 * VB)));
+        asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(t[2 * g]), "=l"(t[2 * g + 1]) : "r"(base + g * (256 * VB)));
       } else {
         uint2 q;
         asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(q.x), "=r"(q.y) : "r"(base + g * (256 * VB)));
         const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&q.x));
         const float2 hi = __half22float2(*reinterpret_cast<const __half2*>(&q.y));
-        t[4 * g] = lo.x; t[4 * g + 1] = lo.y; t[4 * g + 2] = hi.x; t[4 * g + 3] = hi.y;
+        t[2 * g] = pair(lo.x, lo.y);
+        t[2 * g + 1] = pair(hi.x, hi.y);
       }
     }
   };
   auto start_next = [&](long long at, unsigned buf) {
-    if (at + (G - 1) * grid_stride < total) issue(at, buf, std::true_type());
+    if (at < x.full_below) issue(at, buf, std::true_type());
     else if (at < total) issue(at, buf, std::false_type());
     else cp_async_commit();  // an empty group keeps the count in the wait below uniform
   };
 
+  for (int a = 0; a < n_inputs; ++a) {
+    if (in.mode[a] == OP_FIXED) {
+      const T* base = static_cast<const T*>(in.ptr[a]);
+      const unsigned to = smem0 + in.slot[a];
+      unsigned i0 = ((unsigned)i * V) % x.d0;  // the grid is small: 32 bits
+      if (x.fixed_vec) {
+        cp_async_group<VB>(to, base + i0, VB);
+      } else {
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+          copy_element<T>(to + e * ES, base + i0, true);
+          if (++i0 == x.d0) i0 = 0;
+        }
+      }
+    }
+  }
   start_next(i, 0);
   for (unsigned buf = 0; i < total; i += grid_stride * G, buf ^= 1u) {
     start_next(i + grid_stride * G, buf ^ 1u);
     cp_async_wait<1>();  // everything but the newest group has landed: this trip's operands
 
-    float s0[E], s1[ES], s2[ES], s3[ES];  // the stack, top (the accumulator) first; every program starts with a push
-#pragma unroll
-    for (int v = 0; v < ES; ++v) s1[v] = s2[v] = s3[v] = 0.f;
-    auto push = [&]() {
-      if (DEEP) {
-#pragma unroll
-        for (int v = 0; v < ES; ++v) { s3[v] = s2[v]; s2[v] = s1[v]; s1[v] = s0[v % E]; }
-      }
-    };
-    auto pop = [&](float (&t)[E]) {  // DEEP programs only
-#pragma unroll
-      for (int v = 0; v < E; ++v) {
-        t[v] = s1[v % ES];
-        if (DEEP) { s1[v % ES] = s2[v % ES]; s2[v % ES] = s3[v % ES]; }
-      }
-    };
+    Pair s0[H], tmp[NTR][H];  // the accumulator (every program starts with a load) and the temporaries
+    unsigned next = prog.ins[0];  // the word of the next instruction is fetched while the current one runs
     for (int k = 0; k < prog.n_ins; ++k) {
-      const unsigned w = prog.ins[k];
-      const unsigned arg = (w >> 16) & 0xffu;
-      tree_dispatch<0, 64>(w >> 24, [&](auto tag) {
-        constexpr unsigned IDX = decltype(tag)::value;
-        if constexpr (IDX == 0) {
-          push();
-          fetch(buf, arg, s0);
-        } else if constexpr (IDX == 1) {
-          push();
-          const float c = prog.consts[arg & (kMaxConsts - 1)];
+      const unsigned w = next, arg = (w >> 8) & 3u, idx = w & 0xffu;
+      const float p = prog.pq[k].x, q = prog.pq[k].y;
+      next = prog.ins[k + 1];  // one word of padding behind the last
+      if (idx < L_HOT) {
+        tree_dispatch<0, 8>(idx, [&](auto tag) {
+          constexpr unsigned IDX = decltype(tag)::value;
+          if constexpr (IDX == L_FMA) {
+            const Pair pp = pair(p, p), qq = pair(q, q);
 #pragma unroll
-          for (int v = 0; v < E; ++v) s0[v] = c;
-        } else if constexpr (IDX < kDispatchBinary) {
-          apply_unary<(int)(CTB_TILED_NEG + IDX - kDispatchUnary)>(s0);
-        } else if constexpr (IDX < kDispatchCount) {
-          constexpr unsigned VARIANT = (IDX - kDispatchBinary) / 7;
-          constexpr int CODE = (int)(CTB_TILED_ADD + (IDX - kDispatchBinary) % 7);
-          constexpr bool REV = VARIANT & 1u;
-          if constexpr (VARIANT / 2 == 0) {  // an input
-            float t[E];
-            fetch(buf, arg, t);
-            apply_binary<CODE, REV>(s0, t);
-          } else if constexpr (VARIANT / 2 == 1) {  // a constant
-            apply_binary<CODE, REV>(s0, prog.consts[arg & (kMaxConsts - 1)]);
-          } else if constexpr (DEEP) {  // the entry below the accumulator
-            float t[E];
-            pop(t);
-            apply_binary<CODE, REV>(s0, t);
+            for (int h = 0; h < H; ++h) s0[h] = fma_pair(s0[h], pp, qq);
+          } else if constexpr (IDX == L_LOAD_INPUT) {
+            fetch(buf, arg, s0);
+          } else if constexpr (IDX == L_LOAD_CONST) {
+#pragma unroll
+            for (int h = 0; h < H; ++h) s0[h] = pair(q, q);
+          } else {
+            const float sign = w & kSubtract ? -1.f : 1.f;
+            auto apply = [&](Pair (&t)[H]) {
+#pragma unroll
+              for (int h = 0; h < H; ++h) {
+                if constexpr (IDX == L_MUL_INPUT || IDX == L_MUL_TEMP) s0[h] = mul_pair(s0[h], t[h]);
+                else if constexpr (IDX == L_ADD_INPUT || IDX == L_ADD_TEMP) s0[h] = fma_pair(t[h], pair(sign, sign), s0[h]);
+                else s0[h] = t[h];  // L_LOAD_TEMP
+              }
+            };
+            if constexpr (IDX == L_LOAD_TEMP) {
+              with_temp<NT>(tmp, arg, apply);
+            } else if (NT > 0 && (w & kOperandFma)) {
+              Pair t[H];
+              if constexpr (IDX == L_MUL_INPUT || IDX == L_ADD_INPUT) {
+                fetch(buf, arg, t);
+              } else {
+                with_temp<NT>(tmp, arg, [&](Pair (&u)[H]) {
+#pragma unroll
+                  for (int h = 0; h < H; ++h) t[h] = u[h];
+                });
+              }
+              const Pair pp = pair(p, p), qq = pair(q, q);
+#pragma unroll
+              for (int h = 0; h < H; ++h) t[h] = fma_pair(t[h], pp, qq);
+              apply(t);
+            } else if constexpr (IDX == L_MUL_INPUT || IDX == L_ADD_INPUT) {
+              Pair t[H];
+              fetch(buf, arg, t);
+              apply(t);
+            } else {
+              with_temp<NT>(tmp, arg, apply);
+            }
           }
-        }
-      });
-    }
-    const bool full = i + (G - 1) * grid_stride < total;
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-      if (!full && i + g * grid_stride >= total) continue;
-      char* out = DENSE ? dst_p + g * group_bytes : static_cast<char*>(dest) + dest_offset(i + g * grid_stride) * (long long)sizeof(T);
-      const float* r = &s0[g * V];
-      if constexpr (sizeof(T) == 4) {
-        __stcs(reinterpret_cast<float4*>(out), make_float4(r[0], r[1], r[2], r[3]));
+        });
       } else {
-        uint2 q;
-        *reinterpret_cast<__half2*>(&q.x) = __floats2half2_rn(r[0], r[1]);
-        *reinterpret_cast<__half2*>(&q.y) = __floats2half2_rn(r[2], r[3]);
-        __stcs(reinterpret_cast<uint2*>(out), q);
+        tree_dispatch<L_UNARY, L_COUNT>(idx, [&](auto tag) {
+          constexpr unsigned IDX = decltype(tag)::value;
+          if constexpr (IDX < L_BINARY) {
+            apply_unary<(int)(CTB_TILED_NEG + IDX - L_UNARY)>(s0);
+          } else {
+            constexpr unsigned SRC = (IDX - L_BINARY) / 10, POS = (IDX - L_BINARY) % 10;
+            constexpr int CODE = kColdCodes[POS / 2];
+            constexpr bool REV = POS & 1u;
+            if constexpr (CODE == CTB_TILED_SUB && (SRC == 1 || !REV)) {
+              // an L_FMA or L_ADD instruction
+            } else if constexpr (SRC == 0) {
+              Pair t[H];
+              fetch(buf, arg, t);
+              apply_binary<CODE, REV>(s0, [&](int h) { return t[h]; });
+            } else if constexpr (SRC == 1) {
+              apply_binary<CODE, REV>(s0, [&](int) { return pair(q, q); });
+            } else {
+              with_temp<NT>(tmp, arg, [&](Pair (&t)[H]) { apply_binary<CODE, REV>(s0, [&](int h) { return t[h]; }); });
+            }
+          }
+        });
+      }
+      if (w >= kTailFma) {
+        if (w & kTailFma) {
+          const Pair pp = pair(p, p), qq = pair(q, q);
+#pragma unroll
+          for (int h = 0; h < H; ++h) s0[h] = fma_pair(s0[h], pp, qq);
+        }
+        if (NT > 0 && w >> kTailStore)
+          with_temp<NT>(tmp, (w >> kTailStore) - 1u, [&](Pair (&t)[H]) {
+#pragma unroll
+            for (int h = 0; h < H; ++h) t[h] = s0[h];
+          });
       }
     }
-    dst_p += group_bytes * G;
+    if (i < x.full_below && x.dest_vec) {
+      char* out = static_cast<char*>(dest) + i * VB;
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        if constexpr (sizeof(T) == 4) {
+          asm volatile("st.global.cs.v2.b64 [%0], {%1, %2};" ::"l"(out + g * (grid_stride * VB)), "l"(s0[2 * g]), "l"(s0[2 * g + 1])
+                       : "memory");
+        } else {
+          const float2 a = unpair(s0[2 * g]), b = unpair(s0[2 * g + 1]);
+          uint2 h;
+          *reinterpret_cast<__half2*>(&h.x) = __floats2half2_rn(a.x, a.y);
+          *reinterpret_cast<__half2*>(&h.y) = __floats2half2_rn(b.x, b.y);
+          __stcs(reinterpret_cast<uint2*>(out + g * (grid_stride * VB)), h);
+        }
+      }
+    } else {  // a partial group, or a destination without vector stores
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        const long long at = (i + g * grid_stride) * V;
+        const float2 a = unpair(s0[2 * g]), b = unpair(s0[2 * g + 1]);
+        const float r[V] = {a.x, a.y, b.x, b.y};
+#pragma unroll
+        for (int e = 0; e < V; ++e)
+          if (at + e < x.n) store1<T>(dest, at + e, r[e]);
+      }
+    }
   }
   cp_async_wait<0>();
 }
 
-template <typename T, int G, bool DENSE, bool DEEP>
-int launch_pipe(ctb_ctx* ctx, cudaStream_t st, void* dest, const Operands& in, const Program& prog, int n_inputs, long long d0,
-                long long d1, long long d2, long long units) {
-  auto kernel = tiled_broadcast_pipe_kernel<T, G, DENSE, DEEP>;
-  const int smem = std::max(1, n_inputs) * 2 * G * 256 * 4 * (int)sizeof(T);
+template <typename T, int G, int NT>
+int launch_broadcast(ctb_ctx* ctx, cudaStream_t st, void* dest, Operands& in, const Program& prog, int n_inputs, long long d0,
+                     Extents& x) {
+  constexpr int VB = 4 * (int)sizeof(T);
+  // Several waves of CTAs, not one wave of resident ones: CTAs that all start together stay in step (all loading,
+  // then all storing) and measured 10 % slower than CTAs that start at different times.  At most 16 per SM, and as many
+  // as give every CTA the same number of trips (2368 CTAs with three or four trips each: 81.8 us for a bias and tanh
+  // expression on 8192 x 4096, 2048 with four: 68.5).
+  const long long ctas = std::max<long long>(1, ((x.n + 3) / 4 + 256ll * G - 1) / (256ll * G));
+  const long long most = (long long)ctx->sm_count * 16, trips = (ctas + most - 1) / most;
+  long long grid = (ctas + trips - 1) / trips;
+  // An operand that varies along the first dimension only is the same for all groups of a thread when a whole grid is a
+  // multiple of the first extent: a grid of a multiple of m CTAs.  Its four elements are then read once instead of with
+  // every group (8192 x 4096, A .+ b: 20.8 -> 14 instructions per element).
+  auto gcd = [](long long a, long long b) {
+    while (b) { const long long t = a % b; a = b; b = t; }
+    return a;
+  };
+  const long long m = d0 / gcd(d0, 1024);  // 256 threads of four elements per CTA
+  const long long up = (grid + m - 1) / m * m;
+  const long long fixed_grid = up <= std::max(most, std::min(ctas, 4 * most)) ? up : grid / m * m;
+  bool linear = true, fixed = false;
+  for (int a = 0; a < n_inputs; ++a) {
+    const bool vector = in.mode[a] == OP_VECTOR || (in.mode[a] == OP_ELEM && in.stride[a][0] == 1 && !in.stride[a][1] && !in.stride[a][2]);
+    if (vector && fixed_grid > 0) {
+      in.mode[a] = OP_FIXED;
+      fixed = true;
+    } else if (in.mode[a] == OP_VECTOR || in.mode[a] == OP_ROW || in.mode[a] == OP_ELEM) {
+      linear = false;
+    }
+  }
+  if (fixed) {
+    grid = fixed_grid;
+    x.d0 = (unsigned)d0;
+    x.fixed_vec = d0 % 4 == 0;
+    for (int a = 0; a < n_inputs; ++a)
+      if (in.mode[a] == OP_FIXED && (uintptr_t)in.ptr[a] % VB) x.fixed_vec = 0;
+  }
+  unsigned smem = 0;
+  for (int a = 0; a < n_inputs; ++a) {
+    in.slot[a] = smem;
+    if (in.mode[a] != OP_SCALAR) smem += (in.mode[a] == OP_FIXED ? 1 : 2 * G) * 256 * VB;
+  }
+  x.full_below = x.n / 4 - (long long)(G - 1) * grid * 256;  // a trip's last group is (G - 1) grids further on
+  auto kernel = linear ? tiled_broadcast_kernel<T, G, NT, true> : tiled_broadcast_kernel<T, G, NT, false>;
   if (smem > 48 * 1024 &&  // per device, so on every launch that needs it: a host-side table write
       cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return fail(CTB_CUDA_ERROR, "ctb_tiled_broadcast: shared memory attribute: %s", cudaGetErrorString(cudaGetLastError()));
-  // Several waves of CTAs, not one wave of resident ones: CTAs that all start together stay in step (all loading,
-  // then all storing) and measured 10 % slower than CTAs that start at different times.
-  const long long ctas = (units + 256ll * G - 1) / (256ll * G);
-  const int grid = (int)std::max<long long>(1, std::min<long long>(ctas, (long long)ctx->sm_count * 16));
-  kernel<<<grid, 256, smem, st>>>(dest, in, prog, n_inputs, d0, d1, d2);
+  launch_kernel(kernel, (unsigned)grid, 256, smem, st, 0, dest, in, prog, n_inputs, x);
   return CTB_OK;
 }
 
@@ -910,18 +1217,19 @@ int ctb_tiled_broadcast(ctb_ctx* ctx, void* stream, void* dest, const int64_t* s
     if (shape[k] < 0) return fail(CTB_BAD_ARG, "ctb_tiled_broadcast: negative extent");
   Program prog;
   const char* why = "";
-  int need = 1;
-  const int bad = compile_program(program, n_ops, n_inputs, n_constants, &prog, &why, &need);
+  const int bad = lower_program(program, n_ops, n_inputs, constants, n_constants, &prog, &why);
   if (bad == -1000)
     return fail(CTB_UNSUPPORTED, "ctb_tiled_broadcast: the expression needs more than %d intermediate values at once", kStack);
   if (bad) return fail(CTB_BAD_ARG, "ctb_tiled_broadcast: operation %d %s", -bad - 1, why);
-  for (int k = 0; k < n_constants; ++k) prog.consts[k] = constants[k];
   const long long d0 = shape[0], d1 = shape[1], d2 = shape[2];
   if (d0 == 0 || d1 == 0 || d2 == 0) return CTB_OK;  // empty arrays: nothing to launch
   CTB_CHECK_DEV(dest);
   const int es = dtype == CTB_F32 ? 4 : 2;
   Operands in = {};
-  bool vec = d0 % 4 == 0 && (uintptr_t)dest % 16 == 0;
+  Extents x = {};
+  x.n = d0 * d1 * d2;
+  x.dest_vec = (uintptr_t)dest % (4 * es) == 0;
+  bool linear = true, by_element = false;
   for (int a = 0; a < n_inputs; ++a) {
     CTB_CHECK_DEV(inputs[a]);
     in.ptr[a] = inputs[a];
@@ -929,50 +1237,41 @@ int ctb_tiled_broadcast(ctb_ctx* ctx, void* stream, void* dest, const int64_t* s
       in.stride[a][k] = input_strides[3 * a + k];
       if (in.stride[a][k] < 0) return fail(CTB_BAD_ARG, "ctb_tiled_broadcast: negative stride");
     }
-    const long long s0 = in.stride[a][0];
-    if (s0 == 1) {  // vector loads need aligned rows
-      if ((uintptr_t)inputs[a] % (4 * es) || (in.stride[a][1] * es) % (4 * es) || (in.stride[a][2] * es) % (4 * es)) vec = false;
-    } else if (s0 != 0) {
-      vec = false;
-    }
+    const long long s0 = in.stride[a][0], s1 = in.stride[a][1], s2 = in.stride[a][2];
+    const bool like_dest = (d0 == 1 || s0 == 1) && (d1 == 1 || s1 == d0) && (d2 == 1 || s2 == d0 * d1);
+    const bool single = (d0 == 1 || s0 == 0) && (d1 == 1 || s1 == 0) && (d2 == 1 || s2 == 0);
+    const bool aligned = (uintptr_t)inputs[a] % (4 * es) == 0;
+    if (single) in.mode[a] = OP_SCALAR;
+    else if (like_dest) in.mode[a] = aligned ? OP_LINEAR : OP_SHIFTED;
+    else if (d0 % 4 == 0 && s0 == 1 && aligned && s1 == 0 && s2 == 0) in.mode[a] = OP_VECTOR;
+    else if (d0 % 4 == 0 && (s0 == 0 || (s0 == 1 && aligned && s1 % 4 == 0 && s2 % 4 == 0))) in.mode[a] = OP_ROW;
+    else in.mode[a] = OP_ELEM;
+    if (in.mode[a] == OP_ROW || in.mode[a] == OP_ELEM || in.mode[a] == OP_VECTOR) linear = false;
+    if (in.mode[a] == OP_ELEM) by_element = true;
   }
-  // dense: every operand is laid out like the destination or is a single element
-  bool dense = true;
-  for (int a = 0; a < n_inputs; ++a) {
-    const bool like_dest = in.stride[a][0] == 1 && (d1 == 1 || in.stride[a][1] == d0) && (d2 == 1 || in.stride[a][2] == d0 * d1);
-    const bool single = in.stride[a][0] == 0 && (d1 == 1 || in.stride[a][1] == 0) && (d2 == 1 || in.stride[a][2] == 0);
-    if (!like_dest && !single) dense = false;
+  if (by_element)  // one pair of divisors serves both kinds: by element then
+    for (int a = 0; a < n_inputs; ++a)
+      if (in.mode[a] == OP_ROW || in.mode[a] == OP_VECTOR) in.mode[a] = OP_ELEM;
+  if (!linear) {
+    if ((by_element ? x.n : x.n / 4) > 0x7fffffffLL)
+      return fail(CTB_UNSUPPORTED, "ctb_tiled_broadcast: too many elements for an expanded operand");
+    x.row = fast_div((unsigned)(by_element ? d0 : d0 / 4));
+    x.col = fast_div((unsigned)d1);
   }
-  const long long units = (vec ? d0 / 4 : d0) * d1 * d2;
-  if (!dense && units > 0x7fffffffLL) return fail(CTB_UNSUPPORTED, "ctb_tiled_broadcast: too many elements for an expanded operand");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const bool deep = need > 1;
   int rc = CTB_OK;
-  // groups per thread: as many as registers (the stack of a deep program) and shared memory (the operands) allow;
-  // eight groups for a single operand measured slower than four (128 registers, two CTAs per SM)
-#define CTB_TILED_VEC(T, D)                                                                                          \
-  do {                                                                                                               \
-    if (deep) rc = launch_pipe<T, 2, D, true>(ctx, st, dest, in, prog, n_inputs, d0, d1, d2, units);                 \
-    else if (n_inputs <= 3) rc = launch_pipe<T, 4, D, false>(ctx, st, dest, in, prog, n_inputs, d0, d1, d2, units);  \
-    else rc = launch_pipe<T, 2, D, false>(ctx, st, dest, in, prog, n_inputs, d0, d1, d2, units);                     \
+  // groups per thread: as many as registers (the temporaries) and shared memory (the operands) allow; eight groups for a
+  // single operand measured slower than four (128 registers, two CTAs per SM)
+#define CTB_TILED_NT(T)                                                                                             \
+  do {                                                                                                              \
+    if (prog.n_temps > 2) rc = launch_broadcast<T, 2, 4>(ctx, st, dest, in, prog, n_inputs, d0, x);                 \
+    else if (prog.n_temps == 2 || n_inputs > 3) rc = launch_broadcast<T, 2, 2>(ctx, st, dest, in, prog, n_inputs, d0, x); \
+    else if (prog.n_temps == 1) rc = launch_broadcast<T, 4, 1>(ctx, st, dest, in, prog, n_inputs, d0, x);           \
+    else rc = launch_broadcast<T, 4, 0>(ctx, st, dest, in, prog, n_inputs, d0, x);                                  \
   } while (0)
-#define CTB_TILED_SCALAR(T, D)                                                                                       \
-  do {                                                                                                               \
-    const int grid = (int)std::max<long long>(1, std::min<long long>((units + 255) / 256, (long long)ctx->sm_count * 16)); \
-    tiled_broadcast_kernel<T, 1, 1, D, kMaxInputs, true><<<grid, 256, 0, st>>>(dest, in, prog, n_inputs, d0, d1, d2); \
-  } while (0)
-#define CTB_TILED_PICK(T)                                                     \
-  do {                                                                        \
-    if (vec && dense) CTB_TILED_VEC(T, true);                                 \
-    else if (vec) CTB_TILED_VEC(T, false);                                    \
-    else if (dense) CTB_TILED_SCALAR(T, true);                                \
-    else CTB_TILED_SCALAR(T, false);                                          \
-  } while (0)
-  if (dtype == CTB_F32) CTB_TILED_PICK(float);
-  else CTB_TILED_PICK(__half);
-#undef CTB_TILED_PICK
-#undef CTB_TILED_SCALAR
-#undef CTB_TILED_VEC
+  if (dtype == CTB_F32) CTB_TILED_NT(float);
+  else CTB_TILED_NT(__half);
+#undef CTB_TILED_NT
   if (rc) return rc;
   CTB_CHECK_LAUNCH("ctb_tiled_broadcast launch");
   return CTB_OK;
@@ -984,14 +1283,14 @@ int ctb_tiled_compile(const int32_t* program, int n_ops, int n_inputs, int n_con
   if (n_inputs < 0 || n_inputs > kMaxInputs || n_ops < 1 || n_ops > kMaxOps || n_constants < 0 || n_constants > kMaxConsts)
     return fail(CTB_UNSUPPORTED, "ctb_tiled_compile: at most %d inputs, %d operations and %d constants", kMaxInputs, kMaxOps,
                 kMaxConsts);
-  Program prog;
+  Compiler c;
   const char* why = "";
-  const int bad = compile_program(program, n_ops, n_inputs, n_constants, &prog, &why);
+  const int bad = compile_program(program, n_ops, n_inputs, n_constants, &c, &why);
   if (bad == -1000)
     return fail(CTB_UNSUPPORTED, "ctb_tiled_compile: the expression needs more than %d intermediate values at once", kStack);
   if (bad) return fail(CTB_BAD_ARG, "ctb_tiled_compile: operation %d %s", -bad - 1, why);
-  for (int k = 0; k < prog.n_ins; ++k) instructions[k] = prog.ins[k];
-  *n_instructions = prog.n_ins;
+  for (int k = 0; k < c.n_words; ++k) instructions[k] = c.words[k];
+  *n_instructions = c.n_words;
   return CTB_OK;
 }
 

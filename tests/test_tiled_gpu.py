@@ -255,3 +255,61 @@ def test_mapreduce_prod_max_min_mapped_and_edge_cases(cuda):
         T.tsum(T.Tiled(A), dims=(1.0,))
     E = torch.empty(0, 4, device="cuda")                                              # Julia (4, 0)
     assert np.array_equal(T.tsum(T.Tiled(E), dims=2).cpu().numpy(), np.zeros((1, 4), np.float32))
+
+
+def gelu_tree(x, b):
+    v = ("add", x, b)
+    return ("mul", ("mul", 0.5, v), ("add", 1.0, ("tanh", ("mul", 0.7978845608, ("add", v, ("mul", 0.044715, ("mul", ("mul", v, v), v)))))))
+
+
+@pytest.mark.parametrize("dtype,tol", [(np.float32, 2e-6), (np.float16, 1.5e-3)])
+@pytest.mark.parametrize("rows,cols", [(1, 4), (7, 5), (129, 64), (33, 1001), (3, 50001), (700, 4092), (2, 2 ** 20)])
+def test_broadcast_shared_subexpressions_and_bias(cuda, rows, cols, dtype, tol):
+    """A subexpression used several times, and an operand that varies along the first dimension only: row lengths that
+    are a multiple of the vector or not, shorter and longer than what one grid covers; the same with arrays that start
+    off the vector alignment."""
+    import torch
+    T = cuda.tiled
+    a, b = rnd((rows, cols), 70, dtype), rnd((cols,), 71, dtype)
+    want = ref.tiled_broadcast(gelu_tree(a.astype(np.float64), b.astype(np.float64)))
+    for shift in (0, 1):
+        def place(v):
+            flat = torch.empty(v.size + shift, device="cuda", dtype=torch.from_numpy(v).dtype)
+            flat[shift:] = torch.from_numpy(v.reshape(-1)).cuda()
+            return flat[shift:].view(v.shape)
+        A, B, out = place(a), place(b), place(np.full_like(a, np.nan))
+        v = T.Tiled(A) + T.Tiled(B)
+        T.assign(out, 0.5 * v * (1.0 + T.tanh(0.7978845608 * (v + 0.044715 * (v * v * v)))))
+        close(out.cpu().numpy(), want, tol)
+
+
+def test_broadcast_many_shared_values(cuda):
+    """More shared values than temporaries, stores on words that store already, affine operands on either side."""
+    import torch
+    T = cuda.tiled
+    a = rnd((1000,), 72)
+    A = torch.from_numpy(a).cuda()
+    x, X = a.astype(np.float64), T.Tiled(A)
+    s, c, e = T.sin(X), T.cos(X), T.exp(X)
+    S, C, E = np.sin(x), np.cos(x), np.exp(x)
+    for expr, want in [((s * c - e / s) * (c - 2.0 * X) + (s + e), (S * C - E / S) * (C - 2 * x) + (S + E)),
+                       (T.exp(s) * (-X) - (3.0 - X) * c, np.exp(S) * -x - (3 - x) * C),
+                       ((s * s) * (s * s) + s, S ** 4 + S), (-(-(s + 1.0)) * (s + 1.0), (S + 1) ** 2)]:
+        out = torch.empty_like(A)
+        T.assign(out, expr)
+        close(out.cpu().numpy(), want, 4e-6)
+
+
+def test_tanh_accuracy(cuda):
+    """tanh of the array expressions (own evaluation): within 2 ulp of the exact value over the whole range."""
+    import torch
+    T = cuda.tiled
+    x = np.concatenate([np.linspace(-12, 12, 1 << 20), np.geomspace(1e-38, 1.3, 1 << 18), [0.0, -0.0, np.inf, -np.inf, 88.0]])
+    x = x.astype(np.float32)
+    out = torch.empty(x.size, device="cuda")
+    T.assign(out, T.tanh(T.Tiled(torch.from_numpy(x).cuda())))
+    got, want = out.cpu().numpy(), np.tanh(x.astype(np.float64))
+    assert (np.abs(got - want) <= 2 * np.spacing(np.abs(want).astype(np.float32))).all()
+    assert np.array_equal(np.signbit(got), np.signbit(x))
+    T.assign(out, T.tanh(T.Tiled(torch.full_like(out, float("nan")))))
+    assert torch.isnan(out).all()
