@@ -10,12 +10,13 @@
 //   rows that fit the registers of a CTA and are 16-byte aligned take the
 //   variant-0 kernel (one HBM read, one write; a chunk-by-chunk running
 //   (max, sum) over bulk-copied chunks was measured 1.5x slower there because
-//   it evaluates two exponentials per element).  Longer rows that fit shared
-//   memory (up to 200 KB) are kept there whole: a running (max, sum) over the
-//   chunks as they land, then a second pass that scales and stores (still one
-//   HBM read, one write; for these rows the passes over shared memory cost
-//   more than the second exponential).  Anything else: a running (max, sum)
-//   per thread over chunks with 128-bit loads, re-read once.
+//   it evaluates two exponentials per element).  Longer rows, of any alignment,
+//   are kept whole in the shared memory of a cluster of CTAs: a running
+//   (max, sum) over the chunks as they land, then a second pass that scales and
+//   stores (still one HBM read, one write; for these rows the passes over
+//   shared memory cost more than the second exponential).  Rows beyond that
+//   (832 KB): a running (max, sum) per thread over chunks, re-read once.
+// Both variants: rows of up to 1024 elements take a warp each.
 //
 // Both compute in f32 (examples/softmax.jl:32-35,92).  exp(x - max) is evaluated
 // as ex2.approx((x - max)*log2(e)) (relative error about 2^-22 plus the rounding
@@ -184,33 +185,140 @@ __global__ void __launch_bounds__(kThreads) softmax_staged_kernel(T* __restrict_
   if (tid == 0) bulk_wait<0>();  // stores complete before the CTA (and its smem) goes away
 }
 
-// ------------------------------------------------------------------ variant 1, rows that fit shared memory
-// Rows too long for the registers of a CTA but not for its shared memory (up to about 200 KB): one CTA per SM keeps
-// the whole row on chip, so HBM is still read once and written once.  The row arrives as kRowChunks bulk copies, each
-// with its own mbarrier; the threads look for the maximum of a chunk as soon as it has landed, under the copies of
-// the chunks behind it and sum the exponentials in the same pass (online, rescaling when the maximum grows).  A second
-// pass evaluates the exponentials again, scales and stores to global memory; a chunk's part of the buffer is refilled
-// with the next row's chunk as soon as it was read.
-constexpr int kRowThreads = 512;
-constexpr int kRowChunks = 8;
-template <typename T>
-__global__ void __launch_bounds__(kRowThreads) softmax_row_smem_kernel(T* __restrict__ out, const T* __restrict__ in, int N,
-                                                                       int M, long long ld_out, long long ld_in, int* status) {
-  using P = typename Pack<T>::type;
-  extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ __align__(8) uint64_t full[kRowChunks];
-  __shared__ float red[kRowThreads / 32];
+// ------------------------------------------------------------------ short rows
+// Up to 1024 elements: one warp per row, the row in registers (element 32 i + lane, or 4 (32 i + lane) + k when VEC, the
+// rows starting on vector boundaries), shuffles instead of barriers.  Bound by HBM for many rows (8192 x 1000 f32: a CTA
+// per row through a ring of stages spends its time on two block reductions per 4 KB), by one load latency for few.
+template <typename T, int NE, bool VEC>  // NE: elements per lane
+__global__ void __launch_bounds__(128) softmax_warp_kernel(T* __restrict__ out, const T* __restrict__ in, int N, int M,
+                                                           long long ld_out, long long ld_in) {
+  grid_dependency_sync();
+  const int lane = threadIdx.x & 31;
+  for (int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); row < M; row += gridDim.x * (blockDim.x >> 5)) {
+    const T* src = in + (long long)row * ld_in;
+    T* dst = out + (long long)row * ld_out;
+    float x[NE];
+    if constexpr (VEC) {
+#pragma unroll
+      for (int i = 0; i < NE / 4; ++i) {
+        const int p = i * 32 + lane;
+        if (p * 4 < N) {
+          Pack<T>::unpack(reinterpret_cast<const typename Pack<T>::type*>(src)[p], &x[4 * i]);
+        } else {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) x[4 * i + k] = -INFINITY;
+        }
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < NE; ++i) x[i] = i * 32 + lane < N ? (float)src[i * 32 + lane] : -INFINITY;
+    }
+    float mx = -FLT_MAX;
+#pragma unroll
+    for (int i = 0; i < NE; ++i) mx = fmaxf(mx, x[i]);
+    mx = warp_max(mx);
+    float s4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < NE; ++i) {
+      x[i] = exp_sub(x[i], mx);  // 0 beyond the row
+      s4[i & 3] += x[i];
+    }
+    const float inv = 1.0f / warp_sum((s4[0] + s4[1]) + (s4[2] + s4[3]));
+#pragma unroll
+    for (int i = 0; i < NE; ++i) x[i] *= inv;
+    if constexpr (VEC) {
+#pragma unroll
+      for (int i = 0; i < NE / 4; ++i)
+        if ((i * 32 + lane) * 4 < N) reinterpret_cast<typename Pack<T>::type*>(dst)[i * 32 + lane] = Pack<T>::pack(&x[4 * i]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < NE; ++i)
+        if (i * 32 + lane < N) dst[i * 32 + lane] = (T)x[i];
+    }
+  }
+}
+
+// Up to 8192 elements in rows that do not start on vector boundaries: one CTA per row, the row in registers, element by
+// element (a warp still covers whole lines), all of a thread's loads in flight at once.
+template <typename T, int NE>
+__global__ void __launch_bounds__(kThreads) softmax_regs_kernel(T* __restrict__ out, const T* __restrict__ in, int N, int M,
+                                                                long long ld_out, long long ld_in) {
+  __shared__ float red[kWarps];
+  grid_dependency_sync();
   const int tid = threadIdx.x;
-  const int npack = N / 4;
-  // chunk boundaries in packs, multiples of 4 packs (16 bytes for f16, 64 for f32)
-  const int per = ((npack + kRowChunks - 1) / kRowChunks + 3) & ~3;
+  for (int row = blockIdx.x; row < M; row += gridDim.x) {
+    const T* src = in + (long long)row * ld_in;
+    T* dst = out + (long long)row * ld_out;
+    float x[NE];
+    float mx = -FLT_MAX;
+#pragma unroll
+    for (int i = 0; i < NE; ++i) x[i] = i * kThreads + tid < N ? (float)src[i * kThreads + tid] : -INFINITY;
+#pragma unroll
+    for (int i = 0; i < NE; ++i) mx = fmaxf(mx, x[i]);
+    mx = block_max(mx, red);
+    float s4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < NE; ++i) {
+      x[i] = exp_sub(x[i], mx);
+      s4[i & 3] += x[i];
+    }
+    const float inv = 1.0f / block_sum((s4[0] + s4[1]) + (s4[2] + s4[3]), red);
+#pragma unroll
+    for (int i = 0; i < NE; ++i)
+      if (i * kThreads + tid < N) dst[i * kThreads + tid] = (T)(x[i] * inv);
+  }
+}
+
+// ------------------------------------------------------------------ variant 1, long rows of any alignment
+// Rows too long for the registers of a CTA: a cluster of C CTAs keeps the whole row in its shared memory, so HBM is
+// read once and written once.  C is the smallest power of two with at most 104 KB per CTA, so that two or more CTAs share
+// an SM and one loads while another computes or stores (one CTA per SM that held a whole row: 5400 GB/s on 1024 x 32768).
+// The 16-byte aligned middle of the row arrives in chunks of kChunkVecs vectors, one bulk copy and mbarrier each; up to
+// one vector's elements before and after it are loaded one by one by rank 0, so rows may start anywhere (1024 x 50001 f32:
+// 227 us with scalar loads and a second read).  One online pass takes the running maximum and sum of exponentials of each
+// chunk as it lands, the CTAs exchange them through distributed shared memory (one cluster barrier per row, two sets of
+// slots), and a second pass evaluates the exponentials again, scales and stores; a chunk's part of the buffer takes the
+// next row's chunk as soon as it was read.
+constexpr int kRowThreads = 512;
+constexpr int kChunkVecs = 1024;
+constexpr int kMaxChunks = 7;
+constexpr int kMaxCluster = 8;
+template <typename T>
+__device__ __forceinline__ void unpack16(const uint4& q, float (&f)[16 / sizeof(T)]) {
+  if constexpr (sizeof(T) == 4) {
+    f[0] = __uint_as_float(q.x); f[1] = __uint_as_float(q.y); f[2] = __uint_as_float(q.z); f[3] = __uint_as_float(q.w);
+  } else {
+    const __half2* h = reinterpret_cast<const __half2*>(&q);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 v = __half22float2(h[i]);
+      f[2 * i] = v.x;
+      f[2 * i + 1] = v.y;
+    }
+  }
+}
+template <typename T>
+__global__ void __launch_bounds__(kRowThreads) softmax_long_kernel(T* __restrict__ out, const T* __restrict__ in, int N, int M,
+                                                                   long long ld_out, long long ld_in, int per, int C,
+                                                                   int* status) {
+  constexpr int V = 16 / (int)sizeof(T);
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ __align__(8) uint64_t full[kMaxChunks];
+  __shared__ float red[kRowThreads / 32];
+  __shared__ float2 peers[2][kMaxCluster];  // (maximum, sum) of every CTA of the cluster, for even and odd rows
+  const int tid = threadIdx.x;
+  const int rank = C > 1 ? (int)cluster_ctarank() : 0, team = blockIdx.x / C, teams = gridDim.x / C;
   if (tid == 0) {
-    for (int c = 0; c < kRowChunks; ++c) mbar_init(&full[c], 1);
+    for (int c = 0; c < kMaxChunks; ++c) mbar_init(&full[c], 1);
     fence_mbar_init();
   }
   __syncthreads();
+  if (C > 1) {  // the peers' shared memory exists
+    cluster_arrive();
+    cluster_wait();
+  }
   grid_dependency_sync();
-  P* buf = reinterpret_cast<P*>(smem);
+  uint4* buf = reinterpret_cast<uint4*>(smem);
   auto block_reduce = [&](float v, bool is_max) {
     v = is_max ? warp_max(v) : warp_sum(v);
     if ((tid & 31) == 0) red[tid >> 5] = v;
@@ -220,58 +328,102 @@ __global__ void __launch_bounds__(kRowThreads) softmax_row_smem_kernel(T* __rest
     __syncthreads();
     return r;
   };
-  // thread 0 issues the bulk copies of chunk c of `row` (the buffer region of the chunk must be free)
-  auto load_chunk = [&](int row, int c) {
-    const int p0 = c * per, p1 = min(npack, p0 + per);
-    if (p1 <= p0) return;
-    const uint32_t bytes = (uint32_t)(p1 - p0) * 4 * sizeof(T);
-    mbar_expect_tx(&full[c], bytes);
-    bulk_g2s(buf + p0, in + (long long)row * ld_in + (long long)p0 * 4, bytes, &full[c]);
+  // the row's elements before the first 16-byte boundary, and the vectors [v0, v1) of the middle that are this CTA's
+  auto layout = [&](int row, const T*& src, int& head, int& nvec, int& v0, int& v1) {
+    src = in + (long long)row * ld_in;
+    head = min(N, (int)((16 - ((uintptr_t)src & 15)) & 15) / (int)sizeof(T));
+    nvec = (N - head) / V;
+    v0 = min(nvec, rank * per);
+    v1 = min(nvec, v0 + per);
   };
-  if (tid == 0 && (int)blockIdx.x < M)
-    for (int c = 0; c < kRowChunks; ++c) load_chunk(blockIdx.x, c);
+  auto load_chunk = [&](int row, int c) {  // thread 0; the buffer region of the chunk must be free
+    const T* src;
+    int head, nvec, v0, v1;
+    layout(row, src, head, nvec, v0, v1);
+    const int p0 = c * kChunkVecs, p1 = min(v1 - v0, p0 + kChunkVecs);
+    if (p1 <= p0) return;
+    const uint32_t bytes = (uint32_t)(p1 - p0) * 16;
+    mbar_expect_tx(&full[c], bytes);
+    bulk_g2s(buf + p0, src + head + (long long)(v0 + p0) * V, bytes, &full[c]);
+  };
+  if (tid == 0 && team < M)
+    for (int c = 0; c * kChunkVecs < per; ++c) load_chunk(team, c);
   bool alive = true;
-  int it = 0;
-  for (int row = blockIdx.x; row < M && alive; row += gridDim.x, ++it) {
-    // One pass over the chunks as they land: running maximum and sum of exponentials per thread, the sum rescaled
-    // when the maximum grows (the chunk loop of the reference, examples/softmax.jl:48-100), then combined over the CTA
-    // in a fixed order.
+  uint32_t phases = 0;  // bit c: parity of chunk c's next completion (a row may have one chunk fewer than another)
+  for (int row = team, it = 0; row < M; row += teams, ++it) {
+    const T* src;
+    int head, nvec, v0, v1;
+    layout(row, src, head, nvec, v0, v1);
+    const int cnt = v1 - v0, tail = N - head - nvec * V;
+    // elements outside the aligned middle: thread i < head + tail of rank 0 holds one
+    const bool edge = rank == 0 && tid < head + tail;
+    const int at = tid < head ? tid : nvec * V + tid;
+    const float xe = edge ? (float)src[at] : 0.f;
     float m = -FLT_MAX, l = 0.f;
-    for (int c = 0; c < kRowChunks; ++c) {
-      const int p0 = c * per, p1 = min(npack, p0 + per);
-      if (p1 <= p0) break;
-      if (!mbar_wait(&full[c], it & 1, status, DEV_TIMEOUT_TMA)) alive = false;
+    if (edge) {
+      m = xe;
+      l = 1.f;
+    }
+    for (int c = 0; c * kChunkVecs < cnt; ++c) {
+      const int p0 = c * kChunkVecs, p1 = min(cnt, p0 + kChunkVecs);
+      if (alive && !mbar_wait(&full[c], (phases >> c) & 1, status, DEV_TIMEOUT_TMA)) alive = false;
+      phases ^= 1u << c;
       for (int p = p0 + tid; p < p1; p += kRowThreads) {
-        float f[4];
-        Pack<T>::unpack(buf[p], f);
-        const float cm = fmaxf(fmaxf(f[0], f[1]), fmaxf(f[2], f[3]));
+        float f[V];
+        unpack16<T>(buf[p], f);
+        float cm = f[0];
+#pragma unroll
+        for (int k = 1; k < V; ++k) cm = fmaxf(cm, f[k]);
         if (cm > m) {
           l *= exp_sub(m, cm);
           m = cm;
         }
-        l += (exp_sub(f[0], m) + exp_sub(f[1], m)) + (exp_sub(f[2], m) + exp_sub(f[3], m));
+        float s = 0.f;
+#pragma unroll
+        for (int k = 0; k < V; k += 2) s += exp_sub(f[k], m) + exp_sub(f[k + 1], m);
+        l += s;
       }
     }
-    alive = __syncthreads_and(alive);
-    if (!alive) break;
-    const float mx = block_reduce(m, true);
-    const float inv = 1.0f / block_reduce(l * exp_sub(m, mx), false);
-    // Scale and store chunk by chunk, from registers straight to global memory (16 bytes per thread, neighbouring
-    // threads neighbouring addresses); as soon as every thread has read a chunk's part of the buffer, the same part
-    // takes the next row's chunk, so that the next row streams in under the rest of this one.
-    const int next = row + gridDim.x;
-    P* dst = reinterpret_cast<P*>(out + (long long)row * ld_out);
-    for (int c = 0; c < kRowChunks; ++c) {
-      const int p0 = c * per, p1 = min(npack, p0 + per);
-      if (p1 <= p0) break;
+    float mx = block_reduce(m, true);
+    float sum = block_reduce(l * exp_sub(m, mx), false);
+    if (C > 1) {
+      if (tid < C) {
+        const uint32_t dst = map_to_cta(&peers[it & 1][rank], (uint32_t)tid);
+        asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(dst), "f"(mx), "f"(sum) : "memory");
+      }
+      cluster_arrive();
+      cluster_wait();
+      float M2 = -FLT_MAX;
+      for (int k = 0; k < C; ++k) M2 = fmaxf(M2, peers[it & 1][k].x);
+      sum = 0.f;
+      for (int k = 0; k < C; ++k) sum += peers[it & 1][k].y * exp_sub(peers[it & 1][k].x, M2);  // ascending rank
+      mx = M2;
+    }
+    const float inv = 1.0f / sum;
+    const int next = row + teams;
+    T* dst = out + (long long)row * ld_out;
+    if (edge) dst[at] = (T)(exp_sub(xe, mx) * inv);
+    T* mid = dst + head + (long long)v0 * V;
+    const bool vec = ((uintptr_t)mid & 15) == 0;
+    for (int c = 0; c * kChunkVecs < per; ++c) {
+      const int p0 = c * kChunkVecs, p1 = min(cnt, p0 + kChunkVecs);
       for (int p = p0 + tid; p < p1; p += kRowThreads) {
-        float f[4];
-        Pack<T>::unpack(buf[p], f);
+        float f[V];
+        unpack16<T>(buf[p], f);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) f[k] = exp_sub(f[k], mx) * inv;
-        const P v = Pack<T>::pack(f);
-        if constexpr (sizeof(P) == 16) __stcs(reinterpret_cast<float4*>(dst + p), *reinterpret_cast<const float4*>(&v));
-        else __stcs(reinterpret_cast<uint2*>(dst + p), *reinterpret_cast<const uint2*>(&v));
+        for (int k = 0; k < V; ++k) f[k] = exp_sub(f[k], mx) * inv;
+        if (vec) {
+          uint4 q;
+          if constexpr (sizeof(T) == 4) {
+            q = make_uint4(__float_as_uint(f[0]), __float_as_uint(f[1]), __float_as_uint(f[2]), __float_as_uint(f[3]));
+          } else {
+            q = make_uint4(pack_f16x2(f[0], f[1]), pack_f16x2(f[2], f[3]), pack_f16x2(f[4], f[5]), pack_f16x2(f[6], f[7]));
+          }
+          __stcs(reinterpret_cast<uint4*>(mid) + p, q);
+        } else {
+#pragma unroll
+          for (int k = 0; k < V; ++k) mid[(long long)p * V + k] = (T)f[k];
+        }
       }
       __syncthreads();  // all reads of the chunk are done before the bulk copy overwrites it
       if (tid == 0 && next < M) load_chunk(next, c);
@@ -365,7 +517,21 @@ int launch(ctb_ctx* ctx, cudaStream_t st, T* out, const T* in, int N, int M, lon
   if (variant == 0 && !fits)
     return fail(CTB_UNSUPPORTED, "ctb_softmax variant 0: N=%d exceeds the single-tile limit %d; use variant 1", N,
                 4 * kThreads * MAXV);
-  if (bulk_ok && fits) {
+  if (N <= 1024) {
+    // both variants; a warp per CTA while that spreads the rows over more SMs
+    const int warps = std::min(4, std::max(1, M / (2 * ctx->sm_count)));
+    const int grid = std::min((M + warps - 1) / warps, ctx->sm_count * 16);
+#define CTB_SOFTMAX_WARP(NE)                                                                                              \
+  do {                                                                                                                    \
+    if (vec_ok) launch_kernel(softmax_warp_kernel<T, NE, true>, grid, warps * 32, 0, st, 0, out, in, N, M, ldo, ldi);     \
+    else launch_kernel(softmax_warp_kernel<T, NE, false>, grid, warps * 32, 0, st, 0, out, in, N, M, ldo, ldi);           \
+  } while (0)
+    if (N <= 128) CTB_SOFTMAX_WARP(4);
+    else if (N <= 256) CTB_SOFTMAX_WARP(8);
+    else if (N <= 512) CTB_SOFTMAX_WARP(16);
+    else CTB_SOFTMAX_WARP(32);
+#undef CTB_SOFTMAX_WARP
+  } else if (bulk_ok && fits) {
     // Both variants: a row that fits the registers of one CTA is read once and written once whatever the chunk
     // size asks for; the chunk loop of the reference (examples/softmax.jl:48-100) only matters for longer rows.
     const int stage_bytes = (int)((row_bytes + 127) & ~size_t(127));
@@ -378,14 +544,23 @@ int launch(ctb_ctx* ctx, cudaStream_t st, T* out, const T* in, int N, int M, lon
     if (per_sm < 1) per_sm = 1;
     const int grid = min(M, ctx->sm_count * per_sm);
     launch_kernel(k, grid, kThreads, smem, st, 0, out, in, N, M, ldo, ldi, stage_bytes, ctx->dev_status);
-  } else if (bulk_ok && row_bytes <= 200 * 1024) {
-    const size_t smem = (row_bytes + 127) & ~size_t(127);
-    auto k = softmax_row_smem_kernel<T>;
+  } else if (fits) {
+    const int grid = std::min(M, ctx->sm_count * 8);
+    if (N <= 8 * kThreads) launch_kernel(softmax_regs_kernel<T, 8>, grid, kThreads, 0, st, 0, out, in, N, M, ldo, ldi);
+    else if (N <= 16 * kThreads) launch_kernel(softmax_regs_kernel<T, 16>, grid, kThreads, 0, st, 0, out, in, N, M, ldo, ldi);
+    else launch_kernel(softmax_regs_kernel<T, 32>, grid, kThreads, 0, st, 0, out, in, N, M, ldo, ldi);
+  } else if (row_bytes <= (size_t)kMaxCluster * 104 * 1024 && (uintptr_t)in % sizeof(T) == 0) {
+    int C = 1;
+    while (row_bytes > (size_t)C * 104 * 1024) C *= 2;
+    constexpr int V = 16 / (int)sizeof(T);
+    const int per = (N / V + C - 1) / C;
+    const size_t smem = (size_t)per * 16;
+    auto k = softmax_long_kernel<T>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return cuda_fail(e, "ctb_softmax: shared memory opt-in");
-    const int per_sm = std::max(1, (int)((size_t)220 * 1024 / (smem + 2048)));
-    const int grid = min(M, ctx->sm_count * std::min(per_sm, 4));
-    launch_kernel(k, grid, kRowThreads, smem, st, 0, out, in, N, M, ldo, ldi, ctx->dev_status);
+    const int per_sm = std::max(1, std::min(4, (int)((size_t)222 * 1024 / (smem + 2048))));
+    const int teams = std::max(1, std::min(M, ctx->sm_count * per_sm / C));
+    launch_kernel(k, teams * C, kRowThreads, smem, st, C, out, in, N, M, ldo, ldi, per, C, ctx->dev_status);
   } else {
     int per_sm = 8;
     const int grid = min(M, ctx->sm_count * per_sm);

@@ -100,3 +100,26 @@ def test_softmax_rejections(cuda):
         cuda.softmax.softmax_tma_kernel(torch.empty_like(x), x, 16384)
     assert e.value.status == lib.UNSUPPORTED
     cuda.softmax.softmax_chunked_kernel(torch.empty(0, 8, device="cuda"), torch.empty(0, 8, device="cuda"), 8, 8)
+
+
+@pytest.mark.parametrize("M,N", [(3, 1), (700, 127), (5, 128), (2000, 257), (9, 1000), (70, 1024), (70, 1025), (11, 2049),
+                                 (600, 4097), (3, 8191), (3, 8193), (400, 16385), (7, 26624), (5, 26625), (310, 50001),
+                                 (2, 106497), (3, 212999), (2, 213500)])
+@pytest.mark.parametrize("dtype,shift", [(np.float32, 0), (np.float32, 1), (np.float16, 0), (np.float16, 3)])
+def test_softmax_any_length_and_alignment(cuda, M, N, dtype, shift):
+    """Every kernel and the sizes where one takes over from another: a warp per row, registers of a CTA, one, two, four and
+    eight CTAs per row, re-read rows; rows that start anywhere (odd lengths, views off the vector alignment), an output with
+    another alignment than the input."""
+    import torch
+    x = inputs.softmax(M=M, N=N, seed=M + N)["input"].astype(dtype)
+    flat = torch.zeros(M * N + 8, device="cuda", dtype=torch.from_numpy(x).dtype)
+    flat[shift:shift + M * N] = torch.from_numpy(x).reshape(-1).cuda()
+    xin = flat[shift:shift + M * N].view(M, N)
+    want = ref.softmax(x)
+    for oshift in (shift, 2):
+        guard = torch.full((M * N + 8,), 7.0, device="cuda", dtype=xin.dtype)
+        out = guard[oshift:oshift + M * N].view(M, N)
+        run(cuda, xin, 1, out=out)
+        assert ref.max_abs_over_max(out.float().cpu().numpy(), want) <= (TOL if dtype == np.float32 else 1e-3)
+        assert (guard[:oshift] == 7.0).all() and (guard[oshift + M * N:] == 7.0).all()
+    cuda.check_device_status(0)
