@@ -2,6 +2,7 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "ctx.h"
@@ -63,9 +64,19 @@ int* sched_slot(ctb_ctx* ctx) {
   return ctx->sched_pool + 2 * (n % kSchedSlots);
 }
 
-int* ticket_slots(ctb_ctx* ctx) {
-  const unsigned n = __atomic_fetch_add(&ctx->tickets_next, 1u, __ATOMIC_RELAXED);
-  return ctx->tickets + (size_t)kTickets * (n % kTicketSlots);
+StreamScratch stream_scratch(ctb_ctx* ctx, cudaStream_t stream) {
+  int slot = 0;
+  {
+    std::lock_guard<std::mutex> lock(*ctx->slot_lock);
+    const int known = std::min(ctx->slots_used, kStreamSlots);
+    while (slot < known && ctx->slot_stream[slot] != stream) ++slot;
+    if (slot == known) {
+      slot = ctx->slots_used % kStreamSlots;
+      ctx->slot_stream[slot] = stream;
+      ctx->slots_used = ctx->slots_used < 2 * kStreamSlots - 1 ? ctx->slots_used + 1 : kStreamSlots;
+    }
+  }
+  return {reinterpret_cast<float*>(ctx->stream_pool + slot * kStreamScratchBytes), ctx->tickets + (size_t)slot * kTickets};
 }
 
 EncodeTiledFn encode_tiled() {
@@ -140,7 +151,9 @@ int ctb_create(ctb_ctx** out, int device) {
   c->sched_pool = nullptr;
   c->sched_next = 0;
   c->tickets = nullptr;
-  c->tickets_next = 0;
+  c->stream_pool = nullptr;
+  c->slots_used = 0;
+  c->slot_lock = new std::mutex();
   c->flag_wait_ns = 2000000000ull;
   c->tf32_rne = 0;
   c->comm = nullptr;
@@ -148,9 +161,11 @@ int ctb_create(ctb_ctx** out, int device) {
   if (e == cudaSuccess) e = cudaMemset(c->dev_status, 0, sizeof(int));
   if (e == cudaSuccess) e = cudaMalloc(&c->sched_pool, 2 * kSchedSlots * sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(c->sched_pool, 0, 2 * kSchedSlots * sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc(&c->tickets, kTicketSlots * kTickets * sizeof(int));
-  if (e == cudaSuccess) e = cudaMemset(c->tickets, 0, kTicketSlots * kTickets * sizeof(int));
+  if (e == cudaSuccess) e = cudaMalloc(&c->tickets, kStreamSlots * kTickets * sizeof(int));
+  if (e == cudaSuccess) e = cudaMemset(c->tickets, 0, kStreamSlots * kTickets * sizeof(int));
+  if (e == cudaSuccess) e = cudaMalloc(&c->stream_pool, kStreamSlots * kStreamScratchBytes);
   if (e != cudaSuccess) {
+    delete c->slot_lock;
     delete c;
     return cuda_fail(e, "ctb_create: status word");
   }
@@ -166,6 +181,8 @@ void ctb_destroy(ctb_ctx* ctx) {
   if (ctx->dev_status) cudaFree(ctx->dev_status);
   if (ctx->sched_pool) cudaFree(ctx->sched_pool);
   if (ctx->tickets) cudaFree(ctx->tickets);
+  if (ctx->stream_pool) cudaFree(ctx->stream_pool);
+  delete ctx->slot_lock;
   delete ctx;
 }
 

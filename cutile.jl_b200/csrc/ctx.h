@@ -7,6 +7,7 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include <mutex>
 #include <utility>
 
 #include "../../include/cutile_b200.h"
@@ -23,10 +24,15 @@ struct ctb_ctx {
   // that overlap on the device (different streams) do not share one.
   int* sched_pool;
   unsigned sched_next;
-  // Arrival counters of reductions whose last CTA finishes the job: kTicketSlots sets of kTickets ints, zero between
-  // launches (the last CTA returns its counter to zero).  Launches take the sets in turn.
+  // Scratch of kernels whose last CTA adds up the parts that the others leave: kStreamSlots slots of kStreamScratchBytes
+  // and kTickets arrival counters each (zero between launches: the last CTA returns its counter to zero).  A stream keeps
+  // the slot it was given first (stream_scratch), so launches that overlap on the device do not share one; beyond
+  // kStreamSlots streams slots are shared in turn.
+  unsigned char* stream_pool;
   int* tickets;
-  unsigned tickets_next;
+  void* slot_stream[32];
+  int slots_used;
+  std::mutex* slot_lock;
   void* comm;             // ctb_internal::Comm* once an NCCL communicator is attached (multi.cu)
   unsigned long long flag_wait_ns;  // how long a kernel waits for another rank's flag before it gives up
   int tf32_rne;           // 1: f32 GEMM operands are rounded to TF32 (nearest even) by a pass of their own first
@@ -50,11 +56,22 @@ int moe_experts_rows(ctb_ctx* ctx, cudaStream_t st, const void* rows, int64_t ld
                      const void* gates, int64_t R, int64_t H, int64_t I, int64_t E_local, const void* w1_local,
                      const void* w2_local, int tile_m, void* C, int64_t ldc, void* const* c_peer, int64_t c_split);
 constexpr int kSchedSlots = 256;
-constexpr int kTickets = 4096, kTicketSlots = 16;
+constexpr int kTickets = 4096, kStreamSlots = 32;
+constexpr size_t kStreamScratchBytes = 1280 * 1024;
+struct StreamScratch {
+  float* data;   // kStreamScratchBytes
+  int* tickets;  // kTickets counters, zero
+};
 // The next pair of work counters of the context (see ctb_ctx::sched_pool).
 int* sched_slot(ctb_ctx* ctx);
-// The next set of kTickets arrival counters of the context (see ctb_ctx::tickets).
-int* ticket_slots(ctb_ctx* ctx);
+// The scratch slot of a stream (see ctb_ctx::stream_pool).
+StreamScratch stream_scratch(ctb_ctx* ctx, cudaStream_t stream);
+// Attention with at most 16 (group x position) query rows per key/value head (fmha_decode.cu); the arguments are checked.
+bool fmha_decode_fits(int64_t seq_q, int group);
+int fmha_decode(ctb_ctx* ctx, cudaStream_t st, const void* Q, const void* K, const void* V, void* Out, int64_t seq_q,
+                int64_t seq_kv, int64_t heads, int64_t kv_heads, int64_t batch, float qk_scale, int input_pos, bool causal,
+                bool bf16);
+
 
 // cuTensorMapEncodeTiled, resolved through the runtime so that the library has
 // no link-time dependency on libcuda and loads on machines without a driver.

@@ -568,6 +568,11 @@ extern "C" int ctb_fmha_fwd(ctb_ctx* ctx, void* stream, const void* Q, const voi
   if ((uintptr_t)Q % 16 || (uintptr_t)K % 16 || (uintptr_t)V % 16 || (uintptr_t)Out % 16)
     return fail(CTB_BAD_ALIGN, "ctb_fmha_fwd: Q, K, V, Out must be 16-byte aligned");
 
+  // Few query rows per key/value head: the kernel that splits the keys over the GPU.  The line is where the rows of a group
+  // no longer fit its 16-row instructions; a 128-row tile is at least 7/8 padding below it.
+  if (fmha_decode_fits(seq_q, query_group_size))
+    return fmha_decode(ctx, static_cast<cudaStream_t>(stream), Q, K, V, Out, seq_q, seq_kv, heads, kv_heads, batch, qk_scale,
+                       input_pos, causal != 0, dtype == CTB_BF16);
   CUtensorMap tq, tk, tv;
   const uint32_t box[3] = {kD, kTN, 1};
   {

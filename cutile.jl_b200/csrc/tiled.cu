@@ -985,7 +985,7 @@ struct ReduceShape {
   long long outputs, red_len, parts, chunk;
 };
 
-// A reduction that is cut into parts leaves one partial result per (part, output) in the context's scratch, outputs
+// A reduction that is cut into parts leaves one partial result per (part, output) in the stream's scratch, outputs
 // contiguous; the CTA that finishes last for its outputs (a counter per grid column, returned to zero by that CTA) adds
 // the parts up in a fixed order.  One launch instead of two, and the result does not depend on which CTA is last.
 // True for every thread of the last CTA; the partials of the others are visible then.
@@ -1343,14 +1343,21 @@ int ctb_tiled_mapreduce(ctb_ctx* ctx, void* stream, void* dest, const void* src,
   if (mode_a) s.chunk = (s.chunk + 1023) / 1024 * 1024;  // parts start on 16-byte boundaries of an aligned row
   s.parts = (std::max<long long>(1, s.red_len) + s.chunk - 1) / s.chunk;
   float* partial = nullptr;
+  int* tickets = nullptr;
   if (s.parts > 1) {
-    void* ws = nullptr;
-    int r = workspace(ctx, (size_t)s.outputs * s.parts * sizeof(float), &ws, st);
-    if (r) return r;
-    partial = static_cast<float*>(ws);
+    const StreamScratch scratch = stream_scratch(ctx, st);
+    tickets = scratch.tickets;
+    const size_t bytes = (size_t)s.outputs * s.parts * sizeof(float);
+    if (bytes <= kStreamScratchBytes) {
+      partial = scratch.data;
+    } else {
+      void* ws = nullptr;
+      int r = workspace(ctx, bytes, &ws, st);
+      if (r) return r;
+      partial = static_cast<float*>(ws);
+    }
   }
   if (columns > 0x7fffffffLL) return fail(CTB_UNSUPPORTED, "ctb_tiled_mapreduce: too many output elements");
-  int* tickets = s.parts > 1 ? ticket_slots(ctx) : nullptr;
   const dim3 grid((unsigned)columns, (unsigned)s.parts);
   const long long rstride = (reduce_mask & 2) ? s.d[0] : s.d[0] * s.d[1];  // between elements of the reduced index space
 #define CTB_RED_LAUNCH(T, OP, M)                                                                                            \

@@ -104,3 +104,27 @@ def test_fmha_bf16(cuda, batch, heads, seq_q, seq_kv, causal, input_pos, kv_head
     want = ref.fmha(back(Q), back(K), back(V), causal=causal, input_pos=input_pos)
     assert ref.rel_fro(back(out), want) <= 1e-2
     cuda.check_device_status(0)
+
+
+@pytest.mark.parametrize("batch,heads,kv_heads,seq_q,seq_kv,causal,input_pos", [
+    (1, 1, 1, 1, 1, True, 0), (2, 8, 2, 1, 31, True, 30), (3, 16, 2, 1, 256, True, 255), (1, 32, 4, 1, 257, True, 256),
+    (5, 4, 4, 1, 1000, True, 999), (1, 8, 8, 1, 8191, True, 8190), (2, 16, 1, 1, 3000, True, 2999), (2, 16, 4, 4, 700, True, 696),
+    (1, 5, 5, 16, 333, True, 317), (2, 6, 3, 8, 64, True, 0), (2, 8, 4, 3, 500, False, 0), (1, 4, 4, 1, 900, True, 200),
+    (40, 8, 4, 1, 2049, True, 2048)])
+@pytest.mark.parametrize("bf16", [False, True])
+def test_fmha_decode(cuda, batch, heads, kv_heads, seq_q, seq_kv, causal, input_pos, bf16):
+    """Few query rows per key/value head: 1, up to 8 and up to 16 rows, keys in one block, at block edges, over several
+    CTAs and with several pairs per CTA, keys behind the last visible one, twice in a row (the arrival counters are back at
+    zero, the order of summation is fixed)."""
+    import torch
+    dt = torch.bfloat16 if bf16 else torch.float16
+    d = inputs.fmha(batch, heads, seq_q, seq_kv, 64, kv_heads=kv_heads, seed=19)
+    Q, K, V = (torch.from_numpy(d[k].astype(np.float32)).cuda().to(dt) for k in ("Q", "K", "V"))
+    run = lambda: cuda.fmha.cutile_fmha(Q, K, V, causal=causal, input_pos=input_pos, query_group_size=heads // kv_heads)
+    out, again = run(), run()
+    assert torch.equal(out, again)
+    back = lambda t: t.float().cpu().numpy()
+    want = ref.fmha(back(Q), back(K), back(V), causal=causal, input_pos=input_pos)
+    for h in range(heads):
+        assert ref.rel_fro(back(out)[:, h], want[:, h]) <= (1e-2 if bf16 else TOL)
+    cuda.check_device_status(0)
