@@ -185,6 +185,131 @@ fft_kernel(const float2* __restrict__ x, float2* __restrict__ y, const float2* _
   });
 }
 
+// ---- the transform with the standard tables -------------------------------------------------------------------------
+// When the DFT matrices are the exact ones (FftPlan), a line of F points is an in-register FFT of radix-2 butterflies
+// with constant factors instead of F^2 multiply-adds: 5 N log2 N operations.  What bounds it then is the latency of one
+// pass: load, two exchanges through shared memory, store (256 x 4096 points: 15.4 us with the matrices, FMA issue and
+// latency of 16 warps per SM).
+template <int K>  // cos(pi K / 16), K = 0..8
+__host__ __device__ constexpr float cos16() {
+  constexpr double c[9] = {1.0, 0.98078528040323044913, 0.92387953251128675613, 0.83146961230254523708, 0.70710678118654752440,
+                           0.55557023301960222474, 0.38268343236508977173, 0.19509032201612826785, 0.0};
+  return (float)c[K];
+}
+// x * exp(-2 pi i K / F), 0 <= K < F / 2
+template <int K, int F>
+__device__ __forceinline__ float2 rotate(float2 x) {
+  constexpr int A = K * 32 / F;  // the angle is -pi A / 16, 0 <= A < 16
+  if constexpr (A == 0) return x;
+  else if constexpr (A == 8) return make_float2(x.y, -x.x);
+  else {
+    constexpr float c = A < 8 ? cos16<A < 8 ? A : 0>() : -cos16<A < 8 ? 0 : 16 - A>();
+    constexpr float sn = A < 8 ? cos16<A < 8 ? 8 - A : 0>() : cos16<A < 8 ? 0 : A - 8>();
+    if constexpr (A == 4) return make_float2(c * (x.x + x.y), c * (x.y - x.x));
+    else if constexpr (A == 12) return make_float2(c * (x.x - x.y), c * (x.x + x.y));
+    else return make_float2(fmaf(x.x, c, x.y * sn), fmaf(x.y, c, -x.x * sn));
+  }
+}
+template <int F, int K>
+__device__ __forceinline__ void combine(float2 (&y)[F], const float2 (&e)[F / 2], const float2 (&o)[F / 2]) {
+  if constexpr (K < F / 2) {
+    const float2 w = rotate<K, F>(o[K]);
+    y[K] = make_float2(e[K].x + w.x, e[K].y + w.y);
+    y[K + F / 2] = make_float2(e[K].x - w.x, e[K].y - w.y);
+    combine<F, K + 1>(y, e, o);
+  }
+}
+template <int F>
+__device__ __forceinline__ void fft_line(float2 (&x)[F]) {  // in place, natural order in and out
+  if constexpr (F > 1) {
+    float2 e[F / 2], o[F / 2];
+#pragma unroll
+    for (int k = 0; k < F / 2; ++k) {
+      e[k] = x[2 * k];
+      o[k] = x[2 * k + 1];
+    }
+    fft_line<F / 2>(e);
+    fft_line<F / 2>(o);
+    combine<F, 0>(x, e, o);
+  }
+}
+template <int MAXF, class Fn>
+__device__ __forceinline__ void with_factor_up_to(int f, Fn fn) {
+  if (f == 1) fn(std::integral_constant<int, 1>{});
+  else if (f == 2) fn(std::integral_constant<int, 2>{});
+  else if (f == 4) fn(std::integral_constant<int, 4>{});
+  else if (MAXF == 8 || f == 8) fn(std::integral_constant<int, 8>{});
+  else if constexpr (MAXF == 16) fn(std::integral_constant<int, 16>{});
+  else if constexpr (MAXF == 32) {
+    if (f == 16) fn(std::integral_constant<int, 16>{});
+    else fn(std::integral_constant<int, 32>{});
+  }
+}
+
+// The three stages of fft_kernel; a CTA transforms `items` items side by side (small transforms: enough lines for its
+// threads).  MAXF: bound of the factors (registers).
+template <int MAXF>
+__global__ void __launch_bounds__(256) fft_plan_kernel(const float2* __restrict__ x, float2* __restrict__ y,
+                                                       const float2* __restrict__ T0, const float2* __restrict__ T1, int F0,
+                                                       int F1, int F2, int batch, int items) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int N = F0 * F1 * F2, F1F2 = F1 * F2, F0F2 = F0 * F2, F0F1 = F0 * F1;
+  const int padded = pad16(N - 1) + 1;
+  const int mine = min(items, batch - (int)blockIdx.x * items);  // items of this CTA
+  float2* A = reinterpret_cast<float2*>(smem_raw);
+  float2* B = A + items * padded;
+  const float2* __restrict__ xb = x + (size_t)blockIdx.x * items * N;
+  float2* __restrict__ yb = y + (size_t)blockIdx.x * items * N;
+  ctb::grid_dependency_sync();
+
+  with_factor_up_to<MAXF>(F0, [&](auto f) {
+    constexpr int F = decltype(f)::value;
+    for (int line = threadIdx.x; line < mine * F1F2; line += blockDim.x) {
+      const int it = line / F1F2, j = line - it * F1F2;
+      float2 v[F], t[F];
+#pragma unroll
+      for (int n = 0; n < F; ++n) v[n] = __ldcs(xb + it * N + j + F1F2 * n);
+#pragma unroll
+      for (int k = 0; k < F; ++k) t[k] = __ldg(T0 + j + F1F2 * k);
+      fft_line<F>(v);
+      float2* a = A + it * padded;
+#pragma unroll
+      for (int k = 0; k < F; ++k) a[pad16(F * j + k)] = cmul(v[k], t[k]);
+    }
+  });
+  __syncthreads();
+  with_factor_up_to<MAXF>(F1, [&](auto f) {
+    constexpr int F = decltype(f)::value;
+    for (int line = threadIdx.x; line < mine * F0F2; line += blockDim.x) {
+      const int it = line / F0F2, r = line - it * F0F2, n2 = r / F0;
+      const float2* a = A + it * padded;
+      float2 v[F], t[F];
+#pragma unroll
+      for (int k = 0; k < F; ++k) t[k] = __ldg(T1 + n2 + F2 * k);
+#pragma unroll
+      for (int n = 0; n < F; ++n) v[n] = a[pad16(r + F0F2 * n)];
+      fft_line<F>(v);
+      float2* b = B + it * padded;
+#pragma unroll
+      for (int k = 0; k < F; ++k) b[pad16(F * r + k)] = cmul(v[k], t[k]);
+    }
+  });
+  __syncthreads();
+  with_factor_up_to<MAXF>(F2, [&](auto f) {
+    constexpr int F = decltype(f)::value;
+    for (int line = threadIdx.x; line < mine * F0F1; line += blockDim.x) {
+      const int it = line / F0F1, t = line - it * F0F1, k1 = t / F0, k0 = t - k1 * F0;
+      const float2* b = B + it * padded;
+      float2 v[F];
+#pragma unroll
+      for (int n = 0; n < F; ++n) v[n] = b[pad16(k1 + F1 * k0 + F0F1 * n)];
+      fft_line<F>(v);
+#pragma unroll
+      for (int k = 0; k < F; ++k) __stcs(yb + it * N + t + F0F1 * k, v[k]);
+    }
+  });
+}
+
 size_t fft_smem_bytes(int N, int F0, int F1, int F2) {
   const size_t padded = ((size_t)(N - 1) + ((N - 1) >> 4) + 2) & ~(size_t)1;
   return (2 * padded + (size_t)F0 * F0 + (size_t)F1 * F1 + (size_t)F2 * F2 + 4) * sizeof(float2);
@@ -192,20 +317,53 @@ size_t fft_smem_bytes(int N, int F0, int F1, int F2) {
 
 }  // namespace
 
+namespace {
+int check_fft(const char* who, int64_t N, int F0, int F1, int F2, int64_t batch, int BS, int D) {
+  for (int f : {F0, F1, F2})
+    if (f < 1 || !is_pow2(f)) return fail(CTB_UNSUPPORTED_TILE, "%s: factors must be powers of two (got %d)", who, f);
+  for (int f : {F0, F1, F2})
+    if (f > kMaxFactor) return fail(CTB_UNSUPPORTED, "%s: factors up to %d are implemented (got %d)", who, kMaxFactor, f);
+  if (N != (int64_t)F0 * F1 * F2) return fail(CTB_BAD_ARG, "%s: N must equal F0 * F1 * F2", who);
+  if (N > kMaxN) return fail(CTB_UNSUPPORTED, "%s: N up to %d is implemented", who, kMaxN);
+  if (batch < 0 || BS < 1 || batch % BS != 0) return fail(CTB_BAD_ARG, "%s: batch must be a non-negative multiple of BS", who);
+  if (!is_pow2(BS)) return fail(CTB_UNSUPPORTED_TILE, "%s: BS must be a power of two", who);
+  if (D < 2 || !is_pow2(D) || (2 * N) % D != 0)
+    return fail(CTB_BAD_ARG, "%s: 2 * N must be divisible by atom_packing_dim (a power of two >= 2)", who);
+  if (batch > INT32_MAX) return fail(CTB_BAD_ARG, "%s: batch too large", who);
+  return CTB_OK;
+}
+}  // namespace
+
+extern "C" int ctb_fft_plan(ctb_ctx* ctx, void* stream, const void* x, void* y, const void* T0, const void* T1, int64_t N, int F0,
+                            int F1, int F2, int64_t batch, int BS, int D) {
+  CTB_CHECK_CTX(ctx);
+  int r = check_fft("ctb_fft_plan", N, F0, F1, F2, batch, BS, D);
+  if (r) return r;
+  if (batch == 0) return CTB_OK;
+  CTB_CHECK_DEV(x); CTB_CHECK_DEV(y); CTB_CHECK_DEV(T0); CTB_CHECK_DEV(T1);
+  for (const void* p : {x, (const void*)y, T0, T1})
+    if ((uintptr_t)p % 8 != 0) return fail(CTB_BAD_ALIGN, "ctb_fft_plan: arrays must be 8-byte aligned");
+  // items per CTA: about 2048 points in a CTA while that leaves every SM a CTA; a thread per line of the largest factor
+  const int items = (int)std::max<int64_t>(1, std::min<int64_t>({2048 / N, batch / ctx->sm_count, (int64_t)64}));
+  const int maxf = std::max(F0, std::max(F1, F2));
+  const int threads = (int)std::min<int64_t>(256, std::max<int64_t>(32, (items * N / maxf + 31) / 32 * 32));
+  const size_t smem = 2 * (size_t)items * ((size_t)(N - 1) + ((N - 1) >> 4) + 1) * sizeof(float2);
+  auto kern = maxf <= 8 ? fft_plan_kernel<8> : maxf == 16 ? fft_plan_kernel<16> : fft_plan_kernel<32>;
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return cuda_fail(e, "ctb_fft_plan: shared memory attribute");
+  }
+  launch_kernel(kern, (unsigned)((batch + items - 1) / items), threads, smem, static_cast<cudaStream_t>(stream), 0,
+                (const float2*)x, (float2*)y, (const float2*)T0, (const float2*)T1, F0, F1, F2, (int)batch, items);
+  CTB_CHECK_LAUNCH("ctb_fft_plan launch");
+  return CTB_OK;
+}
+
 extern "C" int ctb_fft(ctb_ctx* ctx, void* stream, const void* x, void* y, const void* W0, const void* W1, const void* W2,
                        const void* T0, const void* T1, int64_t N, int F0, int F1, int F2, int64_t batch, int BS, int D) {
   CTB_CHECK_CTX(ctx);
-  for (int f : {F0, F1, F2})
-    if (f < 1 || !is_pow2(f)) return fail(CTB_UNSUPPORTED_TILE, "ctb_fft: factors must be powers of two (got %d)", f);
-  for (int f : {F0, F1, F2})
-    if (f > kMaxFactor) return fail(CTB_UNSUPPORTED, "ctb_fft: factors up to %d are implemented (got %d)", kMaxFactor, f);
-  if (N != (int64_t)F0 * F1 * F2) return fail(CTB_BAD_ARG, "ctb_fft: N must equal F0 * F1 * F2");
-  if (N > kMaxN) return fail(CTB_UNSUPPORTED, "ctb_fft: N up to %d is implemented", kMaxN);
-  if (batch < 0 || BS < 1 || batch % BS != 0) return fail(CTB_BAD_ARG, "ctb_fft: batch must be a non-negative multiple of BS");
-  if (!is_pow2(BS)) return fail(CTB_UNSUPPORTED_TILE, "ctb_fft: BS must be a power of two");
-  if (D < 2 || !is_pow2(D) || (2 * N) % D != 0)
-    return fail(CTB_BAD_ARG, "ctb_fft: 2 * N must be divisible by atom_packing_dim (a power of two >= 2)");
-  if (batch > INT32_MAX) return fail(CTB_BAD_ARG, "ctb_fft: batch too large");
+  int r = check_fft("ctb_fft", N, F0, F1, F2, batch, BS, D);
+  if (r) return r;
   if (batch == 0) return CTB_OK;
   CTB_CHECK_DEV(x); CTB_CHECK_DEV(y); CTB_CHECK_DEV(W0); CTB_CHECK_DEV(W1); CTB_CHECK_DEV(W2); CTB_CHECK_DEV(T0); CTB_CHECK_DEV(T1);
   for (const void* p : {x, (const void*)y, W0, W1, W2, T0, T1})

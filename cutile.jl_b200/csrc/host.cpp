@@ -663,18 +663,18 @@ PyObject* mapreduce(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return THPVariable_Wrap(std::move(dest));
 }
 
-// fft(x complex64 [batch, N], out or None, (W0, W1, W2, T0, T1), N, F0, F1, F2, D) -> out
+// fft(x complex64 [batch, N], out or None, (W0, W1, W2, T0, T1) of make_twiddles, N, F0, F1, F2, D) -> out
 PyObject* fft(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  const Tensor *x, *out, *tab[5];
+  const Tensor *x, *out, *tab[2];
   long long v[5];
   if (n != 8 || !(x = cuda_tensor(a[0])) || !PyTuple_Check(a[2]) || PyTuple_GET_SIZE(a[2]) != 5 || !ints(a + 3, 5, v))
     return decline();
   const int64_t N = v[0], F0 = v[1], F1 = v[2], F2 = v[3];
   if (x->scalar_type() != at::kComplexFloat || x->dim() != 2 || x->size(1) != N || !x->is_contiguous() || x->is_conj())
     return decline();
-  const int64_t want[5] = {2 * F0 * F0, 2 * F1 * F1, 2 * F2 * F2, 2 * F0 * F1 * F2, 2 * F1 * F2};
-  for (int i = 0; i < 5; ++i)
-    if (!(tab[i] = cuda_tensor(PyTuple_GET_ITEM(a[2], i))) || !vec_f32(tab[i], want[i])) return decline();
+  const int64_t want[2] = {2 * F0 * F1 * F2, 2 * F1 * F2};
+  for (int i = 0; i < 2; ++i)
+    if (!(tab[i] = cuda_tensor(PyTuple_GET_ITEM(a[2], 3 + i))) || !vec_f32(tab[i], want[i])) return decline();
   Tensor made;
   if (a[1] == Py_None) {
     made = at::empty(x->sizes(), x->options());
@@ -686,8 +686,8 @@ PyObject* fft(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Call c(*x);
   if (!c.ok()) return nullptr;
   const int s = without_gil([&] {
-    return ctb_fft(c.ctx, c.stream, x->data_ptr(), out->data_ptr(), tab[0]->data_ptr(), tab[1]->data_ptr(), tab[2]->data_ptr(),
-                   tab[3]->data_ptr(), tab[4]->data_ptr(), N, (int)F0, (int)F1, (int)F2, x->size(0), 1, (int)v[4]);
+    return ctb_fft_plan(c.ctx, c.stream, x->data_ptr(), out->data_ptr(), tab[0]->data_ptr(), tab[1]->data_ptr(), N, (int)F0,
+                        (int)F1, (int)F2, x->size(0), 1, (int)v[4]);
   });
   if (s != CTB_OK || a[1] != Py_None) return done(s, s == CTB_OK ? Py_NewRef(a[1]) : nullptr);
   return THPVariable_Wrap(std::move(made));

@@ -119,6 +119,10 @@ int ctb_transpose(ctb_ctx* ctx, void* stream, const void* x, void* y, int64_t m,
  * reference launch, batch % BS == 0) and D (2N % D == 0) are validated and otherwise advisory.  f32 FMA arithmetic. */
 int ctb_fft(ctb_ctx* ctx, void* stream, const void* x, void* y, const void* W0, const void* W1, const void* W2, const void* T0,
             const void* T1, int64_t N, int F0, int F1, int F2, int64_t batch, int BS, int D);
+/* The same transform for the tables of make_twiddles: the DFT matrices are the exact ones and are not passed (lines are
+ * transformed by butterflies instead of matrix products); T0 and T1 as above. */
+int ctb_fft_plan(ctb_ctx* ctx, void* stream, const void* x, void* y, const void* T0, const void* T1, int64_t N, int F0, int F1,
+                 int F2, int64_t batch, int BS, int D);
 
 /* ---- Host-level array operations (ct.Tiled) ---------------------------------- */
 /* ct.Tiled(C) .= f.(ct.Tiled(A), ...)                 src/broadcast.jl:19-23,92-165 (one fused kernel per expression)

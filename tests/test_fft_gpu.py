@@ -101,3 +101,18 @@ def test_fft_rejections(cuda):
     with pytest.raises(cuda.CtbError) as e:
         cuda.fft.fft_kernel(x3, torch.empty_like(x3), *t3, 27, 3, 3, 3, 1, 2)  # tile dimensions are powers of two
     assert e.value.status == lib.UNSUPPORTED_TILE
+
+
+@pytest.mark.parametrize("batch,factors", [(1, (1, 1, 1)), (3, (2, 1, 4)), (2, (2, 2, 2)), (300, (4, 4, 4)), (1000, (8, 4, 2)),
+                                           (5, (4, 8, 16)), (3, (32, 2, 8)), (256, (16, 16, 16)), (7, (32, 16, 16)),
+                                           (3, (16, 32, 8)), (150, (32, 32, 8)), (9, (2, 32, 32)), (301, (1, 16, 2))])
+def test_fft_plan_matches_oracle(cuda, batch, factors):
+    """The butterfly form that FftPlan takes: every factor, several items per CTA and a last CTA with fewer, the largest
+    sizes; and within a few rounding errors of the matrix form."""
+    import torch
+    d = inputs.fft(batch, factors, seed=5 + batch)
+    x = torch.from_numpy(d["input"]).cuda()
+    y = cuda.fft.FftPlan(factors, "cuda")(x).cpu().numpy()
+    assert ref.rel_fro(_planes(y), _planes(ref.fft(d["input"]))) <= 1e-6
+    m, _ = _run(cuda, d)
+    assert ref.rel_fro(_planes(y), _planes(m)) <= 1e-6
