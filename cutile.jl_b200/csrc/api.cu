@@ -163,6 +163,9 @@ int ctb_create(ctb_ctx** out, int device) {
   if (e == cudaSuccess) e = cudaMemset(c->sched_pool, 0, 2 * kSchedSlots * sizeof(int));
   if (e == cudaSuccess) e = cudaMalloc(&c->tickets, kStreamSlots * kTickets * sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(c->tickets, 0, kStreamSlots * kTickets * sizeof(int));
+  // one partial GEMM tile (128 x 256 f32) per SM: split-K products never have to grow the scratch
+  c->workspace_bytes = (size_t)c->sm_count * 128 * 256 * sizeof(float);
+  if (e == cudaSuccess) e = cudaMalloc(&c->workspace, c->workspace_bytes);
   if (e == cudaSuccess) e = cudaMalloc(&c->stream_pool, kStreamSlots * kStreamScratchBytes);
   if (e != cudaSuccess) {
     delete c->slot_lock;

@@ -8,18 +8,19 @@
 // truncation instead of the reference's round-to-nearest-even); f16 inputs run
 // as f16 MMAs with f32 accumulation and an f16 result.
 //
-// One persistent CTA per SM, 6 warps:
+// One persistent CTA per SM, 10 warps:
 //   warp 0     TMA producer: per k-block, A as 128-byte-wide boxes (M contiguous,
 //              "MN-major") and B as one box (K contiguous, "K-major"), 128B swizzle
 //              (32-byte-atom flavour for the tf32 A operand),
-//              into a ring of kStages shared-memory stages guarded by mbarriers;
-//   warp 1     MMA issuer: tcgen05.mma 128 x 256 x (32 bytes of K) from shared-memory
+//              into a ring of shared-memory stages guarded by mbarriers;
+//   warp 1     MMA issuer: tcgen05.mma 128 x bn x (32 bytes of K) from shared-memory
 //              descriptors into one of two 256-column TMEM accumulators;
 //              tcgen05.commit frees the stage / publishes the accumulator;
-//   warps 2-5  epilogue: tcgen05.ld the finished accumulator (lane = row m) and
-//              store C with coalesced 128-byte rows while the MMA warp already
-//              works on the next tile in the other accumulator.
-// Out-of-range parts of edge tiles are zero-filled by TMA and masked on store.
+//   warps 2-9  epilogue: tcgen05.ld the finished accumulator (lane = row m), stage
+//              32 x 32 blocks in shared memory and store them by TMA while the MMA
+//              warp already works on the next tile in the other accumulator.
+// Tiles are bn columns wide, bn a multiple of 32 up to 256 (choose()).
+// Out-of-range parts of edge tiles are zero-filled by TMA and clipped on store.
 //
 // Large problems run gemm_pair_kernel instead: the two CTAs of a 2-CTA cluster share one 256 x 256 tile
 // (tcgen05 cta_group::2, the counterpart of the reference's num_ctas = 2 hint on this architecture,
@@ -40,8 +41,10 @@ namespace {
 
 constexpr int kTileM = 128;
 constexpr int kTileN = 256;
-constexpr int kStages = 4;
-constexpr int kThreads = 192;
+constexpr int kMaxStages = 8;
+constexpr int kRingBytes = 192 * 1024;  // operand stages: as many of a tile's size as fit, at most kMaxStages
+constexpr int kEpiWarps = 8;  // two per TMEM lane quadrant, each takes every other block of 32 columns
+constexpr int kThreads = 64 + 32 * kEpiWarps;
 constexpr int kAccCols = kTileN;  // f32 accumulator columns per tile
 constexpr uint32_t kTmemCols = 512;
 
@@ -62,8 +65,6 @@ struct Cfg {
   static constexpr int A_BOXES = kTileM / CHUNK_M;
   static constexpr int A_BOX_BYTES = BK * 128;  // BK rows of 128 bytes
   static constexpr int A_BYTES = A_BOXES * A_BOX_BYTES;
-  static constexpr int B_BYTES = kTileN * 128;
-  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr uint32_t FMT = sizeof(T) == 4 ? FMT_TF32 : std::is_same<T, __nv_bfloat16>::value ? FMT_BF16 : FMT_F16;
   // An MN-major tf32 operand must use the 128-byte swizzle with 32-byte atoms
   // (4 K-rows per swizzle period); 16-bit types use the ordinary 128-byte swizzle.
@@ -74,13 +75,73 @@ struct Cfg {
 struct Params {
   int M, N, K, batch;
   long long ldc, strideC;
+  int bn;  // columns of a tile: a multiple of 32, at most kTileN
+  int stages, stage_bytes;  // per CTA; a stage is a multiple of 1024 bytes
   int tiles_m, tiles_n, num_tiles;
+  int c_tma;  // C starts on 16-byte boundaries: results leave by tiled bulk stores
   // Split-K (single-CTA kernel, few tiles): a work unit is (tile, split); split s takes the k-blocks
-  // [s * nk / splits, (s + 1) * nk / splits) and leaves its f32 accumulator tile in partial[unit] (column by column,
-  // 128 rows each); gemm_splitk_reduce_kernel adds the splits in ascending order.
+  // [s * nk / splits, (s + 1) * nk / splits) and leaves its f32 accumulator tile in partial[unit], as blocks of
+  // 32 columns x 32 rows (rows contiguous), four blocks per 32 columns; gemm_splitk_reduce_kernel adds the splits in
+  // ascending order.
   int splits;
   float* partial;
 };
+
+// Results on their way out.  An epilogue warp owns 32 rows (lane = row) of 32 columns at a time: it writes them to its
+// staging block in shared memory (a row of the block = 32 consecutive rows of a column of C, no bank conflicts)
+// and lane 0 sends the block off with one tiled bulk store, which clips at the edges of C; the next block's TMEM load runs
+// meanwhile.  Stored from registers, a tile of 128 x 256 cost about 10 us per CTA (12 x 1024 x 512 in bf16 with a single
+// k-block: 23.5 us), more than its main loop for K up to 2000.
+constexpr int kStageBlock = 32 * 32 * 4;             // bytes of a staging block (f32)
+constexpr int kEpiBytes = kEpiWarps * kStageBlock;
+template <typename T>
+__device__ __forceinline__ void stage_block(unsigned char* stage, const uint32_t (&r)[32], int lane) {
+#pragma unroll
+  for (int j = 0; j < 32; ++j) reinterpret_cast<T*>(stage)[j * 32 + lane] = from_f32<T>(__uint_as_float(r[j]));
+}
+// One 32 x 32 block of a tile: r[j] = element (row m0 + lane, column n0 + j) of batch b.
+template <typename T>
+__device__ __forceinline__ void store_block(const Params& p, const void* tmapC, T* C, unsigned char* stage,
+                                            const uint32_t (&r)[32], int m0, int n0, int b, float* partial, int lane) {
+  if (p.c_tma || partial) {
+    if (lane == 0) bulk_wait_read<0>();  // the previous store has read the block
+    __syncwarp();
+    if (partial) stage_block<float>(stage, r, lane);
+    else stage_block<T>(stage, r, lane);
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+      if (partial) bulk_s2g(partial, stage, kStageBlock);
+      else if (m0 < p.M && n0 < p.N) tma_store_3d(tmapC, stage, m0, n0, b);
+      bulk_commit();
+    }
+  } else {
+    const int m = m0 + lane;
+    T* crow = C + (long long)b * p.strideC + m;
+#pragma unroll
+    for (int j = 0; j < 32; ++j)
+      if (m < p.M && n0 + j < p.N) crow[(long long)(n0 + j) * p.ldc] = from_f32<T>(__uint_as_float(r[j]));
+    __syncwarp();
+  }
+}
+
+// A warp's share of a finished accumulator: every other block of 32 columns, the next one's TMEM load in flight while the
+// current one is stored.
+template <typename T>
+__device__ __forceinline__ void store_tile(const Params& p, const void* tmapC, T* C, unsigned char* stage, uint32_t taddr, int half,
+                                           int m0, int n0, int b, float* partial, int lane) {
+  const int nb = p.bn / 32;
+  uint32_t r[2][32];
+  if (half < nb) tmem_ld32(taddr + half * 32, r[0]);
+#pragma unroll
+  for (int i = 0; i < kTileN / 64; ++i) {
+    const int c = 2 * i + half;
+    if (c >= nb) break;  // uniform
+    tc_wait_ld();
+    if (c + 2 < nb) tmem_ld32(taddr + (c + 2) * 32, r[(i + 1) & 1]);
+    store_block<T>(p, tmapC, C, stage, r[i & 1], m0, n0 + c * 32, b, partial ? partial + c * 4096 : nullptr, lane);
+  }
+}
 
 __device__ __forceinline__ void tile_coords(const Params& p, int t, int& b, int& tm, int& tn) {
   const int per_batch = p.tiles_m * p.tiles_n;
@@ -97,24 +158,24 @@ __device__ __forceinline__ void tile_coords(const Params& p, int t, int& b, int&
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 1)
     gemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapB,
-                T* __restrict__ C, const Params p, int* status) {
+                const __grid_constant__ CUtensorMap tmapC, T* __restrict__ C, const Params p, int* status) {
   using G = Cfg<T>;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ __align__(8) uint64_t full[kStages], empty[kStages], acc_full[2], acc_empty[2];
+  __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], acc_full[2], acc_empty[2];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     abort_s = 0;
-    for (int s = 0; s < kStages; ++s) {
+    for (int s = 0; s < kMaxStages; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&acc_full[a], 1);
-      mbar_init(&acc_empty[a], 4);
+      mbar_init(&acc_empty[a], kEpiWarps);
     }
     fence_mbar_init();
     tma_prefetch_desc(&tmapA);
@@ -145,16 +206,16 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (int kb = kb_lo; kb < kb_hi; ++kb) {
         ok = CTB_WARP_WAIT(&empty[stage], phase ^ 1, status, DEV_TIMEOUT_SLOT, abort);
         if (!ok) break;
-        unsigned char* sa = smem + (size_t)stage * G::STAGE_BYTES;
+        unsigned char* sa = smem + stage * p.stage_bytes;
         if (elect_one()) {
-          mbar_expect_tx(&full[stage], G::STAGE_BYTES);
+          mbar_expect_tx(&full[stage], G::A_BYTES + p.bn * 128);
 #pragma unroll
           for (int j = 0; j < G::A_BOXES; ++j)
             tma_load_3d(sa + j * G::A_BOX_BYTES, &tmapA, tm * kTileM + j * G::CHUNK_M, kb * G::BK, b, &full[stage]);
-          tma_load_3d(sa + G::A_BYTES, &tmapB, kb * G::BK, tn * kTileN, b, &full[stage]);
+          tma_load_3d(sa + G::A_BYTES, &tmapB, kb * G::BK, tn * p.bn, b, &full[stage]);
         }
         __syncwarp();
-        if (++stage == kStages) {
+        if (++stage == p.stages) {
           stage = 0;
           phase ^= 1;
         }
@@ -163,7 +224,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else if (warp == 1) {
     // ---- MMA issuer: the whole warp walks the loop, one elected lane issues
-    constexpr uint32_t idesc = make_idesc(G::FMT, kTileM, kTileN, /*A MN-major*/ 1, /*B K-major*/ 0);
+    const uint32_t idesc = make_idesc(G::FMT, kTileM, (uint32_t)p.bn, /*A MN-major*/ 1, /*B K-major*/ 0);
     int stage = 0;
     uint32_t phase = 0;
     int it = 0;
@@ -179,7 +240,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         ok = CTB_WARP_WAIT(&full[stage], phase, status, DEV_TIMEOUT_TMA, abort);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t sa = smem_u32(smem + (size_t)stage * G::STAGE_BYTES);
+        const uint32_t sa = smem_u32(smem + stage * p.stage_bytes);
         const uint32_t sb = sa + G::A_BYTES;
         if (elect_one()) {
 #pragma unroll
@@ -194,7 +255,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           tc_commit(&empty[stage]);
         }
         __syncwarp();
-        if (++stage == kStages) {
+        if (++stage == p.stages) {
           stage = 0;
           phase ^= 1;
         }
@@ -205,6 +266,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else {
     const int sub = warp & 3;  // TMEM lanes [32*sub, 32*sub+32) belong to this warp
+    const int half = (warp - 2) >> 2;
+    unsigned char* epi = smem + kRingBytes + (warp - 2) * kStageBlock;
     int it = 0;
     for (int u = blockIdx.x; u < units; u += gridDim.x, ++it) {
       const int acc = it & 1;
@@ -214,35 +277,14 @@ __global__ void __launch_bounds__(kThreads, 1)
       bool ok = CTB_WARP_WAIT(&acc_full[acc], acc_phase, status, DEV_TIMEOUT_MMA, abort);
       if (!ok) break;
       tc_fence_after();
-      const int m = tm * kTileM + sub * 32 + lane;
-      T* crow = C + (long long)b * p.strideC + m;
-      float* prow = p.partial + (long long)u * (kTileM * kTileN) + sub * 32 + lane;
-      const uint32_t taddr = tmem_base + acc * kAccCols + ((uint32_t)(sub * 32) << 16);
-#pragma unroll 1
-      for (int c = 0; c < kTileN / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld32(taddr + c * 32, r);
-        tc_wait_ld();
-        const int n0 = tn * kTileN + c * 32;
-        if (p.splits > 1) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) prow[(c * 32 + j) * kTileM] = __uint_as_float(r[j]);
-        } else if (m < p.M) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            if (n0 + j < p.N) {
-              if constexpr (sizeof(T) == 4)
-                crow[(long long)(n0 + j) * p.ldc] = __uint_as_float(r[j]);
-              else
-                crow[(long long)(n0 + j) * p.ldc] = from_f32<T>(__uint_as_float(r[j]));
-            }
-          }
-        }
-      }
+      const int m0 = tm * kTileM + sub * 32;
+      store_tile<T>(p, &tmapC, C, epi, tmem_base + acc * kAccCols + ((uint32_t)(sub * 32) << 16), half, m0, tn * p.bn, b,
+                    p.splits > 1 ? p.partial + (long long)u * (kTileM * kTileN) + sub * 1024 : nullptr, lane);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[acc]);
     }
+    bulk_wait<0>();  // this warp's stores are complete
   }
   tc_fence_before();
   __syncthreads();
@@ -253,19 +295,20 @@ __global__ void __launch_bounds__(kThreads, 1)
 }
 
 // Adds the splits of every tile in ascending order and writes C.  A thread takes four consecutive rows of a column
-// (16-byte loads; a warp covers 128 rows = one column of the tile) and requests eight splits at a time.
+// (16-byte loads; eight lanes cover a column's 32 rows of a block) and requests eight splits at a time.
 template <typename T>
 __global__ void __launch_bounds__(256)
     gemm_splitk_reduce_kernel(const float* __restrict__ partial, T* __restrict__ C, const Params p) {
   grid_dependency_sync();
   constexpr int kTileElems = kTileM * kTileN;
-  const long long total = (long long)p.num_tiles * (kTileElems / 4);
+  const int per_tile = kTileM * p.bn / 4;
+  const long long total = (long long)p.num_tiles * per_tile;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int t = (int)(i / (kTileElems / 4)), e = (int)(i - (long long)t * (kTileElems / 4)) * 4;
-    const int col = e / kTileM, row = e - col * kTileM;
+    const int t = (int)(i / per_tile), e = (int)(i - (long long)t * per_tile) * 4;
+    const int block = e >> 10, col = (block >> 2) * 32 + ((e >> 5) & 31), row = (block & 3) * 32 + (e & 31);
     int b, tm, tn;
     tile_coords(p, t, b, tm, tn);
-    const int m = tm * kTileM + row, n = tn * kTileN + col;
+    const int m = tm * kTileM + row, n = tn * p.bn + col;
     if (m >= p.M || n >= p.N) continue;
     const float4* src = reinterpret_cast<const float4*>(partial + (long long)t * p.splits * kTileElems + e);
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -284,14 +327,17 @@ __global__ void __launch_bounds__(256)
     }
     T* dst = C + (long long)b * p.strideC + (long long)n * p.ldc + m;
     const float o[4] = {acc.x, acc.y, acc.z, acc.w};
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      if (m + q < p.M) {
-        if constexpr (sizeof(T) == 4)
-          dst[q] = o[q];
-        else
-          dst[q] = from_f32<T>(o[q]);
+    if (p.c_tma && m + 3 < p.M) {  // C is aligned and m a multiple of four
+      if constexpr (sizeof(T) == 4) {
+        *reinterpret_cast<float4*>(dst) = acc;
+      } else {
+        T h[4] = {from_f32<T>(o[0]), from_f32<T>(o[1]), from_f32<T>(o[2]), from_f32<T>(o[3])};
+        *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(h);
       }
+    } else {
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (m + q < p.M) dst[q] = from_f32<T>(o[q]);
     }
   }
 }
@@ -302,26 +348,16 @@ __global__ void __launch_bounds__(256)
 // columns in its TMEM.  Barriers: full[] lives in rank 0 and counts the bytes of both CTAs' loads; empty[] and
 // acc_full[] exist in both CTAs and are arrived by rank 0's multicast commits; acc_empty[] lives in rank 0 and is
 // arrived by the epilogue warps of both CTAs.
-constexpr int kPairStages = 6;
 constexpr int kPairTileM = 256;
-
-template <typename T>
-struct PairCfg {
-  using G = Cfg<T>;
-  static constexpr int B_ROWS = kTileN / 2;          // columns of the tile held by one CTA
-  static constexpr int B_BYTES = B_ROWS * 128;
-  static constexpr int STAGE_BYTES = G::A_BYTES + B_BYTES;  // per CTA
-};
 
 template <typename T>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     gemm_pair_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapB,
-                     T* __restrict__ C, const Params p, int* status) {
+                     const __grid_constant__ CUtensorMap tmapC, T* __restrict__ C, const Params p, int* status) {
   using G = Cfg<T>;
-  using P = PairCfg<T>;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ __align__(8) uint64_t full[kPairStages], empty[kPairStages], acc_full[2], acc_empty[2];
+  __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], acc_full[2], acc_empty[2];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s;
 
@@ -330,13 +366,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
   if (threadIdx.x == 0) {
     abort_s = 0;
-    for (int s = 0; s < kPairStages; ++s) {
+    for (int s = 0; s < kMaxStages; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&acc_full[a], 1);
-      mbar_init(&acc_empty[a], 8);  // four epilogue warps in each of the two CTAs
+      mbar_init(&acc_empty[a], 2 * kEpiWarps);  // the epilogue warps of both CTAs
     }
     fence_mbar_init();
     tma_prefetch_desc(&tmapA);
@@ -363,14 +399,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     for (int t = pair; t < p.num_tiles; t += num_pairs) {
       int b, tm, tn;
       tile_coords(p, t, b, tm, tn);
-      const int m0 = tm * kPairTileM + (int)rank * kTileM, n0 = tn * kTileN + (int)rank * P::B_ROWS;
+      const int m0 = tm * kPairTileM + (int)rank * kTileM, n0 = tn * p.bn + (int)rank * (p.bn / 2);
       bool ok = true;
       for (int kb = 0; kb < nk; ++kb) {
         ok = CTB_WARP_WAIT(&empty[stage], phase ^ 1, status, DEV_TIMEOUT_SLOT, abort);
         if (!ok) break;
-        unsigned char* sa = smem + (size_t)stage * P::STAGE_BYTES;
+        unsigned char* sa = smem + stage * p.stage_bytes;
         if (elect_one()) {
-          if (rank == 0) mbar_expect_tx(&full[stage], 2 * P::STAGE_BYTES);
+          if (rank == 0) mbar_expect_tx(&full[stage], 2 * (G::A_BYTES + p.bn / 2 * 128));
           const uint32_t bar = map_to_cta(&full[stage], 0);
 #pragma unroll
           for (int j = 0; j < G::A_BOXES; ++j)
@@ -378,7 +414,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
           tma_load_3d_pair(sa + G::A_BYTES, &tmapB, kb * G::BK, n0, b, bar);
         }
         __syncwarp();
-        if (++stage == kPairStages) {
+        if (++stage == p.stages) {
           stage = 0;
           phase ^= 1;
         }
@@ -388,7 +424,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   } else if (warp == 1) {
     if (rank == 0) {
       // ---- MMA issuer (rank 0 only): one instruction drives the tensor cores of both SMs
-      constexpr uint32_t idesc = make_idesc(G::FMT, kPairTileM, kTileN, /*A MN-major*/ 1, /*B K-major*/ 0);
+      const uint32_t idesc = make_idesc(G::FMT, kPairTileM, (uint32_t)p.bn, /*A MN-major*/ 1, /*B K-major*/ 0);
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;
@@ -403,7 +439,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
           ok = CTB_WARP_WAIT(&full[stage], phase, status, DEV_TIMEOUT_TMA, abort);
           if (!ok) break;
           tc_fence_after();
-          const uint32_t sa = smem_u32(smem + (size_t)stage * P::STAGE_BYTES);
+          const uint32_t sa = smem_u32(smem + stage * p.stage_bytes);
           const uint32_t sb = sa + G::A_BYTES;
           if (elect_one()) {
 #pragma unroll
@@ -418,7 +454,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             tc_commit_pair(&empty[stage], 3);
           }
           __syncwarp();
-          if (++stage == kPairStages) {
+          if (++stage == p.stages) {
             stage = 0;
             phase ^= 1;
           }
@@ -430,6 +466,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     }
   } else {
     const int sub = warp & 3;  // TMEM lanes [32*sub, 32*sub+32) belong to this warp
+    const int half = (warp - 2) >> 2;
+    unsigned char* epi = smem + kRingBytes + (warp - 2) * kStageBlock;
     int it = 0;
     for (int t = pair; t < p.num_tiles; t += num_pairs, ++it) {
       const int acc = it & 1;
@@ -439,31 +477,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       bool ok = CTB_WARP_WAIT(&acc_full[acc], acc_phase, status, DEV_TIMEOUT_MMA, abort);
       if (!ok) break;
       tc_fence_after();
-      const int m = tm * kPairTileM + (int)rank * kTileM + sub * 32 + lane;
-      T* crow = C + (long long)b * p.strideC + m;
-      const uint32_t taddr = tmem_base + acc * kAccCols + ((uint32_t)(sub * 32) << 16);
-#pragma unroll 1
-      for (int c = 0; c < kTileN / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld32(taddr + c * 32, r);
-        tc_wait_ld();
-        const int n0 = tn * kTileN + c * 32;
-        if (m < p.M) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            if (n0 + j < p.N) {
-              if constexpr (sizeof(T) == 4)
-                crow[(long long)(n0 + j) * p.ldc] = __uint_as_float(r[j]);
-              else
-                crow[(long long)(n0 + j) * p.ldc] = from_f32<T>(__uint_as_float(r[j]));
-            }
-          }
-        }
-      }
+      const int m0 = tm * kPairTileM + (int)rank * kTileM + sub * 32;
+      store_tile<T>(p, &tmapC, C, epi, tmem_base + acc * kAccCols + ((uint32_t)(sub * 32) << 16), half, m0, tn * p.bn, b,
+                    nullptr, lane);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(map_to_cta(&acc_empty[acc], 0));
     }
+    bulk_wait<0>();  // this warp's stores are complete
   }
   // Neither CTA may leave (or free its TMEM) while the other can still read its shared memory, write its TMEM or
   // signal its barriers: every thread of both CTAs meets here, also after an abort.
@@ -495,7 +516,8 @@ int pair_clusters(ctb_ctx* ctx, size_t smem) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
-    cudaError_t e = cudaOccupancyMaxActiveClusters(&n, gemm_pair_kernel<T>, &cfg);
+    cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, gemm_pair_kernel<T>, &cfg);
     c = (e == cudaSuccess && n > 0) ? n : -1;
     if (e != cudaSuccess) (void)cudaGetLastError();
   }
@@ -518,6 +540,43 @@ __global__ void __launch_bounds__(256) tf32_round_kernel(const uint4* __restrict
     out[i] = v;
   }
   if (blockIdx.x == 0 && (int)threadIdx.x < tail) out_tail[threadIdx.x] = rne(in_tail[threadIdx.x]);
+}
+
+constexpr size_t kSmem = (size_t)kRingBytes + kEpiBytes + 1024;
+
+// Kernel, tile width and number of splits of K, by an estimate of the clocks of the slowest CTA.  Per k-block (128 bytes of
+// K) a tile of bn columns costs 2 bn clocks of tensor core per SM or, if that is more, the arrival of its operands (16 KB
+// of A and bn or, in a pair, bn / 2 rows of 128 bytes of B, at about 55 bytes per clock and SM when all are loading: measured); a tile's
+// results need about 1000 + 4 bn clocks and hide behind the next tile's main loop, so a CTA pays per tile the larger of the two;
+// filling the pipeline and the last tile's results come on top.  A split adds its partial tiles (written and read back
+// through the L2) and a second kernel.  Narrow tiles fill the SMs and waste little of a ragged N, wide ones load less.
+struct Choice {
+  bool pair;
+  int bn, splits;
+  int tile_m() const { return pair ? kPairTileM : kTileM; }
+};
+Choice choose(const ctb_ctx* ctx, long long M, long long N, long long nk, long long batch, int clusters) {
+  Choice best = {false, kTileN, 1};
+  double best_cost = 1e300;
+  for (int pair = 0; pair <= (clusters > 0 && M > kTileM ? 1 : 0); ++pair)
+    for (int bn = 32; bn <= kTileN; bn += 32) {
+      if (bn > 32 && bn - 32 >= N) break;
+      const long long tm = pair ? kPairTileM : kTileM;
+      const long long tiles = ((M + tm - 1) / tm) * ((N + bn - 1) / bn) * batch, slots = pair ? clusters : ctx->sm_count;
+      const double per_kb = std::max(2.0 * bn, (16384.0 + (pair ? 64.0 : 128.0) * bn) / 55.0);
+      for (int splits = 1; splits <= 16; ++splits) {
+        if (splits > 1 && (pair || nk / splits < 4 || tiles * splits > slots)) break;
+        const long long rounds = (tiles * splits + slots - 1) / slots;
+        const double kloop = (double)((nk + splits - 1) / splits) * per_kb, epi = 1000.0 + 4.0 * bn;
+        double cost = rounds * std::max(kloop, epi) + epi + 1500.0;
+        if (splits > 1) cost += 6000.0 + (double)tiles * splits * kTileM * bn * 8.0 / slots / 40.0;
+        if (cost < best_cost * 0.98) {
+          best_cost = cost;
+          best = {pair != 0, bn, splits};
+        }
+      }
+    }
+  return best;
 }
 
 template <typename T>
@@ -553,7 +612,9 @@ int launch(ctb_ctx* ctx, cudaStream_t st, const T* A, const T* B, T* C, int M, i
     A = reinterpret_cast<const T*>(A2);
     B = reinterpret_cast<const T*>(B2);
   }
-  CUtensorMap ta, tb;
+  const int nk = (K + G::BK - 1) / G::BK;
+  const Choice ch = choose(ctx, M, N, nk, batch, pair_clusters<T>(ctx, kSmem));
+  CUtensorMap ta, tb, tc;
   {
     // A memory: [batch][K][M], M contiguous
     uint64_t dims[3] = {(uint64_t)M, (uint64_t)K, (uint64_t)batch};
@@ -564,70 +625,58 @@ int launch(ctb_ctx* ctx, cudaStream_t st, const T* A, const T* B, T* C, int M, i
     if (r) return r;
   }
   {
-    // B memory: [batch][N][K], K contiguous
+    // B memory: [batch][N][K], K contiguous; a CTA of a pair loads half of the tile's columns
     uint64_t dims[3] = {(uint64_t)K, (uint64_t)N, (uint64_t)batch};
     uint64_t str[2] = {(uint64_t)ldb * G::ES, (uint64_t)(batch > 1 ? sB : ldb * (long long)N) * G::ES};
-    uint32_t box[3] = {(uint32_t)G::BK, (uint32_t)kTileN, 1};
+    uint32_t box[3] = {(uint32_t)G::BK, (uint32_t)(ch.pair ? ch.bn / 2 : ch.bn), 1};
     int r = make_tmap(&tb, dt, 3, B, dims, str, box);
     if (r) return r;
   }
   Params p;
   p.M = M; p.N = N; p.K = K; p.batch = batch;
   p.ldc = ldc; p.strideC = sC;
-  {
-    // CTA pairs when there are enough 256 x 256 tiles to occupy at least half of the SM pairs
-    const long long pairs = (long long)((M + kPairTileM - 1) / kPairTileM) * ((N + kTileN - 1) / kTileN) * batch;
-    if (M >= kPairTileM && N >= kTileN && pairs * 4 >= ctx->sm_count && pairs <= INT32_MAX) {
-      using P = PairCfg<T>;
-      CUtensorMap tb2;
-      uint64_t dims[3] = {(uint64_t)K, (uint64_t)N, (uint64_t)batch};
-      uint64_t str[2] = {(uint64_t)ldb * G::ES, (uint64_t)(batch > 1 ? sB : ldb * (long long)N) * G::ES};
-      uint32_t box[3] = {(uint32_t)G::BK, (uint32_t)P::B_ROWS, 1};
-      int r = make_tmap(&tb2, dt, 3, B, dims, str, box);
-      if (r) return r;
-      p.tiles_m = (M + kPairTileM - 1) / kPairTileM;
-      p.tiles_n = (N + kTileN - 1) / kTileN;
-      p.num_tiles = (int)pairs;
-      p.splits = 1;
-      p.partial = nullptr;
-      const size_t smem = (size_t)kPairStages * P::STAGE_BYTES + 1024;
-      auto k = gemm_pair_kernel<T>;
-      cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return cuda_fail(e, "ctb_gemm: shared memory opt-in");
-      const int clusters = pair_clusters<T>(ctx, smem);
-      if (clusters > 0) {
-        const int grid = 2 * (int)std::min<long long>(pairs, clusters);
-        launch_kernel(k, grid, kThreads, smem, st, 0, ta, tb2, C, p, ctx->dev_status);
-        CTB_CHECK_LAUNCH("ctb_gemm launch");
-        return CTB_OK;
-      }
-    }
-  }
-  p.tiles_m = (M + kTileM - 1) / kTileM;
-  p.tiles_n = (N + kTileN - 1) / kTileN;
+  p.bn = ch.bn;
+  p.stage_bytes = G::A_BYTES + (ch.pair ? ch.bn / 2 : ch.bn) * 128;
+  p.stages = std::min(kMaxStages, kRingBytes / p.stage_bytes);
+  p.tiles_m = (M + ch.tile_m() - 1) / ch.tile_m();
+  p.tiles_n = (N + ch.bn - 1) / ch.bn;
   const long long nt = (long long)p.tiles_m * p.tiles_n * batch;
-  if (nt > INT32_MAX) return fail(CTB_UNSUPPORTED, "ctb_gemm: too many tiles");
+  if (nt * ch.splits > INT32_MAX) return fail(CTB_UNSUPPORTED, "ctb_gemm: too many tiles");
   p.num_tiles = (int)nt;
-  // Few tiles and a long K (one rank's share of a batch-sharded problem): split K over the idle SMs, at least four
-  // k-blocks per split.
-  const int nk = (K + G::BK - 1) / G::BK;
-  p.splits = (int)std::max<long long>(1, std::min<long long>(std::min<long long>(ctx->sm_count / nt, nk / 4), 16));
+  p.splits = ch.splits;
   p.partial = nullptr;
+  p.c_tma = (uintptr_t)C % 16 == 0 && ldc * G::ES % 16 == 0 && (batch == 1 || sC * G::ES % 16 == 0);
+  tc = ta;  // not used when C is not aligned
+  if (p.c_tma) {
+    uint64_t dims[3] = {(uint64_t)M, (uint64_t)N, (uint64_t)batch};
+    uint64_t str[2] = {(uint64_t)ldc * G::ES, (uint64_t)(batch > 1 ? sC : ldc * (long long)N) * G::ES};
+    uint32_t box[3] = {32, 32, 1};
+    int r = make_tmap(&tc, dt, 3, C, dims, str, box, CU_TENSOR_MAP_SWIZZLE_NONE);
+    if (r) return r;
+  }
+  if (ch.pair) {
+    auto k = gemm_pair_kernel<T>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+    if (e != cudaSuccess) return cuda_fail(e, "ctb_gemm: shared memory opt-in");
+    const int grid = 2 * (int)std::min<long long>(nt, pair_clusters<T>(ctx, kSmem));
+    launch_kernel(k, grid, kThreads, kSmem, st, 0, ta, tb, tc, C, p, ctx->dev_status);
+    CTB_CHECK_LAUNCH("ctb_gemm launch");
+    return CTB_OK;
+  }
   if (p.splits > 1) {
     void* ws = nullptr;
     int r = workspace(ctx, ws_used + (size_t)nt * p.splits * kTileM * kTileN * sizeof(float), &ws, st);
     if (r) return r;
     p.partial = reinterpret_cast<float*>(static_cast<unsigned char*>(ws) + ws_used);
   }
-  const size_t smem = (size_t)kStages * G::STAGE_BYTES + 1024;
   auto k = gemm_kernel<T>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
   if (e != cudaSuccess) return cuda_fail(e, "ctb_gemm: shared memory opt-in");
   const int grid = (int)std::min<long long>(nt * p.splits, ctx->sm_count);
-  launch_kernel(k, grid, kThreads, smem, st, 0, ta, tb, C, p, ctx->dev_status);
+  launch_kernel(k, grid, kThreads, kSmem, st, 0, ta, tb, tc, C, p, ctx->dev_status);
   CTB_CHECK_LAUNCH("ctb_gemm launch");
   if (p.splits > 1) {
-    const long long work = nt * kTileM * kTileN / 4;
+    const long long work = nt * kTileM * p.bn / 4;
     const int rgrid = (int)std::min<long long>((work + 255) / 256, (long long)ctx->sm_count * 8);
     launch_kernel(gemm_splitk_reduce_kernel<T>, rgrid, 256, 0, st, 0, p.partial, C, p);
     CTB_CHECK_LAUNCH("ctb_gemm split-K reduction launch");

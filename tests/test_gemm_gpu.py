@@ -146,3 +146,26 @@ def test_gemm_bf16(cuda, M, K, N, batch):
         C2 = torch.empty(N, M, device="cuda", dtype=torch.bfloat16)
         cuda.matmul.matmul_kernel(A[0], B[0], C2, 64, 64, 64)
         assert torch.equal(C2, C[0])
+
+
+@pytest.mark.parametrize("M,N,K,batch", [(4, 1, 4, 1), (128, 31, 64, 1), (132, 33, 36, 2), (256, 160, 520, 3), (1000, 515, 776, 2),
+                                         (520, 97, 2048, 1), (96, 669, 1232, 3), (2056, 225, 64, 1), (1288, 1000, 200, 5)])
+@pytest.mark.parametrize("dtype", [np.float32, np.float16])
+@pytest.mark.parametrize("c_shift,c_pad", [(0, 0), (1, 0), (0, 3)])
+def test_gemm_tile_widths_and_result_alignment(cuda, M, N, K, batch, dtype, c_shift, c_pad):
+    """Every tile width the host may pick (ragged M, N and K, split K), results that leave by tiled stores and results whose
+    start or leading dimension is off the 16-byte alignment; nothing is written outside the result."""
+    import torch
+    M, K = (M, K) if dtype == np.float32 else ((M + 7) // 8 * 8, (K + 7) // 8 * 8)
+    d = inputs.batched_gemm(M, K, N, batch, seed=3, dtype=dtype)
+    A, B = torch.from_numpy(d["A"]).cuda(), torch.from_numpy(d["B"]).cuda()
+    ld = M + c_pad
+    flat = torch.full((c_shift + batch * N * ld + 8,), 7.0, device="cuda", dtype=A.dtype)
+    C = flat[c_shift:c_shift + batch * N * ld].view(batch, N, ld)[:, :, :M]
+    cuda.batchmatmul.batch_matmul_kernel(A, B, C, 128, 128, 64)
+    want = ref.batched_gemm(d["A"], d["B"])
+    for b in range(batch):
+        assert ref.rel_fro(C[b].float().cpu().numpy(), want[b]) <= (TOL_TF32 if dtype == np.float32 else TOL_F16)
+    C.fill_(7.0)
+    assert (flat == 7.0).all()
+    cuda.check_device_status(0)
