@@ -55,6 +55,9 @@ size_t moe_experts_rows_workspace(int64_t R, int64_t I, int64_t E_local, int til
 int moe_experts_rows(ctb_ctx* ctx, cudaStream_t st, const void* rows, int64_t ld_rows, const int32_t* ids,
                      const void* gates, int64_t R, int64_t H, int64_t I, int64_t E_local, const void* w1_local,
                      const void* w2_local, int tile_m, void* C, int64_t ldc, void* const* c_peer, int64_t c_split);
+// Scratch of ctb_moe_ffn (moe_ffn.cu) and the check of its tile constants (moe.cu).
+size_t moe_ffn_workspace(int64_t T, int64_t H, int64_t I, int64_t E, int64_t topk);
+int moe_check_tile(const char* who, int tile_m, int tile_n, int tile_k);
 constexpr int kSchedSlots = 256;
 constexpr int kTickets = 4096, kStreamSlots = 32;
 constexpr size_t kStreamScratchBytes = 1280 * 1024;

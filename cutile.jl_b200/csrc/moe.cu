@@ -472,8 +472,7 @@ struct GemmParams {
   const int* expert_ids;  // 1-based expert per block (0 = unused block)
   const int* num_blocks_dev;
   int num_blocks_host;    // >= 0: use this instead of *num_blocks_dev
-  const __half* topk_w;   // routing weights, may be null
-  int w_tokens, w_topk;   // w_tokens == 0: topk_w is flat, indexed by id-1; else (T, topk) column-major
+  const __half* topk_w;   // routing weights, flat by id - 1; may be null
   int replicas, mul_weight;
   int K, N;               // N = output rows per expert (SwiGLU: the weight tensor holds 2N rows)
   int E, tile_m, total;
@@ -786,8 +785,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         if (id < 1 || id > p.total) id = 0;
         float wt = 1.f;
         if (p.mul_weight && id) {
-          const int f = id - 1;
-          wt = __half2float(p.topk_w[p.w_tokens ? (long long)(f % p.w_topk) * p.w_tokens + f / p.w_topk : f]);
+          wt = __half2float(p.topk_w[id - 1]);
         }
         const int col = id ? id - 1 : 0;
         __half* crow = p.c_split ? p.c_peer[col / p.c_split] + (long long)(col % p.c_split) * p.ldc
@@ -1000,7 +998,7 @@ __global__ void moe_ep_barrier_kernel(const EpFlags f, uint32_t* epoch, int worl
 int launch_gemm(ctb_ctx* ctx, cudaStream_t st, int epi, const __half* A, long long lda, int a_rows, const __half* W,
                 int K, int wrows, int N, int E, const __half* topk_w, const int* sorted_ids, const int* expert_ids,
                 const int* nblocks_dev, int nblocks_host, int max_blocks, int replicas, int mul_weight, int tile_m,
-                int total, void* C, long long ldc, int w_tokens = 0, int w_topk = 1, void* const* c_peer = nullptr,
+                int total, void* C, long long ldc, void* const* c_peer = nullptr,
                 int c_split = 0, int expect_blocks = -1) {
   if (expect_blocks < 0) expect_blocks = max_blocks;
   CUtensorMap tw;
@@ -1014,7 +1012,6 @@ int launch_gemm(ctb_ctx* ctx, cudaStream_t st, int epi, const __half* A, long lo
   p.sorted_ids = sorted_ids; p.expert_ids = expert_ids;
   p.num_blocks_dev = nblocks_dev; p.num_blocks_host = nblocks_host;
   p.topk_w = topk_w; p.replicas = replicas; p.mul_weight = mul_weight;
-  p.w_tokens = w_tokens; p.w_topk = w_topk;
   p.K = K; p.N = N; p.E = E; p.tile_m = tile_m; p.total = total;
   p.C = (__half*)C; p.ldc = ldc;
   p.c_vec = (ldc % 8 == 0 && (uintptr_t)C % 16 == 0) ? 1 : 0;
@@ -1083,17 +1080,17 @@ int launch_align(ctb_ctx* ctx, cudaStream_t st, const void* topk_ids, int ids_bi
   return CTB_OK;
 }
 
-int check_tile(const char* who, int tile_m, int tile_n, int tile_k) {
+}  // namespace
+
+namespace ctb_internal {
+
+int moe_check_tile(const char* who, int tile_m, int tile_n, int tile_k) {
   if (!is_pow2(tile_m) || !is_pow2(tile_n) || !is_pow2(tile_k))
     return fail(CTB_UNSUPPORTED_TILE, "%s: tile sizes must be powers of two (got %d,%d,%d)", who, tile_m, tile_n, tile_k);
   if (tile_m < 16 || tile_m > kMaxTileM)
     return fail(CTB_UNSUPPORTED_TILE, "%s: tile_m must be between 16 and %d (got %d)", who, kMaxTileM, tile_m);
   return CTB_OK;
 }
-
-}  // namespace
-
-namespace ctb_internal {
 
 size_t moe_experts_rows_workspace(int64_t R, int64_t I, int64_t E_local, int tile_m) {
   const int64_t blocks_cap = ctb_moe_max_blocks(R, 1, E_local, tile_m);
@@ -1136,7 +1133,7 @@ int moe_experts_rows(ctb_ctx* ctx, cudaStream_t st, const void* rows, int64_t ld
                   act, I);
   if (r) return r;
   return launch_gemm(ctx, st, EPI_F16, act, I, (int)R, (const __half*)w2_local, (int)I, (int)H, (int)H, (int)E_local,
-                     (const __half*)gates, s_tok, s_exp, s_nb, -1, blocks_cap, 1, 1, tile_m, (int)R, C, ldc, 0, 1, c_peer,
+                     (const __half*)gates, s_tok, s_exp, s_nb, -1, blocks_cap, 1, 1, tile_m, (int)R, C, ldc, c_peer,
                      (int)c_split, expect_blocks);
 }
 
@@ -1214,7 +1211,7 @@ int ctb_moe_fused_gemm(ctb_ctx* ctx, void* stream, const void* A, const void* B,
                        int64_t K, int64_t N, int64_t E, int64_t a_cols, int64_t c_cols, int num_token_replicas,
                        int mul_routed_weight, int tile_m, int tile_n, int tile_k) {
   CTB_CHECK_CTX(ctx);
-  int r = check_tile("ctb_moe_fused_gemm", tile_m, tile_n, tile_k);
+  int r = moe_check_tile("ctb_moe_fused_gemm", tile_m, tile_n, tile_k);
   if (r) return r;
   if (K <= 0 || N <= 0 || E <= 0 || a_cols <= 0 || c_cols <= 0 || num_token_replicas <= 0 || num_slots_padded < 0 ||
       num_slots_padded % tile_m)
@@ -1243,55 +1240,6 @@ int ctb_moe_silu_and_mul(ctb_ctx* ctx, void* stream, const void* A, const void* 
   launch_kernel(moe_silu_and_mul_kernel, (unsigned)((tot + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream), 0,
       (const __half*)A, (const __half*)B, (__half*)C, (int)n, cols, lda, ldb, ldc);
   CTB_CHECK_LAUNCH("ctb_moe_silu_and_mul launch");
-  return CTB_OK;
-}
-
-int ctb_moe_ffn(ctb_ctx* ctx, void* stream, const void* hidden, const void* w1, const void* w2,
-                const void* topk_weights, const void* topk_ids, int ids_bits, void* out, int64_t T, int64_t H,
-                int64_t I, int64_t E, int64_t topk, int tile_m, int tile_n, int tile_k) {
-  CTB_CHECK_CTX(ctx);
-  int r = check_tile("ctb_moe_ffn", tile_m, tile_n, tile_k);
-  if (r) return r;
-  if (T <= 0 || H <= 0 || I <= 0 || E <= 0 || topk <= 0 || T * topk > (1 << 24))
-    return fail(CTB_BAD_ARG, "ctb_moe_ffn: bad shape");
-  if (E > kMaxExperts) return fail(CTB_UNSUPPORTED, "ctb_moe_ffn: at most %d experts", kMaxExperts);
-  if (H % 8 || I % 8) return fail(CTB_BAD_ALIGN, "ctb_moe_ffn: hidden and intermediate sizes must be multiples of 8");
-  if (ids_bits != 32 && ids_bits != 64) return fail(CTB_BAD_ARG, "ctb_moe_ffn: ids_bits must be 32 or 64");
-  CTB_CHECK_DEV(hidden); CTB_CHECK_DEV(w1); CTB_CHECK_DEV(w2); CTB_CHECK_DEV(topk_weights); CTB_CHECK_DEV(topk_ids);
-  CTB_CHECK_DEV(out);
-  if ((uintptr_t)hidden % 16 || (uintptr_t)w1 % 16 || (uintptr_t)w2 % 16 || (uintptr_t)out % 16)
-    return fail(CTB_BAD_ALIGN, "ctb_moe_ffn: 16-byte alignment of hidden, w1, w2");
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int total = (int)(T * topk);
-  const int cap = (int)ctb_moe_max_blocks(T, topk, E, tile_m);
-  // scratch: sorted ids | expert ids | block count | activations (I, total) f16 | per-slot outputs (H, total) f16
-  auto up = [](size_t v) { return (v + 255) & ~size_t(255); };
-  const size_t o_tok = 0, o_exp = up((size_t)cap * tile_m * 4), o_nb = o_exp + up((size_t)cap * 4), o_act = o_nb + 256,
-               o_slots = o_act + up((size_t)total * I * 2), bytes = o_slots + up((size_t)total * H * 2);
-  void* ws;
-  r = workspace(ctx, bytes, &ws, st);
-  if (r) return r;
-  unsigned char* w = (unsigned char*)ws;
-  int* s_tok = (int*)(w + o_tok);
-  int* s_exp = (int*)(w + o_exp);
-  int* s_nb = (int*)(w + o_nb);
-  __half* act = (__half*)(w + o_act);
-  __half* slots = (__half*)(w + o_slots);
-  r = launch_align(ctx, st, topk_ids, ids_bits, (int)T, (int)topk, (int)E, tile_m, s_tok, s_exp, s_nb, cap, 0, w1,
-                   warm_bytes(T * topk, 2 * I * H * E * 2));
-  if (r) return r;
-  // gate/up projection with the SwiGLU epilogue: act(:, id) = silu(Wg x) * (Wu x)
-  r = launch_gemm(ctx, st, EPI_SWIGLU, (const __half*)hidden, H, (int)T, (const __half*)w1, (int)H, (int)(2 * I),
-                  (int)I, (int)E, nullptr, s_tok, s_exp, s_nb, -1, cap, (int)topk, 0, tile_m, total, act, I);
-  if (r) return r;
-  // down projection scaled by the routing weight, one f16 column per slot (the reference's cache3)
-  r = launch_gemm(ctx, st, EPI_F16, act, I, total, (const __half*)w2, (int)I, (int)H, (int)H, (int)E,
-                  (const __half*)topk_weights, s_tok, s_exp, s_nb, -1, cap, 1, 1, tile_m, total, slots, H, (int)T,
-                  (int)topk);
-  if (r) return r;
-  const long long n8 = T * (H / 8);
-  launch_kernel(moe_combine_kernel, (unsigned)((n8 + 255) / 256), 256, 0, st, 0, slots, (__half*)out, (int)T, (int)H, (int)topk);
-  CTB_CHECK_LAUNCH("ctb_moe_ffn combine launch");
   return CTB_OK;
 }
 
@@ -1359,7 +1307,7 @@ int ctb_moe_ep_experts(ctb_ctx* ctx, void* stream, const ctb_ep_buffers* bufs, c
   CTB_CHECK_CTX(ctx);
   int r = check_ep("ctb_moe_ep_experts", bufs);
   if (r) return r;
-  r = check_tile("ctb_moe_ep_experts", tile_m, tile_n, tile_k);
+  r = moe_check_tile("ctb_moe_ep_experts", tile_m, tile_n, tile_k);
   if (r) return r;
   const long long R = cap * bufs->world;  // columns of the receive buffers
   if (cap <= 0) return fail(CTB_BAD_ARG, "ctb_moe_ep_experts: bad shape");

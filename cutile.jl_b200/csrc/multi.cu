@@ -768,13 +768,11 @@ int ctb_moe_ffn_ep_group(ctb_group* g, ctb_ep* const* eps, void* const* streams,
 
 // ------------------------------------------------------------------ scratch sizing
 size_t ctb_workspace_bytes(int op, const int64_t* dims, int ndims) {
-  auto up = [](size_t v) { return (v + 255) & ~size_t(255); };
   if (!dims) return 0;
   if (op == CTB_OP_MOE_FFN && ndims >= 6) {  // T, H, I, E, topk, tile_m
     const int64_t T = dims[0], H = dims[1], I = dims[2], E = dims[3], topk = dims[4], tile_m = dims[5];
     if (T <= 0 || H <= 0 || I <= 0 || E <= 0 || topk <= 0 || tile_m <= 0) return 0;
-    const size_t total = (size_t)(T * topk), cap = (size_t)ctb_moe_max_blocks(T, topk, E, (int)tile_m);
-    return up(cap * tile_m * 4) + up(cap * 4) + 256 + up(total * I * 2) + up(total * H * 2);
+    return moe_ffn_workspace(T, H, I, E, topk);
   }
   if (op == CTB_OP_MOE_EP && ndims >= 6) {  // T_local, H, I, E_local, topk, tile_m, [world]
     const int64_t world = ndims >= 7 ? dims[6] : 1;

@@ -159,3 +159,42 @@ def test_moe_rejections(cuda):
     with pytest.raises(cuda.CtbError) as e:
         cuda.moe.cutile_moe(X, w1, w2[:, :, :32].contiguous(), wd, idd, 128, 128, 64)
     assert e.value.status == lib.BAD_ARG
+
+
+# slots per expert around the block sizes: one slot, 16, 17, up to 256 (one block), 257 and more (two, three blocks), one
+# expert with everything, empty experts, row counts off the 128- and 256-row tiles, a reduction length off the k-block,
+# more slots than a CTA of the sort counts itself
+@pytest.mark.parametrize("T,H,E,I,topk,skew", [(1, 64, 4, 64, 1, False), (1, 512, 64, 1024, 8, False), (17, 128, 3, 200, 1, True),
+                                               (257, 264, 2, 72, 1, True), (300, 512, 5, 136, 2, False), (700, 72, 1, 320, 1, False),
+                                               (640, 512, 16, 256, 4, True), (3, 1024, 256, 128, 8, False), (5000, 64, 7, 64, 4, False)])
+@pytest.mark.parametrize("ids64", [False, True])
+def test_cutile_moe_block_shapes(cuda, T, H, E, I, topk, skew, ids64):
+    import torch
+    d = inputs.moe(tokens=T, hidden=H, experts=E, inter=I, topk=topk, seed=6)
+    ids, w = random_routing(T, E, topk, seed=T)
+    if skew:  # most tokens choose the first expert (first choices only: a token's choices stay different)
+        first = np.where(np.arange(T) % 8 < 7, 1, ids[0])
+        clash = (ids == 1) & (np.arange(topk)[:, None] > 0) & (first == 1)
+        ids = np.where(clash, ids[0][None, :], ids)
+        ids[0] = first
+    X, w1, w2 = dev(d, "X", "w1", "w2")
+    args = (X, w1, w2, torch.from_numpy(w).cuda(), torch.from_numpy(ids if ids64 else ids.astype(np.int32)).cuda(), 128, 128, 64)
+    out, again = cuda.moe.cutile_moe(*args), cuda.moe.cutile_moe(*args)
+    assert torch.equal(out, again)
+    want = ref.moe_ffn(d["X"], d["w1"], d["w2"], w, ids)
+    assert ref.rel_fro(out.cpu().numpy(), want) <= TOL
+    cuda.check_device_status(0)
+
+
+def test_cutile_moe_bad_expert_id_is_reported(cuda):
+    import torch
+    d = inputs.moe(tokens=40, hidden=64, experts=4, inter=64, topk=2, seed=1)
+    ids, w = random_routing(40, 4, 2, 0)
+    ids[1, 7] = 5
+    X, w1, w2 = dev(d, "X", "w1", "w2")
+    cuda.moe.cutile_moe(X, w1, w2, torch.from_numpy(w).cuda(), torch.from_numpy(ids).cuda(), 128, 128, 64)
+    with pytest.raises(cuda.CtbError):
+        cuda.check_device_status(0)
+    ids[1, 7] = 1 + ids[0, 7] % 4
+    out = cuda.moe.cutile_moe(X, w1, w2, torch.from_numpy(w).cuda(), torch.from_numpy(ids).cuda(), 128, 128, 64)
+    assert ref.rel_fro(out.cpu().numpy(), ref.moe_ffn(d["X"], d["w1"], d["w2"], w, ids)) <= TOL
