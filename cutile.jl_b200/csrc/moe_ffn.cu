@@ -29,8 +29,12 @@ constexpr int kMaxExperts = 256;
 constexpr int kMaxBlockSlots = 256;  // MMA N
 
 // ------------------------------------------------------------------ sort and gather
-constexpr int kSortThreads = 512, kSortWarps = kSortThreads / 32, kSortCtas = 148;
+constexpr int kSortThreads = 512, kSortCtas = 148;
+constexpr int kSortThreadsEarly = 256;  // registers for a CTA of the gate/up kernel remain
 constexpr int kSortLocal = 16384;  // up to this many slots every CTA counts all of them itself
+// Up to this many slots the gate/up kernel starts beside the sort: it streams 28 MB of weights while the sort runs.  With more
+// slots the weights bound it less than the rows, whose copies take 18 us instead of 6 beside that stream (8192 slots).
+constexpr int kEarlySlots = 2048;
 
 struct Block {  // slots of one expert that one GEMM item takes
   int expert, row0, n, pad;
@@ -44,10 +48,7 @@ struct SortParams {
   Block* table;
   int* num_blocks;  // [0] blocks, [1] slots of the largest
   const int* counts;  // [kSortCtas][E + 1]: slots per expert in every CTA's chunk, then 1 if an id is out of range; or null
-  const unsigned char* warm;  // gate/up weights, for the L2 (null: not)
-  long long warm_expert;      // bytes of one expert's gate or up rows
-  int warm_tile, warm_mtiles;  // bytes of the 64 rows that a CTA of an item streams; row tiles per block
-  int T, topk, E, vecs, total, chunk;
+  int T, topk, E, vecs, total, chunk, early;
   int* status;
 };
 
@@ -81,45 +82,111 @@ __global__ void __launch_bounds__(kSortThreads)
   for (int e = threadIdx.x; e <= E; e += kSortThreads) counts[blockIdx.x * (E + 1) + e] = cnt[e];
 }
 
+// Adds every slot of expert e to tot[e] and, if `base` is given, those with a flat index below `lo` to base[e] (both in
+// shared memory); true if an id is out of range.  All threads of the CTA.
+template <typename IdT>
+__device__ __forceinline__ bool count_slots(const IdT* __restrict__ ids, int T, int topk, int E, int lo, int* tot, int* base) {
+  bool bad = false;
+  const int step = blockDim.x, total = T * topk;
+  for (int m0 = threadIdx.x; m0 < total; m0 += 8 * step) {
+    long long e[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) e[q] = m0 + q * step < total ? (long long)ids[m0 + q * step] - 1 : 0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int m = m0 + q * step;
+      if (m >= total) continue;
+      if (e[q] < 0 || e[q] >= E) {
+        bad = true;
+        continue;
+      }
+      atomicAdd(&tot[e[q]], 1);
+      if (base) {
+        const int slot = m / T;
+        if ((m - slot * T) * topk + slot < lo) atomicAdd(&base[e[q]], 1);
+      }
+    }
+  }
+  return bad;
+}
+// First row and first block of every expert from its number of slots (one warp; first[e] is added to).
+__device__ __forceinline__ void scan_experts(const int* tot, int E, int* first, int* bstart, int lane) {
+  int rows = 0, blocks = 0;
+  for (int e0 = 0; e0 < E; e0 += 32) {
+    const int e = e0 + lane, c = e < E ? tot[e] : 0, padded = (c + 15) & ~15, nb = (c + kMaxBlockSlots - 1) / kMaxBlockSlots;
+    int r = padded, b = nb;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int rr = __shfl_up_sync(0xffffffffu, r, o), bb = __shfl_up_sync(0xffffffffu, b, o);
+      if (lane >= o) { r += rr; b += bb; }
+    }
+    if (e < E) {
+      first[e] += rows + r - padded;
+      bstart[e] = blocks + b - nb;
+    }
+    rows += __shfl_sync(0xffffffffu, r, 31);
+    blocks += __shfl_sync(0xffffffffu, b, 31);
+  }
+  if (lane == 0) bstart[E] = blocks;
+}
+// The blocks of expert e (c slots in nb blocks from row `row0` on); returns the slots of the largest.
+__device__ __forceinline__ int write_blocks(Block* table, int e, int c, int nb, int row0) {
+  const int size = ((c + nb - 1) / nb + 15) & ~15;
+  for (int k = 0; k < nb; ++k) table[k] = {e, row0 + k * size, max((min(size, c - k * size) + 15) & ~15, 16), 0};
+  return size;
+}
+
 // CTA c places the flat slots [c * chunk, (c + 1) * chunk) and copies their rows.  Nothing is exchanged between the CTAs:
 // each counts all slots (or reads the chunks' counts) and so knows where every expert's rows and its own share of them
 // start; the order inside an expert is the flat slot order, as in moe_align_tile_size (examples/moe.jl:142-183).
-// A chain of latencies (7.9 us at 512 slots by itself).  While the rows are copied the L2 fetches the weights that the
-// GEMM's CTAs stream first.
-template <typename IdT>
-__global__ void __launch_bounds__(kSortThreads) moe_sort_gather_kernel(const IdT* __restrict__ ids, const SortParams p) {
+// A chain of latencies: 2.3 us to the counts, 4.3 to the table, then the rows.  The gate/up kernel does not wait for it: it
+// is set up beside this one, counts the slots itself and streams weights meanwhile.
+template <typename IdT, int kThreads>
+__global__ void __launch_bounds__(kThreads) moe_sort_gather_kernel(const IdT* __restrict__ ids, const SortParams p) {
+  constexpr int kWarps = kThreads / 32;
   extern __shared__ int sort_smem[];  // small, so that the next kernel's CTAs fit beside
-  __shared__ int spos[kSortThreads];
+  __shared__ int spos[kThreads];
   __shared__ int bad, nmax;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, E = p.E, cta = blockIdx.x;
-  int *tot = sort_smem, *base = tot + E, *wcount = base + E, *bstart = wcount + kSortWarps * E;  // [E], [E], [warps][E], [E + 1]
-  for (int e = tid; e < E; e += kSortThreads) tot[e] = base[e] = 0;
+  int *tot = sort_smem, *base = tot + E, *wcount = base + E, *bstart = wcount + kWarps * E;  // [E], [E], [warps][E], [E + 1]
+  for (int e = tid; e < E; e += kThreads) tot[e] = base[e] = 0;
   if (tid == 0) bad = nmax = 0;
   __syncthreads();
-  grid_dependency_sync();
+  grid_dependency_wait();
+  if (p.early) grid_dependency_launch();  // the gate/up kernel reads the ids as well
   const int lo = min(p.total, cta * p.chunk), hi = min(p.total, lo + p.chunk);
-  // ---- slots per expert: all of them, and those before this CTA's
-  if (!p.counts) {
-    for (int slot = 0; slot < p.topk; ++slot) {
-      const IdT* col = ids + (long long)slot * p.T;
-      for (int t0 = tid; t0 < p.T; t0 += 8 * kSortThreads) {
-        long long e[8];
+  // Which slots and rows are this CTA's is known from the start: the first are on their way before anything else is asked
+  // for, ahead of the gate/up kernel's weights (behind them they took 5 us longer).
+  uint4 v[8];
+  auto load_rows = [&](int b0, int x0) {
+    const int n = min(kThreads, hi - b0) * p.vecs;
 #pragma unroll
-        for (int q = 0; q < 8; ++q) e[q] = t0 + q * kSortThreads < p.T ? (long long)col[t0 + q * kSortThreads] - 1 : 0;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          if (t0 + q * kSortThreads >= p.T) continue;
-          if (e[q] < 0 || e[q] >= E) {
-            bad = 1;
-          } else {
-            atomicAdd(&tot[e[q]], 1);
-            if ((t0 + q * kSortThreads) * p.topk + slot < lo) atomicAdd(&base[e[q]], 1);
-          }
-        }
+    for (int q = 0; q < 8; ++q) {
+      const int x = x0 + q * kThreads;
+      if (x < n) {
+        const int r = x / p.vecs;
+        v[q] = __ldg(p.X + (long long)((b0 + r) / p.topk) * p.vecs + (x - r * p.vecs));
       }
     }
+  };
+  int e;
+  float weight;
+  auto load_slot = [&](int i) {
+    e = -1;
+    weight = 0.f;
+    if (i < hi) {
+      const int tok = i / p.topk, slot = i - tok * p.topk;
+      e = (int)ids[(long long)slot * p.T + tok] - 1;
+      weight = __half2float(p.topk_w[(long long)slot * p.T + tok]);
+    }
+  };
+  load_slot(lo + tid);
+  load_rows(lo, tid);
+  // ---- slots per expert: all of them, and those before this CTA's
+  if (!p.counts) {
+    if (count_slots(ids, p.T, p.topk, E, lo, tot, base)) bad = 1;
   } else {
-    for (int e = tid; e <= E; e += kSortThreads) {
+    for (int e = tid; e <= E; e += kThreads) {
       int all = 0, before = 0;
 #pragma unroll 8
       for (int c = 0; c < kSortCtas; ++c) {
@@ -142,58 +209,16 @@ __global__ void __launch_bounds__(kSortThreads) moe_sort_gather_kernel(const IdT
       p.num_blocks[0] = 0;
       p.num_blocks[1] = 16;
     }
-    for (int i = lo + tid; i < hi; i += kSortThreads) p.pos_of[i] = 0;
+    for (int i = lo + tid; i < hi; i += kThreads) p.pos_of[i] = 0;
     return;
   }
   // ---- first row and first block of every expert
-  if (warp == 0) {
-    int rows = 0, blocks = 0;
-    for (int e0 = 0; e0 < E; e0 += 32) {
-      const int e = e0 + lane, c = e < E ? tot[e] : 0, padded = (c + 15) & ~15, nb = (c + kMaxBlockSlots - 1) / kMaxBlockSlots;
-      int r = padded, b = nb;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int rr = __shfl_up_sync(0xffffffffu, r, o), bb = __shfl_up_sync(0xffffffffu, b, o);
-        if (lane >= o) { r += rr; b += bb; }
-      }
-      if (e < E) {
-        base[e] += rows + r - padded;
-        bstart[e] = blocks + b - nb;
-      }
-      rows += __shfl_sync(0xffffffffu, r, 31);
-      blocks += __shfl_sync(0xffffffffu, b, 31);
-    }
-    if (lane == 0) bstart[E] = blocks;
-  }
+  if (warp == 0) scan_experts(tot, E, base, bstart, lane);
   __syncthreads();
-  // ---- weights that this CTA's part of the first gate/up item streams
-  if (p.warm) {
-    const int item = cta >> 1, b = item / p.warm_mtiles;
-    if (b < bstart[E]) {
-      int l = 0, h = E - 1;  // last expert whose first block is <= b
-      while (l < h) {
-        const int mid = (l + h + 1) >> 1;
-        if (bstart[mid] <= b) l = mid;
-        else h = mid - 1;
-      }
-      const long long first = ((long long)(item - b * p.warm_mtiles) * 2 + (cta & 1)) * p.warm_tile;
-      const unsigned char* gate = p.warm + (long long)l * 2 * p.warm_expert + first;
-      for (int x = tid * 128; x < min((long long)p.warm_tile, p.warm_expert - first); x += kSortThreads * 128) {
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(gate + x) : "memory");
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(gate + p.warm_expert + x) : "memory");
-      }
-    }
-  }
   if (cta == 0) {  // the block table; this CTA has no slots before it: base is the experts' first row
-    for (int e = tid; e < E; e += kSortThreads) {
-      const int c = tot[e], nb = bstart[e + 1] - bstart[e];
-      if (!nb) continue;
-      const int size = ((c + nb - 1) / nb + 15) & ~15;
-      for (int k = 0; k < nb; ++k) {
-        const int n = (min(size, c - k * size) + 15) & ~15;
-        p.table[bstart[e] + k] = {e, base[e] + k * size, max(n, 16), 0};
-      }
-      atomicMax(&nmax, size);
+    for (int e = tid; e < E; e += kThreads) {
+      const int nb = bstart[e + 1] - bstart[e];
+      if (nb) atomicMax(&nmax, write_blocks(p.table + bstart[e], e, tot[e], nb, base[e]));
     }
     __syncthreads();
     if (tid == 0) {
@@ -202,19 +227,14 @@ __global__ void __launch_bounds__(kSortThreads) moe_sort_gather_kernel(const IdT
     }
     __syncthreads();
   }
-  // ---- this CTA's slots, kSortThreads at a time: stable positions, then the rows
+  // ---- this CTA's slots, kThreads at a time: stable positions, then the rows
   int ebits = 1;
   while ((1 << ebits) < E) ++ebits;
-  for (int b0 = lo; b0 < hi; b0 += kSortThreads) {
-    for (int i = tid; i < kSortWarps * E; i += kSortThreads) wcount[i] = 0;
+  for (int b0 = lo; b0 < hi; b0 += kThreads) {
+    for (int i = tid; i < kWarps * E; i += kThreads) wcount[i] = 0;
     __syncthreads();
     const int i = b0 + tid;
-    int e = -1, tok = 0, slot = 0;
-    if (i < hi) {
-      tok = i / p.topk;
-      slot = i - tok * p.topk;
-      e = (int)ids[(long long)slot * p.T + tok] - 1;
-    }
+    if (b0 != lo) load_slot(i);
     const unsigned grp = same_value(e, ebits);
     const int rank = __popc(grp & ((1u << lane) - 1));
     if (e >= 0 && rank == 0) wcount[warp * E + e] = __popc(grp);
@@ -222,7 +242,7 @@ __global__ void __launch_bounds__(kSortThreads) moe_sort_gather_kernel(const IdT
     if (tid < E) {
       int run = base[tid];
 #pragma unroll
-      for (int w = 0; w < kSortWarps; ++w) {
+      for (int w = 0; w < kWarps; ++w) {
         const int c = wcount[w * E + tid];
         wcount[w * E + tid] = run;
         run += c;
@@ -234,25 +254,20 @@ __global__ void __launch_bounds__(kSortThreads) moe_sort_gather_kernel(const IdT
       const int pos = wcount[warp * E + e] + rank;
       spos[tid] = pos;
       p.pos_of[i] = pos;
-      p.wts[pos] = __half2float(p.topk_w[(long long)slot * p.T + tok]);
+      p.wts[pos] = weight;
     }
     __syncthreads();
-    const int n = min(kSortThreads, hi - b0) * p.vecs;
-    for (int x0 = tid; x0 < n; x0 += 8 * kSortThreads) {
-      uint4 v[8];
-      long long to[8];
+    const int n = min(kThreads, hi - b0) * p.vecs;
+    for (int x0 = tid; x0 < n; x0 += 8 * kThreads) {
+      if (b0 != lo || x0 != tid) load_rows(b0, x0);
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
-        const int x = x0 + q * kSortThreads;
+        const int x = x0 + q * kThreads;
         if (x < n) {
-          const int r = x / p.vecs, c = x - r * p.vecs;
-          v[q] = __ldg(p.X + (long long)((b0 + r) / p.topk) * p.vecs + c);
-          to[q] = (long long)spos[r] * p.vecs + c;
+          const int r = x / p.vecs;
+          p.xs[(long long)spos[r] * p.vecs + (x - r * p.vecs)] = v[q];
         }
       }
-#pragma unroll
-      for (int q = 0; q < 8; ++q)
-        if (x0 + q * kSortThreads < n) p.xs[to[q]] = v[q];
     }
     __syncthreads();
   }
@@ -265,11 +280,12 @@ constexpr int kMaxStages = 12;
 constexpr int kRingBytes = 192 * 1024;
 constexpr int kEpiWarps = 8;                 // two per TMEM lane quadrant, each takes every other block of 32 slots
 constexpr int kGemmThreads = 96 + 32 * kEpiWarps;
-constexpr int kSlotBlock = 16 * 32 * 2;      // 16 slots x 32 rows, f16: a tiled store
-constexpr int kXchgBytes = 32 * 32 * 4;      // values on their way to the other warp of a team
-// Results: gate/up one staging block per warp and an exchange buffer per team, down two staging blocks per warp.  Together
-// with the ring little enough that the CTAs fit beside those of the sort and are set up when it ends.
-constexpr size_t kGemmSmem = 1024 + kRingBytes + kEpiWarps * kSlotBlock + 4 * kXchgBytes;
+constexpr int kTileBytes = 32 * 64 * 2;      // staged results: 32 slots x 64 rows, f16, 128-byte swizzle
+// Warps that share a staging tile: gate/up the four quadrants (a CTA's 64 outputs), down two of them; two tiles each.
+template <bool UP>
+constexpr int kGroupThreads = UP ? 128 : 64;
+template <bool UP>
+constexpr size_t kGemmSmem = 1024 + kRingBytes + (size_t)(UP ? 2 : 4) * 2 * kTileBytes;
 
 // The sorted rows with a box for every number of slots that a CTA may hold (8, 16, ... 128): one copy per k-block.
 struct SlotMaps {
@@ -280,29 +296,49 @@ struct PairParams {
   const int* num_blocks;
   const float* wts;
   int mtiles, K, rows;  // rows: output rows of the projection
+  const void* ids;      // gate/up with at most kEarlySlots slots: the kernel builds its own table (null: it reads the sort's)
+  int ids_bits, T, topk, E;
 };
 
-// Barriers between the two warps of a team (64 threads).
-__device__ __forceinline__ void team_sync(int id) { asm volatile("barrier.cta.sync %0, 64;" ::"r"(id) : "memory"); }
-__device__ __forceinline__ bool team_all(int id, bool v) {
+// Barriers of `threads` threads (whole warps).
+__device__ __forceinline__ void group_sync(int id, int threads) { asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ bool group_all(int id, int threads, bool v) {
   uint32_t r;
-  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.cta.red.and.pred q, %2, 64, p;\n\tselp.b32 %0, 1, 0, q;\n\t}"
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.cta.red.and.pred q, %2, %3, p;\n\tselp.b32 %0, 1, 0, q;\n\t}"
                : "=r"(r)
-               : "r"((uint32_t)v), "r"(id)
+               : "r"((uint32_t)v), "r"(id), "r"(threads)
                : "memory");
   return r != 0;
 }
+// TMEM -> registers, 16 lanes x 32 columns: thread t holds, of the columns 8q + 2 (t mod 4) and the next, lane t / 4 in
+// r[4q], r[4q + 1] and lane t / 4 + 8 in r[4q + 2], r[4q + 3].
+__device__ __forceinline__ void tmem_ld_16x32(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+// Four 8 x 8 matrices of 16-bit elements (register k of thread t: row t / 4, columns 2 (t mod 4) and the next of matrix k),
+// stored transposed: lane l gives the address of column l mod 8 of matrix l / 8.
+__device__ __forceinline__ void stmatrix4_trans(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d)
+               : "memory");
+}
 
 // One item = 256 weight rows x one block of slots, on a 2-CTA cluster.  CTA rank r holds 128 of the rows in its shared
-// memory (gate/up: 64 gate rows and the 64 up rows that belong to them) and half of the block's slots per k-block, and the
-// accumulators of its rows (TMEM lanes) x all slots (columns).  Roles and barriers as in gemm_pair_kernel (gemm.cu): warp 0
-// loads weights, warp 2 slots, warp 1 of rank 0 issues the MMAs of both SMs, warps 3-10 store; two accumulators of 256
-// columns.
-// UP = true (gate/up): out = silu(gate) * up.  The gate values of a row are in lanes 0-63, the up values in lanes 64-127:
-// the warp that holds the gate values of 32 rows and the one that holds the up values (a team) swap halves of 32 slots
-// through shared memory and finish 16 slots each.  UP = false (down): out = value * routing weight.
-// The down projection does not wait for the gate/up kernel before it fills its pipeline with weights: the block table is
-// older, only the activations are new.
+// memory and half of the block's slots per k-block, and the accumulators of its rows (TMEM lanes) x all slots (columns).
+// Roles and barriers as in gemm_pair_kernel (gemm.cu): warp 0 loads weights, warp 2 slots, warp 1 of rank 0 issues the MMAs
+// of both SMs, warps 3-10 store; two accumulators of 256 columns.
+// UP = true (gate/up): out = silu(gate) * up.  A CTA's rows are 64 gate and the 64 up rows that belong to them, in groups of
+// eight in turn (a five-dimensional copy), so that a thread that reads two TMEM lanes eight apart has both values of an
+// output.  UP = false (down): out = value * routing weight.  Results go through shared memory by transposing matrix stores
+// (8 of 128 bytes per 32 slots and 16 outputs; element by element they were 48 of 64 bytes and shared the shared memory with
+// the operands: with 4096 tokens the results cost 27 of 168 us that way, now 14 of 156).
+// Neither projection waits for the kernel before it ahead of its first weights: the block table is older than it (down) or
+// computed from the ids (gate/up); only the rows are new.
+// With few slots several k-blocks make a stage: the waits and issues of a k-block take about 0.25 us, more than its weights.
 template <bool UP>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
     moe_pair_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ SlotMaps tmX,
@@ -311,7 +347,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], acc_full[2], acc_empty[2];
   __shared__ uint32_t tmem_base_s;
-  __shared__ int abort_s;
+  __shared__ int abort_s, nmax_s;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
@@ -338,21 +374,45 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
   cluster_arrive();  // the peer's barriers exist before anything is signalled on them
   cluster_wait();
   tc_fence_after();
-  if (UP) {  // the next kernel on the stream may start its weights once everything before this one is complete
-    grid_dependency_wait();
-    grid_dependency_launch();
-  } else {
-    grid_dependency_launch();
-  }
+  if (!UP) grid_dependency_launch();
   const uint32_t tmem_base = tmem_base_s;
   volatile int* abort = &abort_s;
-  const int items = __ldcg(p.num_blocks) * p.mtiles;
-  const int stage_bytes = kABytes + __ldcg(p.num_blocks + 1) / 2 * 128;
+  const Block* table = p.table;
+  int blocks, nmax;
+  if (UP && p.ids) {  // count the slots as the sort does
+    int* tot = reinterpret_cast<int*>(smem_raw + kGemmSmem<UP>);
+    int *first = tot + p.E, *bstart = first + p.E;
+    Block* own = reinterpret_cast<Block*>(smem_raw + kGemmSmem<UP> + (((3 * p.E + 1) * 4 + 15) & ~15));
+    for (int e = threadIdx.x; e < p.E; e += kGemmThreads) tot[e] = first[e] = 0;
+    if (threadIdx.x == 0) nmax_s = 16;
+    __syncthreads();
+    const bool bad = p.ids_bits == 32 ? count_slots(static_cast<const int*>(p.ids), p.T, p.topk, p.E, 0, tot, (int*)nullptr)
+                                      : count_slots(static_cast<const long long*>(p.ids), p.T, p.topk, p.E, 0, tot, (int*)nullptr);
+    const bool none = __syncthreads_or(bad);
+    if (warp == 0) scan_experts(tot, p.E, first, bstart, lane);
+    __syncthreads();
+    for (int e = threadIdx.x; e < p.E; e += kGemmThreads) {
+      const int nb = bstart[e + 1] - bstart[e];
+      if (nb) atomicMax(&nmax_s, write_blocks(own + bstart[e], e, tot[e], nb, first[e]));
+    }
+    __syncthreads();
+    table = own;
+    blocks = none ? 0 : bstart[p.E];
+    nmax = nmax_s;
+  } else {
+    if (UP) grid_dependency_wait();
+    blocks = __ldcg(p.num_blocks);
+    nmax = __ldcg(p.num_blocks + 1);
+  }
+  const int items = blocks * p.mtiles;
+  const int per_stage = nmax <= 64 ? 2 : 1;  // k-blocks of a stage
+  const int stage_bytes = per_stage * (kABytes + nmax / 2 * 128);
   const int stages = min(kMaxStages, kRingBytes / stage_bytes);
   const int nk = (p.K + kBK - 1) / kBK;
   auto block_of = [&](int it) -> Block {
-    const int4 v = it < items ? __ldcg(reinterpret_cast<const int4*>(p.table + it / p.mtiles)) : make_int4(0, 0, 16, 0);
-    return {v.x, v.y, v.z, 0};
+    if (it >= items) return {0, 0, 16, 0};
+    const Block* b = table + it / p.mtiles;
+    return {b->expert, b->row0, b->n, 0};
   };
 
   if (warp == 0 || warp == 2) {
@@ -360,7 +420,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
     // full barrier.  One copy per warp and k-block and little beside it: with both in one warp, six copies (boxes of 64
     // weight rows and 32 or 8 slots) and a division per k-block the issue took about 800 clocks per k-block and bound the
     // kernel whatever the operands' size.
-    if (!UP && warp == 2) grid_dependency_wait();  // the activations
+    if (warp == 2) {
+      if (lane == 0) tma_prefetch_desc(&tmX.m[block_of(pair).n / 16 - 1]);
+      grid_dependency_wait();  // the rows
+      if (UP) grid_dependency_launch();  // the down projection may start its weights
+    }
     const uint32_t bars = map_to_cta(&full[0], 0);
     int stage = 0;
     uint32_t phase = 0;
@@ -369,18 +433,23 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
       const Block b = block_of(it);
       const int half = b.n / 2;
       const uint32_t bytes = 2 * (kABytes + half * 128);
-      const int wrow = ((it % p.mtiles) * 2 + (int)rank) * (UP ? 64 : 128), xrow = b.row0 + (int)rank * half;
+      const int wrow = ((it % p.mtiles) * 2 + (int)rank) * (UP ? 8 : 128), xrow = b.row0 + (int)rank * half;
       const CUtensorMap* map = &tmX.m[b.n / 16 - 1];
-      for (int kb = 0; kb < nk; ++kb) {
+      for (int kb = 0; kb < nk; kb += per_stage) {
         ok = CTB_WARP_WAIT(&empty[stage], phase ^ 1, status, DEV_TIMEOUT_SLOT, abort);
         if (!ok) break;
+        const int live = min(per_stage, nk - kb);
         if (elect_one()) {
           unsigned char* dst = smem + stage * stage_bytes;
           if (warp == 0) {
-            if (rank == 0) mbar_expect_tx(&full[stage], bytes);
-            tma_load_4d_pair(dst, &tmW, kb * kBK, wrow, 0, b.expert, bars + stage * 8);
+            if (rank == 0) mbar_expect_tx(&full[stage], live * bytes);
+            for (int q = 0; q < live; ++q) {
+              if (UP) tma_load_5d_pair(dst + q * kABytes, &tmW, (kb + q) * kBK, 0, 0, wrow, b.expert, bars + stage * 8);
+              else tma_load_3d_pair(dst + q * kABytes, &tmW, (kb + q) * kBK, wrow, b.expert, bars + stage * 8);
+            }
           } else {
-            tma_load_3d_pair(dst + kABytes, map, kb * kBK, xrow, 0, bars + stage * 8);
+            for (int q = 0; q < live; ++q)
+              tma_load_3d_pair(dst + per_stage * kABytes + q * (nmax / 2 * 128), map, (kb + q) * kBK, xrow, 0, bars + stage * 8);
           }
         }
         __syncwarp();
@@ -405,16 +474,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
         tc_fence_after();
         const uint32_t d = tmem_base + acc * 256;
         bool ok = true;
-        for (int kb = 0; kb < nk; ++kb) {
+        for (int kb = 0; kb < nk; kb += per_stage) {
           ok = CTB_WARP_WAIT(&full[stage], phase, status, DEV_TIMEOUT_TMA, abort);
           if (!ok) break;
           tc_fence_after();
-          const uint32_t sa = smem_u32(smem + stage * stage_bytes), sb = sa + kABytes;
+          const int live = min(per_stage, nk - kb);
+          const uint32_t sa0 = smem_u32(smem + stage * stage_bytes), sb0 = sa0 + per_stage * kABytes;
           if (elect_one()) {
+            for (int q = 0; q < live; ++q) {
+              const uint32_t sa = sa0 + q * kABytes, sb = sb0 + q * (nmax / 2 * 128);
 #pragma unroll
-            for (int k = 0; k < kBK / 16; ++k)
-              mma_f16_ss_pair(d, make_sdesc_sw128(sa + k * 32, 0, 1024), make_sdesc_sw128(sb + k * 32, 0, 1024), idesc,
-                              (kb | k) != 0);
+              for (int k = 0; k < kBK / 16; ++k)
+                mma_f16_ss_pair(d, make_sdesc_sw128(sa + k * 32, 0, 1024), make_sdesc_sw128(sb + k * 32, 0, 1024), idesc,
+                                (kb | q | k) != 0);
+            }
             tc_commit_pair(&empty[stage], 3);
           }
           __syncwarp();
@@ -429,14 +502,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
       }
     }
   } else {
-    // ---- epilogue: lane = output row (UP: gate or up row), 32 slots at a time -> this warp's staging block -> tiled stores
+    // ---- epilogue: 32 slots at a time -> staging tile [slot][64 outputs] of the group -> tiled store
     const int sub = warp & 3, half = (warp - 3) >> 2;  // TMEM lanes [32 sub, 32 sub + 32), every other block of slots
-    unsigned char* epi = smem + kRingBytes;
-    __half* out = reinterpret_cast<__half*>(epi + (warp - 3) * (UP ? kSlotBlock : 2 * kSlotBlock));
-    const int team = half * 2 + (sub & 1);
-    const bool gate = sub < 2;
-    // UP: [16 slots][32 lanes] to the up warp, then the same to the gate warp
-    float* xchg = reinterpret_cast<float*>(epi + kEpiWarps * kSlotBlock + team * kXchgBytes) + lane;
+    const int group = UP ? half : half * 2 + (sub >> 1);
+    const bool issuer = (UP ? sub == 3 : (sub & 1)) && lane == 0;
+    const uint32_t tiles = smem_u32(smem + kRingBytes + group * 2 * kTileBytes);
+    uint32_t flip = 0;  // the staging tile to fill next
     int n = 0;
     Block next = block_of(pair);
     for (int it = pair; it < items; it += num_pairs, ++n) {
@@ -444,64 +515,66 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
       next = block_of(it + num_pairs);
       const int acc = n & 1;
       bool ok = CTB_WARP_WAIT1(&acc_full[acc], (n >> 1) & 1, status, DEV_TIMEOUT_MMA, abort);
-      if (UP) ok = team_all(1 + team, ok);  // both warps of a team go on or both stop
+      ok = group_all(1 + group, kGroupThreads<UP>, ok);  // the warps of a group go on or stop together
       if (!ok) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + acc * 256 + ((uint32_t)(sub * 32) << 16);
-      const int m0 = UP ? (it % p.mtiles) * 128 + (int)rank * 64 + (sub & 1) * 32 : (it % p.mtiles) * 256 + (int)rank * 128 + sub * 32;
-      uint32_t r[2][32];
-      if (half * 32 < b.n) tmem_ld32(taddr + half * 32, r[0]);
+      const int m0 = UP ? (it % p.mtiles) * 128 + (int)rank * 64 : (it % p.mtiles) * 256 + (int)rank * 128 + (sub >> 1) * 64;
+      uint32_t r[2][2][16];
+      auto load = [&](int c, uint32_t (&v)[2][16]) {
+        tmem_ld_16x32(taddr + c, v[0]);
+        tmem_ld_16x32(taddr + (16u << 16) + c, v[1]);
+      };
+      if (half * 32 < b.n) load(half * 32, r[0]);
 #pragma unroll
       for (int i = 0; i < kMaxBlockSlots / 64; ++i) {
         const int c = i * 64 + half * 32;
         if (c >= b.n) break;  // uniform
-        uint32_t(&v)[32] = r[i & 1];
-        float4 w4[8];
-        if constexpr (!UP) {  // routing weights of the 32 slots, the same for all lanes (row0 is a multiple of 16)
+        uint32_t(&v)[2][16] = r[i & 1];
+        float2 wt[4];
+        if constexpr (!UP) {  // routing weights of this thread's slots
 #pragma unroll
-          for (int q = 0; q < 8; ++q)
-            w4[q] = c + q * 4 < b.n ? __ldcg(reinterpret_cast<const float4*>(p.wts + b.row0 + c) + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int q = 0; q < 4; ++q) {
+            const int at = c + q * 8 + 2 * (lane & 3);
+            wt[q] = at < b.n ? __ldcg(reinterpret_cast<const float2*>(p.wts + b.row0 + at)) : make_float2(0.f, 0.f);
+          }
         }
         tc_wait_ld();
-        if (c + 64 < b.n) tmem_ld32(taddr + c + 64, r[(i + 1) & 1]);
-        if constexpr (UP) {
+        if (c + 64 < b.n) load(c + 64, r[(i + 1) & 1]);
+        // lane l gives the address of slot c + l; 16-byte piece k of its 128 bytes lies at k ^ (l mod 8)
+        const uint32_t row = tiles + flip * kTileBytes + lane * 128;
+        auto piece = [&](int k) { return row + (uint32_t)((k ^ (lane & 7)) << 4); };
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            if (gate) xchg[j * 32] = __uint_as_float(v[16 + j]);
-            else xchg[(16 + j) * 32] = __uint_as_float(v[j]);
+        for (int h = 0; h < 2; ++h) {
+          uint32_t o[2][4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const float a0 = __uint_as_float(v[h][4 * q]), a1 = __uint_as_float(v[h][4 * q + 1]);
+            const float b0 = __uint_as_float(v[h][4 * q + 2]), b1 = __uint_as_float(v[h][4 * q + 3]);
+            if constexpr (UP) {  // silu(g) * u with flush-to-zero and an approximate reciprocal (examples/moe.jl:117-124)
+              o[0][q] = pack_f16x2(a0 * rcp_approx_ftz(1.0f + __expf(-a0)) * b0, a1 * rcp_approx_ftz(1.0f + __expf(-a1)) * b1);
+            } else {
+              o[0][q] = pack_f16x2(a0 * wt[q].x, a1 * wt[q].y);
+              o[1][q] = pack_f16x2(b0 * wt[q].x, b1 * wt[q].y);
+            }
           }
-          team_sync(1 + team);
-          if (lane == 0) bulk_wait_read<0>();  // the previous store has read the staging block
-          __syncwarp();
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {  // silu(g) * u with flush-to-zero and an approximate reciprocal (examples/moe.jl:117-124)
-            const float got = xchg[(gate ? 16 + j : j) * 32];
-            const float g = gate ? __uint_as_float(v[j]) : got, u = gate ? got : __uint_as_float(v[16 + j]);
-            out[j * 32 + lane] = __float2half_rn(g * rcp_approx_ftz(1.0f + __expf(-g)) * u);
-          }
-        } else {
-          if (lane == 0) bulk_wait_read<0>();  // the previous stores have read the staging blocks
-          __syncwarp();
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const float4 w = w4[j / 4];
-            const float wt = j % 4 == 0 ? w.x : j % 4 == 1 ? w.y : j % 4 == 2 ? w.z : w.w;
-            out[j * 32 + lane] = __float2half_rn(__uint_as_float(v[j]) * wt);
+          if constexpr (UP) {
+            stmatrix4_trans(piece(sub * 2 + h), o[0][0], o[0][1], o[0][2], o[0][3]);
+          } else {
+            stmatrix4_trans(piece((sub & 1) * 4 + h * 2), o[0][0], o[0][1], o[0][2], o[0][3]);
+            stmatrix4_trans(piece((sub & 1) * 4 + h * 2 + 1), o[1][0], o[1][1], o[1][2], o[1][3]);
           }
         }
         fence_proxy_async_smem();
-        if (UP) team_sync(1 + team);  // the exchange buffer has been read
-        else __syncwarp();
-        if (lane == 0 && m0 < p.rows) {  // rows beyond the tensor are clipped, slots beyond the block are not stored
-          if (UP) {
-            const int first = c + (gate ? 0 : 16);
-            if (first < b.n) tma_store_3d(&tmOut, out, m0, b.row0 + first, 0);
-          } else {
-            tma_store_3d(&tmOut, out, m0, b.row0 + c, 0);
-            if (c + 16 < b.n) tma_store_3d(&tmOut, out + 16 * 32, m0, b.row0 + c + 16, 0);
-          }
+        if (issuer) bulk_wait_read<0>();  // the store before has read the other tile: free for everyone behind the barrier
+        group_sync(1 + group, kGroupThreads<UP>);
+        if (issuer && m0 < p.rows) {  // rows beyond the tensor are clipped, slots beyond the block are not stored
+          const unsigned char* tile = smem + kRingBytes + (group * 2 + flip) * kTileBytes;
+          tma_store_3d(&tmOut, tile, m0, b.row0 + c, 0);
+          if (c + 16 < b.n) tma_store_3d(&tmOut, tile + kTileBytes / 2, m0, b.row0 + c + 16, 0);
           bulk_commit();
         }
+        flip ^= 1;
       }
       tc_fence_before();
       __syncwarp();
@@ -588,7 +661,7 @@ int pair_clusters(ctb_ctx* ctx) {  // clusters of the kernel that the device run
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * ctx->sm_count);
     cfg.blockDim = dim3(kGemmThreads);
-    cfg.dynamicSmemBytes = kGemmSmem;
+    cfg.dynamicSmemBytes = kGemmSmem<UP>;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
@@ -597,7 +670,7 @@ int pair_clusters(ctb_ctx* ctx) {  // clusters of the kernel that the device run
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
-    cudaError_t e = cudaFuncSetAttribute(moe_pair_gemm_kernel<UP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
+    cudaError_t e = cudaFuncSetAttribute(moe_pair_gemm_kernel<UP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem<UP>);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, moe_pair_gemm_kernel<UP>, &cfg);
     if (e != cudaSuccess) {
       (void)cudaGetLastError();
@@ -610,15 +683,21 @@ int pair_clusters(ctb_ctx* ctx) {  // clusters of the kernel that the device run
 
 template <bool UP>
 int launch_projection(ctb_ctx* ctx, cudaStream_t st, const void* W, const void* X, void* out, int64_t K, int64_t wrows, int64_t N,
-                      int64_t E, const Scratch& sc, unsigned char* ws, int64_t max_blocks) {
+                      int64_t E, const Scratch& sc, unsigned char* ws, int64_t max_blocks, const void* ids, int ids_bits, int64_t T,
+                      int64_t topk) {
   CUtensorMap tw, to;
   SlotMaps tx;
-  {
-    // gate/up: a tile is 64 gate rows and the 64 up rows that belong to them; down: 128 rows
-    uint64_t dims[4] = {(uint64_t)K, (uint64_t)N, UP ? 2u : 1u, (uint64_t)E};
-    uint64_t str[3] = {(uint64_t)K * 2, (uint64_t)K * N * 2, (uint64_t)K * wrows * 2};
-    uint32_t box[4] = {kBK, UP ? 64u : 128u, UP ? 2u : 1u, 1};
-    int r = make_tmap(&tw, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, W, dims, str, box);
+  if (UP) {  // 8 gate rows, the 8 up rows that belong to them, the next 8 gate rows, ...
+    uint64_t dims[5] = {(uint64_t)K, 8, 2, (uint64_t)(N / 8), (uint64_t)E};
+    uint64_t str[4] = {(uint64_t)K * 2, (uint64_t)K * N * 2, (uint64_t)K * 16, (uint64_t)K * wrows * 2};
+    uint32_t box[5] = {kBK, 8, 2, 8, 1};
+    int r = make_tmap(&tw, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5, W, dims, str, box);
+    if (r) return r;
+  } else {
+    uint64_t dims[3] = {(uint64_t)K, (uint64_t)wrows, (uint64_t)E};
+    uint64_t str[2] = {(uint64_t)K * 2, (uint64_t)K * wrows * 2};
+    uint32_t box[3] = {kBK, 128, 1};
+    int r = make_tmap(&tw, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, W, dims, str, box);
     if (r) return r;
   }
   for (int k = 0; k < kMaxBlockSlots / 16; ++k) {
@@ -631,8 +710,8 @@ int launch_projection(ctb_ctx* ctx, cudaStream_t st, const void* W, const void* 
   {
     uint64_t dims[3] = {(uint64_t)N, (uint64_t)sc.rows, 1};
     uint64_t str[2] = {(uint64_t)N * 2, (uint64_t)N * sc.rows * 2};
-    uint32_t box[3] = {32, 16, 1};
-    int r = make_tmap(&to, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, out, dims, str, box, CU_TENSOR_MAP_SWIZZLE_NONE);
+    uint32_t box[3] = {64, 16, 1};
+    int r = make_tmap(&to, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, out, dims, str, box);
     if (r) return r;
   }
   PairParams p;
@@ -643,10 +722,13 @@ int launch_projection(ctb_ctx* ctx, cudaStream_t st, const void* W, const void* 
   p.mtiles = (int)((N + (UP ? 127 : 255)) / (UP ? 128 : 256));
   const int clusters = pair_clusters<UP>(ctx);
   if (clusters < 1) return fail(CTB_UNSUPPORTED, "ctb_moe_ffn: the device runs no CTA pairs");
-  cudaError_t e = cudaFuncSetAttribute(moe_pair_gemm_kernel<UP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
+  p.ids = ids;
+  p.ids_bits = ids_bits; p.T = (int)T; p.topk = (int)topk; p.E = (int)E;
+  const size_t smem = kGemmSmem<UP> + (ids ? (((3 * E + 1) * 4 + 15) & ~15) + max_blocks * sizeof(Block) : 0);
+  cudaError_t e = cudaFuncSetAttribute(moe_pair_gemm_kernel<UP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return cuda_fail(e, "ctb_moe_ffn: shared memory opt-in");
   const int grid = 2 * (int)std::min<int64_t>(clusters, max_blocks * p.mtiles);
-  e = launch_kernel(moe_pair_gemm_kernel<UP>, grid, kGemmThreads, kGemmSmem, st, 0, tw, tx, to, p, ctx->dev_status);
+  e = launch_kernel(moe_pair_gemm_kernel<UP>, grid, kGemmThreads, smem, st, 0, tw, tx, to, p, ctx->dev_status);
   if (e != cudaSuccess) return cuda_fail(e, "ctb_moe_ffn projection launch");
   return CTB_OK;
 }
@@ -658,8 +740,10 @@ int launch_sort(cudaStream_t st, const void* topk_ids, const SortParams& sp) {
   if (sp.counts)
     e = launch_kernel(moe_count_kernel<IdT>, kSortCtas, kSortThreads, 0, st, 0, ids, sp.T, sp.topk, sp.E, sp.total, sp.chunk,
                       const_cast<int*>(sp.counts));
-  const size_t smem = (size_t)((3 + kSortWarps) * sp.E + 1) * sizeof(int);
-  if (e == cudaSuccess) e = launch_kernel(moe_sort_gather_kernel<IdT>, kSortCtas, kSortThreads, smem, st, 0, ids, sp);
+  auto kernel = sp.early ? moe_sort_gather_kernel<IdT, kSortThreadsEarly> : moe_sort_gather_kernel<IdT, kSortThreads>;
+  const int threads = sp.early ? kSortThreadsEarly : kSortThreads;
+  const size_t smem = (size_t)((3 + threads / 32) * sp.E + 1) * sizeof(int);
+  if (e == cudaSuccess) e = launch_kernel(kernel, kSortCtas, threads, smem, st, 0, ids, sp);
   return e == cudaSuccess ? (int)CTB_OK : cuda_fail(e, "ctb_moe_ffn sort launch");
 }
 
@@ -701,21 +785,18 @@ extern "C" int ctb_moe_ffn(ctb_ctx* ctx, void* stream, const void* hidden, const
   sp.table = reinterpret_cast<Block*>(ws + sc.table);
   sp.num_blocks = reinterpret_cast<int*>(ws + sc.blocks);
   sp.counts = total > kSortLocal ? reinterpret_cast<int*>(ws + sc.counts) : nullptr;
-  // With few slots the gate/up projection is bound by HBM, idle during the sort: fetch what its CTAs read first.
-  sp.warm = total <= 2048 ? static_cast<const unsigned char*>(w1) : nullptr;
-  sp.warm_expert = (long long)I * H * 2;
-  sp.warm_tile = (int)(64 * H * 2);
-  sp.warm_mtiles = (int)((I + 127) / 128);
+  sp.early = total <= kEarlySlots;
   sp.T = (int)T; sp.topk = (int)topk; sp.E = (int)E; sp.vecs = (int)(H / 8); sp.total = total;
   sp.chunk = (total + kSortCtas - 1) / kSortCtas;
   sp.status = ctx->dev_status;
   r = ids_bits == 32 ? launch_sort<int>(st, topk_ids, sp) : launch_sort<long long>(st, topk_ids, sp);
   if (r) return r;
   // gate/up projection with the SwiGLU epilogue: act(:, row) = silu(Wg x) * (Wu x)
-  r = launch_projection<true>(ctx, st, w1, ws + sc.xs, ws + sc.act, H, 2 * I, I, E, sc, ws, max_blocks);
+  r = launch_projection<true>(ctx, st, w1, ws + sc.xs, ws + sc.act, H, 2 * I, I, E, sc, ws, max_blocks,
+                              sp.early ? topk_ids : nullptr, ids_bits, T, topk);
   if (r) return r;
   // down projection scaled by the routing weight, one f16 row per slot (the reference's cache3)
-  r = launch_projection<false>(ctx, st, w2, ws + sc.act, ws + sc.xs, I, H, H, E, sc, ws, max_blocks);
+  r = launch_projection<false>(ctx, st, w2, ws + sc.act, ws + sc.xs, I, H, H, E, sc, ws, max_blocks, nullptr, 0, T, topk);
   if (r) return r;
   const long long n8 = T * (H / 8);
   cudaError_t e = launch_kernel(moe_sorted_combine_kernel, (unsigned)((n8 + 255) / 256), 256, 0, st, 0, (const __half*)(ws + sc.xs),

@@ -277,12 +277,12 @@ __device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const void* tma
       "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(bar_cluster_addr)
       : "memory");
 }
-__device__ __forceinline__ void tma_load_4d_pair(void* smem_dst, const void* tmap, int x, int y, int z, int w,
+__device__ __forceinline__ void tma_load_5d_pair(void* smem_dst, const void* tmap, int x, int y, int z, int w, int v,
                                                  uint32_t bar_cluster_addr) {
   asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3, %4, %5}], "
-      "[%6];" ::"r"(smem_u32(smem_dst)),
-      "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(w), "r"(bar_cluster_addr)
+      "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 "
+      "[%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(smem_u32(smem_dst)),
+      "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(w), "r"(v), "r"(bar_cluster_addr)
       : "memory");
 }
 __device__ __forceinline__ void mma_f16_ss_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
