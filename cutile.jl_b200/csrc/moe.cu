@@ -97,75 +97,76 @@ __device__ __forceinline__ void route_one(float (&mine)[EPL], int t, int* __rest
 constexpr int kRouterWarps = 16;  // four per scheduler: the logit loop is latency-bound with fewer
 constexpr int kRouterThreads = kRouterWarps * 32;
 constexpr int kMaxRouterE = 256;
-constexpr int kRouterTE = 4;  // experts a warp carries through the hidden dimension at a time
-
-__device__ __forceinline__ void cvt8(const uint4& u, float* f) {
-  const __half2* h = reinterpret_cast<const __half2*>(&u);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 v = __half22float2(h[i]);
-    f[2 * i] = v.x;
-    f[2 * i + 1] = v.y;
-  }
+// a * b + c, a and b f16, c f32: the product is exact, one rounding, as fmaf of the converted values.
+__device__ __forceinline__ void fma_f16_f32(float& c, uint32_t a, uint32_t b, bool high) {
+  const unsigned short ah = (unsigned short)(high ? a >> 16 : a & 0xffff), bh = (unsigned short)(high ? b >> 16 : b & 0xffff);
+  asm("fma.rn.f32.f16 %0, %1, %2, %0;" : "+f"(c) : "h"(ah), "h"(bh));
 }
-
 // A CTA works on groups of G = TT * tw tokens.  Its 16 warps form tw token-warps x ew expert-warps (tw * ew = 16):
-// a warp owns TT tokens and every ew-th block of four experts, computes those logits in the fixed order (lane l
+// a warp owns TT tokens and every ew-th block of TE experts, computes those logits in the fixed order (lane l
 // = partial sum l, its 8 elements of each 256-chunk are one 16-byte shared-memory read, conflict-free without any
 // permutation) and leaves them in shared memory; after a barrier the warps take the group's tokens in turn for
 // top-k and gates.  Few tokens: small groups split over expert-warps, so that a 256-token batch still fills the
-// GPU; many tokens: TT = 4 tokens per warp, so that every weight vector read from shared memory feeds four
-// multiply-adds.  Rows are staged as f16 with cp.async (zero-filled up to a multiple of 256 elements); W_r stays
+// GPU, two experts per warp; many tokens: 4 tokens x 8 experts per warp, 12 vectors read from shared memory for 32 times 8
+// multiply-adds.  Rows are staged as f16, one bulk copy each (padded with zeros to a multiple of 256 elements); W_r stays
 // resident for the CTA's lifetime when it fits, else it passes through in slices of eg experts.
-template <int TT>
+// With few tokens a chain of latencies, with many bound by the multiply-adds, which take the f16 operands as they are.
+// 256 tokens x 1024 x 32 experts: 6.3 us with 16-byte copies and a conversion of each operand, now 4.9; 4096 tokens:
+// 15.5 us, now 10.8.
+template <int TT, int TE>
 __global__ void __launch_bounds__(kRouterThreads)
     moe_router_kernel(const __half* __restrict__ X, const __half* __restrict__ Wr, int* __restrict__ ids,
                       __half* __restrict__ gates, float* __restrict__ logits_out, int T, int H, int E, int topk,
-                      int eg, int tw) {
+                      int eg, int tw, int* status) {
   extern __shared__ __align__(16) unsigned char rsm_raw[];
-  grid_dependency_sync();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  __shared__ __align__(8) uint64_t bar;
   const int nchunk = (H + 255) / 256, Hp = nchunk * 256;
   const int ew = kRouterWarps / tw, G = TT * tw;
   __half* sx = reinterpret_cast<__half*>(rsm_raw);                     // [G][Hp]
   __half* sw = sx + (size_t)G * Hp;                                    // [eg][Hp]
   float* sl = reinterpret_cast<float*>(sw + (size_t)eg * Hp);          // [G][E] logits of the group
-  const int vpr = Hp / 8;                                              // 16-byte vectors per padded row
   const int ngroups = (T + G - 1) / G;
   constexpr int EPL = kRouterEPL;
-  auto stage_rows = [&](__half* dst, const __half* src, int nrows, int row_limit) {
-    for (int i = tid; i < nrows * vpr; i += kRouterThreads) {
-      const int r = i / vpr, v = i - r * vpr;
-      const bool valid = r < row_limit && v * 8 < H;
-      cp_async16(dst + (size_t)r * Hp + v * 8, valid ? (const void*)(src + (long long)r * H + v * 8) : (const void*)src,
-                 valid ? 16u : 0u);
-    }
-  };
+  if (tid == 0) {
+    mbar_init(&bar, 1);
+    fence_mbar_init();
+  }
+  if (H < Hp) {  // the copies never write the padding
+    const int pad = (Hp - H) / 8;
+    for (int i = tid; i < (G + eg) * pad; i += kRouterThreads)
+      reinterpret_cast<uint4*>(sx + (size_t)(i / pad) * Hp + H)[i % pad] = make_uint4(0u, 0u, 0u, 0u);
+  }
+  grid_dependency_sync();
   const bool resident = eg >= E;  // all of W_r stays in shared memory for the CTA's lifetime
-  if (resident) stage_rows(sw, Wr, E, E);
   const int wt = warp / ew, we = warp - wt * ew;
+  bool first = true;
+  uint32_t phase = 0;
 #pragma unroll 1
   for (int grp = blockIdx.x; grp < ngroups; grp += gridDim.x) {
     const int tbase = grp * G;
-    __syncthreads();  // the previous group's token rows and logits have been consumed
-    stage_rows(sx, X + (long long)tbase * H, G, T - tbase);
     const uint4* xrow[TT];
 #pragma unroll
     for (int u = 0; u < TT; ++u) xrow[u] = reinterpret_cast<const uint4*>(sx + (size_t)(wt * TT + u) * Hp) + lane;
 #pragma unroll 1
     for (int g0 = 0; g0 < E; g0 += eg) {
       const int ge = min(eg, E - g0);
-      if (!resident) {
-        __syncthreads();  // the previous expert rows have been consumed
-        stage_rows(sw, Wr + (long long)g0 * H, ge, ge);
+      __syncthreads();  // the rows before these and the logits of the previous group have been consumed
+      const int nx = g0 == 0 ? min(G, T - tbase) : 0, nw = !resident || first ? ge : 0;
+      first = false;
+      if (tid == 0) mbar_expect_tx(&bar, (uint32_t)(nx + nw) * H * 2);
+      for (int i = tid; i < nx + nw; i += kRouterThreads) {
+        if (i < nw) bulk_g2s(sw + (size_t)i * Hp, Wr + (long long)(g0 + i) * H, H * 2, &bar);
+        else bulk_g2s(sx + (size_t)(i - nw) * Hp, X + (long long)(tbase + i - nw) * H, H * 2, &bar);
       }
-      cp_async_wait_all();
-      __syncthreads();
-      // four experts at a time in rolled loops (the body runs a few times per warp: keep it small for the
-      // instruction cache)
-      constexpr int TE = kRouterTE;
+      const bool ok = mbar_wait(&bar, phase, status, DEV_TIMEOUT_TMA);
+      phase ^= 1;
+      if (__syncthreads_or(!ok)) return;
+      // rolled loops: the body runs a few times per warp, keep it small for the instruction cache
 #pragma unroll 1
-      for (int e0 = we * TE; e0 < ge; e0 += ew * TE) {
+      for (int p0 = 0; p0 < ge; p0 += ew * TE) {
+        const int e0 = p0 + we * TE;
+        if (e0 >= ge) break;
         float acc[TT][TE];
 #pragma unroll
         for (int u = 0; u < TT; ++u)
@@ -174,19 +175,22 @@ __global__ void __launch_bounds__(kRouterThreads)
         const uint4* wrow[TE];
 #pragma unroll
         for (int e = 0; e < TE; ++e) wrow[e] = reinterpret_cast<const uint4*>(sw + (size_t)min(e0 + e, ge - 1) * Hp) + lane;
-#pragma unroll 2
+#pragma unroll 1
         for (int c = 0; c < nchunk; ++c) {
-          float xf[TT][8];
+          uint4 xv[TT];
 #pragma unroll
-          for (int u = 0; u < TT; ++u) cvt8(xrow[u][c * 32], xf[u]);
+          for (int u = 0; u < TT; ++u) xv[u] = xrow[u][c * 32];
 #pragma unroll
           for (int e = 0; e < TE; ++e) {
-            float wf[8];
-            cvt8(wrow[e][c * 32], wf);
+            const uint4 wv = wrow[e][c * 32];
+            const uint32_t wp[4] = {wv.x, wv.y, wv.z, wv.w};
 #pragma unroll
             for (int j = 0; j < 8; ++j)  // ascending k inside the lane
 #pragma unroll
-              for (int u = 0; u < TT; ++u) acc[u][e] = fmaf(xf[u][j], wf[j], acc[u][e]);
+              for (int u = 0; u < TT; ++u) {
+                const uint32_t xp[4] = {xv[u].x, xv[u].y, xv[u].z, xv[u].w};
+                fma_f16_f32(acc[u][e], xp[j / 2], wp[j / 2], j & 1);
+              }
           }
         }
         // The 32 partial sums of each of the TT * TE logits meet in the butterfly v += v[lane ^ o], o = 16, 8, 4, 2, 1.
@@ -220,7 +224,7 @@ __global__ void __launch_bounds__(kRouterThreads)
             v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
           }
         }
-        static_assert(NV <= 16, "the last butterfly level must be a plain exchange");
+        static_assert(NV <= 32, "at most one logit per lane is left");
         {
           const int u = held / TE, e = held - u * TE;
           if ((lane & ((32 / NV) - 1)) == 0 && e0 + e < ge) sl[(size_t)(wt * TT + u) * E + g0 + e0 + e] = v[0];
@@ -245,7 +249,6 @@ __global__ void __launch_bounds__(kRouterThreads)
       else route(std::integral_constant<int, EPL>{});
     }
   }
-  cp_async_wait_all();  // a CTA without any group still has its copy of W_r in flight
 }
 
 // ------------------------------------------------------------------ align
@@ -1156,35 +1159,37 @@ int ctb_moe_router(ctb_ctx* ctx, void* stream, const void* hidden, const void* W
   if (T == 0) return CTB_OK;
   CTB_CHECK_DEV(hidden); CTB_CHECK_DEV(W_r); CTB_CHECK_DEV(topk_ids); CTB_CHECK_DEV(topk_weights);
   if ((uintptr_t)hidden % 16 || (uintptr_t)W_r % 16) return fail(CTB_BAD_ALIGN, "ctb_moe_router: 16-byte alignment");
-  // Group shape: (tokens per warp, token-warps).  Cost model: rounds of groups over the SMs x tokens per group x
-  // shared-memory reads per token-expert block, (TT + 4) / TT.
-  static const int cand[5][2] = {{2, 1}, {2, 2}, {2, 4}, {2, 8}, {4, 8}};
-  int best = 0;
+  // Group shape: (tokens per warp, token-warps, experts per warp at a time).  Cost model: rounds of groups over the SMs x
+  // tokens per group x shared-memory reads per logit, (TT + TE) / (TT * TE).  Shared memory: G token rows + eg expert rows
+  // as f16, rows padded to a multiple of 256 elements, + G x E logits.
+  static const int cand[5][3] = {{2, 1, 2}, {2, 2, 2}, {2, 4, 2}, {2, 8, 2}, {4, 8, 8}};
+  const int64_t Hp = (H + 255) / 256 * 256;
+  const size_t budget = 220 * 1024, rowbytes = (size_t)Hp * 2;
+  auto fixed_of = [&](int c) { return (size_t)(cand[c][0] * cand[c][1]) * (rowbytes + (size_t)E * 4); };
+  int best = -1;
   double best_cost = 1e300;
   for (int c = 0; c < 5; ++c) {
+    if (fixed_of(c) + 4 * rowbytes > budget) continue;
     const int G = cand[c][0] * cand[c][1];
     const long long groups = (T + G - 1) / G, rounds = (groups + ctx->sm_count - 1) / ctx->sm_count;
-    const double cost = (double)rounds * G * (cand[c][0] + kRouterTE) / cand[c][0];
+    const double cost = (double)rounds * G * (cand[c][0] + cand[c][2]) / (cand[c][0] * cand[c][2]);
     if (cost < best_cost * 0.999) { best_cost = cost; best = c; }
   }
-  const int TT = cand[best][0], tw = cand[best][1], G = TT * tw;
-  // shared memory: G token rows + eg expert rows as f16, rows padded to a multiple of 256 elements, + G x E logits
-  const int64_t Hp = (H + 255) / 256 * 256;
-  const size_t budget = 220 * 1024, rowbytes = (size_t)Hp * 2, fixed = (size_t)G * rowbytes + (size_t)G * E * 4;
-  if (fixed + kRouterTE * rowbytes > budget)
-    return fail(CTB_UNSUPPORTED, "ctb_moe_router: hidden size %lld too large", (long long)H);
-  const int eg = (int)std::min<size_t>((size_t)E, (budget - fixed) / rowbytes / kRouterTE * kRouterTE);
+  if (best < 0) return fail(CTB_UNSUPPORTED, "ctb_moe_router: hidden size %lld too large", (long long)H);
+  const int TT = cand[best][0], tw = cand[best][1], TE = cand[best][2], G = TT * tw;
+  const size_t fixed = fixed_of(best);
+  const int eg = (int)std::min<size_t>((size_t)E, std::max<size_t>((budget - fixed) / rowbytes / TE * TE, 4));
   const size_t smem = fixed + (size_t)eg * rowbytes;
   const int ngroups = (int)((T + G - 1) / G);
   const int grid = std::min(ngroups, ctx->sm_count);
   cudaError_t ce;
-#define CTB_LAUNCH_ROUTER(TTV)                                                                                  \
-  ce = cudaFuncSetAttribute(moe_router_kernel<TTV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);    \
+#define CTB_LAUNCH_ROUTER(TTV, TEV)                                                                                  \
+  ce = cudaFuncSetAttribute(moe_router_kernel<TTV, TEV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);    \
   if (ce != cudaSuccess) return cuda_fail(ce, "ctb_moe_router: shared memory opt-in");                          \
-  launch_kernel(moe_router_kernel<TTV>, grid, kRouterThreads, smem, static_cast<cudaStream_t>(stream), 0,                     \
+  launch_kernel(moe_router_kernel<TTV, TEV>, grid, kRouterThreads, smem, static_cast<cudaStream_t>(stream), 0,                     \
       (const __half*)hidden, (const __half*)W_r, topk_ids, (__half*)topk_weights, logits, (int)T, (int)H, (int)E, \
-      topk, eg, tw);
-  if (TT == 4) { CTB_LAUNCH_ROUTER(4) } else { CTB_LAUNCH_ROUTER(2) }
+      topk, eg, tw, ctx->dev_status);
+  if (TT == 4) { CTB_LAUNCH_ROUTER(4, 8) } else { CTB_LAUNCH_ROUTER(2, 2) }
 #undef CTB_LAUNCH_ROUTER
   CTB_CHECK_LAUNCH("ctb_moe_router launch");
   return CTB_OK;
