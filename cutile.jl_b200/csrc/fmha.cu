@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(kThreadsD, 1)
       // ---- scheduler + TMA producer of stream s (whole warp in lock step, one elected lane issues)
       auto fetch = [&]() -> int {
         int v = 0;
-        if (lane == 0) v = atomicAdd(&p.sched[0], 1);
+        if (lane == 0) v = atomicAdd(&p.sched[0], 1) + 2 * gridDim.x;
         return __shfl_sync(0xffffffffu, v, 0);
       };
       auto publish = [&](int n, int idx) -> bool {
@@ -244,7 +244,8 @@ __global__ void __launch_bounds__(kThreadsD, 1)
       // The next item is fetched late, when the loads of the current item's last two tiles are issued: work is
       // handed out heaviest first, and an item claimed early is an item that cannot go to a stream that runs dry.
       // (The other roles ask for item n+1 during the last score tile of item n.)
-      int cur = fetch();
+      // The first item needs no counter: the streams of the grid take the first 2 * gridDim.x.
+      int cur = blockIdx.x + s * gridDim.x;
       bool ok = publish(0, cur);
       int g = 0;
       for (int n = 0; ok && cur < p.items; ++n) {
@@ -374,6 +375,7 @@ __global__ void __launch_bounds__(kThreadsD, 1)
       Item it;
       decode(p, idx, it);
       const int vis_last = p.causal ? min(it.q0 + row + p.input_pos, p.seq_kv - 1) : p.seq_kv - 1;  // last visible key
+      const int vis_lo = __shfl_sync(0xffffffffu, vis_last, 0);
       float m_ref = -INFINITY, l = 0.f;
       for (int j = 0; j < it.Tc; ++j, ++ns) {
         CTB_TR(0);
@@ -388,9 +390,11 @@ __global__ void __launch_bounds__(kThreadsD, 1)
         __syncwarp();
         if (lane == 0) mbar_arrive(&B.s_free);  // the next Q*K^T may overwrite S
         CTB_TR(1);
+        const int lim = vis_last - j * kTN, lim_lo = vis_lo - j * kTN;  // last visible column of this row, of the warp's first row
         float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) chunk_max(sr[c], c, j >= it.mask_start, vis_last - j * kTN, mx0, mx1, mx2, mx3);
+        for (int c = 0; c < 4; ++c)
+          chunk_max(sr[c], c, j >= it.mask_start && c * 32 + 31 > lim_lo, lim, mx0, mx1, mx2, mx3);
         // ---- exponent reference: moved (and O, l rescaled) only when the maximum grew by more than 2^8
         const float m_true = fmaxf(m_ref, fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * p.scale_log2);
         const bool grow = m_true - m_ref > 8.0f || m_ref == -INFINITY;

@@ -35,6 +35,13 @@ def test_router_bit_exact(cuda, T, H, E, topk):
     assert ulp.max() <= 1
 
 
+# one token, hidden sizes off the 256-element chunks, several groups of tokens per CTA, experts that are no multiple of what a
+# warp carries, router weights that do not fit in shared memory
+@pytest.mark.parametrize("T,H,E,topk", [(1, 8, 3, 3), (300, 264, 35, 5), (700, 72, 33, 1), (5000, 264, 36, 4), (1300, 1544, 100, 2)])
+def test_router_group_shapes(cuda, T, H, E, topk):
+    test_router_bit_exact(cuda, T, H, E, topk)
+
+
 def test_router_tie_goes_to_smallest_index(cuda):
     import torch
     X = np.zeros((3, 64), np.float16); X[:, 0] = 1
