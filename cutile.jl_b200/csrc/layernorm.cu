@@ -150,7 +150,122 @@ __global__ void __launch_bounds__(kFwdThreads)
   if (tid == 0) bulk_wait<0>();  // stores complete before the CTA (and its shared memory) goes away
 }
 
-// Any N, any alignment: three passes over the row (the later ones hit L1/L2).
+// V neighbouring floats (V = 4: 16-byte aligned).
+template <int V>
+__device__ __forceinline__ void load_vec(const float* p, float (&v)[V]) {
+  if constexpr (V == 4) {
+    const float4 t = *reinterpret_cast<const float4*>(p);
+    v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+  } else {
+    v[0] = *p;
+  }
+}
+template <int V>
+__device__ __forceinline__ void store_vec(float* p, const float (&v)[V]) {
+  if constexpr (V == 4) *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+  else *p = v[0];
+}
+
+// Rows of at most 1024 columns, any alignment: a warp per row, the row in its registers (NE loads of V floats per lane), no
+// barrier.  A row of a few hundred columns is too short for a CTA: two block reductions and a bulk copy each way per row
+// cost more than its bytes (16384 x 256: 28.3 us with a CTA per row, now 7.0; 16384 x 1024: 32.1, now 23.9).
+constexpr int kWarpCols = 1024;
+template <int V, int NE>
+__global__ void __launch_bounds__(kFwdThreads)
+    ln_fwd_warp_kernel(const float* __restrict__ X, const float* __restrict__ W, const float* __restrict__ B,
+                       float* __restrict__ Y, float* __restrict__ Mean, float* __restrict__ Rstd, int N, int M, long long ldx,
+                       long long ldy, float eps) {
+  grid_dependency_sync();
+  const int lane = threadIdx.x & 31, warps = gridDim.x * (kFwdThreads / 32);
+  const float fn = (float)N;
+  for (int row = blockIdx.x * (kFwdThreads / 32) + (threadIdx.x >> 5); row < M; row += warps) {
+    const float* src = X + (long long)row * ldx;
+    float* dst = Y + (long long)row * ldy;
+    float x[NE][V];
+    float s = 0.f;
+#pragma unroll
+    for (int k = 0; k < NE; ++k) {
+      const int c = (lane + 32 * k) * V;
+      if (c < N) load_vec<V>(src + c, x[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < NE; ++k)
+      if ((lane + 32 * k) * V < N) {
+#pragma unroll
+        for (int q = 0; q < V; ++q) s += x[k][q];
+      }
+    const float mean = warp_sum(s) / fn;
+    float v = 0.f;
+#pragma unroll
+    for (int k = 0; k < NE; ++k)
+      if ((lane + 32 * k) * V < N) {
+#pragma unroll
+        for (int q = 0; q < V; ++q) {
+          x[k][q] -= mean;
+          v += x[k][q] * x[k][q];
+        }
+      }
+    const float rstd = 1.0f / sqrtf(warp_sum(v) / fn + eps);
+    if (lane == 0) {
+      Mean[row] = mean;
+      Rstd[row] = rstd;
+    }
+#pragma unroll
+    for (int k = 0; k < NE; ++k) {
+      const int c = (lane + 32 * k) * V;
+      if (c < N) {
+        float w[V], b[V];
+        load_vec<V>(W + c, w);
+        load_vec<V>(B + c, b);
+#pragma unroll
+        for (int q = 0; q < V; ++q) x[k][q] = x[k][q] * rstd * w[q] + b[q];
+        store_vec<V>(dst + c, x[k]);
+      }
+    }
+  }
+}
+
+// Wider rows off the 16-byte grid: a CTA per row, the row in registers, read once.
+template <int NE>
+__global__ void __launch_bounds__(kFwdThreads)
+    ln_fwd_regs_kernel(const float* __restrict__ X, const float* __restrict__ W, const float* __restrict__ B,
+                       float* __restrict__ Y, float* __restrict__ Mean, float* __restrict__ Rstd, int N, int M, long long ldx,
+                       long long ldy, float eps) {
+  __shared__ float red[kFwdThreads / 32];
+  grid_dependency_sync();
+  const int tid = threadIdx.x;
+  const float fn = (float)N;
+  for (int row = blockIdx.x; row < M; row += gridDim.x) {
+    const float* src = X + (long long)row * ldx;
+    float* dst = Y + (long long)row * ldy;
+    float x[NE];
+    float s = 0.f;
+#pragma unroll
+    for (int k = 0; k < NE; ++k) x[k] = tid + k * kFwdThreads < N ? src[tid + k * kFwdThreads] : 0.f;
+#pragma unroll
+    for (int k = 0; k < NE; ++k) s += x[k];
+    const float mean = block_sum1<kFwdThreads / 32>(s, red) / fn;
+    float v = 0.f;
+#pragma unroll
+    for (int k = 0; k < NE; ++k)
+      if (tid + k * kFwdThreads < N) {
+        x[k] -= mean;
+        v += x[k] * x[k];
+      }
+    const float rstd = 1.0f / sqrtf(block_sum1<kFwdThreads / 32>(v, red) / fn + eps);
+    if (tid == 0) {
+      Mean[row] = mean;
+      Rstd[row] = rstd;
+    }
+#pragma unroll
+    for (int k = 0; k < NE; ++k) {
+      const int c = tid + k * kFwdThreads;
+      if (c < N) dst[c] = x[k] * rstd * W[c] + B[c];
+    }
+  }
+}
+
+// Rows of more than 8192 columns off the fast path: three passes over the row (the later ones hit L1/L2).
 __global__ void __launch_bounds__(kFwdThreads) ln_fwd_generic_kernel(const float* __restrict__ X,
                                                                      const float* __restrict__ W,
                                                                      const float* __restrict__ B, float* __restrict__ Y,
@@ -351,69 +466,197 @@ __global__ void __launch_bounds__(kBwdThreads)
   if (tid == 0) bulk_wait<0>();
 }
 
-// Any N <= kBwdThreads*kGenCols, any alignment: one CTA per group, scalar accesses.
-constexpr int kGenCols = 16;
-__global__ void __launch_bounds__(kBwdThreads)
-    ln_bwd_generic_kernel(float* __restrict__ DX, const float* __restrict__ DY, float* __restrict__ DW,
-                          float* __restrict__ DB, const float* __restrict__ X, const float* __restrict__ W,
-                          const float* __restrict__ Mean, const float* __restrict__ Rstd, int N, int M, long long ldx,
-                          long long lddy, long long lddx, int G) {
-  __shared__ float red[2][kBwdWarps];
+// Adds the partial column sums of a cluster's CTAs (`mine` = this CTA's [dW | dB], N floats each, in shared memory) in
+// ascending rank order and writes column g of DW and DB.  All threads; the cluster meets before and after.
+__device__ __forceinline__ void cluster_columns(float* mine, float* __restrict__ DW, float* __restrict__ DB, int N, int g) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const int C = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  cluster.sync();
+  for (int c = rank * blockDim.x + threadIdx.x; c < N; c += C * blockDim.x) {
+    float a = 0.f, b = 0.f;
+    for (int k = 0; k < C; ++k) {
+      const float* theirs = cluster.map_shared_rank(mine, k);
+      a += theirs[c];
+      b += theirs[N + c];
+    }
+    DW[(long long)g * N + c] = a;
+    DB[(long long)g * N + c] = b;
+  }
+  cluster.sync();  // peers may still be reading this CTA's shared memory
+}
+
+// Rows of at most 1024 columns, any alignment: a warp per row, row and partial dW/dB in its registers, no barrier until the
+// end.  Grid and clusters as above: warp w of CTA r of cluster g takes the rows g + G * (r * warps + w + C * warps * j).
+// 16384 x 256: 72.7 us with a CTA per row, now 13.1; 16384 x 1024: 86.0, now 49.1.
+constexpr int kBwdWarpThreads = 256;
+template <int V, int NE>
+__global__ void __launch_bounds__(kBwdWarpThreads)
+    ln_bwd_warp_kernel(float* __restrict__ DX, const float* __restrict__ DY, float* __restrict__ DW, float* __restrict__ DB,
+                       const float* __restrict__ X, const float* __restrict__ W, const float* __restrict__ Mean,
+                       const float* __restrict__ Rstd, int N, int M, long long ldx, long long lddy, long long lddx, int G, int C) {
+  extern __shared__ __align__(16) float part[];  // [warps][2][N]
+  constexpr int kWarps = kBwdWarpThreads / 32;
   grid_dependency_sync();
-  const int tid = threadIdx.x, g = blockIdx.x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = blockIdx.x / C, rank = blockIdx.x - g * C;
   const float inv_n = 1.0f / (float)N;
-  float dw[kGenCols], db[kGenCols];
+  float dw[NE][V], db[NE][V];
 #pragma unroll
-  for (int k = 0; k < kGenCols; ++k) dw[k] = db[k] = 0.f;
-  for (long long row = g; row < M; row += G) {
+  for (int k = 0; k < NE; ++k)
+#pragma unroll
+    for (int q = 0; q < V; ++q) dw[k][q] = db[k][q] = 0.f;
+  for (long long row = g + (long long)G * (rank * kWarps + warp); row < M; row += (long long)G * C * kWarps) {
     const float mean = Mean[row], rstd = Rstd[row];
-    float xh[kGenCols], dy[kGenCols], wd[kGenCols];
-    float c1 = 0.f, c2 = 0.f;
+    float xh[NE][V], dy[NE][V];
 #pragma unroll
-    for (int k = 0; k < kGenCols; ++k) {
-      const int c = tid + k * kBwdThreads;
+    for (int k = 0; k < NE; ++k) {
+      const int c = (lane + 32 * k) * V;
       if (c < N) {
-        xh[k] = (X[row * ldx + c] - mean) * rstd;
-        dy[k] = DY[row * lddy + c];
-        wd[k] = W[c] * dy[k];
-        c1 += xh[k] * wd[k];
-        c2 += wd[k];
+        load_vec<V>(X + row * ldx + c, xh[k]);
+        load_vec<V>(DY + row * lddy + c, dy[k]);
       }
     }
+    float c1 = 0.f, c2 = 0.f;
+#pragma unroll
+    for (int k = 0; k < NE; ++k) {
+      const int c = (lane + 32 * k) * V;
+      if (c < N) {
+        float w[V];
+        load_vec<V>(W + c, w);
+#pragma unroll
+        for (int q = 0; q < V; ++q) {
+          xh[k][q] = (xh[k][q] - mean) * rstd;
+          const float wd = __fmul_rn(w[q], dy[k][q]);
+          c1 += xh[k][q] * wd;
+          c2 += wd;
+        }
+      }
+    }
+    c1 = warp_sum(c1) * inv_n;
+    c2 = warp_sum(c2) * inv_n;
+#pragma unroll
+    for (int k = 0; k < NE; ++k) {
+      const int c = (lane + 32 * k) * V;
+      if (c < N) {
+        float w[V], dx[V];
+        load_vec<V>(W + c, w);
+#pragma unroll
+        for (int q = 0; q < V; ++q) {
+          dx[q] = (__fmul_rn(w[q], dy[k][q]) - (xh[k][q] * c1 + c2)) * rstd;  // the product as c1 and c2 have it
+          dw[k][q] += dy[k][q] * xh[k][q];
+          db[k][q] += dy[k][q];
+        }
+        store_vec<V>(DX + row * lddx + c, dx);
+      }
+    }
+  }
+  float* mine = part + (size_t)warp * 2 * N;
+#pragma unroll
+  for (int k = 0; k < NE; ++k) {
+    const int c = (lane + 32 * k) * V;
+    if (c < N) {
+#pragma unroll
+      for (int q = 0; q < V; ++q) {
+        mine[c + q] = dw[k][q];
+        mine[N + c + q] = db[k][q];
+      }
+    }
+  }
+  __syncthreads();
+  for (int c = threadIdx.x; c < 2 * N; c += kBwdWarpThreads) {  // ascending warps
+    float a = part[c];
+#pragma unroll
+    for (int w = 1; w < kWarps; ++w) a += part[(size_t)w * 2 * N + c];
+    part[c] = a;
+  }
+  cluster_columns(part, DW, DB, N, g);
+}
+
+// Rows (N <= 512 * NE) off the 16-byte grid: a CTA per row as in ln_bwd_kernel, but scalar loads into registers, those of the
+// next row ahead of this row's reductions.  One CTA per group, loads when a row's turn came: 8000 x 2047 261 us, now 46.5;
+// 2000 x 8191 98, now 49.5.
+constexpr int kGenCols = 16;
+template <int NE>
+__global__ void __launch_bounds__(kBwdThreads)
+    ln_bwd_regs_kernel(float* __restrict__ DX, const float* __restrict__ DY, float* __restrict__ DW, float* __restrict__ DB,
+                       const float* __restrict__ X, const float* __restrict__ W, const float* __restrict__ Mean,
+                       const float* __restrict__ Rstd, int N, int M, long long ldx, long long lddy, long long lddx, int G, int C) {
+  extern __shared__ __align__(16) float part[];  // [2][N]
+  __shared__ float red[2][2][kBwdWarps];  // two rows in turn: one barrier per row
+  grid_dependency_sync();
+  const int tid = threadIdx.x, g = blockIdx.x / C, rank = blockIdx.x - g * C;
+  const float inv_n = 1.0f / (float)N;
+  const long long step = (long long)G * C;
+  float dw[NE], db[NE], xn[NE], dyn[NE];
+#pragma unroll
+  for (int k = 0; k < NE; ++k) dw[k] = db[k] = 0.f;
+  float mean_n = 0.f, rstd_n = 0.f;
+  auto fetch = [&](long long row) {
+    if (row >= M) return;
+    mean_n = Mean[row];
+    rstd_n = Rstd[row];
+#pragma unroll
+    for (int k = 0; k < NE; ++k) {
+      const int c = tid + k * kBwdThreads;
+      if (c < N) {
+        xn[k] = X[row * ldx + c];
+        dyn[k] = DY[row * lddy + c];
+      }
+    }
+  };
+  const long long first = g + (long long)G * rank;
+  fetch(first);
+  int flip = 0;
+  for (long long row = first; row < M; row += step, flip ^= 1) {
+    const float mean = mean_n, rstd = rstd_n;
+    float xh[NE], dy[NE];
+    float c1 = 0.f, c2 = 0.f;
+#pragma unroll
+    for (int k = 0; k < NE; ++k) {
+      const int c = tid + k * kBwdThreads;
+      if (c < N) {
+        xh[k] = (xn[k] - mean) * rstd;
+        dy[k] = dyn[k];
+        const float wd = __fmul_rn(W[c], dy[k]);
+        c1 += xh[k] * wd;
+        c2 += wd;
+      }
+    }
+    fetch(row + step);
     c1 = warp_sum(c1);
     c2 = warp_sum(c2);
     if ((tid & 31) == 0) {
-      red[0][tid >> 5] = c1;
-      red[1][tid >> 5] = c2;
+      red[flip][0][tid >> 5] = c1;
+      red[flip][1][tid >> 5] = c2;
     }
     __syncthreads();
     c1 = c2 = 0.f;
 #pragma unroll
     for (int k = 0; k < kBwdWarps; ++k) {
-      c1 += red[0][k];
-      c2 += red[1][k];
+      c1 += red[flip][0][k];
+      c2 += red[flip][1][k];
     }
-    __syncthreads();
     c1 *= inv_n;
     c2 *= inv_n;
 #pragma unroll
-    for (int k = 0; k < kGenCols; ++k) {
+    for (int k = 0; k < NE; ++k) {
       const int c = tid + k * kBwdThreads;
       if (c < N) {
-        DX[row * lddx + c] = (wd[k] - (xh[k] * c1 + c2)) * rstd;
+        DX[row * lddx + c] = (__fmul_rn(W[c], dy[k]) - (xh[k] * c1 + c2)) * rstd;
         dw[k] += dy[k] * xh[k];
         db[k] += dy[k];
       }
     }
   }
 #pragma unroll
-  for (int k = 0; k < kGenCols; ++k) {
+  for (int k = 0; k < NE; ++k) {
     const int c = tid + k * kBwdThreads;
     if (c < N) {
-      DW[(long long)g * N + c] = dw[k];
-      DB[(long long)g * N + c] = db[k];
+      part[c] = dw[k];
+      part[N + c] = db[k];
     }
   }
+  cluster_columns(part, DW, DB, N, g);
 }
 
 // Column sums of the (N, G) partials.  Block = 32 columns x 8 group slices; each
@@ -475,6 +718,22 @@ int launch_bwd(ctb_ctx* ctx, cudaStream_t st, float* DX, const float* DY, float*
   return CTB_OK;
 }
 
+// The kernels without bulk copies: as many CTAs per group (a power of two up to 8) as run at once and find `rows` rows each.
+template <typename Kernel>
+int launch_bwd_regs(ctb_ctx* ctx, Kernel k, int threads, size_t smem, int rows, cudaStream_t st, float* DX, const float* DY, float* DW,
+                    float* DB, const float* X, const float* W, const float* Mean, const float* Rstd, int N, int M, long long ldx,
+                    long long lddy, long long lddx, int G) {
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return cuda_fail(e, "ctb_layernorm_bwd: shared memory opt-in");
+  int per_sm = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem);
+  per_sm = std::max(per_sm, 1);
+  int C = 8;
+  while (C > 1 && ((long long)G * C > (long long)ctx->sm_count * per_sm || (long long)G * C * rows > M)) C >>= 1;
+  e = launch_kernel(k, G * C, threads, smem, st, C, DX, DY, DW, DB, X, W, Mean, Rstd, N, M, ldx, lddy, lddx, G, C);
+  return e == cudaSuccess ? (int)CTB_OK : cuda_fail(e, "ctb_layernorm_bwd_dx_partial_dwdb launch");
+}
+
 bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
 }  // namespace
@@ -492,10 +751,16 @@ int ctb_layernorm_fwd(ctb_ctx* ctx, void* stream, const float* X, const float* W
   if (M == 0) return CTB_OK;
   CTB_CHECK_DEV(X); CTB_CHECK_DEV(W); CTB_CHECK_DEV(B); CTB_CHECK_DEV(Y); CTB_CHECK_DEV(Mean); CTB_CHECK_DEV(Rstd);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const bool fast = N % 4 == 0 && ldx % 4 == 0 && ldy % 4 == 0 && aligned16(X) && aligned16(Y) && aligned16(W) &&
-                    aligned16(B) && N <= 4 * kFwdThreads * 8;
+  const bool vec = N % 4 == 0 && ldx % 4 == 0 && ldy % 4 == 0 && aligned16(X) && aligned16(Y) && aligned16(W) && aligned16(B);
   const int n = (int)N, m = (int)M;
-  if (fast) {
+  // A warp takes a row as long as its loads are few (256 columns) or there are rows enough to hide their latency; below
+  // M = N a CTA per row has the result sooner (8 x 1024: 2.5 against 3.7 us; 600 x 1024: 3.6 against 4.0).
+  if (N <= 256 || (N <= kWarpCols && M >= N)) {
+    auto k = vec ? (n <= 256 ? ln_fwd_warp_kernel<4, 2> : n <= 512 ? ln_fwd_warp_kernel<4, 4> : ln_fwd_warp_kernel<4, 8>)
+                 : (n <= 256 ? ln_fwd_warp_kernel<1, 8> : n <= 512 ? ln_fwd_warp_kernel<1, 16> : ln_fwd_warp_kernel<1, 32>);
+    const int grid = (int)std::min<int64_t>((M + kFwdThreads / 32 - 1) / (kFwdThreads / 32), (int64_t)ctx->sm_count * 8);
+    launch_kernel(k, grid, kFwdThreads, 0, st, 0, X, W, B, Y, Mean, Rstd, n, m, ldx, ldy, eps);
+  } else if (vec && N <= 4 * kFwdThreads * 8) {
     const int nv = (n / 4 + kFwdThreads - 1) / kFwdThreads;
     const int stage_bytes = (int)(((size_t)n * 4 + 127) & ~size_t(127));
     const size_t smem = (size_t)kFwdStages * stage_bytes;
@@ -517,7 +782,9 @@ int ctb_layernorm_fwd(ctb_ctx* ctx, void* stream, const float* X, const float* W
 #undef CTB_LN_FWD
   } else {
     const int grid = (int)std::min<int64_t>(M, (int64_t)ctx->sm_count * 8);
-    launch_kernel(ln_fwd_generic_kernel, grid, kFwdThreads, 0, st, 0, X, W, B, Y, Mean, Rstd, n, m, ldx, ldy, eps);
+    auto k = n <= kFwdThreads * 8 ? ln_fwd_regs_kernel<8> : n <= kFwdThreads * 16 ? ln_fwd_regs_kernel<16>
+             : n <= kFwdThreads * 32 ? ln_fwd_regs_kernel<32> : ln_fwd_generic_kernel;
+    launch_kernel(k, grid, kFwdThreads, 0, st, 0, X, W, B, Y, Mean, Rstd, n, m, ldx, ldy, eps);
   }
   CTB_CHECK_LAUNCH("ctb_layernorm_fwd launch");
   return CTB_OK;
@@ -542,9 +809,19 @@ int ctb_layernorm_bwd_dx_partial_dwdb(ctb_ctx* ctx, void* stream, float* DX, con
   CTB_CHECK_DEV(W);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int n = (int)N, m = (int)M, G = group_size_m;
-  const bool fast = N % 4 == 0 && ldx % 4 == 0 && lddy % 4 == 0 && lddx % 4 == 0 && aligned16(X) && aligned16(DY) &&
-                    aligned16(DX) && aligned16(W) && aligned16(DW) && aligned16(DB) && N <= 4 * kBwdThreads * 4;
-  if (fast) {
+  const bool vec = N % 4 == 0 && ldx % 4 == 0 && lddy % 4 == 0 && lddx % 4 == 0 && aligned16(X) && aligned16(DY) &&
+                   aligned16(DX) && aligned16(W);
+  // A warp per row: as in the forward pass, but the other kernels need two barriers per row and fill up sooner, so the line
+  // lies at M = N / 4 (1024 columns: 300 rows 6.1 against 6.4 us, 64 rows 5.8 against 3.2).  Single floats only up to 512
+  // columns: 64 more registers of partial sums leave too few warps (2400 x 1023: 18.5 against 16.6 us).
+  if (N <= 256 || (4 * M >= N && N <= (vec ? kWarpCols : 512))) {
+    auto k = vec ? (n <= 256 ? ln_bwd_warp_kernel<4, 2> : n <= 512 ? ln_bwd_warp_kernel<4, 4> : ln_bwd_warp_kernel<4, 8>)
+                 : (n <= 256 ? ln_bwd_warp_kernel<1, 8> : ln_bwd_warp_kernel<1, 16>);
+    constexpr int kWarps = kBwdWarpThreads / 32;
+    return launch_bwd_regs(ctx, k, kBwdWarpThreads, (size_t)kWarps * 2 * n * 4, kWarps, st, DX, DY, DW, DB, X, W, Mean, Rstd, n, m,
+                           ldx, lddy, lddx, G);
+  }
+  if (vec && aligned16(DW) && aligned16(DB) && N <= 4 * kBwdThreads * 4) {
     const int nv = (n / 4 + kBwdThreads - 1) / kBwdThreads;
     if (nv <= 1) return launch_bwd<1>(ctx, st, DX, DY, DW, DB, X, W, Mean, Rstd, n, m, ldx, lddy, lddx, G);
     if (nv <= 2) return launch_bwd<2>(ctx, st, DX, DY, DW, DB, X, W, Mean, Rstd, n, m, ldx, lddy, lddx, G);
@@ -553,9 +830,8 @@ int ctb_layernorm_bwd_dx_partial_dwdb(ctb_ctx* ctx, void* stream, float* DX, con
   if (N > kBwdThreads * kGenCols)
     return fail(CTB_UNSUPPORTED, "ctb_layernorm_bwd_dx_partial_dwdb: N=%lld exceeds %d", (long long)N,
                 kBwdThreads * kGenCols);
-  launch_kernel(ln_bwd_generic_kernel, G, kBwdThreads, 0, st, 0, DX, DY, DW, DB, X, W, Mean, Rstd, n, m, ldx, lddy, lddx, G);
-  CTB_CHECK_LAUNCH("ctb_layernorm_bwd_dx_partial_dwdb launch");
-  return CTB_OK;
+  auto k = n <= kBwdThreads * 2 ? ln_bwd_regs_kernel<2> : n <= kBwdThreads * 4 ? ln_bwd_regs_kernel<4> : n <= kBwdThreads * 8 ? ln_bwd_regs_kernel<8> : ln_bwd_regs_kernel<kGenCols>;
+  return launch_bwd_regs(ctx, k, kBwdThreads, (size_t)2 * n * 4, 2, st, DX, DY, DW, DB, X, W, Mean, Rstd, n, m, ldx, lddy, lddx, G);
 }
 
 int ctb_layernorm_bwd_dwdb(ctb_ctx* ctx, void* stream, const float* DW, const float* DB, float* FINAL_DW,

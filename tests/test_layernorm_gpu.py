@@ -54,6 +54,15 @@ def test_layernorm_parity(cuda, M, N, G):
         assert ref.rel_fro(got, want) <= 1e-2  # the reference's own criterion
 
 
+# around the widths that change the kernel (256, 512, 1024, 2048, 4096, 8192 columns), on and off the 16-byte grid, with rows
+# on both sides of the lines M = N and M = N / 4, fewer rows than groups or warps, a group count that is no power of two
+@pytest.mark.parametrize("M,N,G", [(9, 5, 64), (700, 31, 64), (3, 255, 3), (1000, 260, 7), (130, 511, 64), (600, 512, 64),
+                                   (127, 513, 2), (60, 516, 64), (1030, 1023, 64), (300, 1024, 64), (70, 1025, 64),
+                                   (513, 2047, 16), (40, 2051, 64), (100, 4099, 64), (20, 8191, 5)])
+def test_layernorm_row_widths(cuda, M, N, G):
+    test_layernorm_parity(cuda, M, N, G)
+
+
 def test_layernorm_strided(cuda):
     d = inputs.layernorm(M=64, N=512, seed=5)
     Y, Mean, Rstd, DX, DW, DB = run_fwd_bwd(cuda, d, 64, ld=640)
