@@ -34,7 +34,12 @@
 // What bounds the kernel is the exp2 unit: about 14.5 results per clock and SM measured (a
 // 128 x 128 score tile costs each of the four schedulers about 1130 clocks when two warps
 // share the unit, 1275 for a warp on its own), against 512 clocks of tensor-core time per
-// tile.  A polynomial exp2 on the FMA pipe costs more per element than the unit does.
+// tile.  Measured 2700 to 3400 per pair of tiles, as the two streams' other phases (300 to pull S, 400 for the maxima, 250
+// until P is free) fall beside each other's exponentials or not.  8 x 16 heads x 1024 causal: 39.5 us (41.1 with the first
+// items from the counter and all columns of a masked tile compared); 4 x 32 heads x 2001 causal, grouped: 117.3 (118.4).
+// Without gain: a polynomial of degree 5 for an eighth of the exponentials (40.0 / 118.2; for a half 47 / 140), P waited for
+// behind the first quarter of the exponentials, locks that keep the streams' exponentials apart (42.5 / 126), branches
+// around chunks that nobody sees (46 / 135).
 #include <cuda_bf16.h>
 #include <math.h>
 
@@ -244,8 +249,10 @@ __global__ void __launch_bounds__(kThreadsD, 1)
       // The next item is fetched late, when the loads of the current item's last two tiles are issued: work is
       // handed out heaviest first, and an item claimed early is an item that cannot go to a stream that runs dry.
       // (The other roles ask for item n+1 during the last score tile of item n.)
-      // The first item needs no counter: the streams of the grid take the first 2 * gridDim.x.
-      int cur = blockIdx.x + s * gridDim.x;
+      // The first item needs no counter: the streams of the grid take the first 2 * gridDim.x, so that with few items every
+      // SM has one before any has two, and a heavy one shares its SM with a light one (16 heads x 1011 causal, 128 items:
+      // 16.6 us; two on each of 64 SMs, the first asked from the counter, took 21.3).
+      int cur = s == 0 ? blockIdx.x : 2 * gridDim.x - 1 - blockIdx.x;
       bool ok = publish(0, cur);
       int g = 0;
       for (int n = 0; ok && cur < p.items; ++n) {
@@ -612,7 +619,7 @@ extern "C" int ctb_fmha_fwd(ctb_ctx* ctx, void* stream, const void* Q, const voi
     if (r) return r;
   }
   const size_t smem = (size_t)2 * kStreamBytes + kOutStageBytes + 1024;
-  const int grid = std::min((p.items + 1) / 2, ctx->sm_count);  // one persistent CTA per SM, two streams each
+  const int grid = std::min(p.items, ctx->sm_count);  // one persistent CTA per SM, two streams each
   auto kern = dtype == CTB_BF16 ? fmha_kernel<true> : fmha_kernel<false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return cuda_fail(e, "ctb_fmha_fwd: shared memory opt-in");
