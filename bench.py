@@ -401,7 +401,7 @@ class SoftmaxOnline(Softmax):
     def __init__(self):
         Softmax.__init__(self, 1)
         self.name = "softmax_online"
-        self.kernel = "softmax_row_smem_kernel"
+        self.kernel = "softmax_long_kernel"
 
     def describe(self):
         return f"row softmax f32 {self.M}x{self.N} N(0,4) seed 1, chunked variant, row resident in shared memory (rows longer than one register tile)"
@@ -543,7 +543,7 @@ class TiledFused(Workload):
     name = "tiled_fused"
     metric = "tiled_broadcast_gbps"
     unit = "GB/s"
-    kernel = "tiled_broadcast_pipe_kernel"
+    kernel = "tiled_broadcast_kernel"
     n = 1 << 26
 
     def describe(self):
@@ -584,7 +584,7 @@ class TiledSum(Workload):
     name = "tiled_sum"
     metric = "tiled_mapreduce_gbps"
     unit = "GB/s"
-    kernel = "tiled_reduce_kernel"
+    kernel = "tiled_reduce_rows_kernel"
     m = n = 8192
 
     def describe(self):
@@ -621,9 +621,9 @@ class Moe(Workload):
     unit = "TFLOP/s"
     bound = "hbm"
     dtype = "f16"
-    kernel = "moe_gemm_kernel"
+    kernel = "moe_pair_gemm_kernel"
     uses_blas = True
-    launches_per_step = 5  # router, align, gate/up GEMM (+SwiGLU), down GEMM, top-k combine
+    launches_per_step = 5  # router, sort, gate/up GEMM (+SwiGLU), down GEMM, top-k combine
     T, Hd, E, I, topk = 256, 1024, 32, 2048, 2
 
     def describe(self):
