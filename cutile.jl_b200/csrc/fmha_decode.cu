@@ -37,7 +37,7 @@ constexpr int kPartFloats = kMaxRows * (kD + 2);
 struct Params {
   const void* Q;
   void* Out;
-  int seq_q, keys, seq_kv, heads, group, rows;  // keys: visible to at least one query
+  int seq_q, seq_kv, group, rows;
   int input_pos, causal, blocks_per_pair;
   long long blocks;
   float scale_log2;
@@ -327,7 +327,10 @@ int fmha_decode(ctb_ctx* ctx, cudaStream_t st, const void* Q, const void* K, con
   const CUtensorMapDataType tdt = bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   CUtensorMap tk, tv;
   const uint32_t box[3] = {kD, kTileKeys, 1};
-  uint64_t dims[3] = {kD, (uint64_t)seq_kv, (uint64_t)(kv_heads * batch)};
+  // The maps end at the last key that some query sees: rows of a cache behind it may never have been written, and a
+  // probability of zero does not take a NaN or an infinity out of P V.  The copies fill with zeros there and read nothing.
+  const int64_t keys = causal ? std::min<int64_t>(seq_kv, (int64_t)input_pos + seq_q) : seq_kv;
+  uint64_t dims[3] = {kD, (uint64_t)keys, (uint64_t)(kv_heads * batch)};
   uint64_t str[2] = {kD * 2, (uint64_t)seq_kv * kD * 2};
   int r = make_tmap(&tk, tdt, 3, K, dims, str, box);
   if (r) return r;
@@ -335,12 +338,11 @@ int fmha_decode(ctb_ctx* ctx, cudaStream_t st, const void* Q, const void* K, con
   if (r) return r;
   Params p;
   p.Q = Q; p.Out = Out;
-  p.seq_q = (int)seq_q; p.seq_kv = (int)seq_kv; p.heads = (int)heads; p.group = (int)(heads / kv_heads);
+  p.seq_q = (int)seq_q; p.seq_kv = (int)seq_kv; p.group = (int)(heads / kv_heads);
   p.rows = p.group * p.seq_q;
   p.input_pos = input_pos; p.causal = causal ? 1 : 0;
-  p.keys = (int)(causal ? std::min<int64_t>(seq_kv, (int64_t)input_pos + seq_q) : seq_kv);
   p.scale_log2 = qk_scale * 1.4426950408889634f;
-  p.blocks_per_pair = (p.keys + kBlockKeys - 1) / kBlockKeys;
+  p.blocks_per_pair = (int)((keys + kBlockKeys - 1) / kBlockKeys);
   const int64_t pairs = kv_heads * batch;
   p.blocks = pairs * p.blocks_per_pair;
   const int grid = (int)std::min<int64_t>(p.blocks, ctx->sm_count);

@@ -128,3 +128,22 @@ def test_fmha_decode(cuda, batch, heads, kv_heads, seq_q, seq_kv, causal, input_
     for h in range(heads):
         assert ref.rel_fro(back(out)[:, h], want[:, h]) <= (1e-2 if bf16 else TOL)
     cuda.check_device_status(0)
+
+
+@pytest.mark.parametrize("heads,kv_heads,seq_q,seq_kv,input_pos", [
+    (8, 2, 1, 900, 200), (8, 8, 1, 256, 127), (4, 4, 1, 64, 0), (16, 4, 4, 1000, 380), (5, 5, 16, 700, 256)])
+@pytest.mark.parametrize("bf16", [False, True])
+def test_fmha_decode_unwritten_cache(cuda, heads, kv_heads, seq_q, seq_kv, input_pos, bf16):
+    """Rows of a preallocated cache behind the last visible key are never written by the caller: whatever lies there (NaN and
+    infinities included) stays out of the result, which equals that of a cache that ends at the last visible key."""
+    import torch
+    dt = torch.bfloat16 if bf16 else torch.float16
+    d = inputs.fmha(2, heads, seq_q, seq_kv, 64, kv_heads=kv_heads, seed=23)
+    Q, K, V = (torch.from_numpy(d[k].astype(np.float32)).cuda().to(dt) for k in ("Q", "K", "V"))
+    n = input_pos + seq_q
+    run = lambda k, v: cuda.fmha.cutile_fmha(Q, k, v, causal=True, input_pos=input_pos, query_group_size=heads // kv_heads)
+    want = run(K[:, :, :n].contiguous(), V[:, :, :n].contiguous())
+    for bad in (float("nan"), float("inf"), float("-inf")):
+        K[:, :, n:], V[:, :, n:] = bad, bad
+        assert torch.equal(run(K, V), want)
+    cuda.check_device_status(0)
