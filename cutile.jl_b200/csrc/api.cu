@@ -2,7 +2,6 @@
 #include <stdio.h>
 #include <string.h>
 
-#include <algorithm>
 #include <mutex>
 
 #include "ctx.h"
@@ -62,21 +61,6 @@ int workspace(ctb_ctx* ctx, size_t bytes, void** out, cudaStream_t stream) {
 int* sched_slot(ctb_ctx* ctx) {
   const unsigned n = __atomic_fetch_add(&ctx->sched_next, 1u, __ATOMIC_RELAXED);
   return ctx->sched_pool + 2 * (n % kSchedSlots);
-}
-
-StreamScratch stream_scratch(ctb_ctx* ctx, cudaStream_t stream) {
-  int slot = 0;
-  {
-    std::lock_guard<std::mutex> lock(*ctx->slot_lock);
-    const int known = std::min(ctx->slots_used, kStreamSlots);
-    while (slot < known && ctx->slot_stream[slot] != stream) ++slot;
-    if (slot == known) {
-      slot = ctx->slots_used % kStreamSlots;
-      ctx->slot_stream[slot] = stream;
-      ctx->slots_used = ctx->slots_used < 2 * kStreamSlots - 1 ? ctx->slots_used + 1 : kStreamSlots;
-    }
-  }
-  return {reinterpret_cast<float*>(ctx->stream_pool + slot * kStreamScratchBytes), ctx->tickets + (size_t)slot * kTickets};
 }
 
 EncodeTiledFn encode_tiled() {
@@ -150,10 +134,7 @@ int ctb_create(ctb_ctx** out, int device) {
   c->workspace_bytes = 0;
   c->sched_pool = nullptr;
   c->sched_next = 0;
-  c->tickets = nullptr;
-  c->stream_pool = nullptr;
-  c->slots_used = 0;
-  c->slot_lock = new std::mutex();
+  c->scratch = scratch_pool_create(device);
   c->flag_wait_ns = 2000000000ull;
   c->tf32_rne = 0;
   c->comm = nullptr;
@@ -161,14 +142,11 @@ int ctb_create(ctb_ctx** out, int device) {
   if (e == cudaSuccess) e = cudaMemset(c->dev_status, 0, sizeof(int));
   if (e == cudaSuccess) e = cudaMalloc(&c->sched_pool, 2 * kSchedSlots * sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(c->sched_pool, 0, 2 * kSchedSlots * sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc(&c->tickets, kStreamSlots * kTickets * sizeof(int));
-  if (e == cudaSuccess) e = cudaMemset(c->tickets, 0, kStreamSlots * kTickets * sizeof(int));
   // one partial GEMM tile (128 x 256 f32) per SM: split-K products never have to grow the scratch
   c->workspace_bytes = (size_t)c->sm_count * 128 * 256 * sizeof(float);
   if (e == cudaSuccess) e = cudaMalloc(&c->workspace, c->workspace_bytes);
-  if (e == cudaSuccess) e = cudaMalloc(&c->stream_pool, kStreamSlots * kStreamScratchBytes);
   if (e != cudaSuccess) {
-    delete c->slot_lock;
+    scratch_pool_destroy(c->scratch);
     delete c;
     return cuda_fail(e, "ctb_create: status word");
   }
@@ -183,9 +161,7 @@ void ctb_destroy(ctb_ctx* ctx) {
   if (ctx->workspace) cudaFree(ctx->workspace);
   if (ctx->dev_status) cudaFree(ctx->dev_status);
   if (ctx->sched_pool) cudaFree(ctx->sched_pool);
-  if (ctx->tickets) cudaFree(ctx->tickets);
-  if (ctx->stream_pool) cudaFree(ctx->stream_pool);
-  delete ctx->slot_lock;
+  scratch_pool_destroy(ctx->scratch);
   delete ctx;
 }
 

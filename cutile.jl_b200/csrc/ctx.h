@@ -7,10 +7,14 @@
 #include <stddef.h>
 #include <stdint.h>
 
-#include <mutex>
 #include <utility>
 
 #include "../../include/cutile_b200.h"
+
+namespace ctb_internal {
+struct ScratchPool;
+struct ScratchSlot;
+}  // namespace ctb_internal
 
 struct ctb_ctx {
   int device;
@@ -24,15 +28,7 @@ struct ctb_ctx {
   // that overlap on the device (different streams) do not share one.
   int* sched_pool;
   unsigned sched_next;
-  // Scratch of kernels whose last CTA adds up the parts that the others leave: kStreamSlots slots of kStreamScratchBytes
-  // and kTickets arrival counters each (zero between launches: the last CTA returns its counter to zero).  A stream keeps
-  // the slot it was given first (stream_scratch), so launches that overlap on the device do not share one; beyond
-  // kStreamSlots streams slots are shared in turn.
-  unsigned char* stream_pool;
-  int* tickets;
-  void* slot_stream[32];
-  int slots_used;
-  std::mutex* slot_lock;
+  ctb_internal::ScratchPool* scratch;  // see StreamScratch
   void* comm;             // ctb_internal::Comm* once an NCCL communicator is attached (multi.cu)
   unsigned long long flag_wait_ns;  // how long a kernel waits for another rank's flag before it gives up
   int tf32_rne;           // 1: f32 GEMM operands are rounded to TF32 (nearest even) by a pass of their own first
@@ -59,22 +55,37 @@ int moe_experts_rows(ctb_ctx* ctx, cudaStream_t st, const void* rows, int64_t ld
 size_t moe_ffn_workspace(int64_t T, int64_t H, int64_t I, int64_t E, int64_t topk);
 int moe_check_tile(const char* who, int tile_m, int tile_n, int tile_k);
 constexpr int kSchedSlots = 256;
-constexpr int kTickets = 4096, kStreamSlots = 32;
+constexpr int kTickets = 4096;
 constexpr size_t kStreamScratchBytes = 1280 * 1024;
-struct StreamScratch {
-  float* data;   // kStreamScratchBytes
-  int* tickets;  // kTickets counters, zero
+// Scratch of a launch whose last CTA adds up the parts that the others leave, and its arrival counters (zero between
+// launches: they are counted by atomicInc, which wraps at the last arrival).  No other launch that may run at the same time has
+// it, captured ones included (scratch.cu).  The object lives until the kernel is launched.  data is null when none can be
+// had; the operation then takes its form without parts.
+class StreamScratch {
+ public:
+  StreamScratch(ctb_ctx* ctx, cudaStream_t stream);
+  ~StreamScratch();
+  StreamScratch(const StreamScratch&) = delete;
+  StreamScratch& operator=(const StreamScratch&) = delete;
+  float* data = nullptr;        // kStreamScratchBytes
+  unsigned* tickets = nullptr;  // kTickets
+
+ private:
+  ScratchPool* pool_;
+  cudaStream_t stream_;
+  ScratchSlot* slot_ = nullptr;
+  bool mark_ = false;
 };
+ScratchPool* scratch_pool_create(int device);
+void scratch_pool_destroy(ScratchPool* pool);
 // The next pair of work counters of the context (see ctb_ctx::sched_pool).
 int* sched_slot(ctb_ctx* ctx);
-// The scratch slot of a stream (see ctb_ctx::stream_pool).
-StreamScratch stream_scratch(ctb_ctx* ctx, cudaStream_t stream);
 // Attention with at most 16 (group x position) query rows per key/value head (fmha_decode.cu); the arguments are checked.
+// *taken is false, and nothing was launched, when there is no scratch for the parts.
 bool fmha_decode_fits(int64_t seq_q, int group);
 int fmha_decode(ctb_ctx* ctx, cudaStream_t st, const void* Q, const void* K, const void* V, void* Out, int64_t seq_q,
                 int64_t seq_kv, int64_t heads, int64_t kv_heads, int64_t batch, float qk_scale, int input_pos, bool causal,
-                bool bf16);
-
+                bool bf16, bool* taken);
 
 // cuTensorMapEncodeTiled, resolved through the runtime so that the library has
 // no link-time dependency on libcuda and loads on machines without a driver.

@@ -581,9 +581,12 @@ extern "C" int ctb_fmha_fwd(ctb_ctx* ctx, void* stream, const void* Q, const voi
 
   // Few query rows per key/value head: the kernel that splits the keys over the GPU.  The line is where the rows of a group
   // no longer fit its 16-row instructions; a 128-row tile is at least 7/8 padding below it.
-  if (fmha_decode_fits(seq_q, query_group_size))
-    return fmha_decode(ctx, static_cast<cudaStream_t>(stream), Q, K, V, Out, seq_q, seq_kv, heads, kv_heads, batch, qk_scale,
-                       input_pos, causal != 0, dtype == CTB_BF16);
+  if (fmha_decode_fits(seq_q, query_group_size)) {
+    bool taken = false;
+    const int r = fmha_decode(ctx, static_cast<cudaStream_t>(stream), Q, K, V, Out, seq_q, seq_kv, heads, kv_heads, batch,
+                              qk_scale, input_pos, causal != 0, dtype == CTB_BF16, &taken);
+    if (taken) return r;
+  }
   CUtensorMap tq, tk, tv;
   const uint32_t box[3] = {kD, kTN, 1};
   {

@@ -42,7 +42,7 @@ struct Params {
   long long blocks;
   float scale_log2;
   float* part;   // [CTA][first, last pair of its range][rows x (64 outputs), maxima, sums]
-  int* tickets;  // per CTA: parts left of the pair that begins in its range and ends in another's
+  unsigned* tickets;  // per CTA: parts left of the pair that begins in its range and ends in another's
 };
 
 __device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], uint32_t addr) {
@@ -280,10 +280,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int c0 = (int)owner(pair_first, p.blocks, grid), c1 = (int)owner(pair_end - 1, p.blocks, grid);
     __threadfence();
     __syncthreads();
-    if (tid == 0) {
-      last_s = atomicAdd(&p.tickets[c0], 1) == c1 - c0;
-      if (last_s) p.tickets[c0] = 0;
-    }
+    if (tid == 0) last_s = atomicInc(&p.tickets[c0], (unsigned)(c1 - c0)) == (unsigned)(c1 - c0);  // back to zero by the last
     __syncthreads();
     if (last_s) {
       __threadfence();
@@ -323,7 +320,10 @@ bool fmha_decode_fits(int64_t seq_q, int group) { return seq_q * group <= kMaxRo
 
 int fmha_decode(ctb_ctx* ctx, cudaStream_t st, const void* Q, const void* K, const void* V, void* Out, int64_t seq_q,
                 int64_t seq_kv, int64_t heads, int64_t kv_heads, int64_t batch, float qk_scale, int input_pos, bool causal,
-                bool bf16) {
+                bool bf16, bool* taken) {
+  const StreamScratch scratch(ctx, st);
+  *taken = scratch.data != nullptr;
+  if (!*taken) return CTB_OK;
   const CUtensorMapDataType tdt = bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   CUtensorMap tk, tv;
   const uint32_t box[3] = {kD, kTileKeys, 1};
@@ -346,7 +346,6 @@ int fmha_decode(ctb_ctx* ctx, cudaStream_t st, const void* Q, const void* K, con
   const int64_t pairs = kv_heads * batch;
   p.blocks = pairs * p.blocks_per_pair;
   const int grid = (int)std::min<int64_t>(p.blocks, ctx->sm_count);
-  const StreamScratch scratch = stream_scratch(ctx, st);
   if ((size_t)grid * 2 * kPartFloats * sizeof(float) > kStreamScratchBytes || grid > kTickets)
     return fail(CTB_UNSUPPORTED, "ctb_fmha_fwd: more SMs than the split over keys has scratch for");
   p.part = scratch.data;

@@ -13,6 +13,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <optional>
 #include <type_traits>
 
 #include "ctx.h"
@@ -986,17 +987,14 @@ struct ReduceShape {
 };
 
 // A reduction that is cut into parts leaves one partial result per (part, output) in the stream's scratch, outputs
-// contiguous; the CTA that finishes last for its outputs (a counter per grid column, returned to zero by that CTA) adds
+// contiguous; the CTA that finishes last for its outputs (a counter per grid column, which its arrival returns to zero) adds
 // the parts up in a fixed order.  One launch instead of two, and the result does not depend on which CTA is last.
 // True for every thread of the last CTA; the partials of the others are visible then.
-__device__ __forceinline__ bool last_part(int* ticket, long long parts) {
+__device__ __forceinline__ bool last_part(unsigned* ticket, long long parts) {
   __shared__ int last;
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) {
-    last = atomicAdd(ticket, 1) == (int)parts - 1;
-    if (last) *ticket = 0;
-  }
+  if (threadIdx.x == 0) last = atomicInc(ticket, (unsigned)parts - 1) == (unsigned)parts - 1;
   __syncthreads();
   __threadfence();
   return last != 0;
@@ -1010,7 +1008,7 @@ __device__ __forceinline__ bool last_part(int* ticket, long long parts) {
 template <typename T, int OP, bool MAPPED>
 __global__ void __launch_bounds__(256)
     tiled_reduce_rows_kernel(const void* __restrict__ src, float* __restrict__ partial, void* __restrict__ dest,
-                             const ReduceShape s, int f_code, int* tickets) {
+                             const ReduceShape s, int f_code, unsigned* tickets) {
   ctb::grid_dependency_sync();
   constexpr int op = OP;
   auto fmap = [&](float v) { return MAPPED ? unary(f_code, v) : v; };
@@ -1084,7 +1082,7 @@ __global__ void __launch_bounds__(256)
 template <typename T, int OP, bool MAPPED, int VB>
 __global__ void __launch_bounds__(256)
     tiled_reduce_cols_kernel(const void* __restrict__ src, float* __restrict__ partial, void* __restrict__ dest,
-                             const ReduceShape s, long long rstride, int lx, int f_code, int* tickets) {
+                             const ReduceShape s, long long rstride, int lx, int f_code, unsigned* tickets) {
   ctb::grid_dependency_sync();
   constexpr int op = OP;
   auto fmap = [&](float v) { return MAPPED ? unary(f_code, v) : v; };
@@ -1340,22 +1338,31 @@ int ctb_tiled_mapreduce(ctb_ctx* ctx, void* stream, void* dest, const void* src,
   s.parts = std::max<long long>(1, std::min<long long>({(long long)ctx->sm_count * (mode_a ? 8 : 4) / std::max<long long>(1, columns),
                                                         (s.red_len + min_part - 1) / min_part, (long long)1024}));
   if (columns > kTickets) s.parts = 1;  // enough CTAs as it is
-  s.chunk = (std::max<long long>(1, s.red_len) + s.parts - 1) / s.parts;
-  if (mode_a) s.chunk = (s.chunk + 1023) / 1024 * 1024;  // parts start on 16-byte boundaries of an aligned row
-  s.parts = (std::max<long long>(1, s.red_len) + s.chunk - 1) / s.chunk;
+  const StreamScratch* scratch = nullptr;
+  std::optional<StreamScratch> slot;  // until the kernel is launched
+  auto cut = [&]() {
+    s.chunk = (std::max<long long>(1, s.red_len) + s.parts - 1) / s.parts;
+    if (mode_a) s.chunk = (s.chunk + 1023) / 1024 * 1024;  // parts start on 16-byte boundaries of an aligned row
+    s.parts = (std::max<long long>(1, s.red_len) + s.chunk - 1) / s.chunk;
+  };
+  cut();
   float* partial = nullptr;
-  int* tickets = nullptr;
+  unsigned* tickets = nullptr;
   if (s.parts > 1) {
-    const StreamScratch scratch = stream_scratch(ctx, st);
-    tickets = scratch.tickets;
+    scratch = &slot.emplace(ctx, st);
     const size_t bytes = (size_t)s.outputs * s.parts * sizeof(float);
-    if (bytes <= kStreamScratchBytes) {
-      partial = scratch.data;
-    } else {
+    if (scratch->data && bytes <= kStreamScratchBytes) {
+      partial = scratch->data;
+      tickets = scratch->tickets;
+    } else if (scratch->data) {
       void* ws = nullptr;
       int r = workspace(ctx, bytes, &ws, st);
       if (r) return r;
       partial = static_cast<float*>(ws);
+      tickets = scratch->tickets;
+    } else {  // no scratch: one CTA per column takes all of it
+      s.parts = 1;
+      cut();
     }
   }
   if (columns > 0x7fffffffLL) return fail(CTB_UNSUPPORTED, "ctb_tiled_mapreduce: too many output elements");

@@ -414,7 +414,10 @@ int ctb_moe_ffn_ep_group(ctb_group* g, ctb_ep* const* eps, void* const* streams,
  * (CTB_UNSUPPORTED) while the stream is being captured.  Size it once up front instead:
  * ctb_workspace_bytes(op, dims, ndims) with dims = {T, H, I, E, topk, tile_m} for CTB_OP_MOE_FFN and
  * {T_local, H, I, E_local, topk, tile_m, world} for CTB_OP_MOE_EP (0 for an unknown op), then
- * ctb_reserve_workspace.  One context serves one stream at a time. */
+ * ctb_reserve_workspace.  Calls that use this scratch (those above, split-K products of ctb_gemm, f32 products with
+ * rounded operands) are for one stream of a context at a time.  The parts of ctb_fmha_fwd with few query rows and of
+ * ctb_tiled_mapreduce lie in scratch of the stream or of the graph that captures them instead, so these may overlap;
+ * only two executables instantiated from one captured graph must not run at the same time. */
 typedef enum ctb_op { CTB_OP_MOE_FFN = 1, CTB_OP_MOE_EP = 2 } ctb_op;
 size_t ctb_workspace_bytes(int op, const int64_t* dims, int ndims);
 int ctb_reserve_workspace(ctb_ctx* ctx, void* stream, size_t bytes);
