@@ -1338,33 +1338,24 @@ int ctb_tiled_mapreduce(ctb_ctx* ctx, void* stream, void* dest, const void* src,
   s.parts = std::max<long long>(1, std::min<long long>({(long long)ctx->sm_count * (mode_a ? 8 : 4) / std::max<long long>(1, columns),
                                                         (s.red_len + min_part - 1) / min_part, (long long)1024}));
   if (columns > kTickets) s.parts = 1;  // enough CTAs as it is
-  const StreamScratch* scratch = nullptr;
-  std::optional<StreamScratch> slot;  // until the kernel is launched
   auto cut = [&]() {
     s.chunk = (std::max<long long>(1, s.red_len) + s.parts - 1) / s.parts;
     if (mode_a) s.chunk = (s.chunk + 1023) / 1024 * 1024;  // parts start on 16-byte boundaries of an aligned row
     s.parts = (std::max<long long>(1, s.red_len) + s.chunk - 1) / s.chunk;
   };
   cut();
-  float* partial = nullptr;
-  unsigned* tickets = nullptr;
+  // More than one part means at most eight row CTAs with one output or four column CTAs with 128 outputs per SM: 300 KB of
+  // partial results on 148 SMs.
+  std::optional<StreamScratch> scratch;  // until the kernel is launched
   if (s.parts > 1) {
-    scratch = &slot.emplace(ctx, st);
-    const size_t bytes = (size_t)s.outputs * s.parts * sizeof(float);
-    if (scratch->data && bytes <= kStreamScratchBytes) {
-      partial = scratch->data;
-      tickets = scratch->tickets;
-    } else if (scratch->data) {
-      void* ws = nullptr;
-      int r = workspace(ctx, bytes, &ws, st);
-      if (r) return r;
-      partial = static_cast<float*>(ws);
-      tickets = scratch->tickets;
-    } else {  // no scratch: one CTA per column takes all of it
-      s.parts = 1;
+    scratch.emplace(ctx, st);
+    if (!scratch->data || (size_t)(s.outputs * s.parts) * sizeof(float) > kStreamScratchBytes) {
+      s.parts = 1;  // one CTA per column takes all of it
       cut();
     }
   }
+  float* partial = s.parts > 1 ? scratch->data : nullptr;
+  unsigned* tickets = s.parts > 1 ? scratch->tickets : nullptr;
   if (columns > 0x7fffffffLL) return fail(CTB_UNSUPPORTED, "ctb_tiled_mapreduce: too many output elements");
   const dim3 grid((unsigned)columns, (unsigned)s.parts);
   const long long rstride = (reduce_mask & 2) ? s.d[0] : s.d[0] * s.d[1];  // between elements of the reduced index space
