@@ -65,11 +65,11 @@ PyObject* yes() { Py_RETURN_TRUE; }
 
 template <class F>
 int without_gil(F f) {
-  int s;
-  Py_BEGIN_ALLOW_THREADS
-  s = f();
-  Py_END_ALLOW_THREADS
-  return s;
+  struct Release {  // the lock is taken again also when f throws: data_ptr() does for a tensor without storage (vmap, fake)
+    PyThreadState* state = PyEval_SaveThread();
+    ~Release() { PyEval_RestoreThread(state); }
+  } release;
+  return f();
 }
 
 bool as_int(PyObject* o, long long* v) {
@@ -411,8 +411,13 @@ PyObject* new_node(PyTypeObject* type, PyObject* tuple_owned, PyObject* tensor) 
 }
 
 int leaf_ok(PyObject* t) {  // 0 with a Python error set when the tensor cannot be a leaf
-  const Tensor* c = cuda_tensor(t);
-  if (c && c->dim() <= 3 && c->is_contiguous()) return 1;
+  try {
+    const Tensor* c = cuda_tensor(t);
+    if (c && c->dim() <= 3 && c->is_contiguous()) return 1;
+  } catch (const std::exception& e) {  // type slots call this too: nothing may pass them
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+    return 0;
+  }
   PyObject* r = PyObject_CallFunctionObjArgs(g_leaf_error, t, nullptr);
   Py_XDECREF(r);
   return r != nullptr;

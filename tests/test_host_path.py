@@ -55,3 +55,30 @@ def test_native_path_follows_the_current_stream(cuda):
         cuda.softmax.softmax_tma_kernel(o, y, 4096)
     side.synchronize()
     assert (o - want).abs().max().item() < 1e-6
+
+
+@pytest.mark.gpu
+def test_tensors_without_data_raise(cuda):
+    """Fake tensors and those that vmap passes have no address: an ordinary exception, and the interpreter goes on."""
+    import threading
+
+    import torch
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    T = cuda.tiled
+    x = torch.randn(3, 8, 64, device="cuda")
+    o = torch.empty(8, 64, device="cuda")
+    calls = [lambda t: cuda.softmax.softmax_tma_kernel(o, t, 64), lambda t: T.tsum(T.Tiled(t)),
+             lambda t: T.assign(o, T.Tiled(t) + 1.0), lambda t: cuda.vadd.vec_add_kernel_2d(t, t, o, 32, 32),
+             lambda t: cuda.transpose.transpose_kernel(t, torch.empty(64, 8, device="cuda"), 32, 32),
+             lambda t: cuda.fmha.cutile_fmha(*3 * (t.half().reshape(1, 1, 8, 64),))]
+    fake = FakeTensorMode().from_tensor(x[0].clone())
+    for call in calls:
+        with pytest.raises(RuntimeError):
+            call(fake)
+        with pytest.raises(RuntimeError):
+            torch.vmap(call)(x)
+    ran = []
+    t = threading.Thread(target=lambda: ran.append(call(x[0])))
+    t.start()
+    t.join()
+    assert len(ran) == 1 and ran[0].shape == (1, 1, 8, 64)
