@@ -126,6 +126,13 @@ cudaError_t launch_kernel(void (*kernel)(P...), dim3 grid, dim3 block, size_t sm
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
+// Lets `kernel` ask for up to `most` bytes of dynamic shared memory.  `most` is the same for every call of a kernel: the limit is
+// the function's, and a launch in another thread may come between this call and the caller's launch.
+template <typename... P>
+cudaError_t allow_smem(void (*kernel)(P...), size_t most) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
 #define CTB_CHECK_CTX(ctx)                                                              \
   do {                                                                                  \
     if (!(ctx)) return ctb_internal::fail(CTB_BAD_ARG, "%s: null context", __func__);   \

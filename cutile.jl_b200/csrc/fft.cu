@@ -350,7 +350,7 @@ extern "C" int ctb_fft_plan(ctb_ctx* ctx, void* stream, const void* x, void* y, 
   const size_t smem = 2 * (size_t)items * ((size_t)(N - 1) + ((N - 1) >> 4) + 1) * sizeof(float2);
   auto kern = maxf <= 8 ? fft_plan_kernel<8> : maxf == 16 ? fft_plan_kernel<16> : fft_plan_kernel<32>;
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kern, 2 * (size_t)(kMaxN + (kMaxN >> 4)) * sizeof(float2));
     if (e != cudaSuccess) return cuda_fail(e, "ctb_fft_plan: shared memory attribute");
   }
   launch_kernel(kern, (unsigned)((batch + items - 1) / items), threads, smem, static_cast<cudaStream_t>(stream), 0,
@@ -370,7 +370,7 @@ extern "C" int ctb_fft(ctb_ctx* ctx, void* stream, const void* x, void* y, const
     if ((uintptr_t)p % 8 != 0) return fail(CTB_BAD_ALIGN, "ctb_fft: arrays must be 8-byte aligned");
   const size_t smem = fft_smem_bytes((int)N, F0, F1, F2);
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(fft_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(fft_kernel, fft_smem_bytes(kMaxN, kMaxFactor, kMaxFactor, kMaxFactor));
     if (e != cudaSuccess) return cuda_fail(e, "ctb_fft: shared memory attribute");
   }
   const int lines = (int)(N / std::min(F0, std::min(F1, F2)));

@@ -703,7 +703,7 @@ int launch_bwd(ctb_ctx* ctx, cudaStream_t st, float* DX, const float* DY, float*
   const int row_stride = (N * 4 + 127) & ~127;
   const size_t smem = (size_t)kBwdStages * 2 * row_stride;
   auto k = ln_bwd_kernel<NV>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(k, (size_t)kBwdStages * 2 * 16 * kBwdThreads * NV);
   if (e != cudaSuccess) return cuda_fail(e, "ctb_layernorm_bwd: shared memory opt-in");
   // Cluster size: the largest of 8,4,2,1 that keeps every CTA resident at once
   // and gives each CTA at least two rows.
@@ -723,7 +723,7 @@ template <typename Kernel>
 int launch_bwd_regs(ctb_ctx* ctx, Kernel k, int threads, size_t smem, int rows, cudaStream_t st, float* DX, const float* DY, float* DW,
                     float* DB, const float* X, const float* W, const float* Mean, const float* Rstd, int N, int M, long long ldx,
                     long long lddy, long long lddx, int G) {
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(k, (size_t)2 * kBwdThreads * kGenCols * 4);  // kernels of up to 1024 columns: 8 warps x 2 x N floats, the same
   if (e != cudaSuccess) return cuda_fail(e, "ctb_layernorm_bwd: shared memory opt-in");
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem);
@@ -767,7 +767,7 @@ int ctb_layernorm_fwd(ctb_ctx* ctx, void* stream, const float* X, const float* W
 #define CTB_LN_FWD(NVV)                                                                                          \
   {                                                                                                              \
     auto k = ln_fwd_staged_kernel<NVV>;                                                                          \
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);             \
+    cudaError_t e = allow_smem(k, (size_t)kFwdStages * 16 * kFwdThreads * NVV);             \
     if (e != cudaSuccess) return cuda_fail(e, "ctb_layernorm_fwd: shared memory opt-in");                        \
     int per_sm = 0;                                                                                              \
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kFwdThreads, smem);                                \
@@ -909,7 +909,7 @@ int launch_bwd_static(const StaticDev& d, cudaStream_t st, float* DX, const floa
   const int row_stride = (N * 4 + 127) & ~127;
   const size_t smem = (size_t)kBwdStages * 2 * row_stride;
   auto k = ln_bwd_kernel<NV>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(k, (size_t)kBwdStages * 2 * 16 * kBwdThreads * NV);
   if (e != cudaSuccess) return cuda_fail(e, "ctb_layernorm_bwd_static: shared memory opt-in");
   int per_sm = (int)((size_t)220 * 1024 / (smem + 1024));
   per_sm = std::max(1, std::min(per_sm, 2048 / kBwdThreads));

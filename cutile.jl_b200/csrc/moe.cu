@@ -1184,7 +1184,7 @@ int ctb_moe_router(ctb_ctx* ctx, void* stream, const void* hidden, const void* W
   const int grid = std::min(ngroups, ctx->sm_count);
   cudaError_t ce;
 #define CTB_LAUNCH_ROUTER(TTV, TEV)                                                                                  \
-  ce = cudaFuncSetAttribute(moe_router_kernel<TTV, TEV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);    \
+  ce = allow_smem(moe_router_kernel<TTV, TEV>, budget);                                                              \
   if (ce != cudaSuccess) return cuda_fail(ce, "ctb_moe_router: shared memory opt-in");                          \
   launch_kernel(moe_router_kernel<TTV, TEV>, grid, kRouterThreads, smem, static_cast<cudaStream_t>(stream), 0,                     \
       (const __half*)hidden, (const __half*)W_r, topk_ids, (__half*)topk_weights, logits, (int)T, (int)H, (int)E, \

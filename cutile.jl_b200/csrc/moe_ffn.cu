@@ -286,6 +286,10 @@ template <bool UP>
 constexpr int kGroupThreads = UP ? 128 : 64;
 template <bool UP>
 constexpr size_t kGemmSmem = 1024 + kRingBytes + (size_t)(UP ? 2 : 4) * 2 * kTileBytes;
+// The gate/up kernel's own block table behind it: slots, first rows and first blocks of E experts, then the blocks.
+constexpr size_t own_table_bytes(int64_t E, int64_t blocks) { return (size_t)(((3 * E + 1) * 4 + 15) & ~15) + blocks * sizeof(Block); }
+template <bool UP>
+constexpr size_t kGemmSmemMost = kGemmSmem<UP> + (UP ? own_table_bytes(kMaxExperts, kEarlySlots / kMaxBlockSlots + kMaxExperts) : 0);
 
 // The sorted rows with a box for every number of slots that a CTA may hold (8, 16, ... 128): one copy per k-block.
 struct SlotMaps {
@@ -383,7 +387,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
   if (UP && p.ids) {  // count the slots as the sort does
     int* tot = reinterpret_cast<int*>(smem_raw + kGemmSmem<UP>);
     int *first = tot + p.E, *bstart = first + p.E;
-    Block* own = reinterpret_cast<Block*>(smem_raw + kGemmSmem<UP> + (((3 * p.E + 1) * 4 + 15) & ~15));
+    Block* own = reinterpret_cast<Block*>(smem_raw + kGemmSmem<UP> + own_table_bytes(p.E, 0));
     for (int e = threadIdx.x; e < p.E; e += kGemmThreads) tot[e] = first[e] = 0;
     if (threadIdx.x == 0) nmax_s = 16;
     __syncthreads();
@@ -671,7 +675,7 @@ int pair_clusters(ctb_ctx* ctx) {  // clusters of the kernel that the device run
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
-    cudaError_t e = cudaFuncSetAttribute(moe_pair_gemm_kernel<UP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem<UP>);
+    cudaError_t e = allow_smem(moe_pair_gemm_kernel<UP>, kGemmSmemMost<UP>);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, moe_pair_gemm_kernel<UP>, &cfg);
     if (e != cudaSuccess) {
       (void)cudaGetLastError();
@@ -725,8 +729,8 @@ int launch_projection(ctb_ctx* ctx, cudaStream_t st, const void* W, const void* 
   if (clusters < 1) return fail(CTB_UNSUPPORTED, "ctb_moe_ffn: the device runs no CTA pairs");
   p.ids = ids;
   p.ids_bits = ids_bits; p.T = (int)T; p.topk = (int)topk; p.E = (int)E;
-  const size_t smem = kGemmSmem<UP> + (ids ? (((3 * E + 1) * 4 + 15) & ~15) + max_blocks * sizeof(Block) : 0);
-  cudaError_t e = cudaFuncSetAttribute(moe_pair_gemm_kernel<UP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const size_t smem = kGemmSmem<UP> + (ids ? own_table_bytes(E, max_blocks) : 0);
+  cudaError_t e = allow_smem(moe_pair_gemm_kernel<UP>, kGemmSmemMost<UP>);
   if (e != cudaSuccess) return cuda_fail(e, "ctb_moe_ffn: shared memory opt-in");
   const int grid = 2 * (int)std::min<int64_t>(clusters, max_blocks * p.mtiles);
   e = launch_kernel(moe_pair_gemm_kernel<UP>, grid, kGemmThreads, smem, st, 0, tw, tx, to, p, ctx->dev_status);

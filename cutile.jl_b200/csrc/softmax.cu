@@ -283,6 +283,7 @@ constexpr int kRowThreads = 512;
 constexpr int kChunkVecs = 1024;
 constexpr int kMaxChunks = 7;
 constexpr int kMaxCluster = 8;
+constexpr size_t kLongBytes = 104 * 1024;  // of a row, per CTA
 template <typename T>
 __device__ __forceinline__ void unpack16(const uint4& q, float (&f)[16 / sizeof(T)]) {
   if constexpr (sizeof(T) == 4) {
@@ -537,7 +538,7 @@ int launch(ctb_ctx* ctx, cudaStream_t st, T* out, const T* in, int N, int M, lon
     const int stage_bytes = (int)((row_bytes + 127) & ~size_t(127));
     const size_t smem = (size_t)STAGES * stage_bytes;
     auto k = softmax_staged_kernel<T, MAXV, STAGES>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(k, (size_t)STAGES * 4 * kThreads * MAXV * sizeof(T));
     if (e != cudaSuccess) return cuda_fail(e, "ctb_softmax: shared memory opt-in");
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads, smem);
@@ -549,14 +550,14 @@ int launch(ctb_ctx* ctx, cudaStream_t st, T* out, const T* in, int N, int M, lon
     if (N <= 8 * kThreads) launch_kernel(softmax_regs_kernel<T, 8>, grid, kThreads, 0, st, 0, out, in, N, M, ldo, ldi);
     else if (N <= 16 * kThreads) launch_kernel(softmax_regs_kernel<T, 16>, grid, kThreads, 0, st, 0, out, in, N, M, ldo, ldi);
     else launch_kernel(softmax_regs_kernel<T, 32>, grid, kThreads, 0, st, 0, out, in, N, M, ldo, ldi);
-  } else if (row_bytes <= (size_t)kMaxCluster * 104 * 1024 && (uintptr_t)in % sizeof(T) == 0) {
+  } else if (row_bytes <= kMaxCluster * kLongBytes && (uintptr_t)in % sizeof(T) == 0) {
     int C = 1;
-    while (row_bytes > (size_t)C * 104 * 1024) C *= 2;
+    while (row_bytes > C * kLongBytes) C *= 2;
     constexpr int V = 16 / (int)sizeof(T);
     const int per = (N / V + C - 1) / C;
     const size_t smem = (size_t)per * 16;
     auto k = softmax_long_kernel<T>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(k, kLongBytes);
     if (e != cudaSuccess) return cuda_fail(e, "ctb_softmax: shared memory opt-in");
     const int per_sm = std::max(1, std::min(4, (int)((size_t)222 * 1024 / (smem + 2048))));
     const int teams = std::max(1, std::min(M, ctx->sm_count * per_sm / C));

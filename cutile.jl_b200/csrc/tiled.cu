@@ -968,7 +968,7 @@ int launch_broadcast(ctb_ctx* ctx, cudaStream_t st, void* dest, Operands& in, co
   x.full_below = x.n / 4 - (long long)(G - 1) * grid * 256;  // a trip's last group is (G - 1) grids further on
   auto kernel = linear ? tiled_broadcast_kernel<T, G, NT, true> : tiled_broadcast_kernel<T, G, NT, false>;
   if (smem > 48 * 1024 &&  // per device, so on every launch that needs it: a host-side table write
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+      allow_smem(kernel, (size_t)kMaxInputs * 2 * G * 256 * VB) != cudaSuccess)
     return fail(CTB_CUDA_ERROR, "ctb_tiled_broadcast: shared memory attribute: %s", cudaGetErrorString(cudaGetLastError()));
   launch_kernel(kernel, (unsigned)grid, 256, smem, st, 0, dest, in, prog, n_inputs, x);
   return CTB_OK;

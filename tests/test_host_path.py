@@ -82,3 +82,52 @@ def test_tensors_without_data_raise(cuda):
     t.start()
     t.join()
     assert len(ran) == 1 and ran[0].shape == (1, 1, 8, 64)
+
+
+@pytest.mark.gpu
+def test_threads_with_different_sizes(cuda):
+    """Calls of one kernel that need different amounts of shared memory, from several threads at once."""
+    import threading
+
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(2)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    T, jobs = cuda.tiled, []
+
+    def softmax(n):
+        x = r(4, n)
+        jobs.append(lambda: cuda.softmax.softmax_chunked_kernel(torch.empty_like(x), x, n, 1024))
+
+    def layernorm(n):
+        x, w, m = r(8, n), r(n), torch.ones(8, device="cuda")
+        e = lambda: torch.empty(8, n, device="cuda")
+
+        def run():
+            cuda.layernorm.layer_norm_fwd(x, w, w, e(), torch.empty(8, device="cuda"), torch.empty(8, device="cuda"), 1e-5, 1024)
+            cuda.layernorm.layer_norm_bwd_dx_partial_dwdb(e(), x, e(), e(), x, w, m, m, None, 8, 1024)
+        jobs.append(run)
+
+    def sums(k):
+        a = [T.Tiled(r(64, 1024)) for _ in range(k)]
+        jobs.append(lambda: T.materialize(sum(a[1:], a[0] * 2.0)))
+
+    def transform(f):
+        x, plan = torch.view_as_complex(r(4, f[0] * f[1] * f[2], 2)), cuda.fft.FftPlan(f, "cuda")
+        jobs.append(lambda: plan(x))
+    softmax(9000), softmax(26000), softmax(4096), softmax(8192), layernorm(2048), layernorm(1028), layernorm(8192)
+    layernorm(8191), layernorm(2047), layernorm(300), layernorm(1023), sums(2), sums(3), transform((16, 16, 16)), transform((32, 16, 16))
+    wrong = []
+
+    def loop(job):
+        try:
+            for _ in range(300):
+                job()
+        except Exception as e:  # noqa: BLE001
+            wrong.append(e)
+    threads = [threading.Thread(target=loop, args=(j,)) for j in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not wrong, wrong[0]
