@@ -160,10 +160,11 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
       for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
     // ---- the warp's tiles of the pair
-    for (; b < end; ++b, ++n) {
+    for (; b < end; ++b) {
       const int s = n % kStages;
       if (ok) ok = CTB_WARP_WAIT(&full[warp][s], (n / kStages) & 1, status, DEV_TIMEOUT_TMA);
-      if (!ok) continue;
+      if (!ok) continue;  // n stays at the tile that did not come
+      ++n;
       const uint32_t sK = smem_u32(ring + s * (2 * kTileBytes)), sV = sK + kTileBytes;
       const int key0 = (int)(b - pair_first) * kBlockKeys + warp * kTileKeys;
       float sc[4][4];
@@ -308,7 +309,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
   }
   if (!ok)  // a wait ran out: copies still in flight must land before the CTA gives its shared memory back
-    for (int k = n > kStages ? n - kStages : 0; k < issued; ++k)
+    for (int k = n; k < issued; ++k)
       (void)CTB_WARP_WAIT(&full[warp][k % kStages], (k / kStages) & 1, status, DEV_TIMEOUT_TMA);
 }
 

@@ -160,8 +160,11 @@ __global__ void __launch_bounds__(kRouterThreads)
         else bulk_g2s(sx + (size_t)(i - nw) * Hp, X + (long long)(tbase + i - nw) * H, H * 2, &bar);
       }
       const bool ok = mbar_wait(&bar, phase, status, DEV_TIMEOUT_TMA);
+      if (__syncthreads_or(!ok)) {  // the copies must land before the CTA gives its shared memory back
+        (void)mbar_wait(&bar, phase, status, DEV_TIMEOUT_TMA);
+        return;
+      }
       phase ^= 1;
-      if (__syncthreads_or(!ok)) return;
       // rolled loops: the body runs a few times per warp, keep it small for the instruction cache
 #pragma unroll 1
       for (int p0 = 0; p0 < ge; p0 += ew * TE) {

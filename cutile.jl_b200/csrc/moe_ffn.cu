@@ -591,6 +591,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
   // signal its barriers: every thread of both CTAs meets here, also after an abort.
   tc_fence_before();
   __syncthreads();
+  let_copies_land(abort);
   cluster_arrive();
   cluster_wait();
   if (warp == 1) {

@@ -113,6 +113,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
   }
 }
 
+// End of a kernel whose roles share an abort flag, behind a barrier of the CTA: after an abort, copies that were requested and
+// that nobody waits for any more get 10 ms to land (they take microseconds) before the CTA gives its shared memory back.
+__device__ __forceinline__ void let_copies_land(const volatile int* abort) {
+  if (!*abort) return;
+  for (const uint64_t t0 = globaltimer_ns(); globaltimer_ns() - t0 < 10000000ull;) __nanosleep(1000);
+}
+
 // ---------------------------------------------------------------- TMA
 // Untiled bulk copy global -> shared (both 16-byte aligned, bytes % 16 == 0).
 __device__ __forceinline__ void bulk_g2s(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {

@@ -337,6 +337,7 @@ __global__ void __launch_bounds__(kRowThreads) softmax_long_kernel(T* __restrict
     v0 = min(nvec, rank * per);
     v1 = min(nvec, v0 + per);
   };
+  uint32_t pending = 0;  // thread 0: chunks whose copy is under way
   auto load_chunk = [&](int row, int c) {  // thread 0; the buffer region of the chunk must be free
     const T* src;
     int head, nvec, v0, v1;
@@ -346,6 +347,7 @@ __global__ void __launch_bounds__(kRowThreads) softmax_long_kernel(T* __restrict
     const uint32_t bytes = (uint32_t)(p1 - p0) * 16;
     mbar_expect_tx(&full[c], bytes);
     bulk_g2s(buf + p0, src + head + (long long)(v0 + p0) * V, bytes, &full[c]);
+    pending |= 1u << c;
   };
   if (tid == 0 && team < M)
     for (int c = 0; c * kChunkVecs < per; ++c) load_chunk(team, c);
@@ -367,8 +369,11 @@ __global__ void __launch_bounds__(kRowThreads) softmax_long_kernel(T* __restrict
     }
     for (int c = 0; c * kChunkVecs < cnt; ++c) {
       const int p0 = c * kChunkVecs, p1 = min(cnt, p0 + kChunkVecs);
-      if (alive && !mbar_wait(&full[c], (phases >> c) & 1, status, DEV_TIMEOUT_TMA)) alive = false;
-      phases ^= 1u << c;
+      if (alive) alive = mbar_wait(&full[c], (phases >> c) & 1, status, DEV_TIMEOUT_TMA);
+      if (alive) {
+        phases ^= 1u << c;
+        pending &= ~(1u << c);
+      }
       for (int p = p0 + tid; p < p1; p += kRowThreads) {
         float f[V];
         unpack16<T>(buf[p], f);
@@ -427,9 +432,12 @@ __global__ void __launch_bounds__(kRowThreads) softmax_long_kernel(T* __restrict
         }
       }
       __syncthreads();  // all reads of the chunk are done before the bulk copy overwrites it
-      if (tid == 0 && next < M) load_chunk(next, c);
+      if (tid == 0 && next < M && alive) load_chunk(next, c);
     }
   }
+  if (tid == 0)  // a wait ran out: copies under way must land before the CTA gives its shared memory back
+    for (; pending; pending &= pending - 1)
+      (void)mbar_wait(&full[__ffs(pending) - 1], (phases >> (__ffs(pending) - 1)) & 1, status, DEV_TIMEOUT_TMA);
 }
 
 // ------------------------------------------------------------------ variant 1, any row
