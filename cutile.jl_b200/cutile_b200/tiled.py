@@ -7,7 +7,6 @@ whole expression as ONE kernel; ``materialize(expr)`` is the allocating form (``
 and the reduced dimensions kept with extent 1.
 """
 import ctypes as C
-import functools
 
 import torch
 
@@ -18,7 +17,6 @@ _OPS = {"input": 0, "const": 1, "identity": 16, "neg": 17, "abs": 18, "sqrt": 19
         "log2": 23, "sin": 24, "cos": 25, "tanh": 26, "inv": 27, "abs2": 28, "add": 64, "sub": 65, "mul": 66, "div": 67,
         "max": 68, "min": 69, "pow": 70}
 MAX_DIMS = 3
-
 
 
 def _leaf_error(tensor):
@@ -36,13 +34,13 @@ Expr, Tiled = _host.Expr, _host.Tiled  # expression nodes (csrc/host.cpp)
 
 
 def _unary(name):
-    return functools.partial(_host.unary, name)
+    return lambda x: _host.unary(name, x)
 
 
 sin, cos, exp, exp2, log, log2, sqrt, tanh, inv, abs2 = (_unary(n) for n in
                                                          ("sin", "cos", "exp", "exp2", "log", "log2", "sqrt", "tanh", "inv", "abs2"))
-tmax = functools.partial(_host.binary, "max")
-tmin = functools.partial(_host.binary, "min")
+tmax = lambda a, b: _host.binary("max", a, b)
+tmin = lambda a, b: _host.binary("min", a, b)
 
 
 def _jshape(t):

@@ -23,6 +23,13 @@ def test_expression_nodes():
     del e
 
 
+def test_function_forms_take_keywords():
+    from cutile_b200 import tiled as T
+    e = T.Expr.wrap(2.0)
+    assert T.sin(x=e).node == ("sin", e) and T.abs2(x=e).node == ("abs2", e)
+    assert T.tmax(a=e, b=1).node[:2] == ("max", e) and T.tmin(1, b=e).node[2] is e
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("m,n", [(1, 4), (64, 1000), (33, 4096)])
 def test_native_and_checked_calls_agree(cuda, m, n):
