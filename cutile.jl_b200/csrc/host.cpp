@@ -370,6 +370,7 @@ struct Node {
   PyObject_HEAD
   PyObject* node;    // ("leaf", tensor) | ("const", float) | (unary name, Expr) | (binary name, Expr, Expr)
   PyObject* tensor;  // Tiled only
+  PyObject *dict, *weak;
 };
 PyTypeObject* g_expr = nullptr;
 PyTypeObject* g_tiled = nullptr;
@@ -479,28 +480,49 @@ int node_traverse(PyObject* self, visitproc visit, void* arg) {
   Py_VISIT(Py_TYPE(self));
   Py_VISIT(reinterpret_cast<Node*>(self)->node);
   Py_VISIT(reinterpret_cast<Node*>(self)->tensor);
+  Py_VISIT(reinterpret_cast<Node*>(self)->dict);
   return 0;
 }
 int node_clear(PyObject* self) {
   Py_CLEAR(reinterpret_cast<Node*>(self)->node);
   Py_CLEAR(reinterpret_cast<Node*>(self)->tensor);
+  Py_CLEAR(reinterpret_cast<Node*>(self)->dict);
   return 0;
 }
 void node_dealloc(PyObject* self) {
   PyTypeObject* type = Py_TYPE(self);
   PyObject_GC_UnTrack(self);
   Py_TRASHCAN_BEGIN(self, node_dealloc)
+  if (reinterpret_cast<Node*>(self)->weak) PyObject_ClearWeakRefs(self);
   node_clear(self);
   type->tp_free(self);
   Py_DECREF(type);
   Py_TRASHCAN_END
 }
 PyObject* expr_wrap(PyObject*, PyObject* x) { return wrap(x); }
-
+// For copies and pickles: a new object of the type, its attributes, then the members above (no __init__ runs).
+PyObject* node_reduce(PyObject* self, PyObject*) {
+  Node* n = reinterpret_cast<Node*>(self);
+  PyObject* module = PyImport_ImportModule("copyreg");
+  PyObject* make = module ? PyObject_GetAttrString(module, "__newobj__") : nullptr;
+  PyObject* members = make ? PyDict_New() : nullptr;
+  bool ok = members && (!n->node || PyDict_SetItemString(members, "node", n->node) == 0) &&
+            (!n->tensor || PyDict_SetItemString(members, "tensor", n->tensor) == 0);
+  PyObject* r = ok ? Py_BuildValue("O(O)(OO)", make, Py_TYPE(self), n->dict ? n->dict : Py_None, members) : nullptr;
+  Py_XDECREF(members);
+  Py_XDECREF(make);
+  Py_XDECREF(module);
+  return r;
+}
 PyMemberDef kNodeMembers[] = {{"node", Py_T_OBJECT_EX, offsetof(Node, node), 0, "the operation and its operands"},
+                              {"__dictoffset__", Py_T_PYSSIZET, offsetof(Node, dict), Py_READONLY, nullptr},
+                              {"__weaklistoffset__", Py_T_PYSSIZET, offsetof(Node, weak), Py_READONLY, nullptr},
                               {nullptr, 0, 0, 0, nullptr}};
 PyMemberDef kTiledMembers[] = {{"tensor", Py_T_OBJECT_EX, offsetof(Node, tensor), 0, "the array"}, {nullptr, 0, 0, 0, nullptr}};
-PyMethodDef kExprMethods[] = {{"wrap", expr_wrap, METH_O | METH_STATIC, "an Expr of an Expr, a tensor or a number"},
+PyGetSetDef kExprGetSet[] = {{"__dict__", PyObject_GenericGetDict, PyObject_GenericSetDict, nullptr, nullptr},
+                             {nullptr, nullptr, nullptr, nullptr, nullptr}};
+PyMethodDef kExprMethods[] = {{"__reduce__", node_reduce, METH_NOARGS, nullptr},
+                              {"wrap", expr_wrap, METH_O | METH_STATIC, "an Expr of an Expr, a tensor or a number"},
                               {nullptr, nullptr, 0, nullptr}};
 template <class F>
 void* slot(F f) { return reinterpret_cast<void*>(f); }
@@ -508,7 +530,7 @@ PyType_Slot kExprSlots[] = {
     {Py_tp_doc, const_cast<char*>("A node of a broadcast expression: (\"leaf\", tensor) | (\"const\", value) | (unary name, Expr) | "
                                   "(binary name, Expr, Expr).")},
     {Py_tp_init, slot(expr_init)}, {Py_tp_dealloc, slot(node_dealloc)}, {Py_tp_traverse, slot(node_traverse)},
-    {Py_tp_clear, slot(node_clear)}, {Py_tp_members, kNodeMembers}, {Py_tp_methods, kExprMethods},
+    {Py_tp_clear, slot(node_clear)}, {Py_tp_members, kNodeMembers}, {Py_tp_methods, kExprMethods}, {Py_tp_getset, kExprGetSet},
     {Py_nb_add, slot(nb_binary<CTB_TILED_ADD>)}, {Py_nb_subtract, slot(nb_binary<CTB_TILED_SUB>)},
     {Py_nb_multiply, slot(nb_binary<CTB_TILED_MUL>)}, {Py_nb_true_divide, slot(nb_binary<CTB_TILED_DIV>)},
     {Py_nb_power, slot(nb_power)}, {Py_nb_negative, slot(nb_unary<CTB_TILED_NEG>)},

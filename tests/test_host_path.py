@@ -30,6 +30,37 @@ def test_function_forms_take_keywords():
     assert T.tmax(a=e, b=1).node[:2] == ("max", e) and T.tmin(1, b=e).node[2] is e
 
 
+def test_nodes_are_ordinary_objects():
+    """Copies, pickles, weak references and attributes of their own, also in subclasses."""
+    import copy
+    import gc
+    import pickle
+    import weakref
+
+    from cutile_b200 import tiled as T
+    e = T.Expr.wrap(2.0) * 3.0 + T.exp(T.Expr.wrap(0.5))
+    for c in (copy.copy(e), copy.deepcopy(e), pickle.loads(pickle.dumps(e))):
+        assert type(c) is T.Expr and c.node[0] == "add" and c.node[1].node[0] == "mul" and c.node[2].node[1].node == ("const", 0.5)
+    assert copy.copy(e).node[1] is e.node[1]
+    e.label = "sum"
+    assert copy.copy(e).label == "sum" and e.__dict__ == {"label": "sum"}
+    r = weakref.ref(e)
+    assert r() is e
+    e.label = e  # a cycle
+    del e, c
+    gc.collect()
+    assert r() is None
+
+    class Named(T.Expr):
+        def __init__(self, name, *node):
+            super().__init__(*node)
+            self.name = name
+    n = Named("two", "const", 2.0)
+    c = copy.copy(n)
+    assert type(c) is Named and c.name == "two" and c.node == ("const", 2.0)
+    assert n.name == "two" and (n + 1).node[1] is n and weakref.ref(n)() is n
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("m,n", [(1, 4), (64, 1000), (33, 4096)])
 def test_native_and_checked_calls_agree(cuda, m, n):
