@@ -6,6 +6,7 @@ in-tree checkout is self-contained.
 """
 import importlib.util
 import os
+import re
 import subprocess
 import sys
 import sysconfig
@@ -66,24 +67,48 @@ def build(force=False, verbose=False):
     return LIB
 
 
-def build_host(force=False, verbose=False):
-    """The CPython extension: compiled against the headers of the torch that imports it, linked to LIB next to it."""
-    src = os.path.join(HERE, "host.cpp")
-    if not (force or _stale(HOST, [src, os.path.join(INCLUDE, "cutile_b200.h")])):
-        return
-    spec = importlib.util.find_spec("torch")  # its folder, without importing it
+def built_for():
+    """What the host extension is compiled against: the torch that is installed (found without importing it) and this
+    Python.  None without torch."""
+    spec = importlib.util.find_spec("torch")
+    if spec is None:
+        return None
     torch_dir = os.path.dirname(spec.origin)
+    with open(os.path.join(torch_dir, "version.py")) as f:
+        version = re.search(r"^__version__ = '([^']*)'", f.read(), re.M).group(1)
+    return {"dir": torch_dir, "torch": version, "python": sysconfig.get_config_var("SOABI")}
+
+
+def build_host(force=False, verbose=False):
+    """The CPython extension: compiled against the headers of the torch that imports it, linked to LIB next to it.  Built
+    again when its sources, torch or Python have changed.  Without torch there is nothing that could use it."""
+    src = os.path.join(HERE, "host.cpp")
+    env = built_for()
+    if env is None:
+        sys.stderr.write("torch is not installed: the host extension of the Python package is not built\n")
+        return
+    stamp_file, stamp = os.path.join(OBJ_DIR, "host.stamp"), f"{env['torch']} {env['python']}\n"
+    same = False
+    if os.path.exists(stamp_file):
+        with open(stamp_file) as f:
+            same = f.read() == stamp
+    if same and not (force or _stale(HOST, [src, os.path.join(INCLUDE, "cutile_b200.h")])):
+        return
     cuda = os.path.dirname(os.path.dirname(NVCC))
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-D_GLIBCXX_USE_CXX11_ABI=1",
-           "-I", sysconfig.get_paths()["include"], "-I", os.path.join(torch_dir, "include"),
-           "-I", os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"), "-I", os.path.join(cuda, "include"),
-           src, "-o", HOST, "-L", OUT_DIR, "-l:libcutile_b200.so", "-L", os.path.join(torch_dir, "lib"),
+           f'-DCTB_TORCH_VERSION="{env["torch"]}"',
+           "-I", sysconfig.get_paths()["include"], "-I", os.path.join(env["dir"], "include"),
+           "-I", os.path.join(env["dir"], "include", "torch", "csrc", "api", "include"), "-I", os.path.join(cuda, "include"),
+           src, "-o", HOST, "-L", OUT_DIR, "-l:libcutile_b200.so", "-L", os.path.join(env["dir"], "lib"),
            "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if verbose or r.returncode:
         sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
     if r.returncode:
         raise RuntimeError("the host extension failed to build")
+    os.makedirs(OBJ_DIR, exist_ok=True)
+    with open(stamp_file, "w") as f:
+        f.write(stamp)
 
 
 if __name__ == "__main__":

@@ -760,7 +760,8 @@ PyMODINIT_FUNC PyInit__host(void) {
   g_expr = reinterpret_cast<PyTypeObject*>(PyType_FromSpec(&kExprSpec));
   g_tiled = g_expr ? reinterpret_cast<PyTypeObject*>(PyType_FromSpecWithBases(&kTiledSpec, reinterpret_cast<PyObject*>(g_expr)))
                    : nullptr;
-  if (!g_tiled || PyModule_AddObjectRef(m, "Expr", reinterpret_cast<PyObject*>(g_expr)) < 0 ||
+  if (!g_tiled || PyModule_AddStringConstant(m, "TORCH_VERSION", CTB_TORCH_VERSION) < 0 ||
+      PyModule_AddObjectRef(m, "Expr", reinterpret_cast<PyObject*>(g_expr)) < 0 ||
       PyModule_AddObjectRef(m, "Tiled", reinterpret_cast<PyObject*>(g_tiled)) < 0) {
     Py_DECREF(m);
     return nullptr;
