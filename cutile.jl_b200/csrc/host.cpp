@@ -14,6 +14,8 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <cstring>
+
 #include "../../include/cutile_b200.h"
 
 namespace {
@@ -595,7 +597,7 @@ struct Walk {
       if (!PyFloat_Check(x)) return false;
       const double v = PyFloat_AS_DOUBLE(x);
       int i = 0;
-      while (i < n_const && exact[i] != v) ++i;
+      while (i < n_const && std::memcmp(&exact[i], &v, sizeof v)) ++i;  // 0.0 and -0.0 are two constants
       if (i == CTB_TILED_MAX_CONSTS) return false;
       if (i == n_const) {
         exact[n_const] = v;

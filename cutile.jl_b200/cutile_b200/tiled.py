@@ -7,6 +7,7 @@ whole expression as ONE kernel; ``materialize(expr)`` is the allocating form (``
 and the reduced dimensions kept with extent 1.
 """
 import ctypes as C
+import struct
 
 import torch
 
@@ -71,7 +72,7 @@ def broadcast_shape(expr):
 
 
 def _compile(expr):
-    inputs, consts, prog = [], [], []
+    inputs, consts, prog = [], {}, []
 
     def walk(e):
         kind = e.node[0]
@@ -84,16 +85,17 @@ def _compile(expr):
             prog.extend((_OPS["input"], idx))
         elif kind == "const":
             v = e.node[1]
-            if v not in consts:
-                consts.append(v)
-            prog.extend((_OPS["const"], consts.index(v)))
+            bits = struct.pack("d", v)  # 0.0 and -0.0 are two constants
+            if bits not in consts:
+                consts[bits] = v
+            prog.extend((_OPS["const"], list(consts).index(bits)))
         else:
             for c in e.node[1:]:
                 walk(c)
             prog.extend((_OPS[kind], 0))
 
     walk(expr)
-    return inputs, consts, prog
+    return inputs, list(consts.values()), prog
 
 
 def assign(dest, expr, **hints):

@@ -313,3 +313,16 @@ def test_tanh_accuracy(cuda):
     assert np.array_equal(np.signbit(got), np.signbit(x))
     T.assign(out, T.tanh(T.Tiled(torch.full_like(out, float("nan")))))
     assert torch.isnan(out).all()
+
+
+@pytest.mark.parametrize("hints", [{}, {"occupancy": 2}])  # the native path, the Python path
+def test_broadcast_signed_zero_constants(cuda, hints):
+    """0.0 and -0.0 in one expression stay two constants."""
+    import torch
+    T = cuda.tiled
+    a = torch.rand(1000, device="cuda")
+    out = torch.empty_like(a)
+    T.assign(out, T.tmin(T.Tiled(a) + 0.0, T.inv(T.Expr.wrap(-0.0))), **hints)
+    assert torch.equal(out, torch.full_like(a, float("-inf")))
+    T.assign(out, (T.Tiled(a) * -0.0) * 1.0 + (T.Tiled(a) * 0.0) * -1.0, **hints)
+    assert torch.equal(out, torch.zeros_like(a)) and torch.signbit(out).all()
