@@ -2,12 +2,13 @@
 // broadcast expression fused into one kernel) and mapreduce (src/mapreduce.jl: sum / prod / maximum / minimum / a
 // mapped reduction over any set of dimensions).  The reference compiles the Julia expression; a prebuilt library
 // cannot, so the expression arrives as a short postfix program (push input, push constant, unary function, binary
-// operator).  The host turns it into instructions of an accumulator machine (compile_program below: a leaf operand
-// of a binary operator is read in place, only a binary operator between two computed values touches the stack),
-// and every thread runs those instructions on registers for four or eight elements at a time: still one pass over
-// memory, one kernel, whatever the expression.  Arrays have up to three dimensions, column-major, first dimension
-// contiguous; an operand with extent 1 along a dimension is expanded along it (stride 0).  Arithmetic is f32
-// whatever the element type.  Both are bound by HBM bandwidth: bytes of the operands read once plus the result.
+// operator).  The host turns it into words of an accumulator machine with up to four temporaries (lower_program below:
+// a leaf operand of a binary operator is read in place, constants and signs ride on other words, a value that occurs
+// more than once is computed once), and every thread runs those words on registers for eight or sixteen elements at a time:
+// still one pass over memory, one kernel, whatever the expression.  Arrays have up to three dimensions, column-major, first
+// dimension contiguous; an operand with extent 1 along a dimension is expanded along it (stride 0).  Arithmetic is f32
+// whatever the element type.  Both are bound by HBM bandwidth (bytes of the operands read once plus the result) as long as
+// the expression is short.
 #include <cuda_fp16.h>
 #include <math.h>
 
@@ -71,7 +72,7 @@ enum : unsigned {
 };
 constexpr int kColdCodes[5] = {CTB_TILED_SUB, CTB_TILED_DIV, CTB_TILED_MAX, CTB_TILED_MIN, CTB_TILED_POW};
 constexpr int kTemps = 4;
-constexpr int kMaxIns = kMaxOps + kMaxOps / 2;
+constexpr int kMaxIns = CTB_TILED_MAX_WORDS;  // a word per operation, and what the stores of temporaries add
 
 struct Program {
   int n_ins;
@@ -1289,6 +1290,29 @@ int ctb_tiled_compile(const int32_t* program, int n_ops, int n_inputs, int n_con
   if (bad) return fail(CTB_BAD_ARG, "ctb_tiled_compile: operation %d %s", -bad - 1, why);
   for (int k = 0; k < c.n_words; ++k) instructions[k] = c.words[k];
   *n_instructions = c.n_words;
+  return CTB_OK;
+}
+
+int ctb_tiled_lower(const int32_t* program, int n_ops, int n_inputs, const float* constants, int n_constants, uint32_t* words,
+                    float* constants_pq, int* n_words, int* n_temps) {
+  if (!program || !words || !constants_pq || !n_words || !n_temps || (n_constants && !constants))
+    return fail(CTB_BAD_ARG, "ctb_tiled_lower: null argument");
+  if (n_inputs < 0 || n_inputs > kMaxInputs || n_ops < 1 || n_ops > kMaxOps || n_constants < 0 || n_constants > kMaxConsts)
+    return fail(CTB_UNSUPPORTED, "ctb_tiled_lower: at most %d inputs, %d operations and %d constants", kMaxInputs, kMaxOps,
+                kMaxConsts);
+  Program prog;
+  const char* why = "";
+  const int bad = lower_program(program, n_ops, n_inputs, constants, n_constants, &prog, &why);
+  if (bad == -1000)
+    return fail(CTB_UNSUPPORTED, "ctb_tiled_lower: the expression needs more than %d intermediate values at once", kStack);
+  if (bad) return fail(CTB_BAD_ARG, "ctb_tiled_lower: operation %d %s", -bad - 1, why);
+  for (int k = 0; k < prog.n_ins; ++k) {
+    words[k] = prog.ins[k];
+    constants_pq[2 * k] = prog.pq[k].x;
+    constants_pq[2 * k + 1] = prog.pq[k].y;
+  }
+  *n_words = prog.n_ins;
+  *n_temps = prog.n_temps;
   return CTB_OK;
 }
 

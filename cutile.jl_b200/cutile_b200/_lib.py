@@ -61,6 +61,8 @@ SIGNATURES = {
     "ctb_tiled_broadcast": [_p, _p, _p, C.POINTER(_i64), C.POINTER(_p), C.POINTER(_i64), _i, C.POINTER(C.c_int32), _i,
                             C.POINTER(C.c_float), _i, _i],
     "ctb_tiled_compile": [C.POINTER(C.c_int32), _i, _i, _i, C.POINTER(C.c_uint32), C.POINTER(_i)],
+    "ctb_tiled_lower": [C.POINTER(C.c_int32), _i, _i, C.POINTER(C.c_float), _i, C.POINTER(C.c_uint32), C.POINTER(C.c_float),
+                        C.POINTER(_i), C.POINTER(_i)],
     "ctb_tiled_mapreduce": [_p, _p, _p, _p, C.POINTER(_i64), _i, _i, _i, _i],
     "ctb_fft": [_p, _p, _p, _p, _p, _p, _p, _p, _p, _i64, _i, _i, _i, _i64, _i, _i],
     "ctb_fft_plan": [_p, _p, _p, _p, _p, _p, _i64, _i, _i, _i, _i64, _i, _i],

@@ -148,13 +148,29 @@ enum {
 int ctb_tiled_broadcast(ctb_ctx* ctx, void* stream, void* dest, const int64_t* shape, const void* const* inputs,
                         const int64_t* input_strides, int n_inputs, const int32_t* program, int n_ops, const float* constants,
                         int n_constants, int dtype);
-/* Diagnostic: the instruction words ctb_tiled_broadcast would run for this program (no GPU needed).  A word is
- * kind | source << 2 | reversed << 4 | code << 8 | argument << 16 with kind 0 = push the operand, 1 = top = code(top),
- * 2 = top = top code operand (operand code top when reversed); source 0 = the value below the top (popped), 1 =
- * inputs[argument], 2 = constants[argument]; the argument has eight bits, bits 24-31 repeat kind, source, reversed and
- * code as one dense index for the kernel's jump table.  instructions has room for CTB_TILED_MAX_OPS words. */
+/* Diagnostics, no GPU needed.
+ * ctb_tiled_compile: the program as instructions of an accumulator machine with a stack, before subexpressions are shared.  A
+ * word is kind | source << 2 | reversed << 4 | code << 8 | argument << 16 with kind 0 = push the operand, 1 = top =
+ * code(top), 2 = top = top code operand (operand code top when reversed); source 0 = the value below the top (popped), 1 =
+ * inputs[argument], 2 = constants[argument]; bits 24-31 repeat kind, source, reversed and code as one dense index.
+ * instructions has room for CTB_TILED_MAX_OPS words.
+ * ctb_tiled_lower: the words that the kernel of ctb_tiled_broadcast runs, on an accumulator A and n_temps temporaries t.
+ * Bits 0-7 are the operation, 8-9 its argument a; every word has two constants (p, q) of its own:
+ *   0         A = p A + q (one rounding)
+ *   1, 2      A = inputs[a], A = t[a]
+ *   3, 4      A = A x with x = inputs[a], t[a]
+ *   5, 6      A = A + x, or A - x with bit 10 set
+ *   7         A = q
+ *   8 + k     A = unary code CTB_TILED_NEG + k of A
+ *   20 + 10 s + 2 j + r   A = A o x, or x o A with r = 1; o = SUB, DIV, MAX, MIN, POW for j = 0..4; x = inputs[a], q, t[a]
+ *             for s = 0, 1, 2
+ * With bit 11 set, x of operations 3 to 6 enters as p x + q.  Behind the operation, bit 12: A = p A + q; then bits 13 and up,
+ * if k > 0: t[k - 1] = A.  words has room for CTB_TILED_MAX_WORDS, constants_pq for twice as many. */
+#define CTB_TILED_MAX_WORDS 48
 int ctb_tiled_compile(const int32_t* program, int n_ops, int n_inputs, int n_constants, uint32_t* instructions,
                       int* n_instructions);
+int ctb_tiled_lower(const int32_t* program, int n_ops, int n_inputs, const float* constants, int n_constants, uint32_t* words,
+                    float* constants_pq, int* n_words, int* n_temps);
 /* dest = reduction with `op` (CTB_TILED_ADD, _MUL, _MAX or _MIN) of f(src) (a unary code, CTB_TILED_IDENTITY for none)
  * over the dimensions whose bit is set in reduce_mask (bit 0 = first dimension); dest is dense with extent 1 along
  * the reduced dimensions.  Fixed summation order (bitwise repeatable); an empty reduction gives the neutral element. */

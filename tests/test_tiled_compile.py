@@ -1,8 +1,8 @@
-"""The broadcast expression compiler of the library (postfix program -> accumulator-machine instructions), without a
-GPU: ctb_tiled_compile returns the instruction words the kernel would run; a small numpy machine with the documented
-meaning of a word (include/cutile_b200.h) runs them and the result must equal the oracle's value of the expression
-(src/broadcast.jl:19-23: the fused kernel means the plain Julia broadcast).  Bit-exact in float64: the compiler only
-re-orders evaluation and commutes + and *."""
+"""The first stage of the broadcast expression compiler (postfix program -> instructions of an accumulator machine with a
+stack), without a GPU: a small numpy machine with the documented meaning of ctb_tiled_compile's words
+(include/cutile_b200.h) runs them and the result must equal the oracle's value of the expression
+(src/broadcast.jl:19-23: the fused kernel means the plain Julia broadcast).  Bit-exact in float64: this stage only
+re-orders evaluation and commutes + and *.  test_tiled_lower.py covers the program that the kernel runs."""
 import ctypes as C
 
 import numpy as np
