@@ -78,7 +78,9 @@ struct Params {
   int bn;  // columns of a tile: a multiple of 32, at most kTileN
   int stages, stage_bytes;  // per CTA; a stage is a multiple of 1024 bytes
   int tiles_m, tiles_n, num_tiles;
-  int c_tma;  // C starts on 16-byte boundaries: results leave by tiled bulk stores
+  // Results leave by tiled bulk stores (C starts on 16-byte boundaries) in blocks that end at or before this row.  A store
+  // clips in units of 16 bytes: with M off that grid the last block would write into what lies behind C's columns.
+  int tma_rows;
   // Split-K (single-CTA kernel, few tiles): a work unit is (tile, split); split s takes the k-blocks
   // [s * nk / splits, (s + 1) * nk / splits) and leaves its f32 accumulator tile in partial[unit], as blocks of
   // 32 columns x 32 rows (rows contiguous), four blocks per 32 columns; gemm_splitk_reduce_kernel adds the splits in
@@ -103,7 +105,7 @@ __device__ __forceinline__ void stage_block(unsigned char* stage, const uint32_t
 template <typename T>
 __device__ __forceinline__ void store_block(const Params& p, const void* tmapC, T* C, unsigned char* stage,
                                             const uint32_t (&r)[32], int m0, int n0, int b, float* partial, int lane) {
-  if (p.c_tma || partial) {
+  if (partial || m0 + 32 <= p.tma_rows) {
     if (lane == 0) bulk_wait_read<0>();  // the previous store has read the block
     __syncwarp();
     if (partial) stage_block<float>(stage, r, lane);
@@ -328,7 +330,7 @@ __global__ void __launch_bounds__(256)
     }
     T* dst = C + (long long)b * p.strideC + (long long)n * p.ldc + m;
     const float o[4] = {acc.x, acc.y, acc.z, acc.w};
-    if (p.c_tma && m + 3 < p.M) {  // C is aligned and m a multiple of four
+    if (p.tma_rows && m + 3 < p.M) {  // C is aligned and m a multiple of four
       if constexpr (sizeof(T) == 4) {
         *reinterpret_cast<float4*>(dst) = acc;
       } else {
@@ -647,9 +649,10 @@ int launch(ctb_ctx* ctx, cudaStream_t st, const T* A, const T* B, T* C, int M, i
   p.num_tiles = (int)nt;
   p.splits = ch.splits;
   p.partial = nullptr;
-  p.c_tma = (uintptr_t)C % 16 == 0 && ldc * G::ES % 16 == 0 && (batch == 1 || sC * G::ES % 16 == 0);
+  const bool c_aligned = (uintptr_t)C % 16 == 0 && ldc * G::ES % 16 == 0 && (batch == 1 || sC * G::ES % 16 == 0);
+  p.tma_rows = !c_aligned ? 0 : (long long)M * G::ES % 16 == 0 ? INT32_MAX : M;
   tc = ta;  // not used when C is not aligned
-  if (p.c_tma) {
+  if (c_aligned) {
     uint64_t dims[3] = {(uint64_t)M, (uint64_t)N, (uint64_t)batch};
     uint64_t str[2] = {(uint64_t)ldc * G::ES, (uint64_t)(batch > 1 ? sC : ldc * (long long)N) * G::ES};
     uint32_t box[3] = {32, 32, 1};

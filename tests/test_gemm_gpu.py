@@ -169,3 +169,23 @@ def test_gemm_tile_widths_and_result_alignment(cuda, M, N, K, batch, dtype, c_sh
     C.fill_(7.0)
     assert (flat == 7.0).all()
     cuda.check_device_status(0)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float16", "bfloat16"])
+@pytest.mark.parametrize("m,n,k,batch", [(157, 9, 129, 0), (1, 5, 16, 0), (5, 70, 8, 3), (1070, 169, 200, 2), (3, 20, 9000, 0),
+                                         (2043, 1500, 64, 0), (129, 40, 4096, 0)])
+def test_gemm_leaves_what_lies_behind_the_rows(cuda, dtype, m, n, k, batch):
+    """C is a view of a wider array whose rows start on 16-byte boundaries: the columns behind it stay as they are."""
+    import torch
+    dt, lead = getattr(torch, dtype), (batch,) if batch else ()
+    g = torch.Generator(device="cuda").manual_seed(5)
+    unit = 4 if dtype == "float32" else 8
+    up = lambda v: (v + unit - 1) // unit * unit
+    a = (torch.rand(*lead, k, up(m), device="cuda", generator=g) * 2 - 1).to(dt)[..., :m]
+    b = (torch.rand(*lead, n, up(k), device="cuda", generator=g) * 2 - 1).to(dt)[..., :k]
+    for pad in (0, unit):
+        wide = torch.full((*lead, n, up(m) + pad), 7.0, device="cuda", dtype=dt)
+        (cuda.batchmatmul.batch_matmul_kernel if batch else cuda.matmul.matmul_kernel)(a, b, wide[..., :m], 64, 64, 64)
+        assert (wide[..., m:] == 7.0).all()
+        want = b.double() @ a.double()
+        assert ((wide[..., :m].double() - want).norm() / want.norm()).item() <= {"float32": 2e-3, "float16": 2e-3, "bfloat16": 1e-2}[dtype]
