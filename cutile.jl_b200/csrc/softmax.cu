@@ -363,9 +363,9 @@ __global__ void __launch_bounds__(kRowThreads) softmax_long_kernel(T* __restrict
     const int at = tid < head ? tid : nvec * V + tid;
     const float xe = edge ? (float)src[at] : 0.f;
     float m = -FLT_MAX, l = 0.f;
-    if (edge) {
-      m = xe;
-      l = 1.f;
+    if (edge) {  // m stays finite: a masked (-inf) element adds exp(-inf), and so do masked elements behind it
+      m = fmaxf(xe, -FLT_MAX);
+      l = exp_sub(xe, m);
     }
     for (int c = 0; c * kChunkVecs < cnt; ++c) {
       const int p0 = c * kChunkVecs, p1 = min(cnt, p0 + kChunkVecs);

@@ -123,3 +123,29 @@ def test_softmax_any_length_and_alignment(cuda, M, N, dtype, shift):
         assert ref.max_abs_over_max(out.float().cpu().numpy(), want) <= (TOL if dtype == np.float32 else 1e-3)
         assert (guard[:oshift] == 7.0).all() and (guard[oshift + M * N:] == 7.0).all()
     cuda.check_device_status(0)
+
+
+@pytest.mark.parametrize("n", [100, 1000, 1001, 1500, 4097, 8192, 9000, 9001, 26003, 60001, 120001, 300001])
+@pytest.mark.parametrize("half", [False, True])
+def test_softmax_masked_rows(cuda, n, half):
+    """Rows with -inf before, behind and between the values, at every alignment, with the type's lowest value, and one that is
+    masked as a whole (NaN, as 0 / 0): row kernels of every length give what torch gives in f64."""
+    import torch
+    dt = torch.float16 if half else torch.float32
+    g = torch.Generator(device="cuda").manual_seed(n)
+    raw = torch.randn(10 * n + 3, device="cuda", generator=g).to(dt)
+    inf = float("inf")
+    for off in range(3):
+        x = raw.clone()[off:off + 10 * n].view(10, n)
+        for r, part in enumerate((slice(0, 1), slice(0, 40), slice(0, n // 2), slice(0, n - 1), slice(n - 1, n), slice(n - 40, n),
+                                  slice(1, n))):
+            x[r, part] = -inf
+        x[7, ::3] = -inf
+        x[8, : n // 2] = torch.finfo(dt).min
+        x[9] = -inf
+        out = torch.full_like(x, 7.0)
+        cuda.softmax.softmax_chunked_kernel(out, x, n, 1024)
+        want = torch.softmax(x.double(), 1)
+        assert out[9].isnan().all() and want[9].isnan().all()
+        assert ((out[:9].double() - want[:9]).abs().amax(1) <= (1e-3 if half else 2e-6) * want[:9].amax(1)).all()
+        assert (out[:9][x[:9] == -inf] == 0).all()
