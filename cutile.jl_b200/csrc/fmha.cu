@@ -581,6 +581,7 @@ extern "C" int ctb_fmha_fwd(ctb_ctx* ctx, void* stream, const void* Q, const voi
 
   // Few query rows per key/value head: the kernel that splits the keys over the GPU.  The line is where the rows of a group
   // no longer fit its 16-row instructions; a 128-row tile is at least 7/8 padding below it.
+  const int64_t keys = causal ? std::min<int64_t>(seq_kv, (int64_t)input_pos + seq_q) : seq_kv;  // up to the last visible one
   if (fmha_decode_fits(seq_q, query_group_size)) {
     bool taken = false;
     const int r = fmha_decode(ctx, static_cast<cudaStream_t>(stream), Q, K, V, Out, seq_q, seq_kv, heads, kv_heads, batch,
@@ -596,7 +597,9 @@ extern "C" int ctb_fmha_fwd(ctb_ctx* ctx, void* stream, const void* Q, const voi
     if (r) return r;
   }
   {
-    uint64_t dims[3] = {kD, (uint64_t)seq_kv, (uint64_t)(kv_heads * batch)};
+    // to the last visible key: rows of a cache behind it may never have been written, and a probability of zero does not take a
+    // NaN or an infinity out of P V
+    uint64_t dims[3] = {kD, (uint64_t)keys, (uint64_t)(kv_heads * batch)};
     uint64_t str[2] = {kD * 2, (uint64_t)seq_kv * kD * 2};
     int r = make_tmap(&tk, tdt, 3, K, dims, str, box);
     if (r) return r;

@@ -131,9 +131,10 @@ def test_fmha_decode(cuda, batch, heads, kv_heads, seq_q, seq_kv, causal, input_
 
 
 @pytest.mark.parametrize("heads,kv_heads,seq_q,seq_kv,input_pos", [
-    (8, 2, 1, 900, 200), (8, 8, 1, 256, 127), (4, 4, 1, 64, 0), (16, 4, 4, 1000, 380), (5, 5, 16, 700, 256)])
+    (8, 2, 1, 900, 200), (8, 8, 1, 256, 127), (4, 4, 1, 64, 0), (16, 4, 4, 1000, 380), (5, 5, 16, 700, 256),
+    (4, 4, 100, 500, 30), (8, 2, 200, 1000, 333)])  # these with 128-row tiles
 @pytest.mark.parametrize("bf16", [False, True])
-def test_fmha_decode_unwritten_cache(cuda, heads, kv_heads, seq_q, seq_kv, input_pos, bf16):
+def test_fmha_unwritten_cache(cuda, heads, kv_heads, seq_q, seq_kv, input_pos, bf16):
     """Rows of a preallocated cache behind the last visible key are never written by the caller: whatever lies there (NaN and
     infinities included) stays out of the result, which equals that of a cache that ends at the last visible key."""
     import torch
@@ -147,3 +148,4 @@ def test_fmha_decode_unwritten_cache(cuda, heads, kv_heads, seq_q, seq_kv, input
         K[:, :, n:], V[:, :, n:] = bad, bad
         assert torch.equal(run(K, V), want)
     cuda.check_device_status(0)
+
