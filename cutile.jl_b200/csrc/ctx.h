@@ -84,7 +84,7 @@ int* sched_slot(ctb_ctx* ctx);
 // *taken is false, and nothing was launched, when there is no scratch for the parts.
 bool fmha_decode_fits(int64_t seq_q, int group);
 int fmha_decode(ctb_ctx* ctx, cudaStream_t st, const void* Q, const void* K, const void* V, void* Out, int64_t seq_q,
-                int64_t seq_kv, int64_t heads, int64_t kv_heads, int64_t batch, float qk_scale, int input_pos, bool causal,
+                int64_t seq_kv, int64_t heads, int64_t kv_heads, int64_t batch, float qk_scale, int input_pos, int64_t keys, bool causal,
                 bool bf16, bool* taken);
 
 // cuTensorMapEncodeTiled, resolved through the runtime so that the library has

@@ -37,7 +37,7 @@ constexpr int kPartFloats = kMaxRows * (kD + 2);
 struct Params {
   const void* Q;
   void* Out;
-  int seq_q, seq_kv, group, rows;
+  int seq_q, keys, seq_kv, group, rows;  // keys: up to the last one that some query sees
   int input_pos, causal, blocks_per_pair;
   long long blocks;
   float scale_log2;
@@ -113,12 +113,23 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int cta = blockIdx.x, grid = gridDim.x;
   const long long lo = first_block(cta, p.blocks, grid), hi = first_block(cta + 1, p.blocks, grid);
   unsigned char* ring = smem + warp * (kStages * 2 * kTileBytes);
+  // In the last block of a pair the keys end at some warp's tile; the warps behind it have none there.
+  auto tiles_of = [&](int block) { return min(kWarps, (p.keys - block * kBlockKeys + kTileKeys - 1) / kTileKeys); };
   int issued = 0;
-  const int ntiles = (int)(hi - lo);
-  auto issue = [&]() {  // the warp's tile of block lo + issued
-    const long long b = lo + issued;
-    const int pair = (int)(b / p.blocks_per_pair), key0 = (int)(b - (long long)pair * p.blocks_per_pair) * kBlockKeys + warp * kTileKeys;
-    const int s = issued % kStages;
+  // the block of the warp's next tile to ask for: pair, block of the pair, blocks left of the CTA's range
+  int a_pair = (int)(lo / p.blocks_per_pair), a_block = (int)(lo - (long long)a_pair * p.blocks_per_pair), a_left = (int)(hi - lo);
+  auto issue = [&]() {
+    auto next = [&]() {
+      --a_left;
+      if (++a_block == p.blocks_per_pair) {
+        a_block = 0;
+        ++a_pair;
+      }
+    };
+    while (a_left > 0 && warp >= tiles_of(a_block)) next();
+    if (a_left <= 0) return;
+    const int pair = a_pair, key0 = a_block * kBlockKeys + warp * kTileKeys, s = issued % kStages;
+    next();
     if (lane == 0) {
       unsigned char* dst = ring + s * (2 * kTileBytes);
       mbar_expect_tx(&full[warp][s], 2 * kTileBytes);
@@ -127,19 +138,14 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     ++issued;
   };
-  for (int s = 0; s < kStages && s < ntiles; ++s) issue();
+  for (int s = 0; s < kStages; ++s) issue();
 
   // this lane's ldmatrix rows inside a tile: matrix lane / 8, row lane % 8
   const int mi = lane >> 3, mr = lane & 7;
   bool ok = true;
   int n = 0;  // tiles consumed
-  for (long long b = lo; b < hi;) {
-    const int pair = (int)(b / p.blocks_per_pair);
-    const long long pair_first = (long long)pair * p.blocks_per_pair, pair_end = pair_first + p.blocks_per_pair;
-    const long long end = min(hi, pair_end);
-    // ---- Q: rows g and g + 8 (row = head in group * seq_q + position)
-    uint32_t q[4][4];
-    int lim[2];  // last visible key of the two rows
+  // Q of a pair: rows g and g + 8 (row = head in group * seq_q + position)
+  auto load_q = [&](uint32_t (&q)[4][4], int pair) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int row = g + 8 * h;
@@ -152,21 +158,43 @@ __global__ void __launch_bounds__(kThreads, 1)
         q[k][h] = live ? src[k * 8 + t] : 0u;
         q[k][2 + h] = live ? src[k * 8 + 4 + t] : 0u;
       }
-      lim[h] = p.causal ? min(p.input_pos + pos, p.seq_kv - 1) : p.seq_kv - 1;
     }
+  };
+  int lim[2];  // last visible key of the two rows
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int row = g + 8 * h, pos = row - row / p.seq_q * p.seq_q;
+    lim[h] = p.causal ? min(p.input_pos + pos, p.seq_kv - 1) : p.seq_kv - 1;
+  }
+  uint32_t q_next[4][4];  // asked for a pair ahead: with few keys a pair is over before its Q would have come
+  load_q(q_next, (int)(lo / p.blocks_per_pair));
+  int pair = (int)(lo / p.blocks_per_pair) - 1;
+  for (long long b = lo; b < hi;) {
+    ++pair;
+    const long long pair_first = (long long)pair * p.blocks_per_pair, pair_end = pair_first + p.blocks_per_pair;
+    const long long end = min(hi, pair_end);
+    int block = (int)(b - pair_first);
+    const int live = tiles_of(block);  // warps that have keys of this part
+    uint32_t q[4][4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+      for (int h = 0; h < 4; ++h) q[k][h] = q_next[k][h];
+    if (pair_end < hi) load_q(q_next, pair + 1);
     float o[8][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
 #pragma unroll
     for (int j = 0; j < 8; ++j)
 #pragma unroll
       for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
     // ---- the warp's tiles of the pair
-    for (; b < end; ++b) {
+    for (; b < end; ++b, ++block) {
+      if (warp >= tiles_of(block)) continue;
       const int s = n % kStages;
       if (ok) ok = CTB_WARP_WAIT(&full[warp][s], (n / kStages) & 1, status, DEV_TIMEOUT_TMA);
       if (!ok) continue;  // n stays at the tile that did not come
       ++n;
       const uint32_t sK = smem_u32(ring + s * (2 * kTileBytes)), sV = sK + kTileBytes;
-      const int key0 = (int)(b - pair_first) * kBlockKeys + warp * kTileKeys;
+      const int key0 = block * kBlockKeys + warp * kTileKeys;
       float sc[4][4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {  // eight keys at a time
@@ -224,11 +252,12 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
       }
       __syncwarp();  // every lane has read the stage
-      if (issued < ntiles) issue();
+      issue();
     }
     // ---- leaving the pair: the warps' results meet
 #pragma unroll
     for (int h = 0; h < (R == 16 ? 2 : 1); ++h) {
+      if (warp >= live) break;
       l[h] += __shfl_xor_sync(0xffffffffu, l[h], 1);
       l[h] += __shfl_xor_sync(0xffffffffu, l[h], 2);
       if (t == 0) {
@@ -246,10 +275,12 @@ __global__ void __launch_bounds__(kThreads, 1)
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     if (mine) {
 #pragma unroll
-      for (int w = 0; w < kWarps; ++w) M = fmaxf(M, ml[0][w][row]);
+      for (int w = 0; w < kWarps; ++w)
+        if (w < live) M = fmaxf(M, ml[0][w][row]);
       const float ref = M == -INFINITY ? 0.f : M;
 #pragma unroll
       for (int w = 0; w < kWarps; ++w) {  // ascending: a fixed order
+        if (w >= live) break;
         const float f = ex2_approx_ftz(ml[0][w][row] - ref);
         const float4 v = *reinterpret_cast<const float4*>(outs + (w * R + row) * kPitch + d0);
         L += ml[1][w][row] * f;
@@ -320,7 +351,7 @@ namespace ctb_internal {
 bool fmha_decode_fits(int64_t seq_q, int group) { return seq_q * group <= kMaxRows; }
 
 int fmha_decode(ctb_ctx* ctx, cudaStream_t st, const void* Q, const void* K, const void* V, void* Out, int64_t seq_q,
-                int64_t seq_kv, int64_t heads, int64_t kv_heads, int64_t batch, float qk_scale, int input_pos, bool causal,
+                int64_t seq_kv, int64_t heads, int64_t kv_heads, int64_t batch, float qk_scale, int input_pos, int64_t keys, bool causal,
                 bool bf16, bool* taken) {
   const StreamScratch scratch(ctx, st);
   *taken = scratch.data != nullptr;
@@ -328,9 +359,7 @@ int fmha_decode(ctb_ctx* ctx, cudaStream_t st, const void* Q, const void* K, con
   const CUtensorMapDataType tdt = bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   CUtensorMap tk, tv;
   const uint32_t box[3] = {kD, kTileKeys, 1};
-  // The maps end at the last key that some query sees: rows of a cache behind it may never have been written, and a
-  // probability of zero does not take a NaN or an infinity out of P V.  The copies fill with zeros there and read nothing.
-  const int64_t keys = causal ? std::min<int64_t>(seq_kv, (int64_t)input_pos + seq_q) : seq_kv;
+  // The maps end at the last key that some query sees (see ctb_fmha_fwd); the copies fill with zeros there and read nothing.
   uint64_t dims[3] = {kD, (uint64_t)keys, (uint64_t)(kv_heads * batch)};
   uint64_t str[2] = {kD * 2, (uint64_t)seq_kv * kD * 2};
   int r = make_tmap(&tk, tdt, 3, K, dims, str, box);
@@ -339,7 +368,7 @@ int fmha_decode(ctb_ctx* ctx, cudaStream_t st, const void* Q, const void* K, con
   if (r) return r;
   Params p;
   p.Q = Q; p.Out = Out;
-  p.seq_q = (int)seq_q; p.seq_kv = (int)seq_kv; p.group = (int)(heads / kv_heads);
+  p.seq_q = (int)seq_q; p.keys = (int)keys; p.seq_kv = (int)seq_kv; p.group = (int)(heads / kv_heads);
   p.rows = p.group * p.seq_q;
   p.input_pos = input_pos; p.causal = causal ? 1 : 0;
   p.scale_log2 = qk_scale * 1.4426950408889634f;
