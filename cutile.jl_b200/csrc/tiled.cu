@@ -85,10 +85,11 @@ struct Program {
 enum : int {
   OP_LINEAR = 0,  // laid out like the destination, aligned: a vector of four elements per group
   OP_SCALAR = 1,  // a single element
-  OP_ROW = 2,     // expanded, first extent a multiple of four: one aligned vector, or one element, per group
+  OP_ROW = 2,     // expanded, first extent a multiple of four: one aligned vector per group
   OP_SHIFTED = 3, // laid out like the destination, not aligned: element by element
   OP_ELEM = 4,    // anything else: element by element, each with its own coordinates
   OP_VECTOR = 5,  // OP_ROW that varies along the first dimension only (a bias): one aligned vector per group
+  OP_GROUP = 7,   // expanded along the first dimension, whose extent is a multiple of four: one element per group
   OP_FIXED = 6    // varies along the first dimension only, and the grid is such that every group of a thread lies at the
                   // same place of it: four elements per thread, read once
 };
@@ -630,7 +631,7 @@ inline FastDiv fast_div(unsigned d) {
 struct Extents {
   long long n;          // elements of the destination
   long long full_below; // a trip that starts at a group below this has all its groups
-  FastDiv row, col;     // row: groups (OP_ROW, OP_VECTOR) or elements (OP_ELEM) of the first dimension; col: the second extent
+  FastDiv row, col;     // row: groups (OP_ROW, OP_GROUP, OP_VECTOR) or elements (OP_ELEM) of the first dimension; col: the second extent
   unsigned d0;          // OP_FIXED: the first extent
   int fixed_vec;        // OP_FIXED: the four elements are one aligned vector
   int dest_vec;         // the destination is aligned for vector stores
@@ -662,6 +663,9 @@ __global__ void __launch_bounds__(256, NT == 0 || NT == 2 ? 4 : 3)
   const unsigned tid = threadIdx.x;
   const unsigned smem0 = smem_addr(tiled_smem) + tid * VB;
   auto slot = [&](unsigned buf, unsigned a) { return smem0 + in.slot[a] + buf * (G * 256 * VB); };
+  auto element = [&](unsigned buf, unsigned a, int g) {  // of OP_GROUP
+    return smem_addr(tiled_smem) + in.slot[a] + ((buf * G + g) * 256 + tid) * ES;
+  };
 
   long long i = (long long)blockIdx.x * blockDim.x + tid;
 
@@ -699,19 +703,15 @@ __global__ void __launch_bounds__(256, NT == 0 || NT == 2 ? 4 : 3)
 #pragma unroll
           for (int e = 0; e < V; ++e) copy_element<T>(to + g * (256 * VB) + e * ES, e < live ? src + e : base, e < live);
         }
-      } else if (!LINEAR && mode == OP_ROW) {  // the extent is a multiple of four: a group exists as a whole or not at all
+      } else if (!LINEAR && (mode == OP_ROW || mode == OP_GROUP)) {  // a group exists as a whole or not at all
 #pragma unroll
         for (int g = 0; g < G; ++g) {
           const int live = live_of(g);
           const unsigned u = live ? (unsigned)at + g * (unsigned)grid_stride : 0u;
           const unsigned r = x.row.div(u), i0 = (u - r * x.row.d) * V, i2 = x.col.div(r), i1 = r - i2 * x.col.d;
           const T* src = base + (i0 * in.stride[a][0] + i1 * in.stride[a][1] + i2 * in.stride[a][2]);
-          if (in.stride[a][0]) {
-            cp_async_group<VB>(to + g * (256 * VB), src, live * ES);
-          } else {
-#pragma unroll
-            for (int e = 0; e < V; ++e) copy_element<T>(to + g * (256 * VB) + e * ES, src, live != 0);
-          }
+          if (mode == OP_ROW) cp_async_group<VB>(to + g * (256 * VB), src, live * ES);
+          else copy_element<T>(element(buf, a, g), src, live != 0);
         }
       } else if (!LINEAR && mode == OP_ELEM) {
 #pragma unroll
@@ -759,6 +759,21 @@ __global__ void __launch_bounds__(256, NT == 0 || NT == 2 ? 4 : 3)
       for (int g = 0; g < G; ++g) {
         t[2 * g] = lo;
         t[2 * g + 1] = hi;
+      }
+      return;
+    }
+    if (!LINEAR && in.mode[a] == OP_GROUP) {
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        float c;
+        if constexpr (sizeof(T) == 4) {
+          asm volatile("ld.shared.f32 %0, [%1];" : "=f"(c) : "r"(element(buf, a, g)));
+        } else {
+          unsigned short h;
+          asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h) : "r"(element(buf, a, g)));
+          c = __half2float(__ushort_as_half(h));
+        }
+        t[2 * g] = t[2 * g + 1] = pair(c, c);
       }
       return;
     }
@@ -950,7 +965,7 @@ int launch_broadcast(ctb_ctx* ctx, cudaStream_t st, void* dest, Operands& in, co
     if (vector && fixed_grid > 0) {
       in.mode[a] = OP_FIXED;
       fixed = true;
-    } else if (in.mode[a] == OP_VECTOR || in.mode[a] == OP_ROW || in.mode[a] == OP_ELEM) {
+    } else if (in.mode[a] == OP_VECTOR || in.mode[a] == OP_ROW || in.mode[a] == OP_GROUP || in.mode[a] == OP_ELEM) {
       linear = false;
     }
   }
@@ -964,7 +979,8 @@ int launch_broadcast(ctb_ctx* ctx, cudaStream_t st, void* dest, Operands& in, co
   unsigned smem = 0;
   for (int a = 0; a < n_inputs; ++a) {
     in.slot[a] = smem;
-    if (in.mode[a] != OP_SCALAR) smem += (in.mode[a] == OP_FIXED ? 1 : 2 * G) * 256 * VB;
+    if (in.mode[a] == OP_GROUP) smem += 2 * G * 256 * sizeof(T);
+    else if (in.mode[a] != OP_SCALAR) smem += (in.mode[a] == OP_FIXED ? 1 : 2 * G) * 256 * VB;
   }
   x.full_below = x.n / 4 - (long long)(G - 1) * grid * 256;  // a trip's last group is (G - 1) grids further on
   auto kernel = linear ? tiled_broadcast_kernel<T, G, NT, true> : tiled_broadcast_kernel<T, G, NT, false>;
@@ -1243,14 +1259,15 @@ int ctb_tiled_broadcast(ctb_ctx* ctx, void* stream, void* dest, const int64_t* s
     if (single) in.mode[a] = OP_SCALAR;
     else if (like_dest) in.mode[a] = aligned ? OP_LINEAR : OP_SHIFTED;
     else if (d0 % 4 == 0 && s0 == 1 && aligned && s1 == 0 && s2 == 0) in.mode[a] = OP_VECTOR;
-    else if (d0 % 4 == 0 && (s0 == 0 || (s0 == 1 && aligned && s1 % 4 == 0 && s2 % 4 == 0))) in.mode[a] = OP_ROW;
+    else if (d0 % 4 == 0 && s0 == 0) in.mode[a] = OP_GROUP;
+    else if (d0 % 4 == 0 && s0 == 1 && aligned && s1 % 4 == 0 && s2 % 4 == 0) in.mode[a] = OP_ROW;
     else in.mode[a] = OP_ELEM;
-    if (in.mode[a] == OP_ROW || in.mode[a] == OP_ELEM || in.mode[a] == OP_VECTOR) linear = false;
+    if (in.mode[a] == OP_ROW || in.mode[a] == OP_GROUP || in.mode[a] == OP_ELEM || in.mode[a] == OP_VECTOR) linear = false;
     if (in.mode[a] == OP_ELEM) by_element = true;
   }
   if (by_element)  // one pair of divisors serves both kinds: by element then
     for (int a = 0; a < n_inputs; ++a)
-      if (in.mode[a] == OP_ROW || in.mode[a] == OP_VECTOR) in.mode[a] = OP_ELEM;
+      if (in.mode[a] == OP_ROW || in.mode[a] == OP_GROUP || in.mode[a] == OP_VECTOR) in.mode[a] = OP_ELEM;
   if (!linear) {
     if ((by_element ? x.n : x.n / 4) > 0x7fffffffLL)
       return fail(CTB_UNSUPPORTED, "ctb_tiled_broadcast: too many elements for an expanded operand");
