@@ -1030,15 +1030,16 @@ __global__ void __launch_bounds__(256)
   constexpr int op = OP;
   auto fmap = [&](float v) { return MAPPED ? unary(f_code, v) : v; };
   __shared__ float wsum[8];
-  auto block_combine = [&](float acc) {  // valid in thread 0
+  auto block_combine = [&](float acc) {  // valid in thread 0; the CTA has met since an earlier call
 #pragma unroll
     for (int sh = 16; sh > 0; sh >>= 1) acc = binary(op, acc, __shfl_xor_sync(0xffffffffu, acc, sh));
-    __syncthreads();
     if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = acc;
     __syncthreads();
-    float t = wsum[0];
-    for (int w = 1; w < 8; ++w) t = binary(op, t, wsum[w]);
-    return t;
+    if (threadIdx.x == 0) {
+      acc = wsum[0];
+      for (int w = 1; w < 8; ++w) acc = binary(op, acc, wsum[w]);
+    }
+    return acc;
   };
   const long long part = blockIdx.y;
   const long long lo = part * s.chunk, hi = min(s.red_len, lo + s.chunk);
@@ -1050,8 +1051,12 @@ __global__ void __launch_bounds__(256)
   const long long d0 = s.d[0];
   constexpr int V = 16 / sizeof(T);
   float acc = neutral(op);
-  for (long long row = lo / d0; row * d0 < hi; ++row) {  // rows of the reduced index space that this part touches
-    const long long r1 = row % s.red_n[1], r2 = row / s.red_n[1];
+  long long row = lo / d0, r1 = row % s.red_n[1], r2 = row / s.red_n[1];
+  for (; row * d0 < hi; ++row, ++r1) {  // rows of the reduced index space that this part touches
+    if (r1 == s.red_n[1]) {
+      r1 = 0;
+      ++r2;
+    }
     const long long rbase = base + r1 * st1 + r2 * st2;
     const long long c_lo = max(lo - row * d0, 0ll), c_hi = min(hi - row * d0, d0);
     const bool vec = ((rbase + c_lo) * (long long)sizeof(T) + (long long)(uintptr_t)src) % 16 == 0;
@@ -1348,9 +1353,19 @@ int ctb_tiled_mapreduce(ctb_ctx* ctx, void* stream, void* dest, const void* src,
   for (int k = 0; k < 3; ++k) {
     if (shape[k] < 0) return fail(CTB_BAD_ARG, "ctb_tiled_mapreduce: negative extent");
     s.d[k] = shape[k];
+  }
+  // Reduced dimensions behind a reduced first one are contiguous with it: one long row instead of many that may be short.
+  for (int k = 0; k < 2 && (reduce_mask & 1); ++k)
+    if ((reduce_mask & 2) || s.d[1] == 1) {
+      s.d[0] *= s.d[1];
+      s.d[1] = s.d[2];
+      s.d[2] = 1;
+      reduce_mask = 1 | ((reduce_mask >> 1) & 2);
+    }
+  for (int k = 0; k < 3; ++k) {
     const bool red = (reduce_mask >> k) & 1;
-    s.keep_n[k] = red ? 1 : shape[k];
-    s.red_n[k] = red ? shape[k] : 1;
+    s.keep_n[k] = red ? 1 : s.d[k];
+    s.red_n[k] = red ? s.d[k] : 1;
     s.outputs *= s.keep_n[k];
     s.red_len *= s.red_n[k];
   }
