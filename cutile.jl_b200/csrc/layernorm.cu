@@ -471,6 +471,14 @@ __global__ void __launch_bounds__(kBwdThreads)
 __device__ __forceinline__ void cluster_columns(float* mine, float* __restrict__ DW, float* __restrict__ DB, int N, int g) {
   cg::cluster_group cluster = cg::this_cluster();
   const int C = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  if (C == 1) {
+    __syncthreads();
+    for (int c = threadIdx.x; c < N; c += blockDim.x) {
+      DW[(long long)g * N + c] = mine[c];
+      DB[(long long)g * N + c] = mine[N + c];
+    }
+    return;
+  }
   cluster.sync();
   for (int c = rank * blockDim.x + threadIdx.x; c < N; c += C * blockDim.x) {
     float a = 0.f, b = 0.f;
