@@ -315,6 +315,27 @@ def test_tanh_accuracy(cuda):
     assert torch.isnan(out).all()
 
 
+@pytest.mark.parametrize("half", [False, True])
+@pytest.mark.parametrize("shape,col", [((300, 64), (300, 1)), ((7, 4), (7, 1)), ((1, 4096), (1, 1)), ((5, 33, 260), (33, 1)),
+                                       ((5, 33, 260), (5, 1, 1)), ((5, 33, 260), (5, 33, 1)), ((1030, 1028), (1030, 1))])
+def test_broadcast_operand_expanded_along_the_first_dimension(cuda, shape, col, half):
+    """One element per group of four (the first extent is a multiple of four), beside operands of other kinds."""
+    import torch
+    T, dt = cuda.tiled, torch.float16 if half else torch.float32
+    g = torch.Generator(device="cuda").manual_seed(31)
+    r = lambda s: torch.randn(*s, device="cuda", generator=g).to(dt)
+    a, c, row = r(shape), r((1,) * (len(shape) - len(col)) + col), r(shape[-1:])
+    if len(col) < len(shape):
+        c = c.view(col)  # dimensions are aligned from the first (last torch) one
+    out = torch.empty_like(a)
+    A, C, R = (t.double() for t in (a, c, row))
+    for expr, want in ((T.Tiled(a) * T.Tiled(c), A * C), (T.Tiled(a) + T.Tiled(c) * T.Tiled(row), A + C * R),
+                       (T.Tiled(c) - T.Tiled(a[..., :1].contiguous()), (C - A[..., :1]).expand(shape))):
+        T.assign(out, expr)
+        scale = want.abs().max()
+        assert ((out.double() - want).abs().max() / scale).item() <= (1e-3 if half else 2.5e-7)  # rounding of the result (and of c * row)
+
+
 @pytest.mark.parametrize("hints", [{}, {"occupancy": 2}])  # the native path, the Python path
 def test_broadcast_signed_zero_constants(cuda, hints):
     """0.0 and -0.0 in one expression stay two constants."""
