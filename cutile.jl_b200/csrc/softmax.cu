@@ -510,6 +510,38 @@ __global__ void __launch_bounds__(kThreads) softmax_online_kernel(T* __restrict_
   }
 }
 
+// Teams (clusters of C CTAs) of softmax_long_kernel that run at once, with at most four CTAs per SM.  A team more would begin
+// when another has done all its rows.  How many clusters fit depends on how many CTAs an SM takes: asked once per device for each.
+template <typename T>
+int long_teams(ctb_ctx* ctx, size_t smem, int C) {
+  int per_sm = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, softmax_long_kernel<T>, kRowThreads, smem);
+  per_sm = std::max(1, std::min(4, per_sm));
+  if (C == 1) return ctx->sm_count * per_sm;
+  static int cached[16][kMaxCluster + 1][5] = {};
+  int& n = cached[ctx->device & 15][C][per_sm];
+  if (n == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctx->sm_count * 4 / C * C);
+    cfg.blockDim = dim3(kRowThreads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = C;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int m = 0;
+    if (cudaOccupancyMaxActiveClusters(&m, softmax_long_kernel<T>, &cfg) != cudaSuccess || m < 1) {
+      (void)cudaGetLastError();
+      return std::max(1, ctx->sm_count * per_sm / C);
+    }
+    n = std::min(m, ctx->sm_count * per_sm / C);
+  }
+  return n;
+}
+
 template <typename T>
 int launch(ctb_ctx* ctx, cudaStream_t st, T* out, const T* in, int N, int M, long long ldo, long long ldi,
            int variant, int tile_size) {
@@ -567,8 +599,7 @@ int launch(ctb_ctx* ctx, cudaStream_t st, T* out, const T* in, int N, int M, lon
     auto k = softmax_long_kernel<T>;
     cudaError_t e = allow_smem(k, kLongBytes);
     if (e != cudaSuccess) return cuda_fail(e, "ctb_softmax: shared memory opt-in");
-    const int per_sm = std::max(1, std::min(4, (int)((size_t)222 * 1024 / (smem + 2048))));
-    const int teams = std::max(1, std::min(M, ctx->sm_count * per_sm / C));
+    const int teams = std::min(M, long_teams<T>(ctx, smem, C));
     launch_kernel(k, teams * C, kRowThreads, smem, st, C, out, in, N, M, ldo, ldi, per, C, ctx->dev_status);
   } else {
     int per_sm = 8;
