@@ -264,6 +264,16 @@ function fft_kernel(x_packed_in::CuArray{Float32,3}, y_packed_out::CuArray{Float
         dptr(T1), N, F0, F1, F2, batch, BS, D))
 end
 
+"The same for the twiddle tables T0, T1 of make_twiddles; the DFT matrices are the exact ones and are not passed."
+function fft_plan_kernel(x_packed_in::CuArray{Float32,3}, y_packed_out::CuArray{Float32,3}, T0::CuArray{Float32,3},
+                         T1::CuArray{Float32,3}, N::Int, F0::Int, F1::Int, F2::Int, BS::Int, D::Int; opts...)
+    size(x_packed_in) == size(y_packed_out) || throw(ArgumentError("fft_plan_kernel: x and y differ in shape"))
+    batch = length(x_packed_in) ÷ 2N
+    check(ccall((:ctb_fft_plan, LIB), Cint,
+        (Ptr{Cvoid}, Ptr{Cvoid}, Ptr{Cvoid}, Ptr{Cvoid}, Ptr{Cvoid}, Ptr{Cvoid}, Int64, Cint, Cint, Cint, Int64, Cint, Cint),
+        context(), launch_opts(; opts...), dptr(x_packed_in), dptr(y_packed_out), dptr(T0), dptr(T1), N, F0, F1, F2, batch, BS, D))
+end
+
 # ---- building blocks of the expert-parallel MoE ----
 "dst(:, i) = src(:, cld(ids[i], num_token_replicas)); ids out of range give zero rows."
 function moe_gather_rows(dst::CuArray{Float16,2}, src::CuArray{Float16,2}, ids::CuArray{Int32,1}, num_token_replicas::Int)
