@@ -13,12 +13,16 @@
 // S = Q K^T and O += P V are m16n8k16 tensor-core instructions on registers (a 128-row tcgen05 tile would be 88 % padding;
 // the tensor work here is a few per cent of what either path delivers): Q stays in registers for the pair, K enters by
 // ldmatrix, the probabilities go from the accumulator layout straight into the A operand, V by transposed ldmatrix.
+// In the last block of a pair the warps behind the last key ask for nothing and have no part in what follows, and Q of the next
+// pair is asked for before the warps meet: short heads are bound by these latencies (8192 heads of one row and 100 keys: 126 us
+// when every warp took a tile and Q was asked for in its turn, 84 now; 3200 of 16 x 16: 70 and 39).
 // Leaving a pair, the warps' results meet in shared memory; a pair that one CTA covers is written at once, otherwise the
 // part goes to scratch and the CTA that arrives last adds the parts in ascending order.
 #include <cuda_bf16.h>
 #include <math.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "ctx.h"
 #include "ptx.cuh"
@@ -114,7 +118,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   const long long lo = first_block(cta, p.blocks, grid), hi = first_block(cta + 1, p.blocks, grid);
   unsigned char* ring = smem + warp * (kStages * 2 * kTileBytes);
   // In the last block of a pair the keys end at some warp's tile; the warps behind it have none there.
-  auto tiles_of = [&](int block) { return min(kWarps, (p.keys - block * kBlockKeys + kTileKeys - 1) / kTileKeys); };
+  const int last_block = p.blocks_per_pair - 1, last_tiles = min(kWarps, (p.keys - last_block * kBlockKeys + kTileKeys - 1) / kTileKeys);
+  auto tiles_of = [&](int block) { return block == last_block ? last_tiles : kWarps; };
   int issued = 0;
   // the block of the warp's next tile to ask for: pair, block of the pair, blocks left of the CTA's range
   int a_pair = (int)(lo / p.blocks_per_pair), a_block = (int)(lo - (long long)a_pair * p.blocks_per_pair), a_left = (int)(hi - lo);
@@ -166,7 +171,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int row = g + 8 * h, pos = row - row / p.seq_q * p.seq_q;
     lim[h] = p.causal ? min(p.input_pos + pos, p.seq_kv - 1) : p.seq_kv - 1;
   }
-  uint32_t q_next[4][4];  // asked for a pair ahead: with few keys a pair is over before its Q would have come
+  uint32_t q_next[4][4];  // asked for before the warps of the last pair meet: with few keys a pair is over before its Q would have come
   load_q(q_next, (int)(lo / p.blocks_per_pair));
   int pair = (int)(lo / p.blocks_per_pair) - 1;
   for (long long b = lo; b < hi;) {
@@ -180,15 +185,14 @@ __global__ void __launch_bounds__(kThreads, 1)
     for (int k = 0; k < 4; ++k)
 #pragma unroll
       for (int h = 0; h < 4; ++h) q[k][h] = q_next[k][h];
-    if (pair_end < hi) load_q(q_next, pair + 1);
     float o[8][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
 #pragma unroll
     for (int j = 0; j < 8; ++j)
 #pragma unroll
       for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
     // ---- the warp's tiles of the pair
-    for (; b < end; ++b, ++block) {
-      if (warp >= tiles_of(block)) continue;
+    const long long mine_end = end == pair_end && warp >= last_tiles ? end - 1 : end;
+    for (; b < mine_end; ++b, ++block) {
       const int s = n % kStages;
       if (ok) ok = CTB_WARP_WAIT(&full[warp][s], (n / kStages) & 1, status, DEV_TIMEOUT_TMA);
       if (!ok) continue;  // n stays at the tile that did not come
@@ -254,6 +258,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       __syncwarp();  // every lane has read the stage
       issue();
     }
+    b = end;
+    if (pair_end < hi) load_q(q_next, pair + 1);
     // ---- leaving the pair: the warps' results meet
 #pragma unroll
     for (int h = 0; h < (R == 16 ? 2 : 1); ++h) {
@@ -273,19 +279,24 @@ __global__ void __launch_bounds__(kThreads, 1)
     const bool mine = row < R && row < p.rows;
     float M = -INFINITY, L = 0.f;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (mine) {
+    auto meet = [&](auto all_tag) {  // the results of all warps, or of the first `live`
+      constexpr bool ALL = decltype(all_tag)::value;
 #pragma unroll
       for (int w = 0; w < kWarps; ++w)
-        if (w < live) M = fmaxf(M, ml[0][w][row]);
+        if (ALL || w < live) M = fmaxf(M, ml[0][w][row]);
       const float ref = M == -INFINITY ? 0.f : M;
 #pragma unroll
       for (int w = 0; w < kWarps; ++w) {  // ascending: a fixed order
-        if (w >= live) break;
+        if (!ALL && w >= live) break;
         const float f = ex2_approx_ftz(ml[0][w][row] - ref);
         const float4 v = *reinterpret_cast<const float4*>(outs + (w * R + row) * kPitch + d0);
         L += ml[1][w][row] * f;
         acc.x += v.x * f; acc.y += v.y * f; acc.z += v.z * f; acc.w += v.w * f;
       }
+    };
+    if (mine) {
+      if (live == kWarps) meet(std::true_type());
+      else meet(std::false_type());
     }
     auto write_out = [&]() {
       const float inv = rcp_approx_ftz(L);
