@@ -580,13 +580,10 @@ extern "C" int ctb_fmha_fwd(ctb_ctx* ctx, void* stream, const void* Q, const voi
     return fail(CTB_BAD_ALIGN, "ctb_fmha_fwd: Q, K, V, Out must be 16-byte aligned");
 
   // Few query rows per key/value head: the kernel that splits the keys over the GPU.  The line is where the rows of a group
-  // no longer fit its 16-row instructions; a 128-row tile is at least 7/8 padding below it.  That padding is cheaper than the
-  // other kernel's barriers per key/value head when a head is one short tile that no other head reads: many heads of a group
-  // of one, 9 to 16 rows, 33 to 256 keys (4800 heads, 16 rows, 100 keys: 88 us there, 78 here; 256 keys 108 and 98; 600 heads
-  // 20 and 20; 16 keys 55 and 57; 8 rows 76 and 78; a group of two 88 and 143).
+  // no longer fit its 16-row instructions; a 128-row tile is at least 7/8 padding below it (4800 heads of 16 rows: 61 us there and
+  // 78 with 128-row tiles for 40 keys, 72 and 76 for 128, 86 and 98 for 256).
   const int64_t keys = causal ? std::min<int64_t>(seq_kv, (int64_t)input_pos + seq_q) : seq_kv;  // up to the last visible one
-  const bool short_heads = query_group_size == 1 && seq_q > 8 && keys > 32 && keys <= 256 && heads * batch >= 16 * ctx->sm_count;
-  if (fmha_decode_fits(seq_q, query_group_size) && !short_heads) {
+  if (fmha_decode_fits(seq_q, query_group_size)) {
     bool taken = false;
     const int r = fmha_decode(ctx, static_cast<cudaStream_t>(stream), Q, K, V, Out, seq_q, seq_kv, heads, kv_heads, batch,
                               qk_scale, input_pos, keys, causal != 0, dtype == CTB_BF16, &taken);

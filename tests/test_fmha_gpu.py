@@ -132,7 +132,7 @@ def test_fmha_decode(cuda, batch, heads, kv_heads, seq_q, seq_kv, causal, input_
 
 @pytest.mark.parametrize("heads,kv_heads,seq_q,seq_kv,input_pos", [
     (8, 2, 1, 900, 200), (8, 8, 1, 256, 127), (4, 4, 1, 64, 0), (16, 4, 4, 1000, 380), (5, 5, 16, 700, 256),
-    (4, 4, 100, 500, 30), (8, 2, 200, 1000, 333), (1184, 1184, 10, 200, 90)])  # these with 128-row tiles
+    (4, 4, 100, 500, 30), (8, 2, 200, 1000, 333), (1184, 1184, 10, 200, 90)])  # two with 128-row tiles, many heads
 @pytest.mark.parametrize("bf16", [False, True])
 def test_fmha_unwritten_cache(cuda, heads, kv_heads, seq_q, seq_kv, input_pos, bf16):
     """Rows of a preallocated cache behind the last visible key are never written by the caller: whatever lies there (NaN and
@@ -153,7 +153,7 @@ def test_fmha_unwritten_cache(cuda, heads, kv_heads, seq_q, seq_kv, input_pos, b
 @pytest.mark.parametrize("batch,heads,seq_q,seq_kv", [(3, 800, 16, 100), (2, 1184, 9, 33), (2, 1184, 16, 256), (2, 1184, 16, 257),
                                                      (2, 1184, 16, 32), (4, 600, 8, 100), (100, 16, 12, 12)])
 def test_fmha_many_short_heads(cuda, batch, heads, seq_q, seq_kv):
-    """On both sides of the line between the two kernels: few rows, few keys, many heads."""
+    """Few rows, few keys, many heads: warps without keys, several heads per CTA and Q of the next."""
     d = inputs.fmha(batch, heads, seq_q, seq_kv, 64, seed=29)
     out = run(cuda, d, causal=True, input_pos=seq_kv - seq_q)
     want = ref.fmha(d["Q"], d["K"], d["V"], causal=True, input_pos=seq_kv - seq_q)
