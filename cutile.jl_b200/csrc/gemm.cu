@@ -89,34 +89,38 @@ struct Params {
   float* partial;
 };
 
-// Results on their way out.  An epilogue warp owns 32 rows (lane = row) of 32 columns at a time: it writes them to its
+// Results on their way out.  An epilogue warp owns 32 rows (lane = row) of 32 columns at a time: it writes them to a
 // staging block in shared memory (a row of the block = 32 consecutive rows of a column of C, no bank conflicts)
 // and lane 0 sends the block off with one tiled bulk store, which clips at the edges of C; the next block's TMEM load runs
 // meanwhile.  Stored from registers, a tile of 128 x 256 cost about 10 us per CTA (12 x 1024 x 512 in bf16 with a single
-// k-block: 23.5 us), more than its main loop for K up to 2000.
-constexpr int kStageBlock = 32 * 32 * 4;             // bytes of a staging block (f32)
-constexpr int kEpiBytes = kEpiWarps * kStageBlock;
+// k-block: 23.5 us), more than its main loop for K up to 2000.  A warp has two blocks of 2 KB (16 columns in f32) and fills one
+// while the other is read: with one, the last tile's results of 12 x 1000 x 515 x 776 in bf16 took 2.0 us and more.
+constexpr int kStageBlock = 32 * 32 * 2;             // bytes of a staging block
+constexpr int kEpiBytes = kEpiWarps * 2 * kStageBlock;
 template <typename T>
-__device__ __forceinline__ void stage_block(unsigned char* stage, const uint32_t (&r)[32], int lane) {
-#pragma unroll
-  for (int j = 0; j < 32; ++j) reinterpret_cast<T*>(stage)[j * 32 + lane] = from_f32<T>(__uint_as_float(r[j]));
-}
+constexpr int kStageCols = kStageBlock / (32 * (int)sizeof(T));
 // One 32 x 32 block of a tile: r[j] = element (row m0 + lane, column n0 + j) of batch b.
 template <typename T>
-__device__ __forceinline__ void store_block(const Params& p, const void* tmapC, T* C, unsigned char* stage,
+__device__ __forceinline__ void store_block(const Params& p, const void* tmapC, T* C, unsigned char* stage, int& sent,
                                             const uint32_t (&r)[32], int m0, int n0, int b, float* partial, int lane) {
   if (partial) {  // whole lines as they are: through the staging block a CTA with one unit waits for its last store
 #pragma unroll
     for (int j = 0; j < 32; ++j) __stcg(partial + j * 32 + lane, __uint_as_float(r[j]));
   } else if (m0 + 32 <= p.tma_rows) {
-    if (lane == 0) bulk_wait_read<0>();  // the previous store has read the block
-    __syncwarp();
-    stage_block<T>(stage, r, lane);
-    fence_proxy_async_smem();
-    __syncwarp();
-    if (lane == 0) {
-      if (m0 < p.M && n0 < p.N) tma_store_3d(tmapC, stage, m0, n0, b);
-      bulk_commit();
+#pragma unroll
+    for (int h = 0; h < 32; h += kStageCols<T>) {
+      unsigned char* block = stage + (sent++ & 1) * kStageBlock;
+      if (lane == 0) bulk_wait_read<1>();  // the store before the previous one has read this block
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < kStageCols<T>; ++j)
+        reinterpret_cast<T*>(block)[j * 32 + lane] = from_f32<T>(__uint_as_float(r[h + j]));
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        if (m0 < p.M && n0 + h < p.N) tma_store_3d(tmapC, block, m0, n0 + h, b);
+        bulk_commit();
+      }
     }
   } else {
     const int m = m0 + lane;
@@ -131,8 +135,8 @@ __device__ __forceinline__ void store_block(const Params& p, const void* tmapC, 
 // A warp's share of a finished accumulator: every other block of 32 columns, the next one's TMEM load in flight while the
 // current one is stored.
 template <typename T>
-__device__ __forceinline__ void store_tile(const Params& p, const void* tmapC, T* C, unsigned char* stage, uint32_t taddr, int half,
-                                           int m0, int n0, int b, float* partial, int lane) {
+__device__ __forceinline__ void store_tile(const Params& p, const void* tmapC, T* C, unsigned char* stage, int& sent,
+                                           uint32_t taddr, int half, int m0, int n0, int b, float* partial, int lane) {
   const int nb = p.bn / 32;
   uint32_t r[2][32];
   if (half < nb) tmem_ld32(taddr + half * 32, r[0]);
@@ -142,7 +146,7 @@ __device__ __forceinline__ void store_tile(const Params& p, const void* tmapC, T
     if (c >= nb) break;  // uniform
     tc_wait_ld();
     if (c + 2 < nb) tmem_ld32(taddr + (c + 2) * 32, r[(i + 1) & 1]);
-    store_block<T>(p, tmapC, C, stage, r[i & 1], m0, n0 + c * 32, b, partial ? partial + c * 4096 : nullptr, lane);
+    store_block<T>(p, tmapC, C, stage, sent, r[i & 1], m0, n0 + c * 32, b, partial ? partial + c * 4096 : nullptr, lane);
   }
 }
 
@@ -270,8 +274,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   } else {
     const int sub = warp & 3;  // TMEM lanes [32*sub, 32*sub+32) belong to this warp
     const int half = (warp - 2) >> 2;
-    unsigned char* epi = smem + kRingBytes + (warp - 2) * kStageBlock;
-    int it = 0;
+    unsigned char* epi = smem + kRingBytes + (warp - 2) * (2 * kStageBlock);
+    int it = 0, sent = 0;
     for (int u = blockIdx.x; u < units; u += gridDim.x, ++it) {
       const int acc = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1;
@@ -281,7 +285,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (!ok) break;
       tc_fence_after();
       const int m0 = tm * kTileM + sub * 32;
-      store_tile<T>(p, &tmapC, C, epi, tmem_base + acc * kAccCols + ((uint32_t)(sub * 32) << 16), half, m0, tn * p.bn, b,
+      store_tile<T>(p, &tmapC, C, epi, sent, tmem_base + acc * kAccCols + ((uint32_t)(sub * 32) << 16), half, m0, tn * p.bn, b,
                     p.splits > 1 ? p.partial + (long long)u * (kTileM * kTileN) + sub * 1024 : nullptr, lane);
       tc_fence_before();
       __syncwarp();
@@ -471,8 +475,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   } else {
     const int sub = warp & 3;  // TMEM lanes [32*sub, 32*sub+32) belong to this warp
     const int half = (warp - 2) >> 2;
-    unsigned char* epi = smem + kRingBytes + (warp - 2) * kStageBlock;
-    int it = 0;
+    unsigned char* epi = smem + kRingBytes + (warp - 2) * (2 * kStageBlock);
+    int it = 0, sent = 0;
     for (int t = pair; t < p.num_tiles; t += num_pairs, ++it) {
       const int acc = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1;
@@ -482,7 +486,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       if (!ok) break;
       tc_fence_after();
       const int m0 = tm * kPairTileM + (int)rank * kTileM + sub * 32;
-      store_tile<T>(p, &tmapC, C, epi, tmem_base + acc * kAccCols + ((uint32_t)(sub * 32) << 16), half, m0, tn * p.bn, b,
+      store_tile<T>(p, &tmapC, C, epi, sent, tmem_base + acc * kAccCols + ((uint32_t)(sub * 32) << 16), half, m0, tn * p.bn, b,
                     nullptr, lane);
       tc_fence_before();
       __syncwarp();
@@ -660,7 +664,7 @@ int launch(ctb_ctx* ctx, cudaStream_t st, const T* A, const T* B, T* C, int M, i
   if (c_aligned) {
     uint64_t dims[3] = {(uint64_t)M, (uint64_t)N, (uint64_t)batch};
     uint64_t str[2] = {(uint64_t)ldc * G::ES, (uint64_t)(batch > 1 ? sC : ldc * (long long)N) * G::ES};
-    uint32_t box[3] = {32, 32, 1};
+    uint32_t box[3] = {32, (uint32_t)kStageCols<T>, 1};
     int r = make_tmap(&tc, dt, 3, C, dims, str, box, CU_TENSOR_MAP_SWIZZLE_NONE);
     if (r) return r;
   }
