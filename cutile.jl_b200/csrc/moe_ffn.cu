@@ -11,11 +11,12 @@
 //
 // The weights are the M operand of the MMA: a CTA pair (cta_group::2) takes 256 weight rows, the slots of one block of an
 // expert are the N operand, so a block costs what it holds, rounded up to 16 slots.  With the slots as M (128 or 256 rows
-// whatever the block holds) 4096 tokens cost 25 % (50 % in pairs) of padding.  An expert with more than 256 slots is cut
-// into equal blocks.
+// whatever the block holds) 4096 tokens cost 25 % (50 % in pairs) of padding.  An expert with too many slots
+// for one block (blocks_for) is cut into equal ones.
 #include <math.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "ctx.h"
 #include "ptx.cuh"
@@ -26,7 +27,15 @@ using namespace ctb_internal;
 namespace {
 
 constexpr int kMaxExperts = 256;
-constexpr int kMaxBlockSlots = 256;  // MMA N
+constexpr int kMmaSlots = 256;       // MMA N
+constexpr int kMaxBlockSlots = 320;  // slots of a block: two MMAs above kMmaSlots
+// Blocks that an expert's slots are cut into.  A k-block costs a pair about 330 ns up to 224 slots, whatever their number, and
+// the MMA's 1.45 ns per slot above: blocks of 226 slots and more are cheap, and one of up to 320 is cheaper than two of half of it.
+// (ring: the accumulators of moe_pair_gemm_kernel may take more than half of the columns.)
+constexpr __host__ __device__ int blocks_for(bool ring, int slots) {
+  const int n = (slots + kMmaSlots - 1) / kMmaSlots;
+  return ring && n > 1 && slots < n * 226 && slots <= (n - 1) * kMaxBlockSlots ? n - 1 : n;
+}
 
 // ------------------------------------------------------------------ sort and gather
 constexpr int kSortThreads = 512, kSortCtas = 148;
@@ -49,6 +58,7 @@ struct SortParams {
   int* num_blocks;  // [0] blocks, [1] slots of the largest
   const int* counts;  // [kSortCtas][E + 1]: slots per expert in every CTA's chunk, then 1 if an id is out of range; or null
   int T, topk, E, vecs, total, chunk, early;
+  int held;  // token rows that a CTA holds in shared memory; 0: they go through registers
   int* status;
 };
 
@@ -83,8 +93,8 @@ __global__ void __launch_bounds__(kSortThreads)
 }
 
 // Adds every slot of expert e to tot[e] and, if `base` is given, those with a flat index below `lo` to base[e] (both in
-// shared memory); true if an id is out of range.  All threads of the CTA.
-template <typename IdT>
+// shared memory; SPLIT: to base[e] only); true if an id is out of range.  All threads of the CTA.
+template <bool SPLIT, typename IdT>
 __device__ __forceinline__ bool count_slots(const IdT* __restrict__ ids, int T, int topk, int E, int lo, int* tot, int* base) {
   bool bad = false;
   const int step = blockDim.x, total = T * topk;
@@ -100,20 +110,22 @@ __device__ __forceinline__ bool count_slots(const IdT* __restrict__ ids, int T, 
         bad = true;
         continue;
       }
-      atomicAdd(&tot[e[q]], 1);
+      if (!SPLIT) atomicAdd(&tot[e[q]], 1);
       if (base) {
         const int slot = m / T;
-        if ((m - slot * T) * topk + slot < lo) atomicAdd(&base[e[q]], 1);
+        const bool before = (m - slot * T) * topk + slot < lo;
+        if (SPLIT) atomicAdd(before ? &base[e[q]] : &tot[e[q]], 1);
+        else if (before) atomicAdd(&base[e[q]], 1);
       }
     }
   }
   return bad;
 }
 // First row and first block of every expert from its number of slots (one warp; first[e] is added to).
-__device__ __forceinline__ void scan_experts(const int* tot, int E, int* first, int* bstart, int lane) {
+__device__ __forceinline__ void scan_experts(bool ring, const int* tot, int E, int* first, int* bstart, int lane) {
   int rows = 0, blocks = 0;
   for (int e0 = 0; e0 < E; e0 += 32) {
-    const int e = e0 + lane, c = e < E ? tot[e] : 0, padded = (c + 15) & ~15, nb = (c + kMaxBlockSlots - 1) / kMaxBlockSlots;
+    const int e = e0 + lane, c = e < E ? tot[e] : 0, padded = (c + 15) & ~15, nb = blocks_for(ring, c);
     int r = padded, b = nb;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -136,24 +148,43 @@ __device__ __forceinline__ int write_blocks(Block* table, int e, int c, int nb, 
   return size;
 }
 
+// Ints of dynamic shared memory ahead of the rows (whole 128 bytes): slots per expert, those before the CTA's, the warps' counts,
+// first blocks.
+constexpr __host__ __device__ size_t sort_ints(int64_t E, int warps) { return (size_t)((3 + warps) * E + 1 + 31) & ~(size_t)31; }
+constexpr size_t kHeldBytes = 160 * 1024;  // at most
+
 // CTA c places the flat slots [c * chunk, (c + 1) * chunk) and copies their rows.  Nothing is exchanged between the CTAs:
 // each counts all slots (or reads the chunks' counts) and so knows where every expert's rows and its own share of them
 // start; the order inside an expert is the flat slot order, as in moe_align_tile_size (examples/moe.jl:142-183).
+// Without the gate/up kernel beside it a CTA has room for the rows: each token's comes by one bulk copy while the slots are
+// counted and leaves by one per choice, with nothing in registers (4096 tokens, top-2: through registers the kernel took
+// 13.5 us, 5 of them for the rows once their places were known; now 9.5 and 2).
 // A chain of latencies: 2.3 us to the counts, 4.3 to the table, then the rows.  The gate/up kernel does not wait for it: it
 // is set up beside this one, counts the slots itself and streams weights meanwhile.
 template <typename IdT, int kThreads>
 __global__ void __launch_bounds__(kThreads) moe_sort_gather_kernel(const IdT* __restrict__ ids, const SortParams p) {
   constexpr int kWarps = kThreads / 32;
-  extern __shared__ int sort_smem[];  // small, so that the next kernel's CTAs fit beside
+  constexpr bool HELD = kThreads == kSortThreads;  // without the gate/up kernel beside it
+  extern __shared__ __align__(128) int sort_smem[];  // small where the next kernel's CTAs run beside this one's
   __shared__ int spos[kThreads];
   __shared__ int bad, nmax;
+  __shared__ __align__(8) uint64_t rows_in;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, E = p.E, cta = blockIdx.x;
   int *tot = sort_smem, *base = tot + E, *wcount = base + E, *bstart = wcount + kWarps * E;  // [E], [E], [warps][E], [E + 1]
   for (int e = tid; e < E; e += kThreads) tot[e] = base[e] = 0;
-  if (tid == 0) bad = nmax = 0;
+  unsigned char* held = reinterpret_cast<unsigned char*>(sort_smem) + sort_ints(E, kWarps) * sizeof(int);  // [p.held] token rows
+  const uint32_t row_bytes = (uint32_t)p.vecs * 16;
+  if (tid == 0) {
+    bad = nmax = 0;
+    if (HELD) {
+      mbar_init(&rows_in, 1);
+      fence_mbar_init();
+    }
+  }
   __syncthreads();
   grid_dependency_wait();
-  if (p.early) grid_dependency_launch();  // the gate/up kernel reads the ids as well
+  // the gate/up kernel reads the ids as well; if it waits for the table it is at least set up where a CTA of this kernel has ended
+  grid_dependency_launch();
   const int lo = min(p.total, cta * p.chunk), hi = min(p.total, lo + p.chunk);
   // Which slots and rows are this CTA's is known from the start: the first are on their way before anything else is asked
   // for, ahead of the gate/up kernel's weights (behind them they took 5 us longer).
@@ -170,21 +201,34 @@ __global__ void __launch_bounds__(kThreads) moe_sort_gather_kernel(const IdT* __
     }
   };
   int e;
-  float weight;
+  __half weight;  // converted where it is used: nothing waits for it before the rows are requested
   auto load_slot = [&](int i) {
     e = -1;
-    weight = 0.f;
+    weight = __ushort_as_half(0);
     if (i < hi) {
       const int tok = i / p.topk, slot = i - tok * p.topk;
       e = (int)ids[(long long)slot * p.T + tok] - 1;
-      weight = __half2float(p.topk_w[(long long)slot * p.T + tok]);
+      weight = p.topk_w[(long long)slot * p.T + tok];
     }
   };
-  load_slot(lo + tid);
-  load_rows(lo, tid);
+  // Slots at a time: their tokens are at most p.held.
+  const int step = HELD && p.held ? min(kThreads, (p.held - 1) * p.topk) : kThreads;
+  auto hold_rows = [&](int b0) {  // requests the rows of the tokens of the slots [b0, b0 + step)
+    const int t0 = b0 / p.topk, n = (min(b0 + step, hi) - 1) / p.topk + 1 - t0;
+    if (tid == 0) mbar_expect_tx(&rows_in, n * row_bytes);
+    for (int r = tid; r < n; r += kThreads)
+      bulk_g2s(held + (size_t)r * row_bytes, p.X + (long long)(t0 + r) * p.vecs, row_bytes, &rows_in);
+  };
+  if (HELD && p.held) {
+    if (lo < hi) hold_rows(lo);
+    load_slot(lo + tid);
+  } else {
+    load_slot(lo + tid);
+    load_rows(lo, tid);
+  }
   // ---- slots per expert: all of them, and those before this CTA's
   if (!p.counts) {
-    if (count_slots(ids, p.T, p.topk, E, lo, tot, base)) bad = 1;
+    if (count_slots<HELD>(ids, p.T, p.topk, E, lo, tot, base)) bad = 1;
   } else {
     for (int e = tid; e <= E; e += kThreads) {
       int all = 0, before = 0;
@@ -210,10 +254,15 @@ __global__ void __launch_bounds__(kThreads) moe_sort_gather_kernel(const IdT* __
       p.num_blocks[1] = 16;
     }
     for (int i = lo + tid; i < hi; i += kThreads) p.pos_of[i] = 0;
+    if (HELD && p.held && lo < hi) (void)mbar_wait(&rows_in, 0, p.status, DEV_TIMEOUT_TMA);
     return;
   }
+  if (HELD && !p.counts) {
+    for (int e = tid; e < E; e += kThreads) tot[e] += base[e];
+    __syncthreads();
+  }
   // ---- first row and first block of every expert
-  if (warp == 0) scan_experts(tot, E, base, bstart, lane);
+  if (warp == 0) scan_experts(HELD, tot, E, base, bstart, lane);
   __syncthreads();
   if (cta == 0) {  // the block table; this CTA has no slots before it: base is the experts' first row
     for (int e = tid; e < E; e += kThreads) {
@@ -230,11 +279,18 @@ __global__ void __launch_bounds__(kThreads) moe_sort_gather_kernel(const IdT* __
   // ---- this CTA's slots, kThreads at a time: stable positions, then the rows
   int ebits = 1;
   while ((1 << ebits) < E) ++ebits;
-  for (int b0 = lo; b0 < hi; b0 += kThreads) {
+  uint32_t phase = 0;
+  for (int b0 = lo; b0 < hi; b0 += step) {
+    if (HELD && p.held && b0 != lo) {
+      bulk_wait_read<0>();  // the rows before these have left
+      __syncthreads();
+      hold_rows(b0);
+    }
     for (int i = tid; i < kWarps * E; i += kThreads) wcount[i] = 0;
     __syncthreads();
     const int i = b0 + tid;
     if (b0 != lo) load_slot(i);
+    if (HELD && tid >= step) e = -1;
     const unsigned grp = same_value(e, ebits);
     const int rank = __popc(grp & ((1u << lane) - 1));
     if (e >= 0 && rank == 0) wcount[warp * E + e] = __popc(grp);
@@ -254,7 +310,19 @@ __global__ void __launch_bounds__(kThreads) moe_sort_gather_kernel(const IdT* __
       const int pos = wcount[warp * E + e] + rank;
       spos[tid] = pos;
       p.pos_of[i] = pos;
-      p.wts[pos] = weight;
+      p.wts[pos] = __half2float(weight);
+    }
+    if (HELD && p.held) {
+      const bool ok = mbar_wait(&rows_in, phase, p.status, DEV_TIMEOUT_TMA);
+      phase ^= 1;
+      if (ok && e >= 0)
+        bulk_s2g(p.xs + (long long)spos[tid] * p.vecs, held + (size_t)(i / p.topk - b0 / p.topk) * row_bytes, row_bytes);
+      bulk_commit();
+      if (__syncthreads_or(!ok)) {  // the copies must land before the CTA gives its shared memory back
+        (void)mbar_wait(&rows_in, phase ^ 1, p.status, DEV_TIMEOUT_TMA);
+        break;
+      }
+      continue;
     }
     __syncthreads();
     const int n = min(kThreads, hi - b0) * p.vecs;
@@ -271,6 +339,7 @@ __global__ void __launch_bounds__(kThreads) moe_sort_gather_kernel(const IdT* __
     }
     __syncthreads();
   }
+  if (HELD) bulk_wait_read<0>();  // this thread's rows have left shared memory
 }
 
 // ------------------------------------------------------------------ the two projections
@@ -280,6 +349,7 @@ constexpr int kMaxStages = 12;
 constexpr int kRingBytes = 192 * 1024;
 constexpr int kEpiWarps = 8;                 // two per TMEM lane quadrant, each takes every other block of 32 slots
 constexpr int kGemmThreads = 96 + 32 * kEpiWarps;
+constexpr int kParts = 6;                    // leading blocks of 32 columns that the next item may need (place())
 constexpr int kTileBytes = 32 * 64 * 2;      // staged results: 32 slots x 64 rows, f16, 128-byte swizzle
 // Warps that share a staging tile: gate/up the four quadrants (a CTA's 64 outputs), down two of them; two tiles each.
 template <bool UP>
@@ -289,20 +359,39 @@ constexpr size_t kGemmSmem = 1024 + kRingBytes + (size_t)(UP ? 2 : 4) * 2 * kTil
 // The gate/up kernel's own block table behind it: slots, first rows and first blocks of E experts, then the blocks.
 constexpr size_t own_table_bytes(int64_t E, int64_t blocks) { return (size_t)(((3 * E + 1) * 4 + 15) & ~15) + blocks * sizeof(Block); }
 template <bool UP>
-constexpr size_t kGemmSmemMost = kGemmSmem<UP> + (UP ? own_table_bytes(kMaxExperts, kEarlySlots / kMaxBlockSlots + kMaxExperts) : 0);
+constexpr size_t kGemmSmemMost = kGemmSmem<UP> + (UP ? own_table_bytes(kMaxExperts, kEarlySlots / kMmaSlots + kMaxExperts) : 0);
 
 // The sorted rows with a box for every number of slots that a CTA may hold (8, 16, ... 128): one copy per k-block.
 struct SlotMaps {
-  CUtensorMap m[kMaxBlockSlots / 16];
+  CUtensorMap m[kMmaSlots / 16];
 };
 struct PairParams {
   const Block* table;
   const int* num_blocks;
   const float* wts;
   int mtiles, K, rows;  // rows: output rows of the projection
-  const void* ids;      // gate/up with at most kEarlySlots slots: the kernel builds its own table (null: it reads the sort's)
+  const void* ids;      // gate/up with at most kEarlySlots slots (not RING): the kernel builds its own table
   int ids_bits, T, topk, E;
 };
+
+// Where a block's accumulators lie in the 512 TMEM columns, which are a ring: slot s of the block in column
+// (col + s) mod 512, col a multiple of 32.  The slots are taken by at most two MMAs: [0, first) and [first, n).
+struct Place {
+  int col, first, next, skipped;  // next: where the next block may start
+};
+template <bool RING>
+__device__ __forceinline__ Place place(int at, int n) {
+  if (!RING) return {at, n, at ^ 256, 0};  // no block above 256 slots: two halves in turn
+  const int n32 = (n + 31) & ~31, room = 512 - at;
+  Place r;
+  // an MMA takes at most kMmaSlots: columns before or behind the end of the ring stay unused where a part would be larger
+  r.skipped = n32 <= room ? 0 : room > kMmaSlots ? room - kMmaSlots : n - room > kMmaSlots ? room : 0;
+  r.col = (at + r.skipped) & 511;
+  const int left = 512 - r.col;
+  r.first = n32 > left ? left : n > kMmaSlots ? ((n / 2 + 15) & ~15) : n;
+  r.next = (r.col + n32) & 511;
+  return r;
+}
 
 // Barriers of `threads` threads (whole warps).
 __device__ __forceinline__ void group_sync(int id, int threads) { asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
@@ -342,15 +431,21 @@ __device__ __forceinline__ void stmatrix4_trans(uint32_t addr, uint32_t a, uint3
 // the operands: with 4096 tokens the results cost 27 of 168 us that way, now 14 of 156).
 // Neither projection waits for the kernel before it ahead of its first weights: the block table is older than it (down) or
 // computed from the ids (gate/up); only the rows are new.
+// The accumulators of an item follow those of the item before it in the ring of 512 columns: an item may begin when the one two
+// before it has been read and, of the one before it, as many leading columns as it needs.  So a block can have more than 256
+// slots and still start beside its predecessor's results.  With two halves of 256 columns an expert of 257 slots was two
+// blocks, at the price of 256 slots each (a k-block of 144 slots took 330 ns, one of 256 slots 374): half of the experts at 4096
+// tokens, top-2 over 32, where gate/up took 66 us and takes 57 now, down 39 and 35.  With at most kEarlySlots slots (not RING)
+// large blocks are rare, and the two halves cost nothing in the roles' code (1 to 2 us of a step with few tokens).
 // Up to 128 slots per block two k-blocks make a stage: the waits and issues of a stage take about 0.25 us, more than the weights
 // of one k-block (100 tokens 86.3 -> 81.5 us, 1000 tokens 104.4 -> 102.6; larger blocks keep more and smaller stages in flight).
-template <bool UP>
+template <bool UP, bool RING>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
     moe_pair_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ SlotMaps tmX,
                          const __grid_constant__ CUtensorMap tmOut, const PairParams p, int* status) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], acc_full[2], acc_empty[2];
+  __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], acc_full[2], acc_empty[2], part_empty[2][kParts];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s, nmax_s;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -365,6 +460,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
     for (int a = 0; a < 2; ++a) {
       mbar_init(&acc_full[a], 1);
       mbar_init(&acc_empty[a], 2 * kEpiWarps);  // the epilogue warps of both CTAs
+      for (int k = 0; RING && k < kParts; ++k) mbar_init(&part_empty[a][k], kEpiWarps);  // those of both that read block k
     }
     fence_mbar_init();
     tma_prefetch_desc(&tmW);
@@ -384,17 +480,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
   volatile int* abort = &abort_s;
   const Block* table = p.table;
   int blocks, nmax;
-  if (UP && p.ids) {  // count the slots as the sort does
+  if (UP && !RING) {  // count the slots as the sort does
     int* tot = reinterpret_cast<int*>(smem_raw + kGemmSmem<UP>);
     int *first = tot + p.E, *bstart = first + p.E;
     Block* own = reinterpret_cast<Block*>(smem_raw + kGemmSmem<UP> + own_table_bytes(p.E, 0));
     for (int e = threadIdx.x; e < p.E; e += kGemmThreads) tot[e] = first[e] = 0;
     if (threadIdx.x == 0) nmax_s = 16;
     __syncthreads();
-    const bool bad = p.ids_bits == 32 ? count_slots(static_cast<const int*>(p.ids), p.T, p.topk, p.E, 0, tot, (int*)nullptr)
-                                      : count_slots(static_cast<const long long*>(p.ids), p.T, p.topk, p.E, 0, tot, (int*)nullptr);
+    const bool bad = p.ids_bits == 32 ? count_slots<false>(static_cast<const int*>(p.ids), p.T, p.topk, p.E, 0, tot, (int*)nullptr)
+                                      : count_slots<false>(static_cast<const long long*>(p.ids), p.T, p.topk, p.E, 0, tot, (int*)nullptr);
     const bool none = __syncthreads_or(bad);
-    if (warp == 0) scan_experts(tot, p.E, first, bstart, lane);
+    if (warp == 0) scan_experts(RING, tot, p.E, first, bstart, lane);
     __syncthreads();
     for (int e = threadIdx.x; e < p.E; e += kGemmThreads) {
       const int nb = bstart[e + 1] - bstart[e];
@@ -426,7 +522,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
     // weight rows and 32 or 8 slots) and a division per k-block the issue took about 800 clocks per k-block and bound the
     // kernel whatever the operands' size.
     if (warp == 2) {
-      if (lane == 0) tma_prefetch_desc(&tmX.m[block_of(pair).n / 16 - 1]);
+      if (lane == 0) tma_prefetch_desc(&tmX.m[place<RING>(0, block_of(pair).n).first / 16 - 1]);
       grid_dependency_wait();  // the rows
       if (UP) grid_dependency_launch();  // the down projection may start its weights
     }
@@ -434,72 +530,113 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
+    int at = 0;
+    Block next = block_of(pair);
     for (int it = pair; ok && it < items; it += num_pairs) {
-      const Block b = block_of(it);
-      const int half = b.n / 2;
+      const Block b = RING ? next : block_of(it);
+      if (RING) next = block_of(it + num_pairs);
+      const Place pl = place<RING>(at, b.n);
+      at = pl.next;
+      const int half = b.n / 2, rest = b.n - pl.first;
       const uint32_t bytes = 2 * (kABytes + half * 128);
-      const int wrow = ((it % p.mtiles) * 2 + (int)rank) * (UP ? 8 : 128), xrow = b.row0 + (int)rank * half;
-      const CUtensorMap* map = &tmX.m[b.n / 16 - 1];
-      for (int kb = 0; kb < nk; kb += per_stage) {
-        ok = CTB_WARP_WAIT(&empty[stage], phase ^ 1, status, DEV_TIMEOUT_SLOT, abort);
-        if (!ok) break;
-        const int live = min(per_stage, nk - kb);
-        if (elect_one()) {
-          unsigned char* dst = smem + stage * stage_bytes;
-          if (warp == 0) {
-            if (rank == 0) mbar_expect_tx(&full[stage], live * bytes);
-            for (int q = 0; q < live; ++q) {
-              if (UP) tma_load_5d_pair(dst + q * kABytes, &tmW, (kb + q) * kBK, 0, 0, wrow, b.expert, bars + stage * 8);
-              else tma_load_3d_pair(dst + q * kABytes, &tmW, (kb + q) * kBK, wrow, b.expert, bars + stage * 8);
-            }
-          } else {
-            for (int q = 0; q < live; ++q)
-              tma_load_3d_pair(dst + per_stage * kABytes + q * (nmax / 2 * 128), map, (kb + q) * kBK, xrow, 0, bars + stage * 8);
-          }
-        }
-        __syncwarp();
-        if (++stage == stages) {
-          stage = 0;
-          phase ^= 1;
-        }
-      }
-    }
-  } else if (warp == 1) {
-    if (rank == 0) {
-      // ---- MMA issuer (rank 0 only): one instruction drives the tensor cores of both SMs
-      int stage = 0, n = 0;
-      uint32_t phase = 0;
-      Block next = block_of(pair);
-      for (int it = pair; it < items; it += num_pairs, ++n) {
-        const uint32_t idesc = make_idesc(FMT_F16, 256, (uint32_t)next.n, 0, 0);
-        next = block_of(it + num_pairs);
-        const int acc = n & 1;
-        const uint32_t acc_phase = (n >> 1) & 1;
-        if (!CTB_WARP_WAIT(&acc_empty[acc], acc_phase ^ 1, status, DEV_TIMEOUT_SLOT, abort)) break;
-        tc_fence_after();
-        const uint32_t d = tmem_base + acc * 256;
-        bool ok = true;
+      const int wrow = ((it % p.mtiles) * 2 + (int)rank) * (UP ? 8 : 128), xrow = b.row0 + (int)rank * (pl.first / 2);
+      const int xrest = b.row0 + pl.first + (int)rank * (rest / 2);
+      const CUtensorMap *map = &tmX.m[pl.first / 16 - 1], *map_rest = &tmX.m[max(rest, 16) / 16 - 1];
+      // fill(stage's memory, its barrier, first k, k-blocks) requests a stage
+      auto walk = [&](auto fill) {
         for (int kb = 0; kb < nk; kb += per_stage) {
-          ok = CTB_WARP_WAIT(&full[stage], phase, status, DEV_TIMEOUT_TMA, abort);
+          ok = CTB_WARP_WAIT(&empty[stage], phase ^ 1, status, DEV_TIMEOUT_SLOT, abort);
           if (!ok) break;
-          tc_fence_after();
-          const int live = min(per_stage, nk - kb);
-          const uint32_t sa0 = smem_u32(smem + stage * stage_bytes), sb0 = sa0 + per_stage * kABytes;
-          if (elect_one()) {
-            for (int q = 0; q < live; ++q) {
-              const uint32_t sa = sa0 + q * kABytes, sb = sb0 + q * (nmax / 2 * 128);
-#pragma unroll
-              for (int k = 0; k < kBK / 16; ++k)
-                mma_f16_ss_pair(d, make_sdesc_sw128(sa + k * 32, 0, 1024), make_sdesc_sw128(sb + k * 32, 0, 1024), idesc,
-                                (kb | q | k) != 0);
-            }
-            tc_commit_pair(&empty[stage], 3);
-          }
+          if (elect_one()) fill(smem + stage * stage_bytes, bars + stage * 8, kb * kBK, min(per_stage, nk - kb));
           __syncwarp();
           if (++stage == stages) {
             stage = 0;
             phase ^= 1;
           }
+        }
+      };
+      const int x_at = per_stage * kABytes, x_bytes = nmax / 2 * 128;
+      if (warp == 0) {
+        walk([&](unsigned char* dst, uint32_t bar, int k, int live) {
+          if (rank == 0) mbar_expect_tx(&full[stage], live * bytes);
+          for (int q = 0; q < live; ++q) {
+            if (UP) tma_load_5d_pair(dst + q * kABytes, &tmW, k + q * kBK, 0, 0, wrow, b.expert, bar);
+            else tma_load_3d_pair(dst + q * kABytes, &tmW, k + q * kBK, wrow, b.expert, bar);
+          }
+        });
+      } else if (!RING || !rest) {
+        walk([&](unsigned char* dst, uint32_t bar, int k, int live) {
+          for (int q = 0; q < live; ++q) tma_load_3d_pair(dst + x_at + q * x_bytes, map, k + q * kBK, xrow, 0, bar);
+        });
+      } else {
+        walk([&](unsigned char* dst, uint32_t bar, int k, int live) {
+          for (int q = 0; q < live; ++q) {
+            tma_load_3d_pair(dst + x_at + q * x_bytes, map, k + q * kBK, xrow, 0, bar);
+            tma_load_3d_pair(dst + x_at + q * x_bytes + pl.first / 2 * 128, map_rest, k + q * kBK, xrest, 0, bar);
+          }
+        });
+      }
+    }
+  } else if (warp == 1) {
+    if (rank == 0) {
+      // ---- MMA issuer (rank 0 only): one instruction drives the tensor cores of both SMs
+      int stage = 0, n = 0, at = 0, before = 0;  // before: columns of the item before this one
+      uint32_t phase = 0;
+      Block next = block_of(pair);
+      for (int it = pair; it < items; it += num_pairs, ++n) {
+        const Place pl = place<RING>(at, next.n);
+        const int rest = next.n - pl.first, n32 = (next.n + 31) & ~31;
+        const uint32_t idesc = make_idesc(FMT_F16, 256, (uint32_t)pl.first, 0, 0);
+        const uint32_t idesc_rest = make_idesc(FMT_F16, 256, (uint32_t)max(rest, 16), 0, 0);
+        const int shared = (before + pl.skipped + n32 - 512) / 32;  // leading blocks of the item before that this one overwrites
+        at = pl.next;
+        before = RING ? n32 : 0;
+        next = block_of(it + num_pairs);
+        const int acc = n & 1;
+        const uint32_t acc_phase = (n >> 1) & 1;
+        bool ok = CTB_WARP_WAIT(&acc_empty[acc], acc_phase ^ 1, status, DEV_TIMEOUT_SLOT, abort);
+        for (int k = max(shared - 2, 0); ok && k < shared; ++k)  // the blocks go to two groups of warps in turn, in order
+          ok = CTB_WARP_WAIT(&part_empty[acc ^ 1][k], ((n - 1) >> 1) & 1, status, DEV_TIMEOUT_SLOT, abort);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t d = tmem_base + pl.col, d_rest = tmem_base + ((pl.col + pl.first) & 511);
+        auto walk = [&](auto two_tag) {
+          constexpr bool TWO = decltype(two_tag)::value;
+          for (int kb = 0; kb < nk; kb += per_stage) {
+            ok = CTB_WARP_WAIT(&full[stage], phase, status, DEV_TIMEOUT_TMA, abort);
+            if (!ok) break;
+            tc_fence_after();
+            const int live = min(per_stage, nk - kb);
+            const uint32_t sa0 = smem_u32(smem + stage * stage_bytes), sb0 = sa0 + per_stage * kABytes;
+            if (elect_one()) {
+              for (int q = 0; q < live; ++q) {
+                const uint32_t sa = sa0 + q * kABytes, sb = sb0 + q * (nmax / 2 * 128);
+#pragma unroll
+                for (int k = 0; k < kBK / 16; ++k)
+                  mma_f16_ss_pair(d, make_sdesc_sw128(sa + k * 32, 0, 1024), make_sdesc_sw128(sb + k * 32, 0, 1024), idesc,
+                                  (kb | q | k) != 0);
+                if constexpr (TWO) {
+                  const uint32_t sr = sb + pl.first / 2 * 128;
+#pragma unroll
+                  for (int k = 0; k < kBK / 16; ++k)
+                    mma_f16_ss_pair(d_rest, make_sdesc_sw128(sa + k * 32, 0, 1024), make_sdesc_sw128(sr + k * 32, 0, 1024),
+                                    idesc_rest, (kb | q | k) != 0);
+                }
+              }
+              tc_commit_pair(&empty[stage], 3);
+            }
+            __syncwarp();
+            if (++stage == stages) {
+              stage = 0;
+              phase ^= 1;
+            }
+          }
+        };
+        if constexpr (RING) {
+          if (rest) walk(std::true_type());
+          else walk(std::false_type());
+        } else {
+          walk(std::false_type());
         }
         if (!ok) break;
         if (elect_one()) tc_commit_pair(&acc_full[acc], 3);
@@ -513,7 +650,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
     const bool issuer = (UP ? sub == 3 : (sub & 1)) && lane == 0;
     const uint32_t tiles = smem_u32(smem + kRingBytes + group * 2 * kTileBytes);
     uint32_t flip = 0;  // the staging tile to fill next
-    int n = 0;
+    int n = 0, at = 0;
     Block next = block_of(pair);
     for (int it = pair; it < items; it += num_pairs, ++n) {
       const Block b = next;
@@ -523,16 +660,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
       ok = group_all(1 + group, kGroupThreads<UP>, ok);  // the warps of a group go on or stop together
       if (!ok) break;
       tc_fence_after();
-      const uint32_t taddr = tmem_base + acc * 256 + ((uint32_t)(sub * 32) << 16);
+      const Place pl = place<RING>(at, b.n);
+      at = pl.next;
+      const uint32_t taddr = tmem_base + ((uint32_t)(sub * 32) << 16);
+      const uint32_t acc_read = map_to_cta(&part_empty[acc][0], 0);
       const int m0 = UP ? (it % p.mtiles) * 128 + (int)rank * 64 : (it % p.mtiles) * 256 + (int)rank * 128 + (sub >> 1) * 64;
       uint32_t r[2][2][16];
       auto load = [&](int c, uint32_t (&v)[2][16]) {
-        tmem_ld_16x32(taddr + c, v[0]);
-        tmem_ld_16x32(taddr + (16u << 16) + c, v[1]);
+        const uint32_t col = (pl.col + c) & 511;
+        tmem_ld_16x32(taddr + col, v[0]);
+        tmem_ld_16x32(taddr + (16u << 16) + col, v[1]);
       };
       if (half * 32 < b.n) load(half * 32, r[0]);
 #pragma unroll
-      for (int i = 0; i < kMaxBlockSlots / 64; ++i) {
+      for (int i = 0; i < (RING ? kMaxBlockSlots : kMmaSlots) / 64; ++i) {
         const int c = i * 64 + half * 32;
         if (c >= b.n) break;  // uniform
         uint32_t(&v)[2][16] = r[i & 1];
@@ -545,6 +686,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
           }
         }
         tc_wait_ld();
+        if (RING && 2 * i + half < kParts) {  // this block of columns is in registers
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(acc_read + (2 * i + half) * 8);
+        }
         if (c + 64 < b.n) load(c + 64, r[(i + 1) & 1]);
         // lane l gives the address of slot c + l; 16-byte piece k of its 128 bytes lies at k ^ (l mod 8)
         const uint32_t row = tiles + flip * kTileBytes + lane * 128;
@@ -583,7 +729,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(map_to_cta(&acc_empty[acc], 0));
+      if (lane == 0) {
+        for (int k = half; RING && k < kParts; k += 2)  // blocks that this item does not have
+          if (k * 32 >= b.n) mbar_arrive_cluster(acc_read + k * 8);
+        mbar_arrive_cluster(map_to_cta(&acc_empty[acc], 0));
+      }
     }
     bulk_wait<0>();  // this warp's stores are complete
   }
@@ -653,13 +803,13 @@ struct Scratch {  // offsets in the context's scratch
     pos = act + up((size_t)rows * I * 2);
     wts = pos + up((size_t)total * 4);
     table = wts + up((size_t)rows * 4);
-    blocks = table + up((size_t)(total / kMaxBlockSlots + used) * sizeof(Block));
+    blocks = table + up((size_t)(total / kMmaSlots + used) * sizeof(Block));
     counts = blocks + 256;
     bytes = counts + (total > kSortLocal ? up((size_t)kSortCtas * (E + 1) * 4) : 0);
   }
 };
 
-template <bool UP>
+template <bool UP, bool RING>
 int pair_clusters(ctb_ctx* ctx) {  // clusters of the kernel that the device runs at once (asked once per device)
   static int cached[16] = {0};
   int& c = cached[ctx->device & 15];
@@ -676,8 +826,8 @@ int pair_clusters(ctb_ctx* ctx) {  // clusters of the kernel that the device run
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
-    cudaError_t e = allow_smem(moe_pair_gemm_kernel<UP>, kGemmSmemMost<UP>);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, moe_pair_gemm_kernel<UP>, &cfg);
+    cudaError_t e = allow_smem(moe_pair_gemm_kernel<UP, RING>, kGemmSmemMost<UP>);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, moe_pair_gemm_kernel<UP, RING>, &cfg);
     if (e != cudaSuccess) {
       (void)cudaGetLastError();
       return 0;
@@ -687,7 +837,7 @@ int pair_clusters(ctb_ctx* ctx) {  // clusters of the kernel that the device run
   return c;
 }
 
-template <bool UP>
+template <bool UP, bool RING>
 int launch_projection(ctb_ctx* ctx, cudaStream_t st, const void* W, const void* X, void* out, int64_t K, int64_t wrows, int64_t N,
                       int64_t E, const Scratch& sc, unsigned char* ws, int64_t max_blocks, const void* ids, int ids_bits, int64_t T,
                       int64_t topk) {
@@ -706,7 +856,7 @@ int launch_projection(ctb_ctx* ctx, cudaStream_t st, const void* W, const void* 
     int r = make_tmap(&tw, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, W, dims, str, box);
     if (r) return r;
   }
-  for (int k = 0; k < kMaxBlockSlots / 16; ++k) {
+  for (int k = 0; k < kMmaSlots / 16; ++k) {
     uint64_t dims[3] = {(uint64_t)K, (uint64_t)sc.rows, 1};
     uint64_t str[2] = {(uint64_t)K * 2, (uint64_t)K * sc.rows * 2};
     uint32_t box[3] = {kBK, 8u * (k + 1), 1};
@@ -726,15 +876,15 @@ int launch_projection(ctb_ctx* ctx, cudaStream_t st, const void* W, const void* 
   p.wts = reinterpret_cast<const float*>(ws + sc.wts);
   p.K = (int)K; p.rows = (int)N;
   p.mtiles = (int)((N + (UP ? 127 : 255)) / (UP ? 128 : 256));
-  const int clusters = pair_clusters<UP>(ctx);
+  const int clusters = pair_clusters<UP, RING>(ctx);
   if (clusters < 1) return fail(CTB_UNSUPPORTED, "ctb_moe_ffn: the device runs no CTA pairs");
   p.ids = ids;
   p.ids_bits = ids_bits; p.T = (int)T; p.topk = (int)topk; p.E = (int)E;
   const size_t smem = kGemmSmem<UP> + (ids ? own_table_bytes(E, max_blocks) : 0);
-  cudaError_t e = allow_smem(moe_pair_gemm_kernel<UP>, kGemmSmemMost<UP>);
+  cudaError_t e = allow_smem(moe_pair_gemm_kernel<UP, RING>, kGemmSmemMost<UP>);
   if (e != cudaSuccess) return cuda_fail(e, "ctb_moe_ffn: shared memory opt-in");
   const int grid = 2 * (int)std::min<int64_t>(clusters, max_blocks * p.mtiles);
-  e = launch_kernel(moe_pair_gemm_kernel<UP>, grid, kGemmThreads, smem, st, 0, tw, tx, to, p, ctx->dev_status);
+  e = launch_kernel(moe_pair_gemm_kernel<UP, RING>, grid, kGemmThreads, smem, st, 0, tw, tx, to, p, ctx->dev_status);
   if (e != cudaSuccess) return cuda_fail(e, "ctb_moe_ffn projection launch");
   return CTB_OK;
 }
@@ -748,7 +898,8 @@ int launch_sort(cudaStream_t st, const void* topk_ids, const SortParams& sp) {
                       const_cast<int*>(sp.counts));
   auto kernel = sp.early ? moe_sort_gather_kernel<IdT, kSortThreadsEarly> : moe_sort_gather_kernel<IdT, kSortThreads>;
   const int threads = sp.early ? kSortThreadsEarly : kSortThreads;
-  const size_t smem = (size_t)((3 + threads / 32) * sp.E + 1) * sizeof(int);
+  const size_t smem = sort_ints(sp.E, threads / 32) * sizeof(int) + (size_t)sp.held * sp.vecs * 16;
+  if (e == cudaSuccess && smem > 48 * 1024) e = allow_smem(kernel, sort_ints(kMaxExperts, threads / 32) * sizeof(int) + kHeldBytes);
   if (e == cudaSuccess) e = launch_kernel(kernel, kSortCtas, threads, smem, st, 0, ids, sp);
   return e == cudaSuccess ? (int)CTB_OK : cuda_fail(e, "ctb_moe_ffn sort launch");
 }
@@ -781,7 +932,7 @@ extern "C" int ctb_moe_ffn(ctb_ctx* ctx, void* stream, const void* hidden, const
   if (r) return r;
   unsigned char* ws = static_cast<unsigned char*>(wsv);
   const int total = (int)(T * topk);
-  const int64_t max_blocks = total / kMaxBlockSlots + std::min<int64_t>(total, E);
+  const int64_t max_blocks = total / kMmaSlots + std::min<int64_t>(total, E);
   SortParams sp;
   sp.topk_w = static_cast<const __half*>(topk_weights);
   sp.X = static_cast<const uint4*>(hidden);
@@ -794,15 +945,22 @@ extern "C" int ctb_moe_ffn(ctb_ctx* ctx, void* stream, const void* hidden, const
   sp.early = total <= kEarlySlots;
   sp.T = (int)T; sp.topk = (int)topk; sp.E = (int)E; sp.vecs = (int)(H / 8); sp.total = total;
   sp.chunk = (total + kSortCtas - 1) / kSortCtas;
+  // a chunk's tokens if they fit; two are needed for the slots to get on at all
+  const int64_t tokens = (sp.chunk + topk - 1) / topk + 1, fit = (int64_t)kHeldBytes / (H * 2);
+  sp.held = sp.early || fit < 2 ? 0 : (int)std::min(tokens, fit);
   sp.status = ctx->dev_status;
   r = ids_bits == 32 ? launch_sort<int>(st, topk_ids, sp) : launch_sort<long long>(st, topk_ids, sp);
   if (r) return r;
-  // gate/up projection with the SwiGLU epilogue: act(:, row) = silu(Wg x) * (Wu x)
-  r = launch_projection<true>(ctx, st, w1, ws + sc.xs, ws + sc.act, H, 2 * I, I, E, sc, ws, max_blocks,
-                              sp.early ? topk_ids : nullptr, ids_bits, T, topk);
-  if (r) return r;
-  // down projection scaled by the routing weight, one f16 row per slot (the reference's cache3)
-  r = launch_projection<false>(ctx, st, w2, ws + sc.act, ws + sc.xs, I, H, H, E, sc, ws, max_blocks, nullptr, 0, T, topk);
+  auto project = [&](auto ring_tag) -> int {
+    constexpr bool RING = decltype(ring_tag)::value;
+    // gate/up projection with the SwiGLU epilogue: act(:, row) = silu(Wg x) * (Wu x)
+    const int bad = launch_projection<true, RING>(ctx, st, w1, ws + sc.xs, ws + sc.act, H, 2 * I, I, E, sc, ws, max_blocks,
+                                                  RING ? nullptr : topk_ids, ids_bits, T, topk);
+    if (bad) return bad;
+    // down projection scaled by the routing weight, one f16 row per slot (the reference's cache3)
+    return launch_projection<false, RING>(ctx, st, w2, ws + sc.act, ws + sc.xs, I, H, H, E, sc, ws, max_blocks, nullptr, 0, T, topk);
+  };
+  r = sp.early ? project(std::false_type()) : project(std::true_type());
   if (r) return r;
   const long long n8 = T * (H / 8);
   cudaError_t e = launch_kernel(moe_sorted_combine_kernel, (unsigned)((n8 + 255) / 256), 256, 0, st, 0, (const __half*)(ws + sc.xs),

@@ -95,6 +95,32 @@ def test_cutile_moe_reference_cases(cuda, T, H, E, I, topk):
     assert ref.rel_fro(out.cpu().numpy(), want) <= TOL
 
 
+# More than 2048 slots.  Blocks of one and of two MMAs whose accumulators follow each other in the ring of TMEM columns: experts at
+# the edges of 256, 320 and 512 slots, and in turn with small ones; then token rows that do and do not fit a CTA of the sort at
+# once, that fit only through registers, and more slots than a CTA counts itself.
+@pytest.mark.parametrize("H,I,topk,counts", [
+    (128, 2048, 1, (257, 320, 16, 272, 304, 0, 288, 321, 1, 319, 256, 255, 273, 17, 512, 513, 640, 289, 32, 320, 320, 320, 258)),
+    (64, 1536, 1, (320, 33, 320, 320, 304, 304, 304, 16, 300, 1, 320, 320, 48, 290, 290, 290, 290, 700, 452, 226)),
+    (8, 256, 3, 900), (16392, 16, 1, 2100), (41000, 8, 8, 257), (64, 64, 2, 8300)])
+def test_cutile_moe_many_slots(cuda, H, I, topk, counts):
+    import torch
+    g = np.random.default_rng(11)
+    if topk == 1 and isinstance(counts, tuple):
+        ids = g.permutation(np.repeat(np.arange(len(counts)), counts))[None] + 1
+        T, E = ids.shape[1], len(counts)
+        w = g.random((1, T)).astype(np.float16)
+    else:
+        T, E = counts, 9 if topk < 8 else 8
+        ids, w = random_routing(T, E, topk, seed=3)
+    d = inputs.moe(tokens=T, hidden=H, experts=E, inter=I, topk=topk, seed=6)
+    X, w1, w2 = dev(d, "X", "w1", "w2")
+    out = cuda.moe.cutile_moe(X, w1, w2, torch.from_numpy(w).cuda(), torch.from_numpy(ids.astype(np.int32)).cuda(), 128, 128, 64)
+    again = cuda.moe.cutile_moe(X, w1, w2, torch.from_numpy(w).cuda(), torch.from_numpy(ids.astype(np.int64)).cuda(), 128, 128, 64)
+    assert torch.equal(out, again)
+    want = ref.moe_ffn(d["X"], d["w1"], d["w2"], w, ids)
+    assert ref.rel_fro(out.cpu().numpy(), want) <= TOL
+
+
 def test_moe_benchmark_config_with_router(cuda):
     import torch
     d = inputs.moe()  # 256 tokens, hidden 1024, 32 experts, inter 2048, top-2, seed 4
