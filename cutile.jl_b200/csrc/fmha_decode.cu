@@ -7,7 +7,8 @@
 //
 // Work is cut into blocks of 256 keys of one (batch, key/value head) pair.  The blocks of all pairs form one line that
 // the CTAs (one per SM) share out in equal contiguous ranges, whatever the number of pairs and keys is: a CTA works
-// through the end of one pair, whole pairs, the head of another.  Inside a block each of the eight warps owns 32 keys: it
+// through the end of one pair, whole pairs, the head of another.  With no more pairs than SMs the pairs are cut into as many equal
+// parts as there are SMs for, and a CTA has a part of one pair only, unless too many SMs would be idle.  Inside a block each of the eight warps owns 32 keys: it
 // has its own ring of stages that its lane 0 fills by TMA (K tile and V tile, 4 KB each, 128-byte swizzle, up to 192 KB
 // in flight per SM), its own running maximum, sum and output, and waits for nobody until the CTA leaves the pair.
 // S = Q K^T and O += P V are m16n8k16 tensor-core instructions on registers (a 128-row tcgen05 tile would be 88 % padding;
@@ -17,7 +18,8 @@
 // pair is asked for before the warps meet: short heads are bound by these latencies (8192 heads of one row and 100 keys: 126 us
 // when every warp took a tile and Q was asked for in its turn, 84 now; 3200 of 16 x 16: 70 and 39).
 // Leaving a pair, the warps' results meet in shared memory; a pair that one CTA covers is written at once, otherwise the
-// part goes to scratch and the CTA that arrives last adds the parts in ascending order.
+// part goes to scratch and the CTA that arrives last adds the parts, each warp every eighth, in a fixed order (one thread per four
+// outputs took them one after the other, with two divisions each: 32 heads over 4, 8000 keys 18.3 us, now 10.1).
 #include <cuda_bf16.h>
 #include <math.h>
 
@@ -44,6 +46,7 @@ struct Params {
   int seq_q, keys, seq_kv, group, rows;  // keys: up to the last one that some query sees
   int input_pos, causal, blocks_per_pair;
   long long blocks;
+  int split;  // parts of a pair, a CTA each; 0: contiguous ranges
   float scale_log2;
   float* part;   // [CTA][first, last pair of its range][rows x (64 outputs), maxima, sums]
   unsigned* tickets;  // per CTA: parts left of the pair that begins in its range and ends in another's
@@ -115,7 +118,15 @@ __global__ void __launch_bounds__(kThreads, 1)
   grid_dependency_sync();
 
   const int cta = blockIdx.x, grid = gridDim.x;
-  const long long lo = first_block(cta, p.blocks, grid), hi = first_block(cta + 1, p.blocks, grid);
+  long long lo, hi;
+  if (p.split) {
+    const int pr = cta / p.split, k = cta - pr * p.split;
+    lo = (long long)pr * p.blocks_per_pair + k * p.blocks_per_pair / p.split;
+    hi = (long long)pr * p.blocks_per_pair + (k + 1) * p.blocks_per_pair / p.split;
+  } else {
+    lo = first_block(cta, p.blocks, grid);
+    hi = first_block(cta + 1, p.blocks, grid);
+  }
   unsigned char* ring = smem + warp * (kStages * 2 * kTileBytes);
   // In the last block of a pair the keys end at some warp's tile; the warps behind it have none there.
   const int last_block = p.blocks_per_pair - 1, last_tiles = min(kWarps, (p.keys - last_block * kBlockKeys + kTileKeys - 1) / kTileKeys);
@@ -320,31 +331,56 @@ __global__ void __launch_bounds__(kThreads, 1)
         part[kMaxRows * (kD + 1) + row] = L;
       }
     }
-    const int c0 = (int)owner(pair_first, p.blocks, grid), c1 = (int)owner(pair_end - 1, p.blocks, grid);
-    __threadfence();
+    const int c0 = p.split ? pair * p.split : (int)owner(pair_first, p.blocks, grid);
+    const int c1 = p.split ? c0 + p.split - 1 : (int)owner(pair_end - 1, p.blocks, grid);
     __syncthreads();
-    if (tid == 0) last_s = atomicInc(&p.tickets[c0], (unsigned)(c1 - c0)) == (unsigned)(c1 - c0);  // back to zero by the last
+    if (tid == 0) {
+      __threadfence();
+      last_s = atomicInc(&p.tickets[c0], (unsigned)(c1 - c0)) == (unsigned)(c1 - c0);  // back to zero by the last
+      __threadfence();
+    }
     __syncthreads();
     if (last_s) {
-      __threadfence();
+      // warp w takes the parts c0 + w, c0 + w + 8, ...; a lane has two outputs of every row, lane r maximum and sum of row r
+      const bool second = !p.split && first_block(c0, p.blocks, grid) != pair_first;  // c0's range begins before the pair
+      auto part_of = [&](int c) { return p.part + ((long long)c * 2 + (c == c0 && second ? 1 : 0)) * kPartFloats; };
+      const int r = lane & (R - 1);
+      float mw = -INFINITY, lw = 0.f;
+      float2 v[R];
+#pragma unroll
+      for (int k = 0; k < R; ++k) v[k] = make_float2(0.f, 0.f);
+#pragma unroll 8
+      for (int c = c0 + warp; c <= c1; c += kWarps) mw = fmaxf(mw, __ldcg(part_of(c) + kMaxRows * kD + r));
+      const float ref = mw == -INFINITY ? 0.f : mw;
+#pragma unroll 2
+      for (int c = c0 + warp; c <= c1; c += kWarps) {
+        const float* pc = part_of(c);
+        float2 x[R];
+#pragma unroll
+        for (int k = 0; k < R; ++k) x[k] = __ldcg(reinterpret_cast<const float2*>(pc + k * kD) + lane);
+        const float f = ex2_approx_ftz(__ldcg(pc + kMaxRows * kD + r) - ref);
+        lw += __ldcg(pc + kMaxRows * (kD + 1) + r) * f;
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+          const float fk = __shfl_sync(0xffffffffu, f, k);
+          if (k < p.rows) {
+            v[k].x += x[k].x * fk;
+            v[k].y += x[k].y * fk;
+          }
+        }
+      }
+      if (lane < R) {
+        ml[0][warp][lane] = mw;
+        ml[1][warp][lane] = lw;
+      }
+#pragma unroll
+      for (int k = 0; k < R; ++k) *reinterpret_cast<float2*>(outs + (warp * R + k) * kPitch + 2 * lane) = v[k];
+      __syncthreads();
       if (mine) {
-        auto part_of = [&](int c) {
-          const int fp = (int)(first_block(c, p.blocks, grid) / p.blocks_per_pair);
-          return p.part + ((long long)c * 2 + (pair == fp ? 0 : 1)) * kPartFloats;
-        };
         M = -INFINITY;
-        for (int c = c0; c <= c1; ++c) M = fmaxf(M, __ldcg(part_of(c) + kMaxRows * kD + row));
-        const float ref = M == -INFINITY ? 0.f : M;
         L = 0.f;
         acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-        for (int c = c0; c <= c1; ++c) {  // ascending: a fixed order
-          const float* pc = part_of(c);
-          const float f = ex2_approx_ftz(__ldcg(pc + kMaxRows * kD + row) - ref);
-          const float4 v = __ldcg(reinterpret_cast<const float4*>(pc + row * kD + d0));
-          L += __ldcg(pc + kMaxRows * (kD + 1) + row) * f;
-          acc.x += v.x * f; acc.y += v.y * f; acc.z += v.z * f; acc.w += v.w * f;
-        }
+        meet(std::true_type());
         write_out();
       }
     }
@@ -386,7 +422,20 @@ int fmha_decode(ctb_ctx* ctx, cudaStream_t st, const void* Q, const void* K, con
   p.blocks_per_pair = (int)((keys + kBlockKeys - 1) / kBlockKeys);
   const int64_t pairs = kv_heads * batch;
   p.blocks = pairs * p.blocks_per_pair;
-  const int grid = (int)std::min<int64_t>(p.blocks, ctx->sm_count);
+  int grid = (int)std::min<int64_t>(p.blocks, ctx->sm_count);
+  p.split = 0;
+  if (pairs <= ctx->sm_count) {
+    const int64_t split = std::min<int64_t>(p.blocks_per_pair, ctx->sm_count / pairs);
+    const int64_t most = (p.blocks_per_pair + split - 1) / split;  // blocks of the largest part
+    // A block (64 KB) takes an SM 1.46 us when all are loading and 0.93 by itself; ranges that cross from pair to pair cost 4.5 us
+    // more, for the second pair that a CTA leaves.  One key/value head, 8192 keys: 29.2 us in ranges, 7.2 in parts; 120 heads of
+    // 2000: 16.8 and 12.5; 75 heads of 6000, where one part each leaves half of the SMs idle, 25.2 and 26.3.
+    const double parts = (double)most * std::max(0.93, 1.46 * (double)(split * pairs) / ctx->sm_count);
+    if (parts <= 1.46 * (double)p.blocks / grid + 4.5) {
+      p.split = (int)split;
+      grid = (int)(split * pairs);
+    }
+  }
   if ((size_t)grid * 2 * kPartFloats * sizeof(float) > kStreamScratchBytes || grid > kTickets)
     return fail(CTB_UNSUPPORTED, "ctb_fmha_fwd: more SMs than the split over keys has scratch for");
   p.part = scratch.data;

@@ -59,6 +59,27 @@ def test_fmha_scale_and_large_scores(cuda):
     assert ref.rel_fro(out, want) <= TOL
 
 
+# (batch, kv heads, group, query rows, keys): one pair in as many parts as SMs, parts of unequal length, two parts, one part each, as
+# many pairs as SMs and one more, pairs that leave half of the SMs idle in parts (long: ranges), 1, 8, 9 and 16 rows
+@pytest.mark.parametrize("batch,kvh,group,seq_q,keys", [
+    (1, 1, 1, 1, 40000), (1, 1, 4, 4, 300), (1, 3, 1, 9, 5000), (2, 37, 2, 4, 513), (5, 10, 8, 1, 900), (3, 19, 3, 3, 9 * 256),
+    (75, 1, 1, 1, 1024), (75, 1, 1, 1, 9000), (37, 4, 1, 1, 600), (149, 1, 3, 1, 600), (1, 2, 16, 1, 257)])
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
+def test_fmha_few_rows_parts(cuda, dtype, batch, kvh, group, seq_q, keys):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(keys)
+    dt = getattr(torch, dtype)
+    q, k, v = (torch.randn(batch, h, n, 64, device="cuda", generator=g).to(dt)
+               for h, n in ((kvh * group, seq_q), (kvh, keys), (kvh, keys)))
+    out = cuda.fmha.cutile_fmha(q, k, v, causal=True, input_pos=keys - seq_q, query_group_size=group)
+    assert torch.equal(out, cuda.fmha.cutile_fmha(q, k, v, causal=True, input_pos=keys - seq_q, query_group_size=group))
+    for b in range(batch):
+        s = q[b].double() @ k[b].double().repeat_interleave(group, 0).transpose(1, 2) / 8
+        s.masked_fill_(torch.arange(keys, device="cuda") > torch.arange(seq_q, device="cuda")[:, None] + keys - seq_q, -torch.inf)
+        want = torch.softmax(s, -1) @ v[b].double().repeat_interleave(group, 0)
+        assert (out[b] - want).norm() <= (TOL if dtype == "float16" else 1e-2) * want.norm()
+
+
 def test_fmha_causal_prefix_property_full_size(cuda):
     """Size-independent property at the benchmark shape: under the causal mask the output of the first 512
     queries does not depend on the later keys/values, so it equals the result on the truncated problem."""
