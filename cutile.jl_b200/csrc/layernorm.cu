@@ -301,6 +301,7 @@ __global__ void __launch_bounds__(kFwdThreads) ln_fwd_generic_kernel(const float
 constexpr int kBwdThreads = 512;
 constexpr int kBwdWarps = kBwdThreads / 32;
 constexpr int kBwdStages = 3;
+constexpr int kBwdRingStages = 8;  // of ln_bwd_ring_kernel, at most
 
 // Fast path.  Grid = group_size_m * C CTAs in clusters of C; cluster g owns
 // partial column g; CTA rank r of the cluster takes rows g + G*(r + C*j).
@@ -493,9 +494,9 @@ __device__ __forceinline__ void cluster_columns(float* mine, float* __restrict__
   cluster.sync();  // peers may still be reading this CTA's shared memory
 }
 
-// Rows of at most 1024 columns, any alignment: a warp per row, row and partial dW/dB in its registers, no barrier until the
+// Rows of at most 512 columns, any alignment: a warp per row, row and partial dW/dB in its registers, no barrier until the
 // end.  Grid and clusters as above: warp w of CTA r of cluster g takes the rows g + G * (r * warps + w + C * warps * j).
-// 16384 x 256: 72.7 us with a CTA per row, now 13.1; 16384 x 1024: 86.0, now 49.1.
+// 16384 x 256: 72.7 us with a CTA per row, now 13.1.
 constexpr int kBwdWarpThreads = 256;
 template <int V, int NE>
 __global__ void __launch_bounds__(kBwdWarpThreads)
@@ -575,6 +576,141 @@ __global__ void __launch_bounds__(kBwdWarpThreads)
     float a = part[c];
 #pragma unroll
     for (int w = 1; w < kWarps; ++w) a += part[(size_t)w * 2 * N + c];
+    part[c] = a;
+  }
+  cluster_columns(part, DW, DB, N, g);
+}
+
+// Aligned rows of at most 1024 columns: a warp per row as above, but the rows come by bulk copies through a ring of the warp's own in
+// shared memory, whose stage is asked for again as soon as the row is in registers.  With the row's loads issued when its turn
+// came, the warps that the registers leave room for (8 per SM at 1024 columns) kept 64 KB of loads in flight and waited
+// for them; the rings keep 192 KB.  16000 x 1000: 52.1 us, now 35.7;
+// 4000 x 640: 12.6 and 10.7; 1000 x 512: 6.1 and 4.0.
+constexpr size_t kBwdRingBytes = 192 * 1024;
+template <int NE, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 1)
+    ln_bwd_ring_kernel(float* __restrict__ DX, const float* __restrict__ DY, float* __restrict__ DW, float* __restrict__ DB,
+                       const float* __restrict__ X, const float* __restrict__ W, const float* __restrict__ Mean,
+                       const float* __restrict__ Rstd, int N, int M, long long ldx, long long lddy, long long lddx, int G, int C,
+                       int stages, int* status) {
+  extern __shared__ __align__(128) unsigned char smem[];  // [warps][stages][x row | dy row], then [warps][2][N] partial sums
+  __shared__ __align__(8) uint64_t full[WARPS][kBwdRingStages];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = blockIdx.x / C, rank = blockIdx.x - g * C;
+  const uint32_t row_bytes = (uint32_t)N * 4u;
+  if (lane == 0) {
+    for (int s = 0; s < stages; ++s) mbar_init(&full[warp][s], 1);
+    fence_mbar_init();
+  }
+  __syncwarp();
+  grid_dependency_sync();
+  const long long first = g + (long long)G * (rank * WARPS + warp), step = (long long)G * C * WARPS;
+  const int nrows = first < M ? (int)((M - first + step - 1) / step) : 0;
+  unsigned char* ring = smem + (size_t)warp * stages * 2 * row_bytes;
+  int issued = 0;
+  auto issue = [&]() {  // the warp's next row
+    if (issued >= nrows) return;
+    if (lane == 0) {
+      const long long row = first + issued * step;
+      uint64_t* bar = &full[warp][issued % stages];
+      unsigned char* at = ring + (size_t)(issued % stages) * 2 * row_bytes;
+      mbar_expect_tx(bar, 2 * row_bytes);
+      bulk_g2s(at, X + row * ldx, row_bytes, bar);
+      bulk_g2s(at + row_bytes, DY + row * lddy, row_bytes, bar);
+    }
+    ++issued;
+  };
+  for (int s = 0; s < stages; ++s) issue();
+  const float inv_n = 1.0f / (float)N;
+  float w[NE][4], dw[NE][4], db[NE][4];
+#pragma unroll
+  for (int k = 0; k < NE; ++k) {
+    const int c = (lane + 32 * k) * 4;
+    if (c < N) load_vec<4>(W + c, w[k]);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) dw[k][q] = db[k][q] = 0.f;
+  }
+  float mean = 0.f, rstd = 0.f;
+  if (nrows > 0) {
+    mean = Mean[first];
+    rstd = Rstd[first];
+  }
+  bool ok = true;
+  int i = 0;
+  for (; i < nrows; ++i) {
+    const int s = i % stages;
+    const long long row = first + i * step;
+    float mean_next = 0.f, rstd_next = 0.f;
+    if (i + 1 < nrows) {  // issued before the wait so the latency is hidden behind it
+      mean_next = Mean[row + step];
+      rstd_next = Rstd[row + step];
+    }
+    ok = CTB_WARP_WAIT(&full[warp][s], (i / stages) & 1, status, DEV_TIMEOUT_TMA);
+    if (!ok) break;
+    const float* xs = reinterpret_cast<const float*>(ring + (size_t)s * 2 * row_bytes);
+    float xh[NE][4], dy[NE][4];
+#pragma unroll
+    for (int k = 0; k < NE; ++k) {
+      const int c = (lane + 32 * k) * 4;
+      if (c < N) {
+        const float4 x = *reinterpret_cast<const float4*>(xs + c), d = *reinterpret_cast<const float4*>(xs + N + c);
+        xh[k][0] = x.x; xh[k][1] = x.y; xh[k][2] = x.z; xh[k][3] = x.w;
+        dy[k][0] = d.x; dy[k][1] = d.y; dy[k][2] = d.z; dy[k][3] = d.w;
+      }
+    }
+    __syncwarp();  // every lane has read the stage
+    issue();
+    float c1 = 0.f, c2 = 0.f;
+#pragma unroll
+    for (int k = 0; k < NE; ++k) {
+      const int c = (lane + 32 * k) * 4;
+      if (c < N) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          xh[k][q] = (xh[k][q] - mean) * rstd;
+          const float wd = __fmul_rn(w[k][q], dy[k][q]);
+          c1 += xh[k][q] * wd;
+          c2 += wd;
+        }
+      }
+    }
+    c1 = warp_sum(c1) * inv_n;
+    c2 = warp_sum(c2) * inv_n;
+#pragma unroll
+    for (int k = 0; k < NE; ++k) {
+      const int c = (lane + 32 * k) * 4;
+      if (c < N) {
+        float dx[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          dx[q] = (__fmul_rn(w[k][q], dy[k][q]) - (xh[k][q] * c1 + c2)) * rstd;  // the product as c1 and c2 have it
+          dw[k][q] += dy[k][q] * xh[k][q];
+          db[k][q] += dy[k][q];
+        }
+        store_vec<4>(DX + row * lddx + c, dx);
+      }
+    }
+    mean = mean_next;
+    rstd = rstd_next;
+  }
+  for (int k = i; k < issued; ++k)  // a wait ran out: copies still in flight must land before the ring is used otherwise
+    (void)CTB_WARP_WAIT(&full[warp][k % stages], (k / stages) & 1, status, DEV_TIMEOUT_TMA);
+  __syncthreads();
+  float* part = reinterpret_cast<float*>(smem);
+  float* mine = part + (size_t)warp * 2 * N;
+#pragma unroll
+  for (int k = 0; k < NE; ++k) {
+    const int c = (lane + 32 * k) * 4;
+    if (c < N) {
+      *reinterpret_cast<float4*>(mine + c) = make_float4(dw[k][0], dw[k][1], dw[k][2], dw[k][3]);
+      *reinterpret_cast<float4*>(mine + N + c) = make_float4(db[k][0], db[k][1], db[k][2], db[k][3]);
+    }
+  }
+  __syncthreads();
+  for (int c = threadIdx.x; c < 2 * N; c += WARPS * 32) {  // ascending warps
+    float a = part[c];
+#pragma unroll
+    for (int k = 1; k < WARPS; ++k) a += part[(size_t)k * 2 * N + c];
     part[c] = a;
   }
   cluster_columns(part, DW, DB, N, g);
@@ -731,7 +867,7 @@ template <typename Kernel>
 int launch_bwd_regs(ctb_ctx* ctx, Kernel k, int threads, size_t smem, int rows, cudaStream_t st, float* DX, const float* DY, float* DW,
                     float* DB, const float* X, const float* W, const float* Mean, const float* Rstd, int N, int M, long long ldx,
                     long long lddy, long long lddx, int G) {
-  cudaError_t e = allow_smem(k, (size_t)2 * kBwdThreads * kGenCols * 4);  // kernels of up to 1024 columns: 8 warps x 2 x N floats, the same
+  cudaError_t e = allow_smem(k, (size_t)2 * kBwdThreads * kGenCols * 4);  // the kernel with a warp per row: 8 warps x 2 x N floats, at most half of it
   if (e != cudaSuccess) return cuda_fail(e, "ctb_layernorm_bwd: shared memory opt-in");
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem);
@@ -739,6 +875,21 @@ int launch_bwd_regs(ctb_ctx* ctx, Kernel k, int threads, size_t smem, int rows, 
   int C = 8;
   while (C > 1 && ((long long)G * C > (long long)ctx->sm_count * per_sm || (long long)G * C * rows > M)) C >>= 1;
   e = launch_kernel(k, G * C, threads, smem, st, C, DX, DY, DW, DB, X, W, Mean, Rstd, N, M, ldx, lddy, lddx, G, C);
+  return e == cudaSuccess ? (int)CTB_OK : cuda_fail(e, "ctb_layernorm_bwd_dx_partial_dwdb launch");
+}
+
+// One CTA per SM; as many per group (a power of two up to 8) as run at once and give every second warp a row.
+template <int NE, int WARPS>
+int launch_bwd_ring(ctb_ctx* ctx, cudaStream_t st, float* DX, const float* DY, float* DW, float* DB, const float* X, const float* W,
+                    const float* Mean, const float* Rstd, int N, int M, long long ldx, long long lddy, long long lddx, int G) {
+  auto k = ln_bwd_ring_kernel<NE, WARPS>;
+  const int stages = (int)std::min<size_t>(kBwdRingStages, kBwdRingBytes / ((size_t)WARPS * 2 * N * 4));
+  cudaError_t e = allow_smem(k, kBwdRingBytes);
+  if (e != cudaSuccess) return cuda_fail(e, "ctb_layernorm_bwd: shared memory opt-in");
+  int C = 8;
+  while (C > 1 && ((long long)G * C > ctx->sm_count || (long long)G * C * (WARPS / 2) > M)) C >>= 1;
+  e = launch_kernel(k, G * C, WARPS * 32, (size_t)WARPS * stages * 2 * N * 4, st, C, DX, DY, DW, DB, X, W, Mean, Rstd, N, M, ldx, lddy,
+                    lddx, G, C, stages, ctx->dev_status);
   return e == cudaSuccess ? (int)CTB_OK : cuda_fail(e, "ctb_layernorm_bwd_dx_partial_dwdb launch");
 }
 
@@ -820,11 +971,18 @@ int ctb_layernorm_bwd_dx_partial_dwdb(ctb_ctx* ctx, void* stream, float* DX, con
   const bool vec = N % 4 == 0 && ldx % 4 == 0 && lddy % 4 == 0 && lddx % 4 == 0 && aligned16(X) && aligned16(DY) &&
                    aligned16(DX) && aligned16(W);
   // A warp per row: as in the forward pass, but the other kernels need two barriers per row and fill up sooner, so the line
-  // lies at M = N / 4 (1024 columns: 300 rows 6.1 against 6.4 us, 64 rows 5.8 against 3.2).  Single floats only up to 512
-  // columns: 64 more registers of partial sums leave too few warps (2400 x 1023: 18.5 against 16.6 us).
-  if (N <= 256 || (4 * M >= N && N <= (vec ? kWarpCols : 512))) {
-    auto k = vec ? (n <= 256 ? ln_bwd_warp_kernel<4, 2> : n <= 512 ? ln_bwd_warp_kernel<4, 4> : ln_bwd_warp_kernel<4, 8>)
-                 : (n <= 256 ? ln_bwd_warp_kernel<1, 8> : ln_bwd_warp_kernel<1, 16>);
+  // lies at M = N / 4 (1024 columns: 150 rows 5.0 us by either, 300 rows 3.9 against 6.4).  Aligned rows come through rings above
+  // 256 columns.  Below, a row's loads are few and the kernel without rings has more warps, which pays with many rows (16000 x
+  // 128: 7.6 against 10.3 us); between 1024 and 4096 rows it needs clusters and the rings do not (2000 x 256: 6.4 against
+  // 4.6).  Single floats only up to 512 columns: 64 more registers of partial sums leave too few warps (2400 x 1023: 18.5
+  // against 16.6 us).
+  if (vec && N <= kWarpCols && (N > 256 ? 4 * M >= N : M > 1024 && M <= 4096)) {
+    if (n <= 256) return launch_bwd_ring<2, 16>(ctx, st, DX, DY, DW, DB, X, W, Mean, Rstd, n, m, ldx, lddy, lddx, G);
+    if (n <= 512) return launch_bwd_ring<4, 16>(ctx, st, DX, DY, DW, DB, X, W, Mean, Rstd, n, m, ldx, lddy, lddx, G);
+    return launch_bwd_ring<8, 8>(ctx, st, DX, DY, DW, DB, X, W, Mean, Rstd, n, m, ldx, lddy, lddx, G);
+  }
+  if (N <= 256 || (!vec && 4 * M >= N && N <= 512)) {
+    auto k = vec ? ln_bwd_warp_kernel<4, 2> : n <= 256 ? ln_bwd_warp_kernel<1, 8> : ln_bwd_warp_kernel<1, 16>;
     constexpr int kWarps = kBwdWarpThreads / 32;
     return launch_bwd_regs(ctx, k, kBwdWarpThreads, (size_t)kWarps * 2 * n * 4, kWarps, st, DX, DY, DW, DB, X, W, Mean, Rstd, n, m,
                            ldx, lddy, lddx, G);

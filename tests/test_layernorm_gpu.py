@@ -63,8 +63,17 @@ def test_layernorm_row_widths(cuda, M, N, G):
     test_layernorm_parity(cuda, M, N, G)
 
 
-def test_layernorm_strided(cuda):
-    d = inputs.layernorm(M=64, N=512, seed=5)
+# the backward kernel whose warps have rings of rows: no row, one, fewer and more rows per warp than stages, the widths where the
+# rows per lane and the warps change, rows on both sides of the lines 1024 and 4096 below 256 columns
+@pytest.mark.parametrize("M,N,G", [(66, 260, 64), (1500, 512, 8), (3100, 516, 64), (5000, 1024, 3), (4000, 1020, 64),
+                                   (1025, 8, 64), (4096, 252, 64), (4097, 256, 64), (1024, 256, 64), (2000, 300, 200)])
+def test_layernorm_row_rings(cuda, M, N, G):
+    test_layernorm_parity(cuda, M, N, G)
+
+
+@pytest.mark.parametrize("M", [64, 700])
+def test_layernorm_strided(cuda, M):
+    d = inputs.layernorm(M=M, N=512, seed=5)
     Y, Mean, Rstd, DX, DW, DB = run_fwd_bwd(cuda, d, 64, ld=640)
     rY, rMean, rRstd = ref.layernorm_fwd(d["X"], d["W"], d["B"], d["eps"])
     rDX, rDW, rDB = ref.layernorm_bwd(d["X"], d["W"], d["DY"], rMean, rRstd)
