@@ -254,7 +254,15 @@ __device__ __forceinline__ uint32_t map_to_cta(const void* smem_ptr, uint32_t ra
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(smem_u32(smem_ptr)), "r"(rank));
   return out;
 }
+// Stores (a, b) at the place that `slot` has in CTA `rank` of the cluster, asynchronously; the eight bytes count on that CTA's `bar`.
+__device__ __forceinline__ void send_to_cta(const void* slot, float a, float b, const void* bar, uint32_t rank) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(map_to_cta(slot, rank)),
+               "f"(a), "f"(b), "r"(map_to_cta(bar, rank))
+               : "memory");
+}
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+// Meets the cluster without making stores visible to it (a release waits for those of the thread).
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // Arrival on a barrier that may live in the peer CTA, for accumulators that have been read: what it orders is TMEM (by the
 // tcgen05 fences on both sides), not memory, so it releases to its own CTA only.  A release to the cluster waits until the

@@ -276,8 +276,9 @@ __global__ void __launch_bounds__(kThreads) softmax_regs_kernel(T* __restrict__ 
 // The 16-byte aligned middle of the row arrives in chunks of kChunkVecs vectors, one bulk copy and mbarrier each; up to
 // one vector's elements before and after it are loaded one by one by rank 0, so rows may start anywhere (1024 x 50001 f32:
 // 227 us with scalar loads and a second read).  One online pass takes the running maximum and sum of exponentials of each
-// chunk as it lands, the CTAs exchange them through distributed shared memory (one cluster barrier per row, two sets of
-// slots), and a second pass evaluates the exponentials again, scales and stores; a chunk's part of the buffer takes the
+// chunk as it lands, the CTAs send them to each other (asynchronous stores that count on an mbarrier of the receiver, two sets of
+// slots; with a cluster barrier per row, whose release waits for the stores of the row before, 1024 x 50001 f32 took 76.3 us, now
+// 73.4, 800 x 65000 f16 51.3 and 44.9), and a second pass evaluates the exponentials again, scales and stores; a chunk's part of the buffer takes the
 // next row's chunk as soon as it was read.
 constexpr int kRowThreads = 512;
 constexpr int kChunkVecs = 1024;
@@ -305,30 +306,24 @@ __global__ void __launch_bounds__(kRowThreads) softmax_long_kernel(T* __restrict
   constexpr int V = 16 / (int)sizeof(T);
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t full[kMaxChunks];
-  __shared__ float red[kRowThreads / 32];
-  __shared__ float2 peers[2][kMaxCluster];  // (maximum, sum) of every CTA of the cluster, for even and odd rows
+  __shared__ __align__(16) float red[2][2][kRowThreads / 32];  // maximum and sum of every warp, for even and odd rows
+  __shared__ __align__(8) float2 peers[2][kMaxCluster];         // and of every CTA of the cluster
+  __shared__ __align__(8) uint64_t met[2];               // all of peers[] have come
   const int tid = threadIdx.x;
   const int rank = C > 1 ? (int)cluster_ctarank() : 0, team = blockIdx.x / C, teams = gridDim.x / C;
   if (tid == 0) {
     for (int c = 0; c < kMaxChunks; ++c) mbar_init(&full[c], 1);
+    mbar_init(&met[0], 1);
+    mbar_init(&met[1], 1);
     fence_mbar_init();
   }
   __syncthreads();
-  if (C > 1) {  // the peers' shared memory exists
+  if (C > 1) {  // the peers' shared memory and barriers exist
     cluster_arrive();
     cluster_wait();
   }
   grid_dependency_sync();
   uint4* buf = reinterpret_cast<uint4*>(smem);
-  auto block_reduce = [&](float v, bool is_max) {
-    v = is_max ? warp_max(v) : warp_sum(v);
-    if ((tid & 31) == 0) red[tid >> 5] = v;
-    __syncthreads();
-    float r = red[0];
-    for (int i = 1; i < kRowThreads / 32; ++i) r = is_max ? fmaxf(r, red[i]) : r + red[i];  // fixed order
-    __syncthreads();
-    return r;
-  };
   // the row's elements before the first 16-byte boundary, and the vectors [v0, v1) of the middle that are this CTA's
   auto layout = [&](int row, const T*& src, int& head, int& nvec, int& v0, int& v1) {
     src = in + (long long)row * ld_in;
@@ -390,15 +385,23 @@ __global__ void __launch_bounds__(kRowThreads) softmax_long_kernel(T* __restrict
         l += s;
       }
     }
-    float mx = block_reduce(m, true);
-    float sum = block_reduce(l * exp_sub(m, mx), false);
+    auto over_warps = [&](float v, int which) {  // two sets of slots: no barrier behind the reads
+      float* slot = red[it & 1][which];
+      v = which == 0 ? warp_max(v) : warp_sum(v);
+      if ((tid & 31) == 0) slot[tid >> 5] = v;
+      __syncthreads();
+      float r = slot[0];
+#pragma unroll
+      for (int k = 1; k < kRowThreads / 32; ++k) r = which == 0 ? fmaxf(r, slot[k]) : r + slot[k];  // fixed order
+      return r;
+    };
+    float mx = over_warps(m, 0);
+    float sum = over_warps(l * exp_sub(m, mx), 1);
     if (C > 1) {
-      if (tid < C) {
-        const uint32_t dst = map_to_cta(&peers[it & 1][rank], (uint32_t)tid);
-        asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(dst), "f"(mx), "f"(sum) : "memory");
-      }
-      cluster_arrive();
-      cluster_wait();
+      // A peer sends its next row but one only after this CTA has sent its next, that is, read these slots.
+      if (tid == 0) mbar_expect_tx(&met[it & 1], C * (uint32_t)sizeof(float2));
+      if (tid < C) send_to_cta(&peers[it & 1][rank], mx, sum, &met[it & 1], (uint32_t)tid);
+      if (!mbar_wait(&met[it & 1], (it >> 1) & 1, status, DEV_TIMEOUT_TMA)) alive = false;
       float M2 = -FLT_MAX;
       for (int k = 0; k < C; ++k) M2 = fmaxf(M2, peers[it & 1][k].x);
       sum = 0.f;
@@ -438,6 +441,10 @@ __global__ void __launch_bounds__(kRowThreads) softmax_long_kernel(T* __restrict
   if (tid == 0)  // a wait ran out: copies under way must land before the CTA gives its shared memory back
     for (; pending; pending &= pending - 1)
       (void)mbar_wait(&full[__ffs(pending) - 1], (phases >> (__ffs(pending) - 1)) & 1, status, DEV_TIMEOUT_TMA);
+  if (C > 1) {  // no peer sends any more
+    cluster_arrive_relaxed();
+    cluster_wait();
+  }
 }
 
 // ------------------------------------------------------------------ variant 1, any row

@@ -149,3 +149,20 @@ def test_softmax_masked_rows(cuda, n, half):
         assert out[9].isnan().all() and want[9].isnan().all()
         assert ((out[:9].double() - want[:9]).abs().amax(1) <= (1e-3 if half else 2e-6) * want[:9].amax(1)).all()
         assert (out[:9][x[:9] == -inf] == 0).all()
+
+
+@pytest.mark.parametrize("M,N,dtype", [(1200, 27001, "float32"), (500, 53003, "float32"), (250, 110001, "float32"), (250, 212001, "float16")])
+def test_softmax_clusters_many_rows(cuda, M, N, dtype):
+    """Two, four and eight CTAs per row, each with several rows: their two sets of slots and barriers are used again and again, and
+    the maximum lies with another CTA in every row."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(N)
+    x = torch.randn(M, N, device="cuda", generator=g)
+    x[torch.arange(M), (torch.arange(M) * 7919) % N] = 9.0
+    x = x.to(getattr(torch, dtype))
+    out = torch.empty_like(x)
+    for _ in range(2):
+        cuda.softmax.softmax_chunked_kernel(out, x, N, 1024)
+    want = torch.softmax(x.double(), -1)
+    assert ((out - want).abs().amax(1) <= (TOL if dtype == "float32" else 1e-3) * want.amax(1)).all()
+    cuda.check_device_status(0)
