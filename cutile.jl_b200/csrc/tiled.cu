@@ -98,6 +98,7 @@ struct Operands {
   long long stride[kMaxInputs][3];
   int mode[kMaxInputs];
   unsigned slot[kMaxInputs];  // offset in shared memory
+  unsigned temp_slot;         // of the temporaries
 };
 
 // ---- postfix program -> accumulator-machine instructions (host) ---------------------------------------------------
@@ -606,17 +607,6 @@ __device__ __forceinline__ void tree_dispatch(unsigned idx, F&& f) {
   }
 }
 
-// f(temporary k) for the run-time index k < NT
-template <int NT, int Q = 0, int N, int H, typename F>
-__device__ __forceinline__ void with_temp(Pair (&tmp)[N][H], unsigned k, F f) {
-  if constexpr (Q + 1 < NT) {
-    if (k == (unsigned)Q) f(tmp[Q]);
-    else with_temp<NT, Q + 1>(tmp, k, f);
-  } else if constexpr (NT > 0) {
-    f(tmp[NT - 1]);
-  }
-}
-
 // Division of an index below 2^31 by a fixed extent: q = u * mul >> shift (mul = floor(2^shift / d) + 1, exact there).
 struct FastDiv {
   unsigned d, mul;
@@ -640,23 +630,25 @@ struct Extents {
 // A group is four neighbouring elements of the destination, whatever the extents are (the last one may be partial); a
 // thread owns G groups per trip, a whole grid apart.  The operands of the NEXT trip are copied global -> shared by
 // cp.async (no registers, nothing waits on them) while the instructions run on the current trip's copies, so the latency
-// of HBM is off the critical path whatever the occupancy; registers hold the accumulator, the current operand and NT
-// temporaries.  A thread reads only the shared memory it filled itself: no CTA barrier anywhere.
-// Shared memory: per operand [2 buffers][G][256 threads] groups of 4 * sizeof(T) bytes, OP_FIXED [256 threads].
+// of HBM is off the critical path whatever the occupancy; registers hold the accumulator and the current operand,
+// and temporaries lie in shared memory too.  A thread reads only the shared memory it filled itself: no CTA barrier anywhere.
+// Shared memory: per operand [2 buffers][G][256 threads] groups of 4 * sizeof(T) bytes, OP_FIXED [256 threads]; per temporary [G]
+// [256 threads] groups of four floats.
 // A trip whose G groups all exist (all but a thread's last) runs without a bounds test.  LINEAR: every operand is laid out
 // like the destination, single or fixed (OP_LINEAR, OP_SCALAR, OP_SHIFTED, OP_FIXED), no coordinates are computed.
 // What bounds it: HBM for short expressions (A .+ b 6200 GB/s on 8192 x 4096 f32), instruction issue and dispatch latency
 // for long ones: a word costs about 24 issue slots of dispatch per thread (16 elements) and half a slot per element for +
 // and *.  0.5 v (1 + tanh(c (v + k v^3))), v = A .+ b, on 8192 x 4096 f32: 254 us with a stack of registers, one
 // instruction per operator and v evaluated five times; 183 with v in a temporary; 109 with pairs in 64-bit registers
-// (107 -> 69 instructions per element); 82 with the words below (7 words, one temporary, b read once); 68.5 with equal
-// trips.
-template <typename T, int G, int NT, bool LINEAR>
-__global__ void __launch_bounds__(256, NT == 0 || NT == 2 ? 4 : 3)
+// (107 -> 69 instructions per element); 82 with the words below (7 words, one temporary, b read once); 69.6 with equal
+// trips (55 instructions per element, 15 of them moves: a temporary in registers is copied wherever the paths of the words
+// meet); 61.1 with the temporary in shared memory, four loads or stores per word that names it. With two temporaries
+// (u v + u) / (v v + 1), u = A + b, v = A C: 161 and now 104 us; with three, 207 and 121.
+template <typename T, int G, bool TEMPS, bool LINEAR>
+__global__ void __launch_bounds__(256, TEMPS ? 3 : 4)
     tiled_broadcast_kernel(void* __restrict__ dest, const Operands in, const Program prog, int n_inputs, const Extents x) {
   ctb::grid_dependency_sync();
   constexpr int V = 4, H = V * G / 2, ES = (int)sizeof(T), VB = V * ES;
-  constexpr int NTR = NT > 0 ? NT : 1;
   extern __shared__ __align__(16) unsigned char tiled_smem[];
   const long long total = (x.n + V - 1) / V;  // groups
   const long long grid_stride = (long long)gridDim.x * blockDim.x;
@@ -792,6 +784,12 @@ __global__ void __launch_bounds__(256, NT == 0 || NT == 2 ? 4 : 3)
       }
     }
   };
+  const unsigned temps = smem_addr(tiled_smem) + in.temp_slot + tid * 16;  // [temporary][G][256 threads] groups of four floats
+  auto load_temp = [&](unsigned k, Pair (&t)[H]) {
+#pragma unroll
+    for (int g = 0; g < G; ++g)
+      asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(t[2 * g]), "=l"(t[2 * g + 1]) : "r"(temps + (k * G + g) * 4096) : "memory");
+  };
   auto start_next = [&](long long at, unsigned buf) {
     if (at < x.full_below) issue(at, buf, std::true_type());
     else if (at < total) issue(at, buf, std::false_type());
@@ -819,7 +817,7 @@ __global__ void __launch_bounds__(256, NT == 0 || NT == 2 ? 4 : 3)
     start_next(i + grid_stride * G, buf ^ 1u);
     cp_async_wait<1>();  // everything but the newest group has landed: this trip's operands
 
-    Pair s0[H], tmp[NTR][H];  // the accumulator (every program starts with a load) and the temporaries
+    Pair s0[H];  // the accumulator (every program starts with a load)
     unsigned next = prog.ins[0];  // the word of the next instruction is fetched while the current one runs
     for (int k = 0; k < prog.n_ins; ++k) {
       const unsigned w = next, arg = (w >> 8) & 3u, idx = w & 0xffu;
@@ -843,32 +841,21 @@ __global__ void __launch_bounds__(256, NT == 0 || NT == 2 ? 4 : 3)
 #pragma unroll
               for (int h = 0; h < H; ++h) {
                 if constexpr (IDX == L_MUL_INPUT || IDX == L_MUL_TEMP) s0[h] = mul_pair(s0[h], t[h]);
-                else if constexpr (IDX == L_ADD_INPUT || IDX == L_ADD_TEMP) s0[h] = fma_pair(t[h], pair(sign, sign), s0[h]);
-                else s0[h] = t[h];  // L_LOAD_TEMP
+                else s0[h] = fma_pair(t[h], pair(sign, sign), s0[h]);
               }
             };
             if constexpr (IDX == L_LOAD_TEMP) {
-              with_temp<NT>(tmp, arg, apply);
-            } else if (NT > 0 && (w & kOperandFma)) {
-              Pair t[H];
-              if constexpr (IDX == L_MUL_INPUT || IDX == L_ADD_INPUT) {
-                fetch(buf, arg, t);
-              } else {
-                with_temp<NT>(tmp, arg, [&](Pair (&u)[H]) {
-#pragma unroll
-                  for (int h = 0; h < H; ++h) t[h] = u[h];
-                });
-              }
-              const Pair pp = pair(p, p), qq = pair(q, q);
-#pragma unroll
-              for (int h = 0; h < H; ++h) t[h] = fma_pair(t[h], pp, qq);
-              apply(t);
-            } else if constexpr (IDX == L_MUL_INPUT || IDX == L_ADD_INPUT) {
-              Pair t[H];
-              fetch(buf, arg, t);
-              apply(t);
+              if constexpr (TEMPS) load_temp(arg, s0);
             } else {
-              with_temp<NT>(tmp, arg, apply);
+              Pair t[H];
+              if constexpr (IDX == L_MUL_INPUT || IDX == L_ADD_INPUT) fetch(buf, arg, t);
+              else if constexpr (TEMPS) load_temp(arg, t);
+              if (TEMPS && (w & kOperandFma)) {
+                const Pair pp = pair(p, p), qq = pair(q, q);
+#pragma unroll
+                for (int h = 0; h < H; ++h) t[h] = fma_pair(t[h], pp, qq);
+              }
+              if constexpr (TEMPS || IDX == L_MUL_INPUT || IDX == L_ADD_INPUT) apply(t);
             }
           }
         });
@@ -890,7 +877,11 @@ __global__ void __launch_bounds__(256, NT == 0 || NT == 2 ? 4 : 3)
             } else if constexpr (SRC == 1) {
               apply_binary<CODE, REV>(s0, [&](int) { return pair(q, q); });
             } else {
-              with_temp<NT>(tmp, arg, [&](Pair (&t)[H]) { apply_binary<CODE, REV>(s0, [&](int h) { return t[h]; }); });
+              if constexpr (TEMPS) {
+                Pair t[H];
+                load_temp(arg, t);
+                apply_binary<CODE, REV>(s0, [&](int h) { return t[h]; });
+              }
             }
           }
         });
@@ -901,11 +892,12 @@ __global__ void __launch_bounds__(256, NT == 0 || NT == 2 ? 4 : 3)
 #pragma unroll
           for (int h = 0; h < H; ++h) s0[h] = fma_pair(s0[h], pp, qq);
         }
-        if (NT > 0 && w >> kTailStore)
-          with_temp<NT>(tmp, (w >> kTailStore) - 1u, [&](Pair (&t)[H]) {
+        if (TEMPS && w >> kTailStore) {
+          const unsigned to = temps + ((w >> kTailStore) - 1u) * (G * 4096);
 #pragma unroll
-            for (int h = 0; h < H; ++h) t[h] = s0[h];
-          });
+          for (int g = 0; g < G; ++g)
+            asm volatile("st.shared.v2.b64 [%0], {%1, %2};" ::"r"(to + g * 4096), "l"(s0[2 * g]), "l"(s0[2 * g + 1]) : "memory");
+        }
       }
     }
     if (i < x.full_below && x.dest_vec) {
@@ -938,7 +930,7 @@ __global__ void __launch_bounds__(256, NT == 0 || NT == 2 ? 4 : 3)
   cp_async_wait<0>();
 }
 
-template <typename T, int G, int NT>
+template <typename T, int G, bool TEMPS>
 int launch_broadcast(ctb_ctx* ctx, cudaStream_t st, void* dest, Operands& in, const Program& prog, int n_inputs, long long d0,
                      Extents& x) {
   constexpr int VB = 4 * (int)sizeof(T);
@@ -982,10 +974,12 @@ int launch_broadcast(ctb_ctx* ctx, cudaStream_t st, void* dest, Operands& in, co
     if (in.mode[a] == OP_GROUP) smem += 2 * G * 256 * sizeof(T);
     else if (in.mode[a] != OP_SCALAR) smem += (in.mode[a] == OP_FIXED ? 1 : 2 * G) * 256 * VB;
   }
+  in.temp_slot = smem;
+  smem += prog.n_temps * G * 4096;
   x.full_below = x.n / 4 - (long long)(G - 1) * grid * 256;  // a trip's last group is (G - 1) grids further on
-  auto kernel = linear ? tiled_broadcast_kernel<T, G, NT, true> : tiled_broadcast_kernel<T, G, NT, false>;
+  auto kernel = linear ? tiled_broadcast_kernel<T, G, TEMPS, true> : tiled_broadcast_kernel<T, G, TEMPS, false>;
   if (smem > 48 * 1024 &&  // per device, so on every launch that needs it: a host-side table write
-      allow_smem(kernel, (size_t)kMaxInputs * 2 * G * 256 * VB) != cudaSuccess)
+      allow_smem(kernel, (size_t)kMaxInputs * 2 * G * 256 * VB + (TEMPS ? kTemps * G * 4096 : 0)) != cudaSuccess)
     return fail(CTB_CUDA_ERROR, "ctb_tiled_broadcast: shared memory attribute: %s", cudaGetErrorString(cudaGetLastError()));
   launch_kernel(kernel, (unsigned)grid, 256, smem, st, 0, dest, in, prog, n_inputs, x);
   return CTB_OK;
@@ -1281,18 +1275,21 @@ int ctb_tiled_broadcast(ctb_ctx* ctx, void* stream, void* dest, const int64_t* s
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int rc = CTB_OK;
-  // groups per thread: as many as registers (the temporaries) and shared memory (the operands) allow; eight groups for a
-  // single operand measured slower than four (128 registers, two CTAs per SM)
-#define CTB_TILED_NT(T)                                                                                             \
-  do {                                                                                                              \
-    if (prog.n_temps > 2) rc = launch_broadcast<T, 2, 4>(ctx, st, dest, in, prog, n_inputs, d0, x);                 \
-    else if (prog.n_temps == 2 || n_inputs > 3) rc = launch_broadcast<T, 2, 2>(ctx, st, dest, in, prog, n_inputs, d0, x); \
-    else if (prog.n_temps == 1) rc = launch_broadcast<T, 4, 1>(ctx, st, dest, in, prog, n_inputs, d0, x);           \
-    else rc = launch_broadcast<T, 4, 0>(ctx, st, dest, in, prog, n_inputs, d0, x);                                  \
-  } while (0)
-  if (dtype == CTB_F32) CTB_TILED_NT(float);
-  else CTB_TILED_NT(__half);
-#undef CTB_TILED_NT
+  // Groups per thread: four, or two where the shared memory of four (operands twice, temporaries once) would leave room for
+  // fewer than three CTAs per SM.
+  const size_t vb = 256 * 4 * (dtype == CTB_F32 ? 4 : 2);
+  size_t need = (size_t)prog.n_temps * 4 * 4096;
+  for (int a = 0; a < n_inputs; ++a)
+    need += in.mode[a] == OP_SCALAR ? 0 : in.mode[a] == OP_VECTOR ? vb : in.mode[a] == OP_GROUP ? 2 * vb : 8 * vb;
+  const bool four = prog.n_temps ? need <= 72 * 1024 : n_inputs <= 3;
+#define CTB_TILED(T)                                                                                                        \
+  rc = prog.n_temps ? four ? launch_broadcast<T, 4, true>(ctx, st, dest, in, prog, n_inputs, d0, x)                         \
+                           : launch_broadcast<T, 2, true>(ctx, st, dest, in, prog, n_inputs, d0, x)                         \
+                    : four ? launch_broadcast<T, 4, false>(ctx, st, dest, in, prog, n_inputs, d0, x)                        \
+                           : launch_broadcast<T, 2, false>(ctx, st, dest, in, prog, n_inputs, d0, x)
+  if (dtype == CTB_F32) CTB_TILED(float);
+  else CTB_TILED(__half);
+#undef CTB_TILED
   if (rc) return rc;
   CTB_CHECK_LAUNCH("ctb_tiled_broadcast launch");
   return CTB_OK;
