@@ -1003,11 +1003,13 @@ struct ReduceShape {
 // True for every thread of the last CTA; the partials of the others are visible then.
 __device__ __forceinline__ bool last_part(unsigned* ticket, long long parts) {
   __shared__ int last;
-  __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) last = atomicInc(ticket, (unsigned)parts - 1) == (unsigned)parts - 1;
+  if (threadIdx.x == 0) {  // its fences cover what the barrier has ordered before and behind them
+    __threadfence();
+    last = atomicInc(ticket, (unsigned)parts - 1) == (unsigned)parts - 1;
+    __threadfence();
+  }
   __syncthreads();
-  __threadfence();
   return last != 0;
 }
 
