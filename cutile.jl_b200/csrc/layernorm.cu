@@ -973,10 +973,11 @@ int ctb_layernorm_bwd_dx_partial_dwdb(ctb_ctx* ctx, void* stream, float* DX, con
   // A warp per row: as in the forward pass, but the other kernels need two barriers per row and fill up sooner, so the line
   // lies at M = N / 4 (1024 columns: 150 rows 5.0 us by either, 300 rows 3.9 against 6.4).  Aligned rows come through rings above
   // 256 columns.  Below, a row's loads are few and the kernel without rings has more warps, which pays with many rows (16000 x
-  // 128: 7.6 against 10.3 us); between 1024 and 4096 rows it needs clusters and the rings do not (2000 x 256: 6.4 against
-  // 4.6).  Single floats only up to 512 columns: 64 more registers of partial sums leave too few warps (2400 x 1023: 18.5
+  // 128: 7.6 against 10.3 us) and with more groups than SMs (3000 x 256 in 300: 4.9 against 7.7); between 1024 and 4096 rows it
+  // needs clusters and the rings do not (2000 x 256: 6.4 against 4.6; in 16 groups both do, 3000 x 256: 7.8 against 10.1).
+  // Single floats only up to 512 columns: 64 more registers of partial sums leave too few warps (2400 x 1023: 18.5
   // against 16.6 us).
-  if (vec && N <= kWarpCols && (N > 256 ? 4 * M >= N : M > 1024 && M <= 4096)) {
+  if (vec && N <= kWarpCols && (N > 256 ? 4 * M >= N : M > 1024 && M <= 4096 && G >= 32 && G <= ctx->sm_count)) {
     if (n <= 256) return launch_bwd_ring<2, 16>(ctx, st, DX, DY, DW, DB, X, W, Mean, Rstd, n, m, ldx, lddy, lddx, G);
     if (n <= 512) return launch_bwd_ring<4, 16>(ctx, st, DX, DY, DW, DB, X, W, Mean, Rstd, n, m, ldx, lddy, lddx, G);
     return launch_bwd_ring<8, 8>(ctx, st, DX, DY, DW, DB, X, W, Mean, Rstd, n, m, ldx, lddy, lddx, G);
