@@ -7,7 +7,7 @@
 //
 // Work is cut into blocks of 256 keys of one (batch, key/value head) pair.  The blocks of all pairs form one line that
 // the CTAs (one per SM) share out in equal contiguous ranges, whatever the number of pairs and keys is: a CTA works
-// through the end of one pair, whole pairs, the head of another.  With no more pairs than SMs the pairs are cut into as many equal
+// through the end of one pair, whole pairs, the head of another, or through whole pairs only where that is as even.  With no more pairs than SMs the pairs are cut into as many equal
 // parts as there are SMs for, and a CTA has a part of one pair only, unless too many SMs would be idle.  Inside a block each of the eight warps owns 32 keys: it
 // has its own ring of stages that its lane 0 fills by TMA (K tile and V tile, 4 KB each, 128-byte swizzle, up to 192 KB
 // in flight per SM), its own running maximum, sum and output, and waits for nobody until the CTA leaves the pair.
@@ -46,7 +46,7 @@ struct Params {
   int seq_q, keys, seq_kv, group, rows;  // keys: up to the last one that some query sees
   int input_pos, causal, blocks_per_pair;
   long long blocks;
-  int split;  // parts of a pair, a CTA each; 0: contiguous ranges
+  int split;  // parts of a pair, a CTA each; 0: contiguous ranges of blocks; -1: contiguous ranges of whole pairs
   float scale_log2;
   float* part;   // [CTA][first, last pair of its range][rows x (64 outputs), maxima, sums]
   unsigned* tickets;  // per CTA: parts left of the pair that begins in its range and ends in another's
@@ -119,7 +119,10 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   const int cta = blockIdx.x, grid = gridDim.x;
   long long lo, hi;
-  if (p.split) {
+  if (p.split < 0) {
+    lo = first_block(cta, p.blocks / p.blocks_per_pair, grid) * p.blocks_per_pair;
+    hi = first_block(cta + 1, p.blocks / p.blocks_per_pair, grid) * p.blocks_per_pair;
+  } else if (p.split) {
     const int pr = cta / p.split, k = cta - pr * p.split;
     lo = (long long)pr * p.blocks_per_pair + k * p.blocks_per_pair / p.split;
     hi = (long long)pr * p.blocks_per_pair + (k + 1) * p.blocks_per_pair / p.split;
@@ -435,6 +438,13 @@ int fmha_decode(ctb_ctx* ctx, cudaStream_t st, const void* Q, const void* K, con
       p.split = (int)split;
       grid = (int)(split * pairs);
     }
+  } else {
+    // Whole pairs: HBM sets the pace while all are loading; at the end those with a pair more have it to themselves.
+    // 256 heads of 4000 keys 45.9 us in ranges, 42.9 in whole pairs, 256 of 2000 26.9 and 23.4, 512 of 500 16.9 and 15.2;
+    // 160 of 3000, where 12 CTAs have two pairs and 136 one, 25.0 and 29.0.
+    const int64_t all = pairs / grid, more = pairs % grid;
+    const double whole = p.blocks_per_pair * (1.46 * (double)all + (more ? std::max(0.93, 1.46 * (double)more / grid) : 0.));
+    if (whole <= 1.46 * (double)p.blocks / grid + 4.5) p.split = -1;
   }
   if ((size_t)grid * 2 * kPartFloats * sizeof(float) > kStreamScratchBytes || grid > kTickets)
     return fail(CTB_UNSUPPORTED, "ctb_fmha_fwd: more SMs than the split over keys has scratch for");

@@ -60,10 +60,12 @@ def test_fmha_scale_and_large_scores(cuda):
 
 
 # (batch, kv heads, group, query rows, keys): one pair in as many parts as SMs, parts of unequal length, two parts, one part each, as
-# many pairs as SMs and one more, pairs that leave half of the SMs idle in parts (long: ranges), 1, 8, 9 and 16 rows
+# many pairs as SMs and one more, pairs that leave half of the SMs idle in parts (long: ranges), more pairs than SMs in ranges of
+# blocks and of whole pairs (twice as many, and a few more), 1 to 16 rows
 @pytest.mark.parametrize("batch,kvh,group,seq_q,keys", [
     (1, 1, 1, 1, 40000), (1, 1, 4, 4, 300), (1, 3, 1, 9, 5000), (2, 37, 2, 4, 513), (5, 10, 8, 1, 900), (3, 19, 3, 3, 9 * 256),
-    (75, 1, 1, 1, 1024), (75, 1, 1, 1, 9000), (37, 4, 1, 1, 600), (149, 1, 3, 1, 600), (1, 2, 16, 1, 257)])
+    (75, 1, 1, 1, 1024), (75, 1, 1, 1, 9000), (37, 4, 1, 1, 600), (149, 1, 3, 1, 600), (1, 2, 16, 1, 257),
+    (160, 1, 1, 1, 3000), (150, 2, 1, 3, 900), (74, 4, 2, 2, 700), (74, 4, 16, 1, 1100)])
 @pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
 def test_fmha_few_rows_parts(cuda, dtype, batch, kvh, group, seq_q, keys):
     import torch
