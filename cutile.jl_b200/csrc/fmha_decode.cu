@@ -7,10 +7,16 @@
 //
 // Work is cut into blocks of 256 keys of one (batch, key/value head) pair.  The blocks of all pairs form one line that
 // the CTAs (one per SM) share out in equal contiguous ranges, whatever the number of pairs and keys is: a CTA works
-// through the end of one pair, whole pairs, the head of another, or through whole pairs only where that is as even.  With no more pairs than SMs the pairs are cut into as many equal
-// parts as there are SMs for, and a CTA has a part of one pair only, unless too many SMs would be idle.  Inside a block each of the eight warps owns 32 keys: it
-// has its own ring of stages that its lane 0 fills by TMA (K tile and V tile, 4 KB each, 128-byte swizzle, up to 192 KB
-// in flight per SM), its own running maximum, sum and output, and waits for nobody until the CTA leaves the pair.
+// through the end of one pair, whole pairs, the head of another, or through whole pairs only where that is as even.  With no more
+// pairs than SMs the pairs are cut into as many equal parts as there are SMs for, and a CTA has a part of one pair only, unless too
+// many SMs would be idle.  Inside a block each of the eight warps owns 32 keys: it has its own ring of stages that its lane 0 fills
+// by TMA (K tile and V tile, 4 KB each, 128-byte swizzle, up to 192 KB in flight per SM), its own running maximum, sum and output,
+// and waits for nobody until the CTA leaves the pair or comes to a cut.
+// Cuts: probabilities are rounded to 16 bits relative to the warp's running maximum, and each running maximum is one that is exact,
+// so a sum over fewer, longer pieces has the larger error (256 heads of 4000 keys in bf16: 2.18e-3 in whole pairs against 2.15e-3
+// in ranges; 75 heads of 2000: 2.15e-3 and 2.08e-3).  CTAs that have whole pairs or equal parts therefore let their warps meet
+// where a range would end as well, which costs them 0.2 to 1.7 us where there are such cuts (256 heads of 4000 keys 42.2 -> 42.6 us, in
+// ranges 47.2; 75 heads of 2000 10.4 -> 12.1, in ranges 16.2), and the results of whole pairs are those of ranges bit for bit.
 // S = Q K^T and O += P V are m16n8k16 tensor-core instructions on registers (a 128-row tcgen05 tile would be 88 % padding;
 // the tensor work here is a few per cent of what either path delivers): Q stays in registers for the pair, K enters by
 // ldmatrix, the probabilities go from the accumulator layout straight into the A operand, V by transposed ldmatrix.
@@ -39,6 +45,9 @@ constexpr int kTileBytes = kTileKeys * kD * 2;  // one K or V tile of a warp
 constexpr int kPitch = kD + 4;                  // floats between rows of the warps' outputs in shared memory
 constexpr int kMaxRows = 16;
 constexpr int kPartFloats = kMaxRows * (kD + 2);
+// Ends of ranges inside a pair or part, at most: with more pairs than SMs a range is no shorter than a pair (one end), with fewer
+// no shorter than half of a part, rounded down (two).
+constexpr int kMaxCuts = 2;
 
 struct Params {
   const void* Q;
@@ -46,7 +55,8 @@ struct Params {
   int seq_q, keys, seq_kv, group, rows;  // keys: up to the last one that some query sees
   int input_pos, causal, blocks_per_pair;
   long long blocks;
-  int split;  // parts of a pair, a CTA each; 0: contiguous ranges of blocks; -1: contiguous ranges of whole pairs
+  int split;       // parts of a pair, a CTA each; 0: contiguous ranges of blocks; -1: contiguous ranges of whole pairs
+  int cut_ranges;  // CUTS: the number of ranges
   float scale_log2;
   float* part;   // [CTA][first, last pair of its range][rows x (64 outputs), maxima, sums]
   unsigned* tickets;  // per CTA: parts left of the pair that begins in its range and ends in another's
@@ -93,8 +103,9 @@ __host__ __device__ __forceinline__ long long owner(long long b, long long block
   return ((b + 1) * grid - 1) / blocks;
 }
 
-// R: query rows computed, 8 or 16 (the instructions have 16; the upper eight are zeros and skipped when R = 8).
-template <bool BF16, int R>
+// R: query rows computed, 8 or 16 (the instructions have 16; the upper eight are zeros and skipped when R = 8).  CUTS: ends of
+// ranges may lie inside what a CTA has of a pair (without the code for it short heads take 0.15 us less).
+template <bool BF16, int R, bool CUTS>
 __global__ void __launch_bounds__(kThreads, 1)
     fmha_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const Params p,
                        int* status) {
@@ -185,20 +196,33 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int row = g + 8 * h, pos = row - row / p.seq_q * p.seq_q;
     lim[h] = p.causal ? min(p.input_pos + pos, p.seq_kv - 1) : p.seq_kv - 1;
   }
+  float M_cut[kMaxCuts], L_cut[kMaxCuts];  // of the pair's pieces before the next cut
+  float4 acc_cut[kMaxCuts];
+  int cuts = 0;
+  uint32_t q[4][4];
   uint32_t q_next[4][4];  // asked for before the warps of the last pair meet: with few keys a pair is over before its Q would have come
   load_q(q_next, (int)(lo / p.blocks_per_pair));
+  // the next cut and the range of blocks that begins there (32 bits: see the launch)
+  unsigned range = 0;
+  long long cut = hi;
+  auto next_cut = [&]() { cut = ++range * (unsigned)p.blocks / (unsigned)p.cut_ranges; };
+  if constexpr (CUTS) {
+    range = (((unsigned)lo + 1) * (unsigned)p.cut_ranges - 1) / (unsigned)p.blocks;  // that lo lies in
+    next_cut();
+  }
   int pair = (int)(lo / p.blocks_per_pair) - 1;
   for (long long b = lo; b < hi;) {
-    ++pair;
+    if (!CUTS || cuts == 0) {
+      ++pair;
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int h = 0; h < 4; ++h) q[k][h] = q_next[k][h];
+    }
     const long long pair_first = (long long)pair * p.blocks_per_pair, pair_end = pair_first + p.blocks_per_pair;
-    const long long end = min(hi, pair_end);
+    const long long end = CUTS ? min(min(hi, pair_end), cut) : min(hi, pair_end);
     int block = (int)(b - pair_first);
     const int live = tiles_of(block);  // warps that have keys of this part
-    uint32_t q[4][4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-#pragma unroll
-      for (int h = 0; h < 4; ++h) q[k][h] = q_next[k][h];
     float o[8][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
 #pragma unroll
     for (int j = 0; j < 8; ++j)
@@ -273,7 +297,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       issue();
     }
     b = end;
-    if (pair_end < hi) load_q(q_next, pair + 1);
+    if (CUTS ? end == pair_end && end < hi : pair_end < hi) load_q(q_next, pair + 1);
     // ---- leaving the pair: the warps' results meet
 #pragma unroll
     for (int h = 0; h < (R == 16 ? 2 : 1); ++h) {
@@ -311,6 +335,41 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (mine) {
       if (live == kWarps) meet(std::true_type());
       else meet(std::false_type());
+    }
+    if constexpr (CUTS) {
+      if (end == cut && end < hi) next_cut();
+      if (end < min(hi, pair_end)) {
+#pragma unroll
+        for (int k = 0; k < kMaxCuts; ++k)
+          if (cuts == k) {
+            M_cut[k] = M;
+            L_cut[k] = L;
+            acc_cut[k] = acc;
+          }
+        ++cuts;
+        __syncthreads();  // the warps' results are overwritten by the next piece
+        continue;
+      }
+      if (cuts) {  // the pieces in ascending order, as the parts of several CTAs below
+        const float M_last = M, L_last = L;
+        const float4 acc_last = acc;
+#pragma unroll
+        for (int k = 0; k < kMaxCuts; ++k)
+          if (k < cuts) M = fmaxf(M, M_cut[k]);
+        const float ref = M == -INFINITY ? 0.f : M;
+        L = 0.f;
+        acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        auto add = [&](float m, float l, const float4& v) {
+          const float f = ex2_approx_ftz(m - ref);
+          L += l * f;
+          acc.x += v.x * f; acc.y += v.y * f; acc.z += v.z * f; acc.w += v.w * f;
+        };
+#pragma unroll
+        for (int k = 0; k < kMaxCuts; ++k)
+          if (k < cuts) add(M_cut[k], L_cut[k], acc_cut[k]);
+        add(M_last, L_last, acc_last);
+        cuts = 0;
+      }
     }
     auto write_out = [&]() {
       const float inv = rcp_approx_ftz(L);
@@ -426,6 +485,7 @@ int fmha_decode(ctb_ctx* ctx, cudaStream_t st, const void* Q, const void* K, con
   const int64_t pairs = kv_heads * batch;
   p.blocks = pairs * p.blocks_per_pair;
   int grid = (int)std::min<int64_t>(p.blocks, ctx->sm_count);
+  const int ranges = grid;
   p.split = 0;
   if (pairs <= ctx->sm_count) {
     const int64_t split = std::min<int64_t>(p.blocks_per_pair, ctx->sm_count / pairs);
@@ -446,14 +506,24 @@ int fmha_decode(ctb_ctx* ctx, cudaStream_t st, const void* Q, const void* K, con
     const double whole = p.blocks_per_pair * (1.46 * (double)all + (more ? std::max(0.93, 1.46 * (double)more / grid) : 0.));
     if (whole <= 1.46 * (double)p.blocks / grid + 4.5) p.split = -1;
   }
+  // none where all ends of ranges are ends of pairs or parts
+  p.cut_ranges = p.split && p.split != p.blocks_per_pair && p.blocks_per_pair > 1 && pairs % ranges ? ranges : 0;
+  if (p.cut_ranges && p.blocks > UINT32_MAX / (ranges + 1)) {  // the kernel finds the cuts in 32 bits
+    p.split = p.cut_ranges = 0;
+    grid = ranges;
+  }
   if ((size_t)grid * 2 * kPartFloats * sizeof(float) > kStreamScratchBytes || grid > kTickets)
     return fail(CTB_UNSUPPORTED, "ctb_fmha_fwd: more SMs than the split over keys has scratch for");
   p.part = scratch.data;
   p.tickets = scratch.tickets;
   const bool small = p.rows <= 8;
   const size_t smem = 1024 + (size_t)kWarps * (small ? 3 : 2) * 2 * kTileBytes + (size_t)kWarps * (small ? 8 : 16) * kPitch * 4;
-  auto kern = bf16 ? (small ? fmha_decode_kernel<true, 8> : fmha_decode_kernel<true, 16>)
-                   : (small ? fmha_decode_kernel<false, 8> : fmha_decode_kernel<false, 16>);
+  auto pick = [&](auto cuts) {
+    constexpr bool CUTS = decltype(cuts)::value;
+    return bf16 ? (small ? fmha_decode_kernel<true, 8, CUTS> : fmha_decode_kernel<true, 16, CUTS>)
+                : (small ? fmha_decode_kernel<false, 8, CUTS> : fmha_decode_kernel<false, 16, CUTS>);
+  };
+  auto kern = p.cut_ranges ? pick(std::true_type()) : pick(std::false_type());
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return cuda_fail(e, "ctb_fmha_fwd: shared memory opt-in");
   launch_kernel(kern, grid, kThreads, smem, st, 0, tk, tv, p, ctx->dev_status);

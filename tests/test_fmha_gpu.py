@@ -82,6 +82,64 @@ def test_fmha_few_rows_parts(cuda, dtype, batch, kvh, group, seq_q, keys):
         assert (out[b] - want).norm() <= (TOL if dtype == "float16" else 1e-2) * want.norm()
 
 
+def grouped(q, k, v, cuts):
+    """Attention of one query position over pairs [P, heads or 1, keys, 64], in f64 but for the probabilities, which are rounded to
+    the type of v relative to a running maximum: of every 32 keys of each 256, from one of `cuts` (blocks of 256 keys, counted
+    over all pairs) to the next."""
+    import torch
+    P, H, keys = q.shape[0], q.shape[1], k.shape[2]
+    n = -(-keys // 256)
+    s = torch.full((P, H, n * 256), -torch.inf, device="cuda", dtype=torch.float64)
+    s[..., :keys] = (q.double() @ k.double().transpose(2, 3))[:, :, 0] * (0.125 * 1.4426950408889634)
+    s = s.view(P, H, n, 8, 32).permute(2, 0, 3, 1, 4)
+    w = torch.zeros(P, n * 256, 64, device="cuda", dtype=torch.float64)
+    w[:, :keys] = v[:, 0].double()
+    w = w.view(P, n, 8, 32, 64).permute(1, 0, 2, 3, 4)
+    first = torch.zeros(P * n, dtype=torch.bool, device="cuda")
+    first[torch.tensor(sorted(c for c in cuts if c < P * n), device="cuda")] = True
+    first = first.view(P, n)
+    shape = (P, 8, H, 1)
+    M, L, O = torch.full(shape, -torch.inf, device="cuda").double(), torch.zeros(shape, device="cuda").double(), 0.0
+    m, l, o = M.clone(), L.clone(), torch.zeros(P, 8, H, 64, device="cuda").double()
+
+    def merge(M, L, O, m, l, o):
+        top = torch.maximum(M, m)
+        f, g = (torch.exp2(x - torch.where(top == -torch.inf, 0.0, top)) for x in (M, m))
+        return top, L * f + l * g, O * f + o * g
+    for j in range(n):
+        new = first[:, j].view(P, 1, 1, 1)
+        M2, L2, O2 = merge(M, L, O, m, l, o)
+        M, L, O = torch.where(new, M2, M), torch.where(new, L2, L), torch.where(new, O2, O + torch.zeros_like(o))
+        m, l, o = torch.where(new, -torch.inf, m), torch.where(new, 0.0, l), torch.where(new, 0.0, o)
+        top = torch.maximum(m, s[j].amax(-1, keepdim=True))
+        ref = torch.where(top == -torch.inf, 0.0, top)
+        p, f = torch.exp2(s[j] - ref), torch.exp2(m - ref)
+        m, l, o = top, l * f + p.sum(-1, keepdim=True), o * f + p.to(v.dtype).double() @ w[j]
+    M, L, O = merge(M, L, O, m, l, o)
+    f = torch.exp2(M - M.amax(1, keepdim=True))
+    return ((O * f).sum(1) / (L * f).sum(1)).view(P, H, 1, 64).to(v.dtype)
+
+
+# What is rounded to 16 bits is rounded as in equal ranges of blocks, one per SM, whatever a CTA works through: whole pairs (twice),
+# one part of a pair (cut once, twice), two parts, ranges.  Another grouping changes 14 to 31 % of the outputs.  With the same one the
+# kernel's probabilities are off by about 1e-6 (f32 scores times log2(e), approximate exponential), so of 4000 in f16 (half a step:
+# 2.4e-4 to 4.9e-4) a dozen are rounded the other way; each moves an output by 2^-11 / 4000 = 1.2e-7, all of them by 4e-7, and a step of
+# an output of 0.02 is 1e-5: 4 % of the outputs come out otherwise.  In bf16 it is one of 4000, 1e-6 against 8e-5: 1 %.
+@pytest.mark.parametrize("pairs,heads,keys", [(256, 4, 4000), (200, 16, 900), (100, 1, 2000), (75, 4, 1000), (64, 4, 2000), (160, 1, 3000)])
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
+def test_fmha_few_rows_grouping(cuda, dtype, pairs, heads, keys):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(keys)
+    q, k, v = (torch.randn(pairs, h, n, 64, device="cuda", generator=g).to(getattr(torch, dtype))
+               for h, n in ((heads, 1), (1, keys), (1, keys)))
+    sms, n = torch.cuda.get_device_properties(0).multi_processor_count, -(-keys // 256)
+    cuts = {c * pairs * n // sms for c in range(sms)} | set(range(0, pairs * n, n))
+    for k0 in range(1, min(n, sms // pairs) if pairs <= sms else 1):  # equal parts
+        cuts |= {pr * n + k0 * n // min(n, sms // pairs) for pr in range(pairs)}
+    out = cuda.fmha.cutile_fmha(q, k, v, causal=True, input_pos=keys - 1, query_group_size=heads)
+    assert (out != grouped(q, k, v, cuts)).double().mean() < (0.08 if dtype == "float16" else 0.02)
+
+
 def test_fmha_causal_prefix_property_full_size(cuda):
     """Size-independent property at the benchmark shape: under the causal mask the output of the first 512
     queries does not depend on the later keys/values, so it equals the result on the truncated problem."""
