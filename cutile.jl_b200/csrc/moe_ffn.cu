@@ -899,7 +899,8 @@ int launch_sort(cudaStream_t st, const void* topk_ids, const SortParams& sp) {
   auto kernel = sp.early ? moe_sort_gather_kernel<IdT, kSortThreadsEarly> : moe_sort_gather_kernel<IdT, kSortThreads>;
   const int threads = sp.early ? kSortThreadsEarly : kSortThreads;
   const size_t smem = sort_ints(sp.E, threads / 32) * sizeof(int) + (size_t)sp.held * sp.vecs * 16;
-  if (e == cudaSuccess && smem > 48 * 1024) e = allow_smem(kernel, sort_ints(kMaxExperts, threads / 32) * sizeof(int) + kHeldBytes);
+  // without the call the kernel's static shared memory counts against the same 48 KB
+  if (e == cudaSuccess && !sp.early) e = allow_smem(kernel, sort_ints(kMaxExperts, threads / 32) * sizeof(int) + kHeldBytes);
   if (e == cudaSuccess) e = launch_kernel(kernel, kSortCtas, threads, smem, st, 0, ids, sp);
   return e == cudaSuccess ? (int)CTB_OK : cuda_fail(e, "ctb_moe_ffn sort launch");
 }

@@ -121,6 +121,38 @@ def test_cutile_moe_many_slots(cuda, H, I, topk, counts):
     assert ref.rel_fro(out.cpu().numpy(), want) <= TOL
 
 
+FIRST_CALL = """
+import sys
+import numpy as np
+import torch
+import cutile_b200 as ctb
+from oracle import inputs, ref
+from test_moe_gpu import TOL, dev, random_routing
+T, H, E, topk = map(int, sys.argv[1:])
+d = inputs.moe(tokens=T, hidden=H, experts=E, inter=16, topk=topk, seed=4)
+ids, w = random_routing(T, E, topk, seed=1)
+X, w1, w2 = dev(d, "X", "w1", "w2")
+want = ref.moe_ffn(d["X"], d["w1"], d["w2"], w, ids)
+for dtype in (np.int32, np.int64):
+    out = ctb.moe.cutile_moe(X, w1, w2, torch.from_numpy(w).cuda(), torch.from_numpy(ids.astype(dtype)).cuda(), 128, 128, 64)
+    assert ref.rel_fro(out.cpu().numpy(), want) <= TOL
+"""
+
+
+# The sort's shared memory is between 48 KB less its static part and 48 KB (22 token rows of 2 KB and the counts of 32 experts; 8 of
+# 5760 bytes), and no larger call of the process has raised the limit before: a process of its own.
+@pytest.mark.parametrize("T,H,E,topk", [(3000, 1024, 32, 2), (950, 2880, 32, 4)])
+def test_cutile_moe_first_call_of_a_process(cuda, T, H, E, topk):
+    import os
+    import subprocess
+    import sys
+    here = os.path.dirname(os.path.abspath(__file__))
+    root = os.path.dirname(here)
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join([root, os.path.join(root, "cutile.jl_b200"), here]))
+    r = subprocess.run([sys.executable, "-c", FIRST_CALL, *map(str, (T, H, E, topk))], capture_output=True, text=True, timeout=300, env=env)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
 def test_moe_benchmark_config_with_router(cuda):
     import torch
     d = inputs.moe()  # 256 tokens, hidden 1024, 32 experts, inter 2048, top-2, seed 4
