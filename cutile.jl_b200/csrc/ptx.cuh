@@ -75,15 +75,26 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// PEERS: what other CTAs of the cluster have stored is visible behind it; else what this CTA and the copies have.
+template <bool PEERS = false>
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.b32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
+  if constexpr (PEERS)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
   return ok != 0;
 }
 __device__ __forceinline__ uint64_t globaltimer_ns() {
@@ -96,12 +107,13 @@ constexpr uint64_t kWaitLimitNs = 2000000000ull;  // 2 s: far beyond any legitim
 // Bounded wait.  Gives up after kWaitLimitNs, or as soon as *abort (a flag in
 // shared memory that every role of the CTA polls) is set; on expiry records
 // `code` in *status, sets *abort and returns false.
+template <bool PEERS = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* status, int code,
                                           volatile int* abort = nullptr) {
-  if (mbar_try_wait(bar, parity)) return true;
+  if (mbar_try_wait<PEERS>(bar, parity)) return true;
   const uint64_t t0 = globaltimer_ns();
   for (uint32_t i = 1;; ++i) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (mbar_try_wait<PEERS>(bar, parity)) return true;
     if ((i & 63u) == 0) {
       if (abort && *abort) return false;
       if (globaltimer_ns() - t0 > kWaitLimitNs) {

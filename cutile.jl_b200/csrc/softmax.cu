@@ -401,7 +401,7 @@ __global__ void __launch_bounds__(kRowThreads) softmax_long_kernel(T* __restrict
       // A peer sends its next row but one only after this CTA has sent its next, that is, read these slots.
       if (tid == 0) mbar_expect_tx(&met[it & 1], C * (uint32_t)sizeof(float2));
       if (tid < C) send_to_cta(&peers[it & 1][rank], mx, sum, &met[it & 1], (uint32_t)tid);
-      if (!mbar_wait(&met[it & 1], (it >> 1) & 1, status, DEV_TIMEOUT_TMA)) alive = false;
+      if (!mbar_wait<true>(&met[it & 1], (it >> 1) & 1, status, DEV_TIMEOUT_TMA)) alive = false;
       float M2 = -FLT_MAX;
       for (int k = 0; k < C; ++k) M2 = fmaxf(M2, peers[it & 1][k].x);
       sum = 0.f;
