@@ -306,7 +306,9 @@ __global__ void __launch_bounds__(kRowThreads) softmax_long_kernel(T* __restrict
   constexpr int V = 16 / (int)sizeof(T);
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t full[kMaxChunks];
-  __shared__ __align__(16) float red[2][2][kRowThreads / 32];  // maximum and sum of every warp, for even and odd rows
+  // Maximum and sum of every warp, for even and odd rows.  Read one by one: as vectors they bring the f32 kernel to 37 registers,
+  // three CTAs per SM instead of four (700 x 8200 12.3 us instead of 11.4, 300 x 27001 17.4 and 14.8).
+  __shared__ float red[2][2][kRowThreads / 32];
   __shared__ __align__(8) float2 peers[2][kMaxCluster];         // and of every CTA of the cluster
   __shared__ __align__(8) uint64_t met[2];               // all of peers[] have come
   const int tid = threadIdx.x;
@@ -602,7 +604,11 @@ int launch(ctb_ctx* ctx, cudaStream_t st, T* out, const T* in, int N, int M, lon
     while (row_bytes > C * kLongBytes) C *= 2;
     constexpr int V = 16 / (int)sizeof(T);
     const int per = (N / V + C - 1) / C;
-    const size_t smem = (size_t)per * 16;
+    size_t smem = (size_t)per * 16;
+    // Room for four CTAs on an SM is for many rows.  Where all rows run at once on up to three per SM, room for three is faster (f32
+    // 150 x 8200 6.7 us with four, 6.0 with three, 150 x 27001 12.0 and 10.3; probably because the next kernel's CTAs come as early as
+    // there is room and lie closer on some SMs than on others), unless a CTA has an SM to itself (f16 75 x 26000 7.2 and 8.1).
+    if ((long long)M * C > ctx->sm_count && 10ll * M * C <= 27ll * ctx->sm_count) smem = std::max(smem, (size_t)60 * 1024);
     auto k = softmax_long_kernel<T>;
     cudaError_t e = allow_smem(k, kLongBytes);
     if (e != cudaSuccess) return cuda_fail(e, "ctb_softmax: shared memory opt-in");
