@@ -311,12 +311,14 @@ __global__ void __launch_bounds__(kRowThreads) softmax_long_kernel(T* __restrict
   __shared__ float red[2][2][kRowThreads / 32];
   __shared__ __align__(8) float2 peers[2][kMaxCluster];         // and of every CTA of the cluster
   __shared__ __align__(8) uint64_t met[2];               // all of peers[] have come
+  __shared__ volatile int given_up;                      // they have not: no further arrival, message or wait
   const int tid = threadIdx.x;
   const int rank = C > 1 ? (int)cluster_ctarank() : 0, team = blockIdx.x / C, teams = gridDim.x / C;
   if (tid == 0) {
     for (int c = 0; c < kMaxChunks; ++c) mbar_init(&full[c], 1);
     mbar_init(&met[0], 1);
     mbar_init(&met[1], 1);
+    given_up = 0;
     fence_mbar_init();
   }
   __syncthreads();
@@ -399,11 +401,13 @@ __global__ void __launch_bounds__(kRowThreads) softmax_long_kernel(T* __restrict
     };
     float mx = over_warps(m, 0);
     float sum = over_warps(l * exp_sub(m, mx), 1);
-    if (C > 1) {
+    if (C > 1 && given_up) {  // the same for all threads: written ahead of the barriers of this row
+      alive = false;
+    } else if (C > 1) {
       // A peer sends its next row but one only after this CTA has sent its next, that is, read these slots.
       if (tid == 0) mbar_expect_tx(&met[it & 1], C * (uint32_t)sizeof(float2));
       if (tid < C) send_to_cta(&peers[it & 1][rank], mx, sum, &met[it & 1], (uint32_t)tid);
-      if (!mbar_wait<true>(&met[it & 1], (it >> 1) & 1, status, DEV_TIMEOUT_TMA)) alive = false;
+      if (!mbar_wait<true>(&met[it & 1], (it >> 1) & 1, status, DEV_TIMEOUT_TMA)) given_up = 1;
       float M2 = -FLT_MAX;
       for (int k = 0; k < C; ++k) M2 = fmaxf(M2, peers[it & 1][k].x);
       sum = 0.f;
@@ -443,9 +447,10 @@ __global__ void __launch_bounds__(kRowThreads) softmax_long_kernel(T* __restrict
   if (tid == 0)  // a wait ran out: copies under way must land before the CTA gives its shared memory back
     for (; pending; pending &= pending - 1)
       (void)mbar_wait(&full[__ffs(pending) - 1], (phases >> (__ffs(pending) - 1)) & 1, status, DEV_TIMEOUT_TMA);
-  if (C > 1) {  // no peer sends any more
+  if (C > 1) {  // no peer sends any more, and what they have sent is there unless a wait ran out
     cluster_arrive_relaxed();
     cluster_wait();
+    let_copies_land(&given_up);
   }
 }
 
