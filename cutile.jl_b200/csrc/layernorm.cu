@@ -586,6 +586,7 @@ __global__ void __launch_bounds__(kBwdWarpThreads)
 // came, the warps that the registers leave room for (8 per SM at 1024 columns) kept 64 KB of loads in flight and waited
 // for them; the rings keep 192 KB.  16000 x 1000: 52.1 us, now 35.7;
 // 4000 x 640: 12.6 and 10.7; 1000 x 512: 6.1 and 4.0.
+// The warps' sums are added in pairs: 16 in a row made dW and dB of up to 512 columns 5 to 15 % less exact than those above.
 constexpr size_t kBwdRingBytes = 192 * 1024;
 template <int NE, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 1)
@@ -707,11 +708,15 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
     }
   }
   __syncthreads();
-  for (int c = threadIdx.x; c < 2 * N; c += WARPS * 32) {  // ascending warps
-    float a = part[c];
+  for (int c = threadIdx.x; c < 2 * N; c += WARPS * 32) {
+    float a[WARPS];
 #pragma unroll
-    for (int k = 1; k < WARPS; ++k) a += part[(size_t)k * 2 * N + c];
-    part[c] = a;
+    for (int k = 0; k < WARPS; ++k) a[k] = part[(size_t)k * 2 * N + c];
+#pragma unroll
+    for (int half = WARPS / 2; half > 0; half /= 2)
+#pragma unroll
+      for (int k = 0; k < half; ++k) a[k] += a[k + half];
+    part[c] = a[0];
   }
   cluster_columns(part, DW, DB, N, g);
 }
