@@ -494,9 +494,9 @@ __device__ __forceinline__ void cluster_columns(float* mine, float* __restrict__
   cluster.sync();  // peers may still be reading this CTA's shared memory
 }
 
-// Rows of at most 512 columns, any alignment: a warp per row, row and partial dW/dB in its registers, no barrier until the
+// Rows of at most 1024 columns (512 off the 16-byte grid): a warp per row, row and partial dW/dB in its registers, no barrier until the
 // end.  Grid and clusters as above: warp w of CTA r of cluster g takes the rows g + G * (r * warps + w + C * warps * j).
-// 16384 x 256: 72.7 us with a CTA per row, now 13.1.
+// 16384 x 256: 72.7 us with a CTA per row, now 13.1; 16384 x 1024: 86.0 and 49.1.
 constexpr int kBwdWarpThreads = 256;
 template <int V, int NE>
 __global__ void __launch_bounds__(kBwdWarpThreads)
@@ -584,8 +584,7 @@ __global__ void __launch_bounds__(kBwdWarpThreads)
 // Aligned rows of at most 1024 columns: a warp per row as above, but the rows come by bulk copies through a ring of the warp's own in
 // shared memory, whose stage is asked for again as soon as the row is in registers.  With the row's loads issued when its turn
 // came, the warps that the registers leave room for (8 per SM at 1024 columns) kept 64 KB of loads in flight and waited
-// for them; the rings keep 192 KB.  16000 x 1000: 52.1 us, now 35.7;
-// 4000 x 640: 12.6 and 10.7; 1000 x 512: 6.1 and 4.0.
+// for them; the rings keep 192 KB.  In 64 groups 16000 x 1024 48.1 us, here 34.5; 4000 x 640 14.6 and 12.2; 1000 x 512 5.9 and 3.9.
 // The warps' sums are added in pairs: 16 in a row made dW and dB of up to 512 columns 5 to 15 % less exact than those above.
 constexpr size_t kBwdRingBytes = 192 * 1024;
 template <int NE, int WARPS>
@@ -867,35 +866,138 @@ int launch_bwd(ctb_ctx* ctx, cudaStream_t st, float* DX, const float* DY, float*
   return CTB_OK;
 }
 
-// The kernels without bulk copies: as many CTAs per group (a power of two up to 8) as run at once and find `rows` rows each.
+// CTAs per group: a power of two up to 8, at most `most` in all, each with at least `rows` rows.
+int cluster_size(int G, long long most, int rows, int M) {
+  int C = 8;
+  while (C > 1 && ((long long)G * C > most || (long long)G * C * rows > M)) C >>= 1;
+  return C;
+}
+
+// Most that the kernels without bulk copies ask for: 2 x N floats, or 8 warps x 2 x N floats with a warp per row, the same.
+constexpr size_t kBwdRegsBytes = (size_t)2 * kBwdThreads * kGenCols * 4;
+// The kernels without bulk copies: as many CTAs per group as run at once and find `rows` rows each.
 template <typename Kernel>
 int launch_bwd_regs(ctb_ctx* ctx, Kernel k, int threads, size_t smem, int rows, cudaStream_t st, float* DX, const float* DY, float* DW,
                     float* DB, const float* X, const float* W, const float* Mean, const float* Rstd, int N, int M, long long ldx,
                     long long lddy, long long lddx, int G) {
-  cudaError_t e = allow_smem(k, (size_t)2 * kBwdThreads * kGenCols * 4);  // the kernel with a warp per row: 8 warps x 2 x N floats, at most half of it
+  cudaError_t e = allow_smem(k, kBwdRegsBytes);
   if (e != cudaSuccess) return cuda_fail(e, "ctb_layernorm_bwd: shared memory opt-in");
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem);
-  per_sm = std::max(per_sm, 1);
-  int C = 8;
-  while (C > 1 && ((long long)G * C > (long long)ctx->sm_count * per_sm || (long long)G * C * rows > M)) C >>= 1;
+  const int C = cluster_size(G, (long long)ctx->sm_count * std::max(per_sm, 1), rows, M);
   e = launch_kernel(k, G * C, threads, smem, st, C, DX, DY, DW, DB, X, W, Mean, Rstd, N, M, ldx, lddy, lddx, G, C);
   return e == cudaSuccess ? (int)CTB_OK : cuda_fail(e, "ctb_layernorm_bwd_dx_partial_dwdb launch");
 }
 
-// One CTA per SM; as many per group (a power of two up to 8) as run at once and give every second warp a row.
+// Clusters of C CTAs of a kernel that the device runs at once (asked once per device).  Not CTAs / C: what is left over in a GPC runs
+// none, and two rounds take twice as long (2000 x 260 by rings in 16 groups: 9.4 us with C = 8, of which 15 run, 6.6 with C = 4).
+template <auto kKernel>
+int running_clusters(ctb_ctx* ctx, int threads, size_t smem, size_t most, int C) {
+  static int cached[16][9] = {};
+  int& c = cached[ctx->device & 15][C];
+  if (c == 0) {
+    int n = 0, per_sm = 0;
+    cudaError_t e = allow_smem(kKernel, most);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kKernel, threads, smem);
+    if (C == 1) {
+      n = per_sm * ctx->sm_count;
+    } else if (e == cudaSuccess) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(std::max(1, ctx->sm_count * per_sm / C) * C);
+      cfg.blockDim = dim3(threads);
+      cfg.dynamicSmemBytes = smem;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = C;
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      e = cudaOccupancyMaxActiveClusters(&n, kKernel, &cfg);
+    }
+    if (e != cudaSuccess) {
+      (void)cudaGetLastError();
+      return 0;
+    }
+    c = n;
+  }
+  return c;
+}
+
+// Time of the backward pass in us: start, more of it with the columns, a meeting of the cluster, then per round and row of a warp, the same
+// with the columns, the arrays' 12 bytes per element at HBM's rate as far as they add to it, and a further round of CTAs.
+struct BwdTime {
+  double start, start_n, meet, row, row_n, hbm, again;
+  double of(int N, int M, int C, long long rounds, long long rows) const {
+    const double n = N / 1000.0;
+    return start + start_n * n + (C > 1 ? meet : 0) + rounds * rows * (row + row_n * n) + hbm * (12.0 * M * N / 6.5e6) +
+           again * (rounds - 1);
+  }
+};
+// CTAs per group with which the ring kernel is taken, 0 for the kernel without rings.  The constants are fitted to the times of
+// both at 2103 points (64 to 1024 columns, 64 to 16000 rows, 1 to 512 groups, one to eight CTAs; mean error 6 to 8 %).  Where the
+// rings are expected to be faster by 4 % they are taken: that is 0.83 of the time without rings in the mean, and slower by more than 3 %
+// in ten points (1000 x 128 in 64 groups 3.05 and 2.94 us; the worst 16000 x 384 in 512 groups, 1.13).  Rings wherever rows are
+// aligned would be slower in 300, most with few columns, with more groups than SMs (one CTA of the ring kernel has all of an SM: 2000 x
+// 260 in 512 groups 10.0 and 6.2 us) and with few rows per group.
+template <int NE, int WARPS>
+int ring_ctas(ctb_ctx* ctx, int N, int M, int G) {
+  constexpr BwdTime kRings = NE == 2   ? BwdTime{1.70, 1.06, 1.60, 0.78, 0.51, 0.45, 1.28}
+                             : NE == 4 ? BwdTime{1.74, 0.97, 1.97, 1.06, 0.16, 0.46, 1.56}
+                                       : BwdTime{1.61, 1.12, 1.91, 1.12, 0.14, 0.34, 1.84};
+  constexpr BwdTime kWithout = NE == 2   ? BwdTime{1.66, 1.37, 1.25, 0.41, 1.06, 1.25, 2.01}
+                               : NE == 4 ? BwdTime{1.68, 1.43, 1.62, 0.91, 0.53, 0.89, 1.52}
+                                         : BwdTime{1.23, 2.01, 1.90, 1.08, 0.97, 0.65, 1.52};
+  constexpr int kWarps = kBwdWarpThreads / 32;
+  constexpr auto kOther = ln_bwd_warp_kernel<4, NE>;
+  auto over = [](long long a, long long b) { return (a + b - 1) / b; };
+  auto other = [&](int c) { return running_clusters<kOther>(ctx, kBwdWarpThreads, (size_t)kWarps * 2 * 128 * NE * 4, kBwdRegsBytes, c); };
+  auto ring = [&](int c) { return running_clusters<ln_bwd_ring_kernel<NE, WARPS>>(ctx, WARPS * 32, kBwdRingBytes, kBwdRingBytes, c); };
+  const int C0 = cluster_size(G, other(1), kWarps, M), n0 = other(C0);
+  if (n0 < 1) return 0;
+  double best = 0.96 * kWithout.of(N, M, C0, over(G, n0), over(M, (long long)G * C0 * kWarps));
+  int C = 0;
+  for (int c = 1; c <= 8 && (c == 1 || G * c <= ctx->sm_count); c *= 2) {
+    const long long chain = over(M, (long long)G * c * WARPS);
+    // A warp adds its rows one by one: what adding the warps in pairs gains makes up for a longer chain only while that is short
+    // (16000 x 1024 in 18 groups, 28 rows instead of 14: dW and dB 3 to 5 % less exact).
+    if (chain > 12 && c * WARPS < C0 * kWarps) continue;
+    const int n = ring(c);
+    if (n < 1) continue;
+    const double t = kRings.of(N, M, c, over(G, n), chain);
+    if (t < best) {
+      best = t;
+      C = c;
+    }
+  }
+  return C;
+}
+
 template <int NE, int WARPS>
 int launch_bwd_ring(ctb_ctx* ctx, cudaStream_t st, float* DX, const float* DY, float* DW, float* DB, const float* X, const float* W,
-                    const float* Mean, const float* Rstd, int N, int M, long long ldx, long long lddy, long long lddx, int G) {
+                    const float* Mean, const float* Rstd, int N, int M, long long ldx, long long lddy, long long lddx, int G, int C) {
   auto k = ln_bwd_ring_kernel<NE, WARPS>;
   const int stages = (int)std::min<size_t>(kBwdRingStages, kBwdRingBytes / ((size_t)WARPS * 2 * N * 4));
   cudaError_t e = allow_smem(k, kBwdRingBytes);
   if (e != cudaSuccess) return cuda_fail(e, "ctb_layernorm_bwd: shared memory opt-in");
-  int C = 8;
-  while (C > 1 && ((long long)G * C > ctx->sm_count || (long long)G * C * (WARPS / 2) > M)) C >>= 1;
   e = launch_kernel(k, G * C, WARPS * 32, (size_t)WARPS * stages * 2 * N * 4, st, C, DX, DY, DW, DB, X, W, Mean, Rstd, N, M, ldx, lddy,
                     lddx, G, C, stages, ctx->dev_status);
   return e == cudaSuccess ? (int)CTB_OK : cuda_fail(e, "ctb_layernorm_bwd_dx_partial_dwdb launch");
+}
+
+// A warp per row, with rings or without; NE vectors of V floats per lane and row.
+template <int V, int NE>
+int launch_bwd_rows(ctb_ctx* ctx, cudaStream_t st, float* DX, const float* DY, float* DW, float* DB, const float* X, const float* W,
+                    const float* Mean, const float* Rstd, int N, int M, long long ldx, long long lddy, long long lddx, int G) {
+  if constexpr (V == 4) {
+    constexpr int kRingWarps = NE == 8 ? 8 : 16;
+    const int C = M > 0 ? ring_ctas<NE, kRingWarps>(ctx, N, M, G) : 0;
+    if (C > 0)
+      return launch_bwd_ring<NE, kRingWarps>(ctx, st, DX, DY, DW, DB, X, W, Mean, Rstd, N, M, ldx, lddy, lddx, G, C);
+  }
+  constexpr int kWarps = kBwdWarpThreads / 32;
+  return launch_bwd_regs(ctx, ln_bwd_warp_kernel<V, NE>, kBwdWarpThreads, (size_t)kWarps * 2 * N * 4, kWarps, st, DX, DY, DW, DB, X, W,
+                         Mean, Rstd, N, M, ldx, lddy, lddx, G);
 }
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
@@ -976,22 +1078,12 @@ int ctb_layernorm_bwd_dx_partial_dwdb(ctb_ctx* ctx, void* stream, float* DX, con
   const bool vec = N % 4 == 0 && ldx % 4 == 0 && lddy % 4 == 0 && lddx % 4 == 0 && aligned16(X) && aligned16(DY) &&
                    aligned16(DX) && aligned16(W);
   // A warp per row: as in the forward pass, but the other kernels need two barriers per row and fill up sooner, so the line
-  // lies at M = N / 4 (1024 columns: 150 rows 5.0 us by either, 300 rows 3.9 against 6.4).  Aligned rows come through rings above
-  // 256 columns.  Below, a row's loads are few and the kernel without rings has more warps, which pays with many rows (16000 x
-  // 128: 7.6 against 10.3 us) and with more groups than SMs (3000 x 256 in 300: 4.9 against 7.7); between 1024 and 4096 rows it
-  // needs clusters and the rings do not (2000 x 256: 6.4 against 4.6; in 16 groups both do, 3000 x 256: 7.8 against 10.1).
-  // Single floats only up to 512 columns: 64 more registers of partial sums leave too few warps (2400 x 1023: 18.5
-  // against 16.6 us).
-  if (vec && N <= kWarpCols && (N > 256 ? 4 * M >= N : M > 1024 && M <= 4096 && G >= 32 && G <= ctx->sm_count)) {
-    if (n <= 256) return launch_bwd_ring<2, 16>(ctx, st, DX, DY, DW, DB, X, W, Mean, Rstd, n, m, ldx, lddy, lddx, G);
-    if (n <= 512) return launch_bwd_ring<4, 16>(ctx, st, DX, DY, DW, DB, X, W, Mean, Rstd, n, m, ldx, lddy, lddx, G);
-    return launch_bwd_ring<8, 8>(ctx, st, DX, DY, DW, DB, X, W, Mean, Rstd, n, m, ldx, lddy, lddx, G);
-  }
-  if (N <= 256 || (!vec && 4 * M >= N && N <= 512)) {
-    auto k = vec ? ln_bwd_warp_kernel<4, 2> : n <= 256 ? ln_bwd_warp_kernel<1, 8> : ln_bwd_warp_kernel<1, 16>;
-    constexpr int kWarps = kBwdWarpThreads / 32;
-    return launch_bwd_regs(ctx, k, kBwdWarpThreads, (size_t)kWarps * 2 * n * 4, kWarps, st, DX, DY, DW, DB, X, W, Mean, Rstd, n, m,
-                           ldx, lddy, lddx, G);
+  // lies at M = N / 4 (1024 columns, with rings: 150 rows 5.0 us by either, 300 rows 3.9 against 6.4).  Single floats only up to 512
+  // columns: 64 more registers of partial sums leave too few warps (2400 x 1023: 18.5 against 16.6 us).
+  if (N <= 256 || (4 * M >= N && N <= (vec ? kWarpCols : 512))) {
+    auto launch = vec ? (n <= 256 ? launch_bwd_rows<4, 2> : n <= 512 ? launch_bwd_rows<4, 4> : launch_bwd_rows<4, 8>)
+                      : (n <= 256 ? launch_bwd_rows<1, 8> : launch_bwd_rows<1, 16>);
+    return launch(ctx, st, DX, DY, DW, DB, X, W, Mean, Rstd, n, m, ldx, lddy, lddx, G);
   }
   if (vec && aligned16(DW) && aligned16(DB) && N <= 4 * kBwdThreads * 4) {
     const int nv = (n / 4 + kBwdThreads - 1) / kBwdThreads;
