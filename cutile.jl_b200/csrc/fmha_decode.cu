@@ -16,7 +16,7 @@
 // so a sum over fewer, longer pieces has the larger error (256 heads of 4000 keys in bf16: 2.18e-3 in whole pairs against 2.15e-3
 // in ranges; 75 heads of 2000: 2.15e-3 and 2.08e-3).  CTAs that have whole pairs or equal parts therefore let their warps meet
 // where a range would end as well, which costs them 0.2 to 1.7 us where there are such cuts (256 heads of 4000 keys 42.2 -> 42.6 us, in
-// ranges 47.2; 75 heads of 2000 10.4 -> 12.1, in ranges 16.2), and the results of whole pairs are those of ranges bit for bit.
+// ranges 47.2; 75 heads of 2000 10.4 -> 11.8, in ranges 16.2), and the results of whole pairs are those of ranges bit for bit.
 // S = Q K^T and O += P V are m16n8k16 tensor-core instructions on registers (a 128-row tcgen05 tile would be 88 % padding;
 // the tensor work here is a few per cent of what either path delivers): Q stays in registers for the pair, K enters by
 // ldmatrix, the probabilities go from the accumulator layout straight into the A operand, V by transposed ldmatrix.
