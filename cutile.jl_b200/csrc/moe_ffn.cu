@@ -320,6 +320,7 @@ __global__ void __launch_bounds__(kThreads) moe_sort_gather_kernel(const IdT* __
       bulk_commit();
       if (__syncthreads_or(!ok)) {  // the copies must land before the CTA gives its shared memory back
         (void)mbar_wait(&rows_in, phase ^ 1, p.status, DEV_TIMEOUT_TMA);
+        for (int j = b0 + step + tid; j < hi; j += kThreads) p.pos_of[j] = 0;  // the combine kernel finds valid positions
         break;
       }
       continue;
