@@ -82,6 +82,7 @@ struct Program {
   // Offset of the temporaries in shared memory.  Here and not among the operands, where four bytes more move the words and their
   // constants: f32 expressions without temporaries took 6 to 13 % longer (1000 x 1000, A + B: 3.6 us, then 4.0).
   unsigned temp_slot;
+  bool operand_fma;  // some word has kOperandFma: the kernel without temporaries does not look for it
 };
 
 // How an operand is read (chosen on the host).
@@ -304,6 +305,7 @@ int lower_program(const int32_t* program, int n_ops, int n_inputs, const float* 
   }
   int next = stack_need() - 1;  // stack entries take the first temporaries
   out->n_temps = next + shared;
+  out->operand_fma = false;
   for (int i = 0; i < c.n_nodes; ++i)
     if (c.nodes[i].temp >= 0) c.nodes[i].temp = next++;
   for (int i = 0; i < c.n_nodes; ++i)
@@ -365,7 +367,7 @@ int lower_program(const int32_t* program, int n_ops, int n_inputs, const float* 
         put(code == CTB_TILED_MUL ? (in ? L_MUL_INPUT : L_MUL_TEMP) : (in ? L_ADD_INPUT : L_ADD_TEMP),
             index | (code == CTB_TILED_SUB ? kSubtract >> 8 : 0u) | kOperandFma >> 8, aff.y, true);
         out->pq[out->n_ins - 1].x = aff.x;
-        out->n_temps = std::max(out->n_temps, 1);  // the kernel without temporaries does not look for it
+        out->operand_fma = true;
       } else if (from == SRC_CONST && code <= CTB_TILED_MUL) {
         const float v = constants[index];
         if (code == CTB_TILED_ADD) fma(1.f, v);
@@ -1285,9 +1287,9 @@ int ctb_tiled_broadcast(ctb_ctx* ctx, void* stream, void* dest, const int64_t* s
   size_t need = (size_t)prog.n_temps * 4 * 4096;
   for (int a = 0; a < n_inputs; ++a)
     need += in.mode[a] == OP_SCALAR ? 0 : in.mode[a] == OP_VECTOR ? vb : in.mode[a] == OP_GROUP ? 2 * vb : 8 * vb;
-  const bool four = prog.n_temps ? need <= 72 * 1024 : n_inputs <= 3;
+  const bool temps = prog.n_temps || prog.operand_fma, four = temps ? need <= 72 * 1024 : n_inputs <= 3;
 #define CTB_TILED(T)                                                                                                        \
-  rc = prog.n_temps ? four ? launch_broadcast<T, 4, true>(ctx, st, dest, in, prog, n_inputs, d0, x)                         \
+  rc = temps ? four ? launch_broadcast<T, 4, true>(ctx, st, dest, in, prog, n_inputs, d0, x)                         \
                            : launch_broadcast<T, 2, true>(ctx, st, dest, in, prog, n_inputs, d0, x)                         \
                     : four ? launch_broadcast<T, 4, false>(ctx, st, dest, in, prog, n_inputs, d0, x)                        \
                            : launch_broadcast<T, 2, false>(ctx, st, dest, in, prog, n_inputs, d0, x)

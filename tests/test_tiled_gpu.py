@@ -350,11 +350,13 @@ def test_broadcast_signed_zero_constants(cuda, hints):
 
 
 @pytest.mark.parametrize("rows,cols", [(1, 3), (5, 4), (37, 1001), (700, 2048), (2500, 4096)])
-@pytest.mark.parametrize("temps,inputs", [(1, 1), (1, 3), (2, 1), (2, 2), (3, 3), (4, 1), (4, 4)])
+@pytest.mark.parametrize("temps,inputs", [(1, 1), (1, 2), (1, 3), (2, 1), (2, 2), (3, 2), (3, 3), (4, 1), (4, 4)])
 @pytest.mark.parametrize("dtype", ["float32", "float16"])
 def test_broadcast_temporaries(cuda, rows, cols, temps, inputs, dtype):
-    """One to four shared values over one to four arrays (four or two groups per thread, a partial group, one and several trips):
-    sums and products of f32, each rounded once, so the result is that of the operators one by one, bit for bit."""
+    """One to four shared values over one to four arrays (a partial group, one and several trips): sums and products of f32, each
+    rounded once, so the result is that of the operators one by one, bit for bit."""
+    import ctypes as C
+
     import torch
     T = cuda.tiled
     g = torch.Generator(device="cuda").manual_seed(rows + temps)
@@ -362,11 +364,18 @@ def test_broadcast_temporaries(cuda, rows, cols, temps, inputs, dtype):
 
     def expression(x, largest, smallest):
         ops = (lambda p, q: p * q, lambda p, q: p + q, largest, smallest)
-        v = [ops[k](x[k % inputs], x[(k + 1) % inputs]) for k in range(temps)]  # each is used below, most of them twice
-        total = v[0] * v[-1]
-        for k in range(temps):
-            total = total * 0.5 + v[k]
-        return total * v[1] if 1 < temps < 4 else total
+        v = [ops[k](x[k % inputs], x[(k + 1) % inputs]) for k in range(temps)]
+        total = v[0]
+        for k, u in enumerate(v[1:] + v):  # each twice
+            total = total + u if k % 2 else total * u
+        return total
+    from cutile_b200 import _lib as L
+    expr = expression([T.Tiled(x) for x in a], T.tmax, T.tmin)
+    prog = T._compile(expr)[2]
+    n, n_temps, words, pq = C.c_int(), C.c_int(), (C.c_uint32 * 48)(), (C.c_float * 96)()
+    assert L.lib.ctb_tiled_lower((C.c_int32 * len(prog))(*prog), len(prog) // 2, inputs, (C.c_float * 1)(), 0, words, pq,
+                                 C.byref(n), C.byref(n_temps)) == 0
+    assert n_temps.value == temps
     out = torch.empty(rows, cols, device="cuda", dtype=a[0].dtype)
-    T.assign(out, expression([T.Tiled(x) for x in a], T.tmax, T.tmin))
+    T.assign(out, expr)
     assert torch.equal(out, expression([x.float() for x in a], torch.maximum, torch.minimum).to(out.dtype))
