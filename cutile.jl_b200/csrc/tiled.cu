@@ -934,17 +934,18 @@ __global__ void __launch_bounds__(256, TEMPS ? 3 : 4)
   cp_async_wait<0>();
 }
 
-template <typename T, int G, bool TEMPS>
-int launch_broadcast(ctb_ctx* ctx, cudaStream_t st, void* dest, Operands& in, Program& prog, int n_inputs, long long d0,
-                     Extents& x) {
-  constexpr int VB = 4 * (int)sizeof(T);
+// CTAs of a broadcast with `groups` groups of four elements per thread and trip.
+struct Grid {
+  long long ctas, fixed;  // fixed: with operands that vary along the first dimension only; 0: they are read with every group
+};
+Grid broadcast_grid(ctb_ctx* ctx, long long n, long long d0, int groups) {
   // Several waves of CTAs, not one wave of resident ones: CTAs that all start together stay in step (all loading,
   // then all storing) and measured 10 % slower than CTAs that start at different times.  At most 16 per SM, and as many
   // as give every CTA the same number of trips (2368 CTAs with three or four trips each: 81.8 us for a bias and tanh
   // expression on 8192 x 4096, 2048 with four: 68.5).
-  const long long ctas = std::max<long long>(1, ((x.n + 3) / 4 + 256ll * G - 1) / (256ll * G));
+  const long long ctas = std::max<long long>(1, ((n + 3) / 4 + 256ll * groups - 1) / (256ll * groups));
   const long long most = (long long)ctx->sm_count * 16, trips = (ctas + most - 1) / most;
-  long long grid = (ctas + trips - 1) / trips;
+  const long long grid = (ctas + trips - 1) / trips;
   // An operand that varies along the first dimension only is the same for all groups of a thread when a whole grid is a
   // multiple of the first extent: a grid of a multiple of m CTAs.  Its four elements are then read once instead of with
   // every group (8192 x 4096, A .+ b: 20.8 -> 14 instructions per element).
@@ -954,11 +955,25 @@ int launch_broadcast(ctb_ctx* ctx, cudaStream_t st, void* dest, Operands& in, Pr
   };
   const long long m = d0 / gcd(d0, 1024);  // 256 threads of four elements per CTA
   const long long up = (grid + m - 1) / m * m;
-  const long long fixed_grid = up <= std::max(most, std::min(ctas, 4 * most)) ? up : grid / m * m;
+  return {grid, up <= std::max(most, std::min(ctas, 4 * most)) ? up : grid / m * m};
+}
+bool along_first(const Operands& in, int a) {
+  return in.mode[a] == OP_VECTOR || (in.mode[a] == OP_ELEM && in.stride[a][0] == 1 && !in.stride[a][1] && !in.stride[a][2]);
+}
+// Bytes of shared memory of an operand with elements of `es` bytes.
+size_t operand_bytes(int mode, int groups, int es) {
+  return mode == OP_SCALAR ? 0 : (size_t)256 * es * (mode == OP_FIXED ? 4 : mode == OP_GROUP ? 2 * groups : 8 * groups);
+}
+
+template <typename T, int G, bool TEMPS>
+int launch_broadcast(ctb_ctx* ctx, cudaStream_t st, void* dest, Operands& in, Program& prog, int n_inputs, long long d0,
+                     Extents& x) {
+  constexpr int VB = 4 * (int)sizeof(T);
+  const Grid grids = broadcast_grid(ctx, x.n, d0, G);
+  long long grid = grids.ctas;
   bool linear = true, fixed = false;
   for (int a = 0; a < n_inputs; ++a) {
-    const bool vector = in.mode[a] == OP_VECTOR || (in.mode[a] == OP_ELEM && in.stride[a][0] == 1 && !in.stride[a][1] && !in.stride[a][2]);
-    if (vector && fixed_grid > 0) {
+    if (along_first(in, a) && grids.fixed > 0) {
       in.mode[a] = OP_FIXED;
       fixed = true;
     } else if (in.mode[a] == OP_VECTOR || in.mode[a] == OP_ROW || in.mode[a] == OP_GROUP || in.mode[a] == OP_ELEM) {
@@ -966,7 +981,7 @@ int launch_broadcast(ctb_ctx* ctx, cudaStream_t st, void* dest, Operands& in, Pr
     }
   }
   if (fixed) {
-    grid = fixed_grid;
+    grid = grids.fixed;
     x.d0 = (unsigned)d0;
     x.fixed_vec = d0 % 4 == 0;
     for (int a = 0; a < n_inputs; ++a)
@@ -975,8 +990,7 @@ int launch_broadcast(ctb_ctx* ctx, cudaStream_t st, void* dest, Operands& in, Pr
   unsigned smem = 0;
   for (int a = 0; a < n_inputs; ++a) {
     in.slot[a] = smem;
-    if (in.mode[a] == OP_GROUP) smem += 2 * G * 256 * sizeof(T);
-    else if (in.mode[a] != OP_SCALAR) smem += (in.mode[a] == OP_FIXED ? 1 : 2 * G) * 256 * VB;
+    smem += (unsigned)operand_bytes(in.mode[a], G, sizeof(T));
   }
   prog.temp_slot = smem;
   smem += prog.n_temps * G * 4096;
@@ -1281,21 +1295,40 @@ int ctb_tiled_broadcast(ctb_ctx* ctx, void* stream, void* dest, const int64_t* s
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int rc = CTB_OK;
-  // Groups per thread: four, or two where the shared memory of four (operands twice, temporaries once) would leave room for
-  // fewer than three CTAs per SM.
-  const size_t vb = 256 * 4 * (dtype == CTB_F32 ? 4 : 2);
-  size_t need = (size_t)prog.n_temps * 4 * 4096;
-  for (int a = 0; a < n_inputs; ++a)
-    need += in.mode[a] == OP_SCALAR ? 0 : in.mode[a] == OP_VECTOR ? vb : in.mode[a] == OP_GROUP ? 2 * vb : 8 * vb;
-  const bool temps = prog.n_temps || prog.operand_fma, four = temps ? need <= 72 * 1024 : n_inputs <= 3;
-#define CTB_TILED(T)                                                                                                        \
-  rc = temps ? four ? launch_broadcast<T, 4, true>(ctx, st, dest, in, prog, n_inputs, d0, x)                         \
-                           : launch_broadcast<T, 2, true>(ctx, st, dest, in, prog, n_inputs, d0, x)                         \
-                    : four ? launch_broadcast<T, 4, false>(ctx, st, dest, in, prog, n_inputs, d0, x)                        \
-                           : launch_broadcast<T, 2, false>(ctx, st, dest, in, prog, n_inputs, d0, x)
-  if (dtype == CTB_F32) CTB_TILED(float);
-  else CTB_TILED(__half);
-#undef CTB_TILED
+  // Groups per thread.  With temporaries the most of four, three and two with which three CTAs fit the shared memory of an SM
+  // (operands twice, those that stay the same and temporaries once): 8192 x 4096 f32, bias and tanh of A + B, 76.7 us with two, 71.2
+  // with three, 76.9 with four; a bias instead of B stays the same, and four fit (60.7, 74.7 with two).  Without temporaries four for
+  // up to three operands, although three arrays of f32 leave room for two CTAs only.
+  const bool temps = prog.n_temps || prog.operand_fma;
+  auto need = [&](int groups) {
+    const bool stays = broadcast_grid(ctx, x.n, d0, groups).fixed > 0;
+    size_t bytes = (size_t)prog.n_temps * groups * 4096;
+    for (int a = 0; a < n_inputs; ++a) bytes += operand_bytes(stays && along_first(in, a) ? OP_FIXED : in.mode[a], groups, es);
+    return bytes;
+  };
+  auto grid_of = [&](int groups) { return broadcast_grid(ctx, x.n, d0, groups); };
+  int groups = n_inputs <= 3 ? 4 : 2;
+  if (temps) {
+    groups = need(4) <= 72 * 1024 ? 4 : need(3) <= 72 * 1024 ? 3 : 2;
+    // Not three where operands that stay the same ask for a grid that gives the CTAs unequal trips (4000 x 2001: 2001 CTAs of three groups
+    // have 1.3 trips, 31.5 us; of two 1.95, 24.8).
+    bool stays = false;
+    for (int a = 0; a < n_inputs; ++a) stays = stays || along_first(in, a);
+    if (groups == 3 && stays && grid_of(3).fixed * 10 > grid_of(3).ctas * 11) groups = 2;
+  }
+  // Two as well where more would leave fewer than two CTAs per SM, or two and a half with three groups (1000 x 1001 f32, bias and tanh, with
+  // two 8.1 us, with four 11.9; not so 300 x 4096, 300 CTAs of four groups: 6.0 and 5.4).
+  if (2 * grid_of(groups).ctas < (groups == 3 ? 5ll : 4ll) * ctx->sm_count) groups = 2;
+  auto launch = [&](auto zero) {
+    using T = decltype(zero);
+    if (temps)
+      return groups == 4   ? launch_broadcast<T, 4, true>(ctx, st, dest, in, prog, n_inputs, d0, x)
+             : groups == 3 ? launch_broadcast<T, 3, true>(ctx, st, dest, in, prog, n_inputs, d0, x)
+                           : launch_broadcast<T, 2, true>(ctx, st, dest, in, prog, n_inputs, d0, x);
+    return groups == 4 ? launch_broadcast<T, 4, false>(ctx, st, dest, in, prog, n_inputs, d0, x)
+                       : launch_broadcast<T, 2, false>(ctx, st, dest, in, prog, n_inputs, d0, x);
+  };
+  rc = dtype == CTB_F32 ? launch(0.f) : launch(__half());
   if (rc) return rc;
   CTB_CHECK_LAUNCH("ctb_tiled_broadcast launch");
   return CTB_OK;

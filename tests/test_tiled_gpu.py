@@ -349,6 +349,8 @@ def test_broadcast_signed_zero_constants(cuda, hints):
     assert torch.equal(out, torch.zeros_like(a)) and torch.signbit(out).all()
 
 
+# groups per thread: by the shared memory of the temporaries and arrays (f32: four with (1, 1) and (2, 1), three with (1, 2), (2, 2) and
+# (4, 1), else two; f16: three with (3, 2), (3, 3) and (4, 1), two with (4, 4), else four), and two with few elements
 @pytest.mark.parametrize("rows,cols", [(1, 3), (5, 4), (37, 1001), (700, 2048), (2500, 4096)])
 @pytest.mark.parametrize("temps,inputs", [(1, 1), (1, 2), (1, 3), (2, 1), (2, 2), (3, 2), (3, 3), (4, 1), (4, 4)])
 @pytest.mark.parametrize("dtype", ["float32", "float16"])
