@@ -19,6 +19,7 @@
 #include <type_traits>
 
 #include "ctx.h"
+#include "moe_place.h"
 #include "ptx.cuh"
 
 using namespace ctb;
@@ -27,15 +28,6 @@ using namespace ctb_internal;
 namespace {
 
 constexpr int kMaxExperts = 256;
-constexpr int kMmaSlots = 256;       // MMA N
-constexpr int kMaxBlockSlots = 320;  // slots of a block: two MMAs above kMmaSlots
-// Blocks that an expert's slots are cut into.  A k-block costs a pair about 330 ns up to 224 slots, whatever their number, and
-// the MMA's 1.45 ns per slot above: blocks of 226 slots and more are cheap, and one of up to 320 is cheaper than two of half of it.
-// (ring: the accumulators of moe_pair_gemm_kernel may take more than half of the columns.)
-constexpr __host__ __device__ int blocks_for(bool ring, int slots) {
-  const int n = (slots + kMmaSlots - 1) / kMmaSlots;
-  return ring && n > 1 && slots < n * 226 && slots <= (n - 1) * kMaxBlockSlots ? n - 1 : n;
-}
 
 // ------------------------------------------------------------------ sort and gather
 constexpr int kSortThreads = 512, kSortCtas = 148;
@@ -350,7 +342,6 @@ constexpr int kMaxStages = 12;
 constexpr int kRingBytes = 192 * 1024;
 constexpr int kEpiWarps = 8;                 // two per TMEM lane quadrant, each takes every other block of 32 slots
 constexpr int kGemmThreads = 96 + 32 * kEpiWarps;
-constexpr int kParts = 6;                    // leading blocks of 32 columns that the next item may need (place())
 constexpr int kTileBytes = 32 * 64 * 2;      // staged results: 32 slots x 64 rows, f16, 128-byte swizzle
 // Warps that share a staging tile: gate/up the four quadrants (a CTA's 64 outputs), down two of them; two tiles each.
 template <bool UP>
@@ -374,25 +365,6 @@ struct PairParams {
   const void* ids;      // gate/up with at most kEarlySlots slots (not RING): the kernel builds its own table
   int ids_bits, T, topk, E;
 };
-
-// Where a block's accumulators lie in the 512 TMEM columns, which are a ring: slot s of the block in column
-// (col + s) mod 512, col a multiple of 32.  The slots are taken by at most two MMAs: [0, first) and [first, n).
-struct Place {
-  int col, first, next, skipped;  // next: where the next block may start
-};
-template <bool RING>
-__device__ __forceinline__ Place place(int at, int n) {
-  if (!RING) return {at, n, at ^ 256, 0};  // no block above 256 slots: two halves in turn
-  const int n32 = (n + 31) & ~31, room = 512 - at;
-  Place r;
-  // an MMA takes at most kMmaSlots: columns before or behind the end of the ring stay unused where a part would be larger
-  r.skipped = n32 <= room ? 0 : room > kMmaSlots ? room - kMmaSlots : n - room > kMmaSlots ? room : 0;
-  r.col = (at + r.skipped) & 511;
-  const int left = 512 - r.col;
-  r.first = n32 > left ? left : n > kMmaSlots ? ((n / 2 + 15) & ~15) : n;
-  r.next = (r.col + n32) & 511;
-  return r;
-}
 
 // Barriers of `threads` threads (whole warps).
 __device__ __forceinline__ void group_sync(int id, int threads) { asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
