@@ -349,13 +349,36 @@ def test_broadcast_signed_zero_constants(cuda, hints):
     assert torch.equal(out, torch.zeros_like(a)) and torch.signbit(out).all()
 
 
+@pytest.mark.parametrize("rows,cols", [(1, 3), (5, 4), (37, 1001), (700, 2048), (2500, 4096)])
+@pytest.mark.parametrize("temps,inputs", [(1, 1), (1, 3), (2, 1), (2, 2), (3, 3), (4, 1), (4, 4)])
+@pytest.mark.parametrize("dtype", ["float32", "float16"])
+def test_broadcast_temporaries(cuda, rows, cols, temps, inputs, dtype):
+    """One to four shared values over one to four arrays (four or two groups per thread, a partial group, one and several trips):
+    sums and products of f32, each rounded once, so the result is that of the operators one by one, bit for bit."""
+    import torch
+    T = cuda.tiled
+    g = torch.Generator(device="cuda").manual_seed(rows + temps)
+    a = [torch.randn(rows, cols, device="cuda", generator=g).to(getattr(torch, dtype)) for _ in range(inputs)]
+
+    def expression(x, largest, smallest):
+        ops = (lambda p, q: p * q, lambda p, q: p + q, largest, smallest)
+        v = [ops[k](x[k % inputs], x[(k + 1) % inputs]) for k in range(temps)]  # each is used below, most of them twice
+        total = v[0] * v[-1]
+        for k in range(temps):
+            total = total * 0.5 + v[k]
+        return total * v[1] if 1 < temps < 4 else total
+    out = torch.empty(rows, cols, device="cuda", dtype=a[0].dtype)
+    T.assign(out, expression([T.Tiled(x) for x in a], T.tmax, T.tmin))
+    assert torch.equal(out, expression([x.float() for x in a], torch.maximum, torch.minimum).to(out.dtype))
+
+
 # groups per thread: by the shared memory of the temporaries and arrays (f32: four with (1, 1) and (2, 1), three with (1, 2), (2, 2) and
 # (4, 1), else two; f16: three with (3, 2), (3, 3) and (4, 1), two with (4, 4), else four), and two with few elements
 @pytest.mark.parametrize("rows,cols", [(1, 3), (5, 4), (37, 1001), (700, 2048), (2500, 4096)])
 @pytest.mark.parametrize("temps,inputs", [(1, 1), (1, 2), (1, 3), (2, 1), (2, 2), (3, 2), (3, 3), (4, 1), (4, 4)])
 @pytest.mark.parametrize("dtype", ["float32", "float16"])
-def test_broadcast_temporaries(cuda, rows, cols, temps, inputs, dtype):
-    """One to four shared values over one to four arrays (a partial group, one and several trips): sums and products of f32, each
+def test_broadcast_temporaries_counted(cuda, rows, cols, temps, inputs, dtype):
+    """One to four shared values, as many temporaries, over one to four arrays (a partial group, one and several trips): sums and products of f32, each
     rounded once, so the result is that of the operators one by one, bit for bit."""
     import ctypes as C
 

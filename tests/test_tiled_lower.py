@@ -162,6 +162,9 @@ def test_what_the_kernel_is_said_to_run():
     assert len(words) == 7 and n_temps == 1
     words, n_temps = check(("add", ("mul", ("c", 0), ("in", 0)), ("c", 1)), random_inputs(np.random.default_rng(1)), [2.0, 1.0])
     assert len(words) == 2 and n_temps == 0
+
+
+def test_scaled_operand_takes_no_temporary():
     # (x + c) (y + d): y enters as y + d, without a temporary
     tree = ("mul", ("add", ("in", 0), ("c", 0)), ("add", ("in", 1), ("c", 1)))
     words, n_temps = check(tree, random_inputs(np.random.default_rng(2)), [2.0, 1.0])
