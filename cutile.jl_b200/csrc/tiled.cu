@@ -1306,19 +1306,22 @@ int ctb_tiled_broadcast(ctb_ctx* ctx, void* stream, void* dest, const int64_t* s
     for (int a = 0; a < n_inputs; ++a) bytes += operand_bytes(stays && along_first(in, a) ? OP_FIXED : in.mode[a], groups, es);
     return bytes;
   };
-  auto grid_of = [&](int groups) { return broadcast_grid(ctx, x.n, d0, groups); };
   int groups = n_inputs <= 3 ? 4 : 2;
-  if (temps) {
-    groups = need(4) <= 72 * 1024 ? 4 : need(3) <= 72 * 1024 ? 3 : 2;
-    // Not three where operands that stay the same ask for a grid that gives the CTAs unequal trips (4000 x 2001: 2001 CTAs of three groups
-    // have 1.3 trips, 31.5 us; of two 1.95, 24.8).
-    bool stays = false;
-    for (int a = 0; a < n_inputs; ++a) stays = stays || along_first(in, a);
-    if (groups == 3 && stays && grid_of(3).fixed * 10 > grid_of(3).ctas * 11) groups = 2;
+  if (temps) groups = need(4) <= 72 * 1024 ? 4 : need(3) <= 72 * 1024 ? 3 : 2;
+  bool stays = false;  // the grid is one that lets operands stay the same
+  for (int a = 0; a < n_inputs; ++a) stays = stays || along_first(in, a);
+  const Grid grid = broadcast_grid(ctx, x.n, d0, groups);
+  if (stays && grid.fixed > 0) {
+    // Such a grid may be far larger than the elements need, and a thread then has one group and computes more: two where four groups
+    // have twice the CTAs (bias and tanh of 1000 x 1001 in f32 7.5 us, with four 11.4; of 452 x 1988 in f16 4.2 and 7.5), or three a tenth more
+    // (4000 x 2001: 2001 CTAs of three groups have 1.3 trips, 31.5 us; of two 1.95, 24.8). Otherwise four also with few elements: every
+    // CTA reads the operand that stays (bias and tanh of 11064 x 72 7.0 us, 11.0 with two; the bias alone 5.1 and 10.1).
+    if (groups == 3 ? grid.fixed * 10 > grid.ctas * 11 : grid.fixed >= grid.ctas * 2) groups = 2;
+  } else if (2 * grid.ctas < (groups == 3 ? 5ll : 4ll) * ctx->sm_count) {
+    // Two as well where more would leave fewer than two CTAs per SM, or two and a half with three groups (f32 1000 x 1001: tanh
+    // of 2 A + 1 2.8 us, with four 3.6; A + B 2.6 and 3.1).
+    groups = 2;
   }
-  // Two as well where more would leave fewer than two CTAs per SM, or two and a half with three groups (1000 x 1001 f32, bias and tanh, with
-  // two 8.1 us, with four 11.9; not so 300 x 4096, 300 CTAs of four groups: 6.0 and 5.4).
-  if (2 * grid_of(groups).ctas < (groups == 3 ? 5ll : 4ll) * ctx->sm_count) groups = 2;
   auto launch = [&](auto zero) {
     using T = decltype(zero);
     if (temps)

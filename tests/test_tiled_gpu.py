@@ -372,14 +372,30 @@ def test_broadcast_temporaries(cuda, rows, cols, temps, inputs, dtype):
     assert torch.equal(out, expression([x.float() for x in a], torch.maximum, torch.minimum).to(out.dtype))
 
 
+# an operand that is the same for all groups of a thread: with a grid that the elements fill and with one of twice the CTAs
+@pytest.mark.parametrize("rows,cols", [(11064, 72), (2450, 356), (1000, 1001), (452, 1988), (3, 1001), (9, 40)])
+@pytest.mark.parametrize("shared", [False, True])
+@pytest.mark.parametrize("dtype", ["float32", "float16"])
+def test_broadcast_bias_grids(cuda, rows, cols, shared, dtype):
+    """A sum with a bias, or its square through a temporary: each operator rounded once in f32, so bit for bit."""
+    import torch
+    T = cuda.tiled
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    a, b = (torch.randn(*s, device="cuda", generator=g).to(getattr(torch, dtype)) for s in ((rows, cols), (cols,)))
+    out = torch.empty_like(a)
+    v, w = T.Tiled(a) + T.Tiled(b), a.float() + b.float()
+    T.assign(out, v * v if shared else v)
+    assert torch.equal(out, (w * w if shared else w).to(out.dtype))
+
+
 # groups per thread: by the shared memory of the temporaries and arrays (f32: four with (1, 1) and (2, 1), three with (1, 2), (2, 2) and
 # (4, 1), else two; f16: three with (3, 2), (3, 3) and (4, 1), two with (4, 4), else four), and two with few elements
 @pytest.mark.parametrize("rows,cols", [(1, 3), (5, 4), (37, 1001), (700, 2048), (2500, 4096)])
 @pytest.mark.parametrize("temps,inputs", [(1, 1), (1, 2), (1, 3), (2, 1), (2, 2), (3, 2), (3, 3), (4, 1), (4, 4)])
 @pytest.mark.parametrize("dtype", ["float32", "float16"])
 def test_broadcast_temporaries_counted(cuda, rows, cols, temps, inputs, dtype):
-    """One to four shared values, as many temporaries, over one to four arrays (a partial group, one and several trips): sums and products of f32, each
-    rounded once, so the result is that of the operators one by one, bit for bit."""
+    """One to four shared values, as many temporaries, over one to four arrays (a partial group, one and several trips): sums and
+    products of f32, each rounded once, so the result is that of the operators one by one, bit for bit."""
     import ctypes as C
 
     import torch
