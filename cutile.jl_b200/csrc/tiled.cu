@@ -1307,16 +1307,22 @@ int ctb_tiled_broadcast(ctb_ctx* ctx, void* stream, void* dest, const int64_t* s
     return bytes;
   };
   int groups = n_inputs <= 3 ? 4 : 2;
-  if (temps) groups = need(4) <= 72 * 1024 ? 4 : need(3) <= 72 * 1024 ? 3 : 2;
   bool stays = false;  // the grid is one that lets operands stay the same
   for (int a = 0; a < n_inputs; ++a) stays = stays || along_first(in, a);
+  if (temps) {
+    groups = need(4) <= 72 * 1024 ? 4 : need(3) <= 72 * 1024 ? 3 : 2;
+    // Four also where two CTAs per SM are all there are: every CTA reads the operand that stays (f32 tanh of a square of A B + bias,
+    // 2450 x 356 5.9 us, 7.2 with three, 8.5 with two; 11064 x 72 7.4, 8.7, 11.2).
+    const Grid four = broadcast_grid(ctx, x.n, d0, 4);
+    if (stays && four.fixed > 0 && four.fixed <= 2 * ctx->sm_count && four.fixed < 2 * four.ctas && need(4) <= 112 * 1024) groups = 4;
+  }
   const Grid grid = broadcast_grid(ctx, x.n, d0, groups);
   if (stays && grid.fixed > 0) {
     // Such a grid may be far larger than the elements need, and a thread then has one group and computes more: two where four groups
-    // have twice the CTAs (bias and tanh of 1000 x 1001 in f32 7.5 us, with four 11.4; of 452 x 1988 in f16 4.2 and 7.5), or three a tenth more
-    // (4000 x 2001: 2001 CTAs of three groups have 1.3 trips, 31.5 us; of two 1.95, 24.8). Otherwise four also with few elements: every
-    // CTA reads the operand that stays (bias and tanh of 11064 x 72 7.0 us, 11.0 with two; the bias alone 5.1 and 10.1).
-    if (groups == 3 ? grid.fixed * 10 > grid.ctas * 11 : grid.fixed >= grid.ctas * 2) groups = 2;
+    // have twice the CTAs (bias and tanh of 1000 x 1001 in f32 7.5 us, with four 11.4; of 452 x 1988 in f16 4.2 and 7.5), or three a fifth more
+    // (4000 x 2001: 2001 CTAs of three groups have 1.3 trips, 31.5 us; of two 1.95, 24.8; but 3459 x 356, 445 CTAs for 401, 7.5 and 8.8).
+    // Otherwise four also with few elements (bias and tanh of 11064 x 72 7.0 us, 11.0 with two; the bias alone 5.1 and 10.1).
+    if (groups == 3 ? grid.fixed * 10 > grid.ctas * 12 : grid.fixed >= grid.ctas * 2) groups = 2;
   } else if (2 * grid.ctas < (groups == 3 ? 5ll : 4ll) * ctx->sm_count) {
     // Two as well where more would leave fewer than two CTAs per SM, or two and a half with three groups (f32 1000 x 1001: tanh
     // of 2 A + 1 2.8 us, with four 3.6; A + B 2.6 and 3.1).

@@ -374,16 +374,18 @@ def test_broadcast_temporaries(cuda, rows, cols, temps, inputs, dtype):
 
 # an operand that is the same for all groups of a thread: with a grid that the elements fill and with one of twice the CTAs
 @pytest.mark.parametrize("rows,cols", [(11064, 72), (2450, 356), (1000, 1001), (452, 1988), (3, 1001), (9, 40)])
-@pytest.mark.parametrize("shared", [False, True])
+@pytest.mark.parametrize("shared,arrays", [(False, 1), (True, 1), (True, 2)])
 @pytest.mark.parametrize("dtype", ["float32", "float16"])
-def test_broadcast_bias_grids(cuda, rows, cols, shared, dtype):
+def test_broadcast_bias_grids(cuda, rows, cols, shared, arrays, dtype):
     """A sum with a bias, or its square through a temporary: each operator rounded once in f32, so bit for bit."""
     import torch
     T = cuda.tiled
     g = torch.Generator(device="cuda").manual_seed(rows)
-    a, b = (torch.randn(*s, device="cuda", generator=g).to(getattr(torch, dtype)) for s in ((rows, cols), (cols,)))
+    a, c, b = (torch.randn(*s, device="cuda", generator=g).to(getattr(torch, dtype)) for s in ((rows, cols), (rows, cols), (cols,)))
     out = torch.empty_like(a)
     v, w = T.Tiled(a) + T.Tiled(b), a.float() + b.float()
+    if arrays == 2:
+        v, w = v + T.Tiled(c), w + c.float()
     T.assign(out, v * v if shared else v)
     assert torch.equal(out, (w * w if shared else w).to(out.dtype))
 
