@@ -949,11 +949,7 @@ Grid broadcast_grid(ctb_ctx* ctx, long long n, long long d0, int groups) {
   // An operand that varies along the first dimension only is the same for all groups of a thread when a whole grid is a
   // multiple of the first extent: a grid of a multiple of m CTAs.  Its four elements are then read once instead of with
   // every group (8192 x 4096, A .+ b: 20.8 -> 14 instructions per element).
-  auto gcd = [](long long a, long long b) {
-    while (b) { const long long t = a % b; a = b; b = t; }
-    return a;
-  };
-  const long long m = d0 / gcd(d0, 1024);  // 256 threads of four elements per CTA
+  const long long m = d0 / std::min(d0 & -d0, 1024ll);  // over the common divisor with 256 threads of four elements
   const long long up = (grid + m - 1) / m * m;
   return {grid, up <= std::max(most, std::min(ctas, 4 * most)) ? up : grid / m * m};
 }
@@ -1300,21 +1296,23 @@ int ctb_tiled_broadcast(ctb_ctx* ctx, void* stream, void* dest, const int64_t* s
   // with three, 76.9 with four; a bias instead of B stays the same, and four fit (60.7, 74.7 with two).  Without temporaries four for
   // up to three operands, although three arrays of f32 leave room for two CTAs only.
   const bool temps = prog.n_temps || prog.operand_fma;
+  bool stays = false;  // some operand may stay the same
+  for (int a = 0; a < n_inputs; ++a) stays = stays || along_first(in, a);
   auto need = [&](int groups) {
-    const bool stays = broadcast_grid(ctx, x.n, d0, groups).fixed > 0;
+    const bool fixed = stays && broadcast_grid(ctx, x.n, d0, groups).fixed > 0;
     size_t bytes = (size_t)prog.n_temps * groups * 4096;
-    for (int a = 0; a < n_inputs; ++a) bytes += operand_bytes(stays && along_first(in, a) ? OP_FIXED : in.mode[a], groups, es);
+    for (int a = 0; a < n_inputs; ++a) bytes += operand_bytes(fixed && along_first(in, a) ? OP_FIXED : in.mode[a], groups, es);
     return bytes;
   };
   int groups = n_inputs <= 3 ? 4 : 2;
-  bool stays = false;  // the grid is one that lets operands stay the same
-  for (int a = 0; a < n_inputs; ++a) stays = stays || along_first(in, a);
   if (temps) {
     groups = need(4) <= 72 * 1024 ? 4 : need(3) <= 72 * 1024 ? 3 : 2;
     // Four also where two CTAs per SM are all there are: every CTA reads the operand that stays (f32 tanh of a square of A B + bias,
     // 2450 x 356 5.9 us, 7.2 with three, 8.5 with two; 11064 x 72 7.4, 8.7, 11.2).
-    const Grid four = broadcast_grid(ctx, x.n, d0, 4);
-    if (stays && four.fixed > 0 && four.fixed <= 2 * ctx->sm_count && four.fixed < 2 * four.ctas && need(4) <= 112 * 1024) groups = 4;
+    if (stays && groups < 4 && need(4) <= 112 * 1024) {
+      const Grid four = broadcast_grid(ctx, x.n, d0, 4);
+      if (four.fixed > 0 && four.fixed <= 2 * ctx->sm_count && four.fixed < 2 * four.ctas) groups = 4;
+    }
   }
   const Grid grid = broadcast_grid(ctx, x.n, d0, groups);
   if (stays && grid.fixed > 0) {
